@@ -21,7 +21,10 @@ __all__ = list(_OPS + _LIB)
 
 def __getattr__(name):
     if name in _OPS:
-        return getattr(importlib.import_module(".ops", __name__), name)
-    if name in _LIB:
-        return getattr(importlib.import_module("._lib", __name__), name)
-    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+        value = getattr(importlib.import_module(".ops", __name__), name)
+    elif name in _LIB:
+        value = getattr(importlib.import_module("._lib", __name__), name)
+    else:
+        raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+    globals()[name] = value  # found directly from now on
+    return value

@@ -14,6 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmiori_b200.so")
 SHIM_LIB = os.path.join(HERE, "libmiori_shim.so")
+BINDING = os.path.join(HERE, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -42,8 +43,28 @@ def _sources(root: str, exts: tuple[str, ...]) -> list[str]:
     return out
 
 
+def _build_binding() -> None:
+    """The operators' native call path: a CPython extension against torch's C++ headers."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", sysconfig.get_paths()["include"]]
+    for d in [*cpp_extension.include_paths(), os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]:
+        cmd += ["-isystem", d]
+    cmd += ["-o", BINDING, os.path.join(CSRC, "binding.cpp")]
+    for d in cpp_extension.library_paths():
+        cmd += ["-L", d, f"-Wl,-rpath,{d}"]
+    cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-ldl"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("binding build failed:\n" + r.stdout + r.stderr)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the CUDA library (and the C++ operator shim) if sources are newer."""
+    """Compile the CUDA library, the operators' binding and the C++ operator shim if sources are newer."""
     srcs = _sources(CSRC, (".cu", ".cuh", ".h")) + [os.path.join(HERE, "..", "include", "miori_b200.h")]
     if force or _stale(LIB, srcs):
         cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB, os.path.join(CSRC, "miori_b200.cu")]
@@ -58,6 +79,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(r.stderr)
         if r.returncode != 0:
             raise RuntimeError("nvcc failed:\n" + r.stdout + r.stderr)
+    header = os.path.join(HERE, "..", "include", "miori_b200.h")
+    if force or _stale(BINDING, [os.path.join(CSRC, "binding.cpp"), header]):
+        _build_binding()
     shim_dir = os.path.join(HERE, "shim")
     shim_srcs = _sources(shim_dir, (".cpp", ".h", ".hpp"))
     shim_cpp = [s for s in shim_srcs if s.endswith(".cpp")]
