@@ -932,7 +932,7 @@ def extras(torch, miori_b200, synth, dev, G, peaks, timed):
     by = packed_bytes(N, K, 4, G)
     ex["stream_gemv4_m1_n131072_k2048"] = {"us": 1e3 * ms, "gbs": by / (ms * 1e-3) / 1e9,
                                            "frac_of_hbm_peak": by / (ms * 1e-3) / 1e9 / peaks["hbm_gbs"],
-                                           "kernel": "gemv_umma_kernel<4,1> (tcgen05.mma.kind::i8), two CTAs per SM"}
+                                           "kernel": "gemv_tma_kernel, one activation row"}
     del big
     # RMSNorm in front of a projection: norm kernel + GEMV against the GEMV with the norm fused into
     # its activation staging, M=1, one layer's four shapes over pools of distinct weights (> L2)
@@ -954,12 +954,8 @@ def extras(torch, miori_b200, synth, dev, G, peaks, timed):
             for q, s, b in pool:
                 miori_b200.gemv4_rmsnorm(q, s, b, xf, gam, 1e-5, group=G, flags=flags, out=y)
 
-        def one_kernel_tcgen05():
-            for q, s, b in pool:
-                miori_b200.gemv4_rmsnorm(q, s, b, xf, gam, 1e-5, group=G, flags=flags | 0x100000, out=y)
         res = {}
-        for name, fn in (("norm_then_gemv_us", two_kernels), ("fused_us", one_kernel),
-                         ("fused_tcgen05_us", one_kernel_tcgen05)):
+        for name, fn in (("norm_then_gemv_us", two_kernels), ("fused_us", one_kernel)):
             fn()
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g):
@@ -971,8 +967,8 @@ def extras(torch, miori_b200, synth, dev, G, peaks, timed):
                                "layer_norm_then_gemv_us": sum(v["norm_then_gemv_us"] for v in fused.values()),
                                "layer_fused_us": sum(v["fused_us"] for v in fused.values()),
                                "how": "CUDA graphs of PDL launches; the unfused pair is the default GEMV after "
-                                      "miori_rmsnorm, the fused one miori_gemv4_rmsnorm (by default the TMA + mma.sync "
-                                      "kernel with the norm in its staging pass; the tcgen05 kernel when forced)"}
+                                      "miori_rmsnorm, the fused one miori_gemv4_rmsnorm (the same kernel with the norm in "
+                                      "its staging pass)"}
     # SiLU x up behind the fused gate + up projection (2048 -> 2 x 8192): GEMV + activation kernel
     # against the GEMV with the activation as its epilogue, over a pool of distinct weights (> L2)
     N, K = 16384, 2048
@@ -1015,7 +1011,7 @@ def extras(torch, miori_b200, synth, dev, G, peaks, timed):
     ex["silu_fusion_gate_up"] = {"per_m": gated,
                                  "how": "CUDA graphs of PDL launches; miori_gemv4 on w1 and on w3 then miori_silu_mul (three "
                                         "launches), miori_gemv4 on the fused weights then miori_silu_mul (two, one row), "
-                                        "and miori_gemv4_silu (TMA + mma.sync kernel, gated epilogue)"}
+                                        "and miori_gemv4_silu (the same kernel, gated epilogue)"}
     # post_norm_add behind the o and w2 projections (M = 1): GEMV + norm kernel against the GEMV with the
     # norm as its epilogue, over pools of distinct weights (> L2)
     post = {}

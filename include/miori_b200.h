@@ -43,7 +43,7 @@ extern "C" {
                                   predecessor on the stream drains; it prefetches weights (which
                                   must be immutable while in flight) and waits for the
                                   predecessor before touching x / A or writing y / C */
-#define MIORI_GEMV_EXACT 4u    /* force the fp32-dequant GEMV path for every M (default: M<=4) */
+#define MIORI_GEMV_EXACT 4u    /* fp32 dequantization for every M (what every launch does) */
 const char* miori_last_error(void);
 /* Library version string, e.g. "miori_b200 0.1 sm_100a". */
 const char* miori_version(void);
@@ -91,13 +91,11 @@ int miori_stream_sync(void* stream);
  *      347-360, 376-390, 424-454, 524-574. ----------------------------------------- */
 
 /* y[m][n] = sum_k (code[n][k]*s[n][k/group] + b[n][k/group]) * x[m][k], 1 <= M <= 32.
- * The result of a row m does not depend on M (reference shaders/batch.metal:142-144)
- * within the same numeric path: M <= 4 dequantizes in fp32 (as gemv4 / gemv4_b do; at
- * group 64 the 4-bit kernel sums a group's two halves in a different order for M = 3, 4
- * than for M <= 2, so those agree to fp32 rounding rather than bit for bit, while group
- * 32 is bit-identical for all M <= 4); M > 4 multiplies bf16-rounded weights on the
- * tensor cores (as the reference does for wide batches through its bf16 cache,
- * src/batch.cpp:223-230) unless MIORI_GEMV_EXACT is set.  Requires K % group == 0, group in {32,64}; q,s,b,x 16-byte
+ * Every M dequantizes in fp32 (as the reference's gemv4 / gemv4_b do); MIORI_GEMV_EXACT, which once
+ * asked for that above four rows, changes nothing.  The result of a row m does not depend on M
+ * (reference shaders/batch.metal:142-144) within a class of batch sizes, 1..2 and 3..8 rows (4-bit
+ * weights in groups of 64) or 1..4 and 5..8 (others), 9..16, 17..32: across classes rows agree to fp32
+ * rounding, not bit for bit.  Requires K % group == 0, group in {32,64}; q,s,b,x 16-byte
  * aligned.  Only M rows of x are read and M rows of y written (the reference's
  * gemv4_b always touches four, shaders/batch.metal:178-179). */
 int miori_gemv4(const void* q, const void* s, const void* b, const void* x, void* y,
@@ -323,8 +321,8 @@ int miori_argmax(const void* v, uint32_t n, uint32_t flags, void* out_index, voi
  * for g, u the fp32 results of rows i and N/2 + i, bit for bit what miori_gemv4 followed by
  * miori_silu_mul gives.  Saves the activation's launch and the fp32 round trip of 2 N values per
  * row (docs/MILESTONES.md:87, "SiLU x up epilogue").  N a multiple of 16, M <= 16 (wider batches
- * go through the bf16 cache, whose GEMM has no such epilogue); runs on the TMA + mma.sync kernel,
- * shapes it does not take get MIORI_E_INVALID. */
+ * go through the bf16 cache, whose GEMM has no such epilogue); scale rows of a
+ * multiple of 16 bytes, (K / group) % 8 == 0; other shapes get MIORI_E_INVALID. */
 int miori_gemv4_silu(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N,
                      uint32_t K, uint32_t M, uint32_t group, uint32_t flags, void* stream);
 /* The gate + up projection with both neighbours: y = bf16(silu(g) * u) of W * bf16(rmsnorm(x)), x fp32
@@ -339,18 +337,16 @@ int miori_gemv4_rmsnorm_silu(const void* q, const void* s, const void* b, const 
  * over out in place, so the result is bit for bit that of miori_gemv4 followed by
  * miori_post_norm_add.  `counter` is one 32-bit word of device memory that is zero before the first
  * launch; the kernel leaves it zero.  Launches that may run concurrently need counters of their
- * own.  Shapes the TMA + mma.sync kernel does not take get MIORI_E_INVALID. */
+ * own.  Requires (K / group) % 8 == 0; other shapes get MIORI_E_INVALID. */
 int miori_gemv4_post_norm_add(const void* q, const void* s, const void* b, const void* x,
                               const void* residual, const void* gamma, float eps, void* counter,
                               void* out, uint32_t N, uint32_t K, uint32_t M, uint32_t group,
                               uint32_t flags, void* stream);
 /* miori_gemv4 / miori_gemv8 with the RMSNorm of the activations fused into their staging:
  * y = W * bf16(rmsnorm(x)), x fp32 [M][K], gamma bf16 [K].  Saves the norm's launch and the
- * round trip of its output (the fusion the reference planned, docs/MILESTONES.md:87).  4-bit
- * weights with up to four rows of K <= 2048 and fp32 out run on the TMA + mma.sync kernel (every CTA
- * sums the rows' squares for itself, then normalises while it stages), everything else on the tcgen05
- * kernel; shapes
- * neither takes get MIORI_E_INVALID.  The result is the unfused pair's up to the fp32 order of the sum
+ * round trip of its output (the fusion the reference planned, docs/MILESTONES.md:87): every CTA sums
+ * the rows' squares for itself, then normalises while it stages.  Requires (K / group) % 8 == 0; other
+ * shapes get MIORI_E_INVALID.  The result is the unfused pair's up to the fp32 order of the sum
  * of squares. */
 int miori_gemv4_rmsnorm(const void* q, const void* s, const void* b, const void* x, const void* gamma,
                         float eps, void* y, uint32_t N, uint32_t K, uint32_t M, uint32_t group,

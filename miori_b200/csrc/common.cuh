@@ -97,14 +97,28 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// The same, but the thread may sleep up to WAIT_SLEEP_NS in the instruction before it comes back false:
+// a waiting warp then takes no issue slots from the working ones.
+constexpr uint32_t WAIT_SLEEP_NS = 1000000u;
+__device__ __forceinline__ bool mbar_try_long(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(WAIT_SLEEP_NS)
+        : "memory");
+    return ok != 0;
+}
 // Bounded wait.  Returns false if the CTA is aborting (this or another role gave up); on
 // expiry it raises the CTA's abort flag and records a device error with code `where`.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort,
                                           uint32_t where) {
-    if (mbar_try(bar, parity)) return true;
+    if (mbar_try_long(bar, parity)) return true;
     const long long t0 = clock64();
     for (;;) {
-        if (mbar_try(bar, parity)) return true;
+        if (mbar_try_long(bar, parity)) return true;
         if (*abort) return false;
         if (clock64() - t0 > WAIT_LIMIT_CYCLES) {
             *abort = 1u;

@@ -30,12 +30,21 @@
 // Every wait is bounded.
 #pragma once
 #include "common.cuh"
-#include "gemv_mma.cuh"
 #include "gemv_tma.cuh"
 #include "tma_host.cuh"
 
 namespace miori_b200 {
 namespace gemvcache {
+
+// D += A B, 16 x 8 x 16, bf16 operands, fp32 accumulators.
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 
 constexpr int WARPS = 16;
 constexpr int THREADS = (WARPS + 1) * 32;
@@ -73,7 +82,6 @@ gemv_cache_kernel(const __grid_constant__ CUtensorMap tmap_w, const uint16_t* __
     // a slab's slot is s % XF in every tile, so the ring must divide the slabs of a tile
     static_assert(!STREAM || (SLABS > X_AHEAD && SLABS % XF == 0), "streaming is for long rows");
     using C = Cfg<NT>;
-    using namespace gemvmma;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bars[MAX_STAGES];
     __shared__ __align__(8) uint64_t empty_bars[MAX_STAGES];

@@ -1,57 +1,114 @@
-// Weight-streaming GEMV with the weights staged through shared memory by TMA.
+// Weight-streaming GEMV for 1 <= M <= 32 activation rows on the packed 4- or 8-bit weights.
 //
-// One CTA per SM (two for long streams) owns every gridDim-th 16-row tile.  Each slab -- 16 rows x 1 KiB of
-// packed codes plus the rows' scales and biases, three cp.async.bulk.tensor requests -- goes
-// into a ring of shared-memory stages; completion is counted in bytes on a "full" mbarrier
-// per stage and consumers hand stages back through an "empty" mbarrier.  The ring is filled
-// BEFORE the kernel waits for its predecessor (programmatic dependent launch): weights are
-// immutable, so a CTA that starts as its predecessor's CTA exits has its first slabs in flight
-// while the grids hand over.  After the wait the CTA stages x (see gemv_mma.cuh for the arithmetic
-// and the k permutation).
+//   y[m][n] = sum_g ( s[n][g] * sum_{k in g} code[n][k] * x[m][k]  +  b[n][g] * sum_{k in g} x[m][k] )
 //
-// The 16 warps work in four independent groups of four; a group owns whole tiles, each of
-// its warps multiplies 4 of the 16 steps of a slab out of shared memory, and the four
-// partial sums per output are combined through shared memory behind a group-private named
-// barrier by a fixed shuffle tree (so a row's value does not depend on M).  There is no
-// CTA-wide barrier in the main loop.  A 17th warp is the TMA producer: one of its threads
-// refills a stage as soon as its group hands it back.  Out-of-range rows and columns are
-// zero-filled by TMA, which makes every code, scale and bias there contribute exactly 0.
+// The inner sum runs on mma.sync.m16n8k16 with fp16 operands and fp32 accumulators:
+//   * a code in the low bits of a 16-bit half IS an fp16 value: the subnormal code * 2^-24.  So a word
+//     of eight 4-bit codes becomes its four A registers with one shift and four ANDs, the codes in bits
+//     4 .. 7 of a half counting 16 times (their activations are staged divided by 16), a word of four
+//     8-bit codes becomes two registers with one shift and two ANDs.  No offset is added to the codes, so
+//     none has to be subtracted from the sums;
+//   * a scale group's activations are multiplied by the power of two that puts the largest into
+//     [2^15, 2^16): bf16's eight bits are exact in fp16 for every activation of at least 2^-28 of the
+//     group's largest (the error below that is under 2^-36 of the largest).
+// Every lane of the accumulator then applies the group's fp32 scale and bias: fp32 dequantization, the
+// arithmetic class of the reference's gemv4 / gemv4_b / gemv8, for every M.  (The same product with
+// e4m3 operands, whose subnormals hold a 4-bit code in a byte, needs half the MMAs; mma.sync takes 25
+// cycles for one on sm_100a against 2 for fp16.)
 //
-// Optional neighbours of the projection, each a template parameter so that the plain instantiation
-// is compiled as if they did not exist: NORMED (RMSNorm of fp32 activations inside the staging pass),
+// What bounds it: HBM for long 8-bit streams, the issue slots (some 90 warp instructions per KiB of codes)
+// for long 4-bit ones, the hand-over between dependent launches and the trip of x through L2 for short
+// ones.  Measured in chains of dependent launches over weights larger than L2, before (codes as bf16
+// 128 + code, one producer) and now, us: 8-bit head 131072 x 2048 at 1, 4, 16 rows 53.1, 60.3, 93 -> 44.1
+// (6.46 TB/s, 0.99 of a plain copy), 45.2, 75; 4-bit 16384 x 2048 at 1, 4, 8 rows 7.44, 8.80, 10.2 ->
+// 6.54, 7.14, 7.75; 2048 x 8192 at 1, 4 rows 6.58, 9.56 -> 4.62, 6.15; 2048 x 2048 at 1 row 2.64 -> 2.40.
+//
+// One CTA per SM owns every gridDim-th 16-row tile.  A slab -- 16 rows x up to 1 KiB of codes -- is one
+// 2-D TMA copy into a shared-memory ring; a tile's scales and biases (contiguous in memory) are two
+// bulk copies into a ring of their own.  Completion is counted in bytes on mbarriers, buffers are
+// handed back through "empty" mbarriers.  The rings are filled BEFORE the kernel waits for its
+// predecessor (programmatic dependent launch): weights are immutable, so a CTA that starts as its
+// predecessor's CTA exits has its first slabs in flight while the grids hand over.
+//
+// The 16 compute warps work in four independent groups of four; a group owns whole tiles, each of its
+// warps multiplies a run of four neighbouring 64-byte steps of a slab, and the four partial sums per
+// output are combined through shared memory behind a group-private named barrier by a fixed shuffle
+// tree.  There is no CTA-wide barrier in the main loop.  Every group has a producer warp of its own,
+// which only issues copies: with one producer for the CTA its hundred dependent instructions per slab and
+// tile bounded long streams (151 MB of 4-bit weights: 46 us, 31 now), not the math.  Out-of-range rows
+// and columns are zero-filled by TMA and staged as zeros.
+//
+// The eight MMA columns.  With more than four activation rows they are rows, and the quad's lanes read
+// 4 or 8 bytes each so that a chain of MMAs covers one scale group.  With one, two or four rows the lanes
+// read 16 bytes and the columns are (slot, row) with 8, 4 or 2 slots: a slot is one scale group of the
+// run, its activations are zero in the lanes and steps that hold other groups, so one accumulator
+// collects the sums of up to eight groups, each column its own, and scales are applied once per eight
+// groups instead of once per group.  The sums of a row then meet in the same order for one to four rows:
+// lane and register hold the groups of one residue modulo eight, added up in a fixed tree.
+//
+// Optional neighbours of the projection, each a template value so that the plain instantiation is
+// compiled as if they did not exist: NORMED (RMSNorm of fp32 activations inside the staging pass),
 // GATED (SiLU x up behind the fused gate + up rows), POSTNORM (post-norm and residual add by the CTA
-// that finishes last), ARGMAX (greedy pick of a sharded head).
+// that finishes last), SHARDED / ARGMAX (exchange with the peer GPUs, greedy pick of a sharded head).
 #pragma once
 #include "common.cuh"
-#include "gemv_mma.cuh"
 #include "norm.cuh"
 #include "peers.cuh"
 #include "tma_host.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace miori_b200 {
 namespace gemvtma {
 
-constexpr int GROUPS = 4;                  // independent groups of 4 warps
-constexpr int WARPS = 4 * GROUPS;           // compute warps
-constexpr int THREADS = (WARPS + 1) * 32;  // plus one producer warp
-constexpr int MAX_STAGES = 12;
-constexpr int ROW_BYTES = 1024;            // packed bytes of one row in one slab
-constexpr int Q_BYTES = 16 * ROW_BYTES;
-constexpr int SB_BYTES = 16 * 128;         // scales (or biases) of 16 rows, up to 64 groups each
-constexpr int STAGE_BYTES = Q_BYTES + 2 * SB_BYTES;  // 20480
-// staged x in 16-byte units: the 4 chunks of a step sit at unit offsets 0,4,10,14 of an
-// 18-unit step and rows have an odd pitch, so the 8 lanes of a quarter warp (2 rows x 4
-// chunks) read 8 distinct bank groups with plain immediate offsets
-constexpr int STEP_UNITS = 18;
-constexpr int SLAB_X_BYTES = 16 * STEP_UNITS * 16;                 // staged x per k-slab and row
-constexpr int ZERO_BYTES = 3 * 4 * STEP_UNITS * 16 + 4 * 16 + 64;  // zeros read by masked lanes
+constexpr int GROUPS = 4;                        // independent groups of 4 warps
+constexpr int WARPS = 4 * GROUPS;                // compute warps
+constexpr int COMPUTE = WARPS * 32;
+constexpr int THREADS = COMPUTE + GROUPS * 32;   // plus one producer warp per group
+constexpr int MAX_NSG = 8;                       // code stages (and scale buffers) of one group
+constexpr uint32_t SLAB_ROW = 1024;              // packed bytes of one row in a full slab
+constexpr uint32_t STEP_BYTES = 64;              // packed bytes of one row in a step
 
-template <int MP>
+constexpr int cmin(int a, int b) { return a < b ? a : b; }
+constexpr int cmax(int a, int b) { return a > b ? a : b; }
+
+// How a launch maps codes and activation rows to MMA operands.  ROWS: 1, 2, 4, 8, 16 or 32.
+template <int BITS_, int GROUP_, int ROWS_>
+struct Shape {
+    static constexpr int BITS = BITS_, GROUP = GROUP_, ROWS = ROWS_;
+    static constexpr int GPS = (int)STEP_BYTES * 8 / BITS / GROUP;  // scale groups per step: 1, 2 or 4
+    static constexpr bool SLOTTED = ROWS < 8;
+    static constexpr int NT = cmax(1, ROWS / 8);                    // sets of eight columns
+    static constexpr int RC = cmin(ROWS, 8);                        // activation rows per set
+    // slotted: columns are (slot, row); a pass covers SPA steps into SETS accumulators
+    static constexpr int SLOTS = 8 / RC;
+    static constexpr int SPA = cmin(4, cmax(1, SLOTS / GPS));
+    static constexpr int SETS = cmax(1, GPS / SLOTS);
+    static constexpr int NCLS = cmin(8, 4 * GPS);                   // residue classes of groups kept apart
+    static constexpr int ACCN = SLOTTED ? cmax(1, NCLS / SLOTS) : NT;
+    // bytes a lane reads of a row per chain, chains per step
+    static constexpr int W = SLOTTED ? 16 : 16 / GPS;
+    static constexpr int CH = 16 / W;
+    static constexpr int NW = W / 4;
+    static constexpr int XB = W * 8 / BITS * 2;                     // bytes of staged x per lane and chain
+    static constexpr uint32_t KC = SLAB_ROW * 8 / BITS;             // codes per full slab
+    static constexpr uint32_t SK = STEP_BYTES * 8 / BITS;           // codes per step
+    // Row pitches in shared memory are these many bytes past a multiple of 128, so that the rows that a
+    // quarter-warp (16-byte loads), half-warp (8) or warp (4) reads fall into different banks.
+    static constexpr uint32_t QPAD = W == 16 ? 64 : W == 8 ? 32 : 16;
+    static constexpr uint32_t XPAD = XB == 16 ? 64 : 16;
+};
+
+// zeros read by the lanes whose codes belong to another slot
+constexpr uint32_t ZERO_BYTES = 64;
+
+// Partial outputs of a group's four warps: [buffers][16 * ROWS outputs][4 warps] floats.  Two buffers, so
+// that one barrier per tile is enough; one where two would cost stages of the code ring.
+template <int ROWS>
 struct Red {
-    static constexpr int WS = 16 * MP + 1;           // padded stride of one warp's partials
-    static constexpr int GROUP_FLOATS = 2 * 4 * WS;  // double-buffered, 4 warps
+    static constexpr int BUFS = ROWS <= 8 ? 2 : 1;
+    static constexpr int FLOATS = 16 * ROWS * 4;
 };
 
 // Shared-memory loads by 32-bit shared address (one instruction each, no generic addressing).
@@ -62,289 +119,273 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
     return v;
 }
-__device__ __forceinline__ uint32_t lds16(uint32_t a) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ float ldsf32(uint32_t a) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-    return v;
-}
-
 __device__ __forceinline__ uint2 lds64(uint32_t a) {
     uint2 v;
     asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
     return v;
 }
+__device__ __forceinline__ float4 ldsf128(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t a) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+    return v;
+}
+template <int BYTES>
+__device__ __forceinline__ void lds_words(uint32_t (&r)[BYTES / 4], uint32_t a) {
+    static_assert(BYTES == 4 || BYTES == 8 || BYTES % 16 == 0, "");
+    if constexpr (BYTES == 4) {
+        r[0] = lds32(a);
+    } else if constexpr (BYTES == 8) {
+        const uint2 v = lds64(a);
+        r[0] = v.x, r[1] = v.y;
+    } else {
+#pragma unroll
+        for (int i = 0; i < BYTES / 16; ++i) {
+            const uint4 v = lds128(a + 16u * i);
+            r[4 * i] = v.x, r[4 * i + 1] = v.y, r[4 * i + 2] = v.z, r[4 * i + 3] = v.w;
+        }
+    }
+}
+__device__ __forceinline__ void named_barrier(uint32_t id, uint32_t threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// D += A B, 16 x 8 x 16, fp16 operands, fp32 accumulators.
+__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                        uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void mma_f16_z(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                          uint32_t b0, uint32_t b1) {  // D = A B
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+}
+
+// The A registers of one lane for one chain: codes of rows g and g + 8.
+template <int BITS, int NW>
+struct AFrag {
+    static constexpr int AR = BITS == 4 ? 4 : 2;  // registers per word and row
+    static constexpr int MMAS = NW * AR / 2;
+    uint32_t r0[NW][AR], r1[NW][AR];
+    __device__ __forceinline__ void unpack(const uint32_t (&q0)[NW], const uint32_t (&q1)[NW]) {
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            const uint32_t h0 = q0[w] >> 8, h1 = q1[w] >> 8;
+            if constexpr (BITS == 4) {
+                r0[w][0] = q0[w] & 0x000F000Fu, r0[w][1] = q0[w] & 0x00F000F0u, r0[w][2] = h0 & 0x000F000Fu, r0[w][3] = h0 & 0x00F000F0u;
+                r1[w][0] = q1[w] & 0x000F000Fu, r1[w][1] = q1[w] & 0x00F000F0u, r1[w][2] = h1 & 0x000F000Fu, r1[w][3] = h1 & 0x00F000F0u;
+            } else {
+                r0[w][0] = q0[w] & 0x00FF00FFu, r0[w][1] = h0 & 0x00FF00FFu;
+                r1[w][0] = q1[w] & 0x00FF00FFu, r1[w][1] = h1 & 0x00FF00FFu;
+            }
+        }
+    }
+    // MMA i of the chain against its two B registers
+    __device__ __forceinline__ void mma(bool first, int i, float (&d)[4], uint32_t b0, uint32_t b1) const {
+        const int w = i / (AR / 2), p = i % (AR / 2) * 2;
+        if (first) mma_f16_z(d, r0[w][p], r1[w][p], r0[w][p + 1], r1[w][p + 1], b0, b1);
+        else mma_f16(d, r0[w][p], r1[w][p], r0[w][p + 1], r1[w][p + 1], b0, b1);
+    }
+};
+
+// ---- staging of the activations ------------------------------------------------------------
+
 // two floats -> packed fp16 pair (lo, hi), round to nearest even
 __device__ __forceinline__ uint32_t f16x2_bits(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
-// a float rounded to fp16 and back: the value the tensor core will see
-__device__ __forceinline__ float through_f16(float v) {
-    float r;
-    asm("{\n\t.reg .b16 h;\n\tcvt.rn.f16.f32 h, %1;\n\tcvt.f32.f16 %0, h;\n\t}" : "=f"(r) : "f"(v));
-    return r;
-}
 
-__device__ __forceinline__ void named_barrier(uint32_t id, uint32_t threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-__device__ __forceinline__ uint32_t x_unit(uint32_t step, uint32_t t, uint32_t wd) {
-    return step * STEP_UNITS + 4u * t + 2u * (t >> 1) + wd;
-}
-
-// Stage x for the MMA B operand: permuted to the k order of the A fragments (8-bit codes: as
-// fp16 scaled by `mul`), laid out by x_unit(); for EXACT also the fp32 sum of x over every chunk
-// (PAIR: over every pair of chunks, i.e. every 64-weight group).
-// `ld8(m, u)` returns the eight bf16 activations 8u .. 8u+7 of row m (4-bit codes; the plain
-// loader reads x, the norm-fused one normalises fp32 activations on the fly).
-template <int BITS, bool EXACT, int MP, bool PAIR, class LD>
-__device__ __forceinline__ void stage_x_padded(const uint16_t* __restrict__ x, uint4* xs,
-                                               float* xsum, uint32_t M, uint32_t K,
-                                               uint32_t steps_p, uint32_t pitch, uint32_t cpr,
-                                               const float* mul_rows, LD ld8) {
-    constexpr int CW = 128 / BITS, KU = BITS == 4 ? 8 : 4;
-    const uint32_t upr = steps_p * 16u;  // logical units per row
-    for (uint32_t i = threadIdx.x; i < (uint32_t)MP * upr; i += THREADS) {
-        const uint32_t m = i / upr, u = i - m * upr;
-        uint4 o = make_uint4(0u, 0u, 0u, 0u);
-        if (m < M && u * KU < K) {
-            if (BITS == 4) {
-                const uint4 v = ld8(m, u);
-                o.x = __byte_perm(v.x, v.z, 0x5410);  // (x0,x4)
-                o.y = __byte_perm(v.x, v.z, 0x7632);  // (x1,x5)
-                o.z = __byte_perm(v.y, v.w, 0x5410);  // (x2,x6)
-                o.w = __byte_perm(v.y, v.w, 0x7632);  // (x3,x7)
-            } else {
-                // 8-bit codes go to the tensor core as fp16 (1024 + code), so x goes as fp16 too,
-                // scaled by the row's power of two that keeps its largest value below 2^15; the
-                // unit holds (x0,x2) and (x1,x3), the k order of the byte pairs the unpack makes
-                const uint2 v = __ldg(reinterpret_cast<const uint2*>(x + (size_t)m * K) + u);
-                const float mul = mul_rows[m];
-                o.x = f16x2_bits(bf16lo(v.x) * mul, bf16lo(v.y) * mul);
-                o.y = f16x2_bits(bf16hi(v.x) * mul, bf16hi(v.y) * mul);
-            }
-        }
-        xs[(size_t)m * pitch + x_unit(u >> 4, (u >> 2) & 3u, u & 3u)] = o;
-    }
-    if (EXACT) {
-        const uint32_t chunks = K / CW;
-        for (uint32_t i = threadIdx.x; i < (uint32_t)MP * cpr; i += THREADS) {
-            const uint32_t m = i / cpr, c = i - m * cpr;
-            float sum = 0.0f;
-            if (m < M && c < chunks) {
-                const float mul = BITS == 8 ? mul_rows[m] : 1.0f;
-                // PAIR: both chunks of a 64-weight group carry the sum over the whole group
-                const uint32_t c0 = PAIR ? (c & ~1u) : c;
-                const uint4* xp = reinterpret_cast<const uint4*>(x + (size_t)m * K + (size_t)c0 * CW);
+// Stage one unit -- eight consecutive activations of a row as bf16 -- for the MMA B operand: scaled fp16
+// pairs in the order of the A registers and, by the first lane of each scale group, the group's {power
+// of two that undoes the scaling, sum of x} / 512 (so that the power of two stays finite for every
+// input; the outputs are multiplied at the end).  The GROUP / 8 lanes of a group hold neighbouring
+// units; every lane of the warp calls.
+constexpr float UNSCALE = 512.0f;
+template <int BITS, int GROUP>
+__device__ __forceinline__ void stage_unit(const uint4& v, bool live, uint32_t x_addr, bool first, uint32_t ms_addr) {
+    const uint32_t a = v.x & 0x7FFF7FFFu, b = v.y & 0x7FFF7FFFu, c = v.z & 0x7FFF7FFFu, d = v.w & 0x7FFF7FFFu;
+    const uint32_t mx2 = __vmaxu2(__vmaxu2(a, b), __vmaxu2(c, d));
+    uint32_t mx = max(mx2 & 0xFFFFu, mx2 >> 16);
+    const float f[8] = {bf16lo(v.x), bf16hi(v.x), bf16lo(v.y), bf16hi(v.y), bf16lo(v.z), bf16hi(v.z), bf16lo(v.w), bf16hi(v.w)};
+    float sum = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
 #pragma unroll
-                for (int j = 0; j < (PAIR ? 2 : 1) * CW / 8; ++j) {
-                    const uint4 v = BITS == 4 ? ld8(m, c0 * (CW / 8) + j) : __ldg(xp + j);
-                    if (BITS == 4) {
-                        sum += bf16lo(v.x); sum += bf16hi(v.x); sum += bf16lo(v.y); sum += bf16hi(v.y);
-                        sum += bf16lo(v.z); sum += bf16hi(v.z); sum += bf16lo(v.w); sum += bf16hi(v.w);
-                    } else {  // the sum of exactly the fp16 values staged above
-                        sum += through_f16(bf16lo(v.x) * mul); sum += through_f16(bf16hi(v.x) * mul);
-                        sum += through_f16(bf16lo(v.y) * mul); sum += through_f16(bf16hi(v.y) * mul);
-                        sum += through_f16(bf16lo(v.z) * mul); sum += through_f16(bf16hi(v.z) * mul);
-                        sum += through_f16(bf16lo(v.w) * mul); sum += through_f16(bf16hi(v.w) * mul);
-                    }
-                }
-            }
-            xsum[i] = sum;
-        }
+    for (int o = 1; o < GROUP / 8; o <<= 1) {
+        mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    }
+    const uint32_t e = max(mx >> 7, 15u);  // exponent field of the largest; tiny groups stay below 2^15
+    const float scale = __uint_as_float((269u - e) << 23);
+    uint32_t o[4];
+    if constexpr (BITS == 4) {
+        const float low = 0.0625f * scale;  // for the codes that count 16 times
+        o[0] = f16x2_bits(f[0] * scale, f[4] * scale), o[1] = f16x2_bits(f[1] * low, f[5] * low);
+        o[2] = f16x2_bits(f[2] * scale, f[6] * scale), o[3] = f16x2_bits(f[3] * low, f[7] * low);
+    } else {
+        o[0] = f16x2_bits(f[0] * scale, f[2] * scale), o[1] = f16x2_bits(f[1] * scale, f[3] * scale);
+        o[2] = f16x2_bits(f[4] * scale, f[6] * scale), o[3] = f16x2_bits(f[5] * scale, f[7] * scale);
+    }
+    if (live) {
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(x_addr), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+        if (first)
+            asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ms_addr), "f"(__uint_as_float(e << 23)), "f"(sum * (1.0f / UNSCALE)) : "memory");
     }
 }
 
-// The same staging in one pass: a thread loads a unit, stores it permuted, and the 4 (PAIR: 8)
-// lanes that hold a chunk (a 64-weight group) add up its fp32 sum with shuffles, so x is read once
-// and there is one load latency instead of two.  Two units per thread and trip, both loads issued
-// before either is used, so that a long row (K = 8192: four units per thread) costs two load
-// latencies, not four.  Whole warps iterate (THREADS and the units per row are multiples of 32
-// resp. 16, so lane groups never straddle a chunk).
-template <int BITS, bool EXACT, int MP, bool PAIR, class LD>
-__device__ __forceinline__ void stage_x_onepass(uint4* xs, float* xsum, uint32_t M, uint32_t K,
-                                                uint32_t steps_p, uint32_t pitch, uint32_t cpr, LD ld8) {
-    static_assert(BITS == 4, "one-pass staging exists for 4-bit codes only (8-bit x is staged as scaled fp16)");
-    static_assert(MP <= 4, "row index by comparison");
-    constexpr int KU = 8;
-    const uint32_t upr = steps_p * 16u;  // logical units per row
-    const uint32_t total = (uint32_t)MP * upr, lane = threadIdx.x & 31u;
-    for (uint32_t i0 = threadIdx.x - lane; i0 < total; i0 += 2u * THREADS) {
-        uint32_t i[2], m[2], u[2];
-        bool live[2];
-        uint4 v[2];
+// Where the staged activations of a CTA lie.
+struct XArea {
+    uint32_t x;      // shared address: [M][pitch] bytes
+    uint32_t pitch;
+    uint32_t ms;     // shared address: [K / GROUP][ROWS] float2
+};
+template <class S>
+__device__ __forceinline__ void stage_unit_at(const XArea& xa, const uint4& v, bool live, uint32_t m, uint32_t u) {
+    constexpr uint32_t UPG = S::GROUP / 8;
+    stage_unit<S::BITS, S::GROUP>(v, live, xa.x + m * xa.pitch + 16u * u, (u & (UPG - 1u)) == 0u,
+                                  xa.ms + ((u / UPG) * S::ROWS + m) * 8u);
+}
+
+// Stage M rows of K bf16 activations, several units per thread and trip with all loads issued first: every
+// CTA of the grid asks L2 for the same lines at the same moment, and each dependent trip pays that queue
+// again.  (Fewer for one row, which has at most two units per thread up to K = 8192: code that runs once
+// per launch costs its instruction fetches, 0.1 us here.  Loading the next trip's units before working on
+// this trip's, and copying all units first and working in place in a short loop, were both slower by 0.1
+// to 1 us from two rows up.)  inv_upr = ceil(2^32 / (K / 8)).
+template <class S>
+__device__ __forceinline__ void stage_x(const XArea& xa, const uint16_t* __restrict__ x, uint32_t M, uint32_t K, uint32_t inv_upr) {
+    const uint32_t upr = K >> 3, total = M * upr, lane = threadIdx.x & 31u;
+    constexpr int AHEAD = S::ROWS == 1 ? 2 : 4;
+    for (uint32_t i0 = threadIdx.x - lane; i0 < total; i0 += AHEAD * COMPUTE) {
+        uint4 v[AHEAD];
+        uint32_t m[AHEAD], u[AHEAD];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            i[h] = i0 + lane + (uint32_t)h * THREADS;
-            m[h] = (i[h] >= upr ? 1u : 0u) + (MP > 2 ? (i[h] >= 2u * upr ? 1u : 0u) + (i[h] >= 3u * upr ? 1u : 0u) : 0u);
-            u[h] = i[h] - m[h] * upr;
-            live[h] = i[h] < total && m[h] < M && u[h] * KU < K;
+        for (int h = 0; h < AHEAD; ++h) {
+            const uint32_t i = i0 + lane + (uint32_t)h * COMPUTE;
+            m[h] = S::ROWS == 1 ? 0u : __umulhi(i, inv_upr);
+            u[h] = i - m[h] * upr;
             v[h] = make_uint4(0u, 0u, 0u, 0u);
-            if (live[h]) v[h] = ld8(m[h], u[h]);
+            if (i < total) v[h] = __ldg(reinterpret_cast<const uint4*>(x) + i);
         }
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (i0 + (uint32_t)h * THREADS >= total) break;  // warp-uniform
-            uint4 o;
-            o.x = __byte_perm(v[h].x, v[h].z, 0x5410);  // (x0,x4)
-            o.y = __byte_perm(v[h].x, v[h].z, 0x7632);  // (x1,x5)
-            o.z = __byte_perm(v[h].y, v[h].w, 0x5410);  // (x2,x6)
-            o.w = __byte_perm(v[h].y, v[h].w, 0x7632);  // (x3,x7)
-            if (i[h] < total) xs[(size_t)m[h] * pitch + x_unit(u[h] >> 4, (u[h] >> 2) & 3u, u[h] & 3u)] = o;
-            if (EXACT) {
-                float sum = ((bf16lo(v[h].x) + bf16hi(v[h].x)) + (bf16lo(v[h].y) + bf16hi(v[h].y))) +
-                            ((bf16lo(v[h].z) + bf16hi(v[h].z)) + (bf16lo(v[h].w) + bf16hi(v[h].w)));
-                sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-                sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
-                if (PAIR) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 4);
-                if (i[h] < total && (u[h] & 3u) == 0u) xsum[m[h] * cpr + (u[h] >> 2)] = sum;
+        for (int h = 0; h < AHEAD; ++h) {
+            if (i0 + (uint32_t)h * COMPUTE >= total) break;  // warp-uniform
+            stage_unit_at<S>(xa, v[h], i0 + lane + (uint32_t)h * COMPUTE < total, m[h], u[h]);
+        }
+    }
+}
+
+// The stand-alone norm kernel's arithmetic for two activations: x * inv * gamma, rounded to bf16.
+__device__ __forceinline__ uint32_t normed2(float lo, float hi, float inv, uint32_t g2) {
+    return float_to_bf16_bits(lo * inv * bf16lo(g2)) | (float_to_bf16_bits(hi * inv * bf16hi(g2)) << 16);
+}
+__device__ __forceinline__ uint4 normed8(const float4& a, const float4& c, float inv, const uint4& g) {
+    return make_uint4(normed2(a.x, a.y, inv, g.x), normed2(a.z, a.w, inv, g.y), normed2(c.x, c.y, inv, g.z),
+                      normed2(c.z, c.w, inv, g.w));
+}
+
+// Meeting point of the compute warps.
+__device__ __forceinline__ void compute_sync() { named_barrier(15u, COMPUTE); }
+
+// Staging with the RMSNorm in it (shaders/ops.metal:86-115): x is fp32.  Up to four rows of K <= 4096 take
+// one trip to L2: thread u loads unit u of every row together with its norm weights, the warps add up
+// the rows' squares (shuffles, 16 warp sums per row through shared memory, every thread adds them in
+// order) and each thread normalises what it holds.  Anything larger sums the squares of four rows at a
+// time first and normalises in the loader of the plain staging.  Called by the compute warps.
+template <class S>
+__device__ __forceinline__ void stage_x_normed(const XArea& xa, const float* __restrict__ x,
+                                               const uint16_t* __restrict__ gamma, float eps, uint32_t M, uint32_t K,
+                                               uint32_t inv_upr, float (&part)[4][WARPS], float (&inv_row)[32]) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, upr = K >> 3;
+    const float4* x4 = reinterpret_cast<const float4*>(x);
+    const uint4* g4 = reinterpret_cast<const uint4*>(gamma);
+    constexpr uint32_t R = S::ROWS < 4 ? S::ROWS : 4;
+    if (S::ROWS <= 4 && upr <= (uint32_t)COMPUTE) {
+        const bool mine = tid < upr;
+        float4 a[R], c[R];
+        uint4 g = make_uint4(0u, 0u, 0u, 0u);
+        if (mine) g = __ldg(g4 + tid);
+#pragma unroll
+        for (uint32_t m = 0; m < R; ++m) {
+            a[m] = c[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (mine && m < M) {
+                a[m] = __ldg(x4 + ((size_t)m * upr + tid) * 2u);
+                c[m] = __ldg(x4 + ((size_t)m * upr + tid) * 2u + 1u);
             }
         }
-    }
-}
-
-// One-pass staging for more than four staged rows, for rows short enough that every thread handles one or two
-// units (K <= 2048): a thread loads a unit, stores it permuted, and the 4 (PAIR: 8) lanes that hold
-// a chunk (a 64-weight group) add up its fp32 sum with shuffles, so x is read once and there is
-// one load latency instead of two.  Whole warps iterate (THREADS and the units per row are
-// multiples of 32 resp. 16, so lane groups never straddle a chunk).  For long rows the two-pass
-// version above is faster: its loads are independent across iterations.
-template <int BITS, bool EXACT, int MP, bool PAIR, class LD>
-__device__ __forceinline__ void stage_x_onepass_wide(uint4* xs, float* xsum, uint32_t M, uint32_t K,
-                                                uint32_t steps_p, uint32_t pitch, uint32_t cpr, LD ld8) {
-    static_assert(BITS == 4, "one-pass staging exists for 4-bit codes only (8-bit x is staged as scaled fp16)");
-    constexpr int KU = 8;
-    const uint32_t upr = steps_p * 16u;  // logical units per row
-    const uint32_t total = (uint32_t)MP * upr, lane = threadIdx.x & 31u;
-    for (uint32_t i0 = threadIdx.x - lane; i0 < total; i0 += THREADS) {
-        const uint32_t i = i0 + lane;
-        const uint32_t m = i / upr, u = i - m * upr;
-        uint4 o = make_uint4(0u, 0u, 0u, 0u);
-        float sum = 0.0f;
-        if (i < total && m < M && u * KU < K) {
-            const uint4 v = ld8(m, u);
-            o.x = __byte_perm(v.x, v.z, 0x5410);  // (x0,x4)
-            o.y = __byte_perm(v.x, v.z, 0x7632);  // (x1,x5)
-            o.z = __byte_perm(v.y, v.w, 0x5410);  // (x2,x6)
-            o.w = __byte_perm(v.y, v.w, 0x7632);  // (x3,x7)
-            if (EXACT)
-                sum = ((bf16lo(v.x) + bf16hi(v.x)) + (bf16lo(v.y) + bf16hi(v.y))) +
-                      ((bf16lo(v.z) + bf16hi(v.z)) + (bf16lo(v.w) + bf16hi(v.w)));
-        }
-        if (i < total) xs[(size_t)m * pitch + x_unit(u >> 4, (u >> 2) & 3u, u & 3u)] = o;
-        if (EXACT) {
-            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
-            if (PAIR) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 4);
-            if (i < total && (u & 3u) == 0u) xsum[m * cpr + (u >> 2)] = sum;
-        }
-    }
-}
-
-// Staging with the RMSNorm in it (shaders/ops.metal:86-115), rows of K <= 2048: x is fp32.  Thread
-// i < K/4 loads piece i (four activations) of every row together with its four norm weights -- one
-// trip to L2 for everything, which matters because every CTA of the grid asks for the same lines at
-// the same moment -- the warps add up the rows' squares (shuffles, 16 warp sums per row through
-// shared memory, every thread adds them in order), and each thread normalises its piece with the
-// stand-alone kernel's arithmetic, x * inv * gamma rounded to bf16.  Lane pairs then form the
-// eight-activation units of the plain staging (permuted store, and for EXACT the fp32 sum over
-// every chunk resp. chunk pair, added up in the plain staging's order).
-template <bool EXACT, int MP, bool PAIR>
-__device__ __forceinline__ void stage_x_normed(const float* __restrict__ x, const uint16_t* __restrict__ gamma,
-                                               float eps, uint4* xs, float* xsum, uint32_t M, uint32_t K,
-                                               uint32_t pitch, uint32_t cpr, float* part) {
-    static_assert(MP <= 4, "rows of the norm prologue");
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t qpr = K >> 2;  // pieces per row, at most 512
-    const bool mine = tid < qpr;
-    float4 v[MP];
-    uint2 gq = make_uint2(0u, 0u);
-    if (mine) gq = __ldg(reinterpret_cast<const uint2*>(gamma) + tid);
 #pragma unroll
-    for (int m = 0; m < MP; ++m) {
-        v[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (mine && (uint32_t)m < M) v[m] = __ldg(reinterpret_cast<const float4*>(x) + (size_t)m * qpr + tid);
-    }
-    // units past K and rows past M read as zeros
-    for (uint32_t i = tid; i < (uint32_t)MP * pitch; i += THREADS) xs[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (EXACT)
-        for (uint32_t i = tid; i < (uint32_t)MP * cpr; i += THREADS) xsum[i] = 0.0f;
-    if (warp < 16u) {
-#pragma unroll
-        for (int m = 0; m < MP; ++m) {
-            float ss = __fmaf_rn(v[m].w, v[m].w, __fmaf_rn(v[m].z, v[m].z, __fmaf_rn(v[m].y, v[m].y, v[m].x * v[m].x)));
+        for (uint32_t m = 0; m < R; ++m) {
+            if (m >= M) break;
+            float ss = a[m].x * a[m].x;
+            ss = __fmaf_rn(a[m].y, a[m].y, ss), ss = __fmaf_rn(a[m].z, a[m].z, ss), ss = __fmaf_rn(a[m].w, a[m].w, ss);
+            ss = __fmaf_rn(c[m].x, c[m].x, ss), ss = __fmaf_rn(c[m].y, c[m].y, ss), ss = __fmaf_rn(c[m].z, c[m].z, ss);
+            ss = __fmaf_rn(c[m].w, c[m].w, ss);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-            if (lane == 0) part[m * 16 + warp] = ss;
+            if (lane == 0) part[m][warp] = ss;
         }
+        compute_sync();
+        if (warp * 32u >= upr) return;
+#pragma unroll
+        for (uint32_t m = 0; m < R; ++m) {
+            if (m >= M) break;
+            float tot = 0.0f;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) tot += part[m][w];
+            const float inv = rsqrtf(tot / (float)K + eps);
+            stage_unit_at<S>(xa, normed8(a[m], c[m], inv, g), mine, m, tid);
+        }
+        return;
     }
-    __syncthreads();
-    if (warp >= 16u) return;
+    const uint32_t qpr = K >> 2;
+    for (uint32_t m0 = 0; m0 < M; m0 += 4u) {
+        float ss[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (uint32_t i = tid; i < qpr; i += COMPUTE) {
 #pragma unroll
-    for (int m = 0; m < MP; ++m) {
-        if ((uint32_t)m >= M) break;  // CTA-uniform
-        float tot = 0.0f;
+            for (uint32_t r = 0; r < 4u; ++r) {
+                if (m0 + r < M) {
+                    const float4 v = __ldg(x4 + (size_t)(m0 + r) * qpr + i);
+                    ss[r] = __fmaf_rn(v.w, v.w, __fmaf_rn(v.z, v.z, __fmaf_rn(v.y, v.y, __fmaf_rn(v.x, v.x, ss[r]))));
+                }
+            }
+        }
 #pragma unroll
-        for (int w = 0; w < 16; ++w) tot += part[m * 16 + w];
-        const float inv = rsqrtf(tot / (float)K + eps);
-        const uint32_t lo = float_to_bf16_bits(v[m].x * inv * bf16lo(gq.x)) |
-                            (float_to_bf16_bits(v[m].y * inv * bf16hi(gq.x)) << 16);
-        const uint32_t hi = float_to_bf16_bits(v[m].z * inv * bf16lo(gq.y)) |
-                            (float_to_bf16_bits(v[m].w * inv * bf16hi(gq.y)) << 16);
-        // the even lane of a pair collects the unit: activations 8u .. 8u+7, u = tid / 2
-        const uint32_t olo = __shfl_down_sync(0xFFFFFFFFu, lo, 1), ohi = __shfl_down_sync(0xFFFFFFFFu, hi, 1);
-        const uint32_t u = tid >> 1;
-        if (mine && (tid & 1u) == 0u) {
-            uint4 o;
-            o.x = __byte_perm(lo, olo, 0x5410);  // (x0,x4)
-            o.y = __byte_perm(lo, olo, 0x7632);  // (x1,x5)
-            o.z = __byte_perm(hi, ohi, 0x5410);  // (x2,x6)
-            o.w = __byte_perm(hi, ohi, 0x7632);  // (x3,x7)
-            xs[(size_t)m * pitch + x_unit(u >> 4, (u >> 2) & 3u, u & 3u)] = o;
+        for (uint32_t r = 0; r < 4u; ++r) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ss[r] += __shfl_xor_sync(0xFFFFFFFFu, ss[r], o);
+            if (lane == 0) part[r][warp] = ss[r];
         }
-        if (EXACT) {
-            float sum = (bf16lo(lo) + bf16hi(lo)) + (bf16lo(hi) + bf16hi(hi));
-            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);  // the unit
-            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
-            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 4);  // the chunk of 32
-            if (PAIR) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 8);
-            if (mine && (tid & 7u) == 0u) xsum[m * cpr + (tid >> 3)] = sum;
+        compute_sync();
+        if (tid < 4u && m0 + tid < M) {
+            float tot = 0.0f;
+            for (int w = 0; w < WARPS; ++w) tot += part[tid][w];
+            inv_row[m0 + tid] = rsqrtf(tot / (float)K + eps);
         }
+        compute_sync();
+    }
+#pragma unroll 2
+    for (uint32_t i0 = tid - lane; i0 < M * upr; i0 += COMPUTE) {  // whole warps
+        const uint32_t i = i0 + lane, m = S::ROWS == 1 ? 0u : __umulhi(i, inv_upr), u = i - m * upr;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (i < M * upr) v = normed8(__ldg(x4 + 2 * (size_t)i), __ldg(x4 + 2 * (size_t)i + 1), inv_row[m], __ldg(g4 + u));
+        stage_unit_at<S>(xa, v, i < M * upr, m, u);
     }
 }
-
-// ROOMY: compiled for one CTA per SM (up to 120 registers instead of 56).  Problems of at most
-// two tiles per SM run 4-18 % faster that way (no spills, freer scheduling); long streams prefer
-// two CTAs per SM.
-// PAIR (4-bit, group 64, EXACT, NT = 1): the two 32-weight chunks of a scale group sit in
-// neighbouring lanes, so the MMA columns are (chunk pair, activation row) instead of (chunk,
-// row) and one column set serves four activation rows.  Used for M = 3, 4 at group 64; the sums
-// of a group's two chunks then meet inside the tensor core instead of after the scale, so a row
-// agrees with its M <= 2 value to fp32 rounding, not bit for bit.
-#ifdef MIORI_TMA_TRACE
-// Profiling build only: %globaltimer marks of the first and the last CTA of the first 256 launches.
-__device__ unsigned long long g_tma_marks[256 * 2 * 8];
-__device__ unsigned int g_tma_launch[4];
-__device__ unsigned long long g_tma_pmarks[256 * 2 * 4];  // the producer thread's marks
-__device__ __forceinline__ unsigned long long gtimer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-#define TMA_MARK(i)                                                                              \
-    do {                                                                                         \
-        if (trace_slot < 256u) g_tma_marks[(trace_slot * 2 + trace_which) * 8 + (i)] = gtimer(); \
-    } while (0)
-#else
-#define TMA_MARK(i) do { } while (0)
-#endif
 
 // What the post-norm epilogue needs besides the GEMV's own arguments (null residual: off).
 struct PostNorm {
@@ -360,693 +401,589 @@ struct PreNorm {
     float eps = 0.0f;
 };
 
-// ARGMAX (with SHARDED, one activation row): the head of a greedy decode step.  The rows go to this
-// rank's y only -- no packets -- and every thread tracks the best (value, index) of what it stores;
-// the candidates meet in a 64-bit atomic maximum, and the CTA that finishes last exchanges this
-// rank's best with the peers (peers.cuh: peer_argmax_exchange), so the kernel ends with the winning
-// token on every rank and nothing else has crossed NVLink.
-template <int BITS, bool EXACT, int NT, bool OUT_BF16, bool SHARDED, bool ROOMY, bool PAIR, bool ARGMAX = false,
-          bool GATED = false, bool POSTNORM = false, bool NORMED = false>
-__global__ void __launch_bounds__(THREADS, (NT == 1 && !ROOMY) ? 2 : 1)
-gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q,
-                const __grid_constant__ CUtensorMap tmap_s,
-                const __grid_constant__ CUtensorMap tmap_b, const uint8_t* __restrict__ qlin,
-                const uint16_t* __restrict__ slin, const uint16_t* __restrict__ blin,
-                const uint16_t* __restrict__ x, void* __restrict__ y, uint32_t N, uint32_t K,
-                uint32_t M, uint32_t gshift, uint32_t ngrp, uint32_t nsg, uint32_t kpar,
-                const PeerArgs pa, uint32_t n_total, uint32_t row0, size_t y_off,
-                unsigned long long* __restrict__ best, const PostNorm pn, const PreNorm pre) {
-    static_assert(!ARGMAX || SHARDED, "the arg-max epilogue lives in the sharded instantiation");
-    // POSTNORM: y = residual + v * rsqrt(mean(v^2) + eps) * gamma over each whole output row v of
-    // the GEMV (shaders/ops.metal:605-631).  Every CTA stores its part of v into y; the CTA that
-    // arrives last then runs the stand-alone kernel's row pass over y in place.
-    static_assert(!POSTNORM || (!OUT_BF16 && !SHARDED && !GATED), "the post-norm epilogue: fp32 out, one GPU");
-    // NORMED: x points at fp32 activations; the staging pass stages bf16(x * rsqrt(mean(x^2) + eps) *
-    // gamma) (shaders/ops.metal:86-115), each CTA computing the rows' sums of squares for itself.
-    static_assert(!NORMED || (BITS == 4 && EXACT && !SHARDED && !POSTNORM), "the norm prologue: 4-bit, up to four rows, one GPU");
-    // GATED: the weight rows are a gate half [0, N/2) and an up half [N/2, N) (the fused w1/w3
-    // projection); a tile is eight rows of each, so that after the tile's reduction one thread
-    // pair holds gate and up of the same output, and y is bf16 [M][N/2] of silu(gate) * up.
-    static_assert(!GATED || (BITS == 4 && OUT_BF16 && !SHARDED), "the gated epilogue: 4-bit, bf16 out, one GPU");
-    using namespace gemvmma;
-    const uint32_t nstage = ngrp * nsg;  // every active group owns a private ring of nsg stages
-    constexpr int CW = 128 / BITS;          // codes per 16-byte chunk
-    constexpr int SK = 4 * CW;              // k per step
-    constexpr int KC = 16 * SK;             // k per slab: 16 steps, 4 per warp of a group
-    static_assert(!PAIR || (EXACT && NT == 1 && BITS == 4), "PAIR is an EXACT 4-bit single-set mode");
-    constexpr int MP = EXACT ? (PAIR ? 4 : 2 * NT) : 8 * NT;
-    constexpr float OFF = BITS == 4 ? 128.0f : 1024.0f;  // what the unpack adds to every code
-    constexpr uint32_t MASK = 0x000F000Fu, MAGIC = 0x43004300u;  // bf16 128.0 in both halves
+// What is fused around the product.
+//   SHARDED: rows [row0, row0 + N) of an n_total-row output, exchanged with the peer GPUs
+//   ARGMAX:  the head of a greedy decode step (one activation row).  The rows go to this rank's y only --
+//            no packets -- and every thread tracks the best (value, index) of what it stores; the
+//            candidates meet in a 64-bit atomic maximum, and the CTA that finishes last exchanges this
+//            rank's best with the peers (peers.cuh: peer_argmax_exchange), so the kernel ends with the
+//            winning token on every rank and nothing else has crossed NVLink
+//   GATED:   the weight rows are a gate half [0, N/2) and an up half [N/2, N) (the fused w1/w3
+//            projection); a tile is eight rows of each, so that after the tile's reduction one thread
+//            pair holds gate and up of the same output, and y is bf16 [M][N/2] of silu(gate) * up
+//   POSTNORM: y = residual + v * rsqrt(mean(v^2) + eps) * gamma over each whole output row v of the GEMV
+//            (shaders/ops.metal:605-631).  Every CTA stores its part of v into y; the CTA that arrives
+//            last then runs the stand-alone kernel's row pass over y in place
+//   NORMED:  x is fp32; bf16(x * rsqrt(mean(x^2) + eps) * gamma) is what is multiplied
+enum Fuse { NONE, SHARDED, ARGMAX, GATED, POSTNORM, NORMED, NORMED_GATED };
+
+struct Args {
+    const uint16_t *s, *b;  // scales and biases, [N][K / GROUP]
+    const uint16_t* x;      // activations, bf16 [M][K] (fp32 when NORMED)
+    void* y;
+    uint32_t N, K, M;
+    uint32_t ngrp, nsg;     // active groups of four warps; code stages per group
+    uint32_t nsb;           // scale buffers of every set of groups that share a tile
+    uint32_t kpar;          // groups that share a tile (1, 2 or 4), each taking every kpar-th slab
+    uint32_t slab_row;      // bytes of a row in a slab: SLAB_ROW, or a shorter whole row rounded up to 128
+    uint32_t inv_upr;       // ceil(2^32 / (K / 8))
+    uint32_t out_bf16;
+    uint32_t n_total, row0; // the whole output's rows and this launch's first one
+    size_t y_off;
+    unsigned long long* best;
+    PeerArgs pa;
+    PostNorm post;
+    PreNorm pre;
+};
+
+// The dynamic shared memory, identical on host and device (bytes from a 128-byte aligned base).
+struct Layout {
+    uint32_t qpitch, stage_bytes, sb_half, x_pitch;
+    uint32_t sb, x, ms, zeros, red, total;
+};
+template <class S>
+__host__ __device__ inline Layout layout(uint32_t K, uint32_t M, uint32_t stages, uint32_t sb_bufs, uint32_t slab_row) {
+    Layout L;
+    L.qpitch = slab_row + S::QPAD;
+    L.stage_bytes = 16u * L.qpitch;
+    L.sb_half = 32u * (K / S::GROUP);  // 16 rows of scales (or of biases)
+    const uint32_t kpad = (K + S::SK - 1u) / S::SK * S::SK;
+    L.x_pitch = (2u * kpad + 127u) / 128u * 128u + S::XPAD;
+    uint32_t at = stages * L.stage_bytes;
+    L.sb = at;
+    at += sb_bufs * 2u * L.sb_half;
+    at = (at + 127u) / 128u * 128u;
+    L.x = at;
+    at += M * L.x_pitch;
+    L.ms = at;
+    at += (kpad / S::GROUP + 8u) * S::ROWS * 8u;  // (a last pass may read, not use, a few groups more)
+    at = (at + 15u) / 16u * 16u;
+    L.zeros = at;
+    at += ZERO_BYTES;
+    L.red = at;  // 16-byte aligned
+    at += GROUPS * Red<S::ROWS>::BUFS * Red<S::ROWS>::FLOATS * 4u;
+    L.total = at;
+    return L;
+}
+
+template <class S, Fuse F>
+__global__ void __launch_bounds__(THREADS, 1)
+gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ Args A) {
+    constexpr bool GATED_ = F == GATED || F == NORMED_GATED, NORMED_ = F == NORMED || F == NORMED_GATED;
+    constexpr bool SHARDED_ = F == SHARDED, ARGMAX_ = F == ARGMAX, POSTNORM_ = F == POSTNORM;
+    constexpr int BITS = S::BITS, NT = S::NT, ROWS = S::ROWS, GPS = S::GPS, RC = S::RC;
+    const uint32_t N = A.N, K = A.K, M = A.M, kpar = A.kpar, nsg = A.nsg, ngrp = A.ngrp;
 
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t g = lane >> 2, t = lane & 3u;
-    const uint32_t grp = warp >> 2, wg = warp & 3u;
+    const uint32_t grp = warp < WARPS ? warp >> 2 : warp - WARPS;  // group of four warps, or its producer
     const uint32_t tiles = (N + 15u) >> 4;
-    const uint32_t kslabs = (K + KC - 1) / KC;
-    const uint32_t steps_p = kslabs * 16u;                 // padded steps along K
-    const uint32_t pitch = steps_p * STEP_UNITS + 1u;      // staged x row pitch (units, odd)
-    const uint32_t cpr = steps_p * 4u;                     // chunks per padded row
-    const uint32_t gps = KC >> gshift;                     // groups per slab row
-    // Linear mode (K fits one slab): the 16 rows of a tile are contiguous in memory, so a slab
-    // is three plain bulk copies and rows keep their global pitch in shared memory.  Otherwise
-    // rows are gathered by 2-D tiled TMA at a fixed 1 KiB / gps pitch.
-    const bool linear = qlin != nullptr;
-    const uint32_t chunks = K / CW, ng = K >> gshift;
-    const bool ktail = linear && chunks < 64u;  // K shorter than one slab of 64 chunks
-    const uint32_t qpitch = linear ? K * BITS / 8 : (uint32_t)ROW_BYTES;
-    const uint32_t spitch = linear ? ng : gps;
+    const uint32_t row_bytes = K * BITS / 8u, ng = K / S::GROUP;
+    const uint32_t kslabs = (row_bytes + SLAB_ROW - 1u) / SLAB_ROW;
 
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t full_bars[MAX_STAGES];
-    __shared__ __align__(8) uint64_t empty_bars[MAX_STAGES];
+    __shared__ __align__(8) uint64_t full_bars[GROUPS * MAX_NSG], empty_bars[GROUPS * MAX_NSG];
+    __shared__ __align__(8) uint64_t sb_full[GROUPS * MAX_NSG], sb_empty[GROUPS * MAX_NSG];
     __shared__ volatile uint32_t abort_flag;
-    __shared__ uint32_t x_maxbits[4];  // 8-bit codes: largest |x| bit pattern of each staged row
-    __shared__ float x_mul[4];         // 8-bit codes: per-row power-of-two scale of the fp16 staging
-    __shared__ float x_rescale[4];     // ... and its inverse, applied at the store
-    uint8_t* ring = smem_raw;                                            // [nstage][STAGE_BYTES]
-    uint4* xs = reinterpret_cast<uint4*>(ring + (size_t)nstage * STAGE_BYTES);  // [MP][pitch]
-    uint4* zeros = xs + (size_t)MP * pitch;                              // ZERO_BYTES of zeros
-    float* xsum = reinterpret_cast<float*>(zeros + ZERO_BYTES / 16);     // [MP][cpr] (EXACT)
-    float* red = xsum + (EXACT ? (size_t)MP * cpr : 0);                  // [GROUPS] group areas
-    float* kred = red + (size_t)GROUPS * Red<MP>::GROUP_FLOATS;          // [2][GROUPS][16*MP]
 
     pdl_launch_dependents();
-#ifdef MIORI_TMA_TRACE
-    const unsigned int trace_which = blockIdx.x == 0 ? 0u : 1u;
-    unsigned int trace_slot = 0xffffffffu;
-    if (threadIdx.x == 0 && (blockIdx.x == 0 || blockIdx.x == gridDim.x - 1))
-        trace_slot = atomicAdd(&g_tma_launch[trace_which], 1u);
-    TMA_MARK(0);
-#endif
 
-    // This CTA's tiles.  Slabs are enumerated in sets of ngrp tiles (one
-    // per active group), k-slab major inside a set, so that consecutive slabs belong to
-    // different groups.  Group gi's k-th slab lives in stage gi*nsg + k % nsg: a stage is only
-    // ever waited on by one group, in order, so barrier parities are never ambiguous.
-    // tiles are dealt round-robin (tile = blockIdx.x + j*gridDim.x): at any moment the CTAs
-    // stream one contiguous window of the weight matrix, which HBM serves best
-    // When a CTA has fewer tiles than groups and K spans several slabs, kpar groups share a
-    // tile: each takes every kpar-th k-slab (a "virtual tile") and their partial outputs are
-    // summed in a fixed order at the end.  kslabs is a multiple of kpar.
-    const uint32_t kshift = kpar >> 1;  // kpar is 1, 2 or 4: log2 without a division
-    const uint32_t ntiles = ((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x) << kshift;  // virtual
-    const uint32_t kslabs_v = kslabs >> kshift;
-    const uint32_t total = ntiles * kslabs_v;
-        const uint32_t stage_tx = Q_BYTES + 2u * 16u * gps * 2u;  // bytes tiled TMA delivers per slab
+    // This CTA's tiles are dealt round-robin (tile = blockIdx.x + j * gridDim.x): at any moment the
+    // CTAs stream one contiguous window of the weight matrix, which HBM serves best.  Group gi takes the
+    // virtual tiles gi, gi + ngrp, ...  When a CTA has fewer tiles than groups and K spans several slabs,
+    // kpar neighbouring groups share a tile: virtual tile v is tile v / kpar and slabs v % kpar,
+    // v % kpar + kpar, ... of it, and the partial outputs are summed in a fixed order at the end (kslabs
+    // and ngrp are multiples of kpar).  The group's k-th slab lives in its stage k % nsg; the scales of
+    // its i-th tile in buffer i % nsb of the first of the groups that share it.
+    const uint32_t kshift = kpar >> 1;  // log2
+    const uint32_t my_tiles = (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x;
+    const uint32_t vtiles = my_tiles << kshift, kp = grp & (kpar - 1u);
+    const Layout L = layout<S>(K, M, ngrp * nsg, (ngrp >> kshift) * A.nsb, A.slab_row);
+    const uint32_t base = smem_addr(smem_raw), qpitch = L.qpitch;
+    const uint32_t bar0 = grp * nsg, sb0 = (grp >> kshift) * A.nsb;  // this group's first barriers
 
-    // producer side (lane 0 of the producer warp only)
-    uint32_t issued = 0;
-    // Producer cursor, advanced incrementally (no divisions on the issue path): the next slab
-    // to issue is k-slab p_ks of the p_gi-th tile of the set starting at tile index p_set0;
-    // p_kmod = k % nsg and p_use = k / nsg for the owning group's slab counter k.
-    uint32_t p_set0 = 0, p_ks = 0, p_gi = 0, p_kmod = 0, p_use = 0;
-    // issue every slab whose stage is free, without blocking
-    auto try_refill = [&](uint32_t upto) {
-        while (issued < upto) {
-            const uint32_t stage = p_gi * nsg + p_kmod;
-            if (p_use != 0u) {
-                if (!mbar_try(smem_addr(&empty_bars[stage]), (p_use - 1u) & 1u)) break;
+    if (warp >= WARPS) {
+        // ---- producer of group `grp`: one lane.  Nothing here depends on the predecessor kernel.
+        if (lane == 0) {
+            abort_flag = 0u;  // by every producer: each reads it without having met the others
+            if (grp < ngrp) {
+                for (uint32_t i = 0; i < nsg; ++i) {
+                    mbar_init(smem_addr(&full_bars[bar0 + i]), 1);
+                    mbar_init(smem_addr(&empty_bars[bar0 + i]), 4);
+                }
+                if (kp == 0u)
+                    for (uint32_t i = 0; i < A.nsb; ++i) {
+                        mbar_init(smem_addr(&sb_full[sb0 + i]), 1);
+                        mbar_init(smem_addr(&sb_empty[sb0 + i]), 4u * kpar);
+                    }
+            }
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncwarp();
+        asm volatile("bar.arrive 14, %0;" ::"n"(THREADS) : "memory");
+        if (lane == 0 && grp < ngrp) {
+            // next buffers, and the parities of their previous releases
+            uint32_t st = 0, st_par = 1u, sb = 0, sb_par = 1u;
+            bool st_wait = false, sb_wait = false, ok = true;
+            // a buffer has to come back: the consumers start after the predecessor, and so does the time limit
+            auto reuse = [&](uint64_t* empty, uint32_t parity, uint32_t where) {
+                pdl_wait_prior();
+                ok = mbar_wait(smem_addr(empty), parity, &abort_flag, where);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            }
-            const uint32_t bar = smem_addr(&full_bars[stage]);
-            const uint32_t dst = smem_addr(ring + (size_t)stage * STAGE_BYTES);
-            const uint32_t vt = p_set0 + p_gi;
-            const uint32_t row = (blockIdx.x + (vt >> kshift) * gridDim.x) * 16u;
-            const uint32_t ks = (vt & (kpar - 1u)) + (p_ks << kshift);
-            if (GATED && linear) {  // N is a multiple of 16: eight whole rows of each half
-                const uint32_t r8 = row >> 1, up8 = (N >> 1) + r8;
-                mbar_expect_tx(bar, 16u * (qpitch + 4u * spitch));
-                bulk_g2s(dst, qlin + (size_t)r8 * qpitch, 8u * qpitch, bar);
-                bulk_g2s(dst + 8u * qpitch, qlin + (size_t)up8 * qpitch, 8u * qpitch, bar);
-                bulk_g2s(dst + Q_BYTES, slin + (size_t)r8 * spitch, 16u * spitch, bar);
-                bulk_g2s(dst + Q_BYTES + 16u * spitch, slin + (size_t)up8 * spitch, 16u * spitch, bar);
-                bulk_g2s(dst + Q_BYTES + SB_BYTES, blin + (size_t)r8 * spitch, 16u * spitch, bar);
-                bulk_g2s(dst + Q_BYTES + SB_BYTES + 16u * spitch, blin + (size_t)up8 * spitch, 16u * spitch, bar);
-            } else if (GATED) {  // the tensor maps' boxes are eight rows high
-                const int r8 = (int)(row >> 1), up8 = (int)((N >> 1) + (row >> 1));
-                mbar_expect_tx(bar, stage_tx);
-                tma_load_2d(dst, &tmap_q, (int)(ks * (ROW_BYTES / 4)), r8, bar);
-                tma_load_2d(dst + 8u * ROW_BYTES, &tmap_q, (int)(ks * (ROW_BYTES / 4)), up8, bar);
-                tma_load_2d(dst + Q_BYTES, &tmap_s, (int)(ks * gps), r8, bar);
-                tma_load_2d(dst + Q_BYTES + 16u * gps, &tmap_s, (int)(ks * gps), up8, bar);
-                tma_load_2d(dst + Q_BYTES + SB_BYTES, &tmap_b, (int)(ks * gps), r8, bar);
-                tma_load_2d(dst + Q_BYTES + SB_BYTES + 16u * gps, &tmap_b, (int)(ks * gps), up8, bar);
-            } else if (linear) {
-                const uint32_t nrows = min(16u, N - row);  // rows past N keep stale (unused) data
-                mbar_expect_tx(bar, nrows * (qpitch + 4u * spitch));
-                bulk_g2s(dst, qlin + (size_t)row * qpitch, nrows * qpitch, bar);
-                bulk_g2s(dst + Q_BYTES, slin + (size_t)row * spitch, nrows * spitch * 2u, bar);
-                bulk_g2s(dst + Q_BYTES + SB_BYTES, blin + (size_t)row * spitch, nrows * spitch * 2u, bar);
-            } else {
-                mbar_expect_tx(bar, stage_tx);
-                tma_load_2d(dst, &tmap_q, (int)(ks * (ROW_BYTES / 4)), (int)row, bar);
-                tma_load_2d(dst + Q_BYTES, &tmap_s, (int)(ks * gps), (int)row, bar);
-                tma_load_2d(dst + Q_BYTES + SB_BYTES, &tmap_b, (int)(ks * gps), (int)row, bar);
-            }
-            ++issued;
-            // advance the cursor: next group of the set, then next k-slab, then next set
-            const uint32_t nt = min(ngrp, ntiles - p_set0);
-            if (++p_gi == nt) {
-                p_gi = 0;
-                if (++p_kmod == nsg) { p_kmod = 0; ++p_use; }
-                if (++p_ks == kslabs_v) { p_ks = 0; p_set0 += ngrp; }
-            }
-        }
-    };
-
-    const bool producer = threadIdx.x == WARPS * 32;
-    if (producer) {
-#ifdef MIORI_TMA_TRACE
-        unsigned int pslot = 0xffffffffu;
-        if (blockIdx.x == 0 || blockIdx.x == gridDim.x - 1) pslot = atomicAdd(&g_tma_launch[2 + trace_which], 1u);
-#define TMA_PMARK(i) do { if (pslot < 256u) g_tma_pmarks[(pslot * 2 + trace_which) * 4 + (i)] = gtimer(); } while (0)
-        TMA_PMARK(0);
-#else
-#define TMA_PMARK(i) do { } while (0)
-#endif
-        abort_flag = 0u;
-        x_maxbits[0] = x_maxbits[1] = x_maxbits[2] = x_maxbits[3] = 0u;
-        for (uint32_t i = 0; i < nstage; ++i) {
-            mbar_init(smem_addr(&full_bars[i]), 1);
-            mbar_init(smem_addr(&empty_bars[i]), 4);
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        TMA_PMARK(1);
-        try_refill(total);  // fills the rings: up to nstage slabs in flight before the wait
-        TMA_PMARK(2);
-#ifdef MIORI_TMA_TRACE
-        for (int spin = 0; spin < 100000 && !mbar_try(smem_addr(&full_bars[0]), 0u); ++spin) { }
-        TMA_PMARK(3);
-#endif
-    }
-
-    pdl_wait_prior();  // x (and y) belong to the predecessor until here
-    TMA_MARK(1);
-
-    // N-sharded launch (pa.world > 1): this rank's rows [row0, row0 + N) of an n_total-row output
-    // go into its own y (at user offset y_off of its arena) and, as {value, launch number}
-    // packets, into every peer's inbox; before the CTA exits it collects its share of the peers'
-    // rows (peers.cuh).  The launch number is re-read from the control block at the point of
-    // use, so the single-GPU path carries no extra registers through the loop; SHARDED is a
-    // template parameter rather than a run-time test because the single-GPU instantiation then
-    // compiles exactly as if the peer path did not exist (a run-time branch cost 3-16 %).
-    const uint32_t world = SHARDED ? pa.world : 0u;
-    unsigned long long my_best = 0ull;  // ARGMAX: key of the best element this thread has stored
-    // one output element: y[m][row0 + row]
-    auto store_out = [&](uint32_t m, uint32_t row, float v) {
-        if (BITS == 8) v *= x_rescale[m];
-        const size_t idx = (size_t)m * n_total + row0 + row;
-        const uint32_t bits = OUT_BF16 ? float_to_bf16_bits(v) : __float_as_uint(v);
-        if (OUT_BF16) reinterpret_cast<uint16_t*>(y)[idx] = (uint16_t)bits;
-        else reinterpret_cast<uint32_t*>(y)[idx] = bits;
-        if constexpr (ARGMAX) {  // compare what was stored (the rounded value when the output is bf16)
-            if (v == v) {
-                const unsigned long long key = peer_best_key(OUT_BF16 ? bits << 16 : bits, row0 + row);
-                my_best = key > my_best ? key : my_best;
-            }
-        } else if constexpr (SHARDED) {
-            if (world > 1u) {
-                const uint32_t e = peer_epoch(pa);
-                const size_t elem = y_off / (OUT_BF16 ? 2u : 4u) + idx;
-                for (uint32_t p = 0; p < world; ++p)
-                    if (p != pa.rank) peer_send(peer_slot(pa, peer_arena(pa, p), e, elem), bits, e);
-            }
-        }
-    };
-
-    // GATED: y[m][row] = bf16(silu(gate) * up) of the N/2-column output, with the arithmetic of the
-    // stand-alone activation kernel (shaders/ops.metal:129-139)
-    auto store_gated = [&](uint32_t m, uint32_t row, float gate, float up) {
-        const float sg = gate / (1.0f + expf(-gate));
-        reinterpret_cast<uint16_t*>(y)[(size_t)m * (N >> 1) + row] = (uint16_t)float_to_bf16_bits(sg * up);
-    };
-    (void)store_gated;
-
-    // one-pass staging where it measured faster: one slab of K, and either the roomy
-    // instantiation or at most two staged rows
-    if constexpr (BITS == 8) {
-        // per-row power-of-two scale for the fp16 staging: the row's largest |x| lands in
-        // [2^14, 2^15); the outputs are multiplied back at the store.  Per row, so that a row's
-        // result does not depend on its neighbours in the batch.
-        static_assert(MP <= 4, "8-bit rows staged per launch");
-        __syncthreads();  // x_maxbits was cleared before the wait
-        const uint32_t upr8 = K / 8u;  // 16-byte pieces per row
-        const uint4* x4 = reinterpret_cast<const uint4*>(x);
-        for (uint32_t m = 0; m < M; ++m) {
-            uint32_t mx = 0;
-            for (uint32_t i = threadIdx.x; i < upr8; i += THREADS) {
-                const uint4 v = __ldg(x4 + (size_t)m * upr8 + i);
-                const uint32_t a = v.x & 0x7FFF7FFFu, b = v.y & 0x7FFF7FFFu, c = v.z & 0x7FFF7FFFu,
-                               d = v.w & 0x7FFF7FFFu;
-                mx = max(max(max(mx, a & 0xFFFFu), max(a >> 16, b & 0xFFFFu)),
-                         max(max(b >> 16, c & 0xFFFFu), max(max(c >> 16, d & 0xFFFFu), d >> 16)));
-            }
-            mx = __reduce_max_sync(0xFFFFFFFFu, mx);
-            if (lane == 0 && mx) atomicMax(&x_maxbits[m], mx);
-        }
-        __syncthreads();
-        if (threadIdx.x < 4u) {
-            const uint32_t top = x_maxbits[threadIdx.x];
-            int sh = top ? (int)((top >> 7) & 0xFFu) - 141 : 0;  // bf16 exponent field - 127 - 14
-            sh = max(-100, min(110, sh));
-            x_mul[threadIdx.x] = __uint_as_float((uint32_t)(127 - sh) << 23);
-            x_rescale[threadIdx.x] = __uint_as_float((uint32_t)(127 + sh) << 23);
-        }
-        __syncthreads();
-    }
-    __shared__ float nm_part[NORMED ? 4 * (WARPS + 1) : 1];
-    __shared__ float nm_inv[4];
-    if constexpr (NORMED) {
-        if (K <= 2048u)
-            stage_x_normed<EXACT, MP, PAIR>(reinterpret_cast<const float*>(x), pre.gamma, pre.eps, xs, xsum, M, K,
-                                            pitch, cpr, nm_part);
-    }
-    if (NORMED && K > 2048u) {
-        // longer rows: sums of squares of the (at most four) rows first -- all loads in flight together,
-        // warps reduce by shuffles, one thread per row adds the warp sums in order -- then the plain
-        // staging passes with a loader that normalises
-        static_assert(!NORMED || MP <= 4, "rows of the norm prologue");
-        const float4* x4 = reinterpret_cast<const float4*>(x);
-        const uint32_t qpr = K >> 2;  // float4 pieces per row (K is a multiple of 32)
-        float ss[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        for (uint32_t i = threadIdx.x; i < qpr; i += THREADS) {
-#pragma unroll
-            for (uint32_t m = 0; m < 4u; ++m) {
-                if (m < M) {
-                    const float4 v = __ldg(x4 + (size_t)m * qpr + i);
-                    ss[m] = __fmaf_rn(v.w, v.w, __fmaf_rn(v.z, v.z, __fmaf_rn(v.y, v.y, __fmaf_rn(v.x, v.x, ss[m]))));
-                }
-            }
-        }
-#pragma unroll
-        for (uint32_t m = 0; m < 4u; ++m) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ss[m] += __shfl_xor_sync(0xFFFFFFFFu, ss[m], o);
-            if (lane == 0) nm_part[m * (WARPS + 1) + warp] = ss[m];
-        }
-        __syncthreads();
-        if (threadIdx.x < 4u) {
-            float tot = 0.0f;
-            for (uint32_t w = 0; w <= (uint32_t)WARPS; ++w) tot += nm_part[threadIdx.x * (WARPS + 1) + w];
-            nm_inv[threadIdx.x] = rsqrtf(tot / (float)K + pre.eps);
-        }
-        __syncthreads();
-    }
-    // the eight bf16 activations 8u .. 8u+7 of row m
-    auto ld8 = [&](uint32_t m, uint32_t u) -> uint4 {
-        if constexpr (NORMED) {
-            const float4* xr = reinterpret_cast<const float4*>(x) + (size_t)m * (K >> 2) + 2u * u;
-            const float4 a = __ldg(xr), c = __ldg(xr + 1);
-            const uint4 gm = __ldg(reinterpret_cast<const uint4*>(pre.gamma) + u);
-            const float inv = nm_inv[m];
-            // the stand-alone norm kernel's arithmetic: x * inv * gamma, rounded to bf16
-            auto two = [&](float lo, float hi, uint32_t g2) {
-                return float_to_bf16_bits(lo * inv * bf16lo(g2)) | (float_to_bf16_bits(hi * inv * bf16hi(g2)) << 16);
+                return ok;
             };
-            return make_uint4(two(a.x, a.y, gm.x), two(a.z, a.w, gm.y), two(c.x, c.y, gm.z), two(c.z, c.w, gm.w));
+            uint32_t row = (blockIdx.x + (grp >> kshift) * gridDim.x) * 16u;
+            const uint32_t row_step = (ngrp >> kshift) * gridDim.x * 16u;
+            for (uint32_t vt = grp; vt < vtiles && ok; vt += ngrp, row += row_step) {
+                // The tile's scales and biases come with its first slab, on the slab's barrier (their buffer is
+                // free when that slab's stage is: plan_launch).  Groups that share a tile share one copy, made
+                // by the first of them, with barriers of its own.
+                const bool shared = kpar > 1u;
+                uint32_t sb_bar = smem_addr(&full_bars[bar0 + st]), extra = 2u * L.sb_half;
+                const uint32_t sdst = base + L.sb + (sb0 + sb) * 2u * L.sb_half;
+                const uint32_t r0 = GATED_ ? row >> 1 : row;  // GATED: N is a multiple of 16, eight whole rows of each half
+                const uint8_t* src_s = reinterpret_cast<const uint8_t*>(A.s) + (size_t)r0 * (2u * ng);
+                const uint8_t* src_b = reinterpret_cast<const uint8_t*>(A.b) + (size_t)r0 * (2u * ng);
+                if (row + 16u > N && kp == 0u) {  // a ragged last tile: whole 16-byte pieces by bulk copy ...
+                    if (!shared && st_wait && !reuse(&empty_bars[bar0 + st], st_par, 0x16)) break;
+                    if (shared && sb_wait && !reuse(&sb_empty[sb0 + sb], sb_par, 0x15)) break;
+                    const uint32_t n = (N - row) * ng;
+                    extra = (2u * n & ~15u) * 2u;
+                    for (uint32_t i = n & ~7u; i < n; ++i) {  // ... the rest by this thread, before it arrives
+                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(sdst + 2u * i), "h"(reinterpret_cast<const uint16_t*>(src_s)[i]) : "memory");
+                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(sdst + L.sb_half + 2u * i), "h"(reinterpret_cast<const uint16_t*>(src_b)[i]) : "memory");
+                    }
+                }
+                auto copy_sb = [&] {
+                    if (GATED_) {
+                        const uint32_t half = L.sb_half >> 1;
+                        const size_t up = (size_t)(N >> 1) * (2u * ng);
+                        bulk_g2s(sdst, src_s, half, sb_bar);
+                        bulk_g2s(sdst + half, src_s + up, half, sb_bar);
+                        bulk_g2s(sdst + L.sb_half, src_b, half, sb_bar);
+                        bulk_g2s(sdst + L.sb_half + half, src_b + up, half, sb_bar);
+                    } else if (extra) {
+                        bulk_g2s(sdst, src_s, extra >> 1, sb_bar);
+                        bulk_g2s(sdst + L.sb_half, src_b, extra >> 1, sb_bar);
+                    }
+                };
+                if (shared && kp == 0u) {
+                    sb_bar = smem_addr(&sb_full[sb0 + sb]);
+                    if (sb_wait && !reuse(&sb_empty[sb0 + sb], sb_par, 0x15)) break;
+                    mbar_expect_tx(sb_bar, extra);
+                    copy_sb();
+                }
+                for (uint32_t ks = kp; ks < kslabs; ks += kpar) {
+                    const uint32_t bar = smem_addr(&full_bars[bar0 + st]), dst = base + (bar0 + st) * L.stage_bytes;
+                    if (st_wait && !reuse(&empty_bars[bar0 + st], st_par, 0x14)) break;
+                    const int c0 = (int)(ks * (SLAB_ROW / 8u));
+                    const bool with_sb = !shared && ks == 0u;
+                    mbar_expect_tx(bar, L.stage_bytes + (with_sb ? extra : 0u));
+                    if (GATED_) {  // the tensor map's boxes are eight rows high
+                        tma_load_2d(dst, &tmap_q, c0, (int)r0, bar);
+                        tma_load_2d(dst + 8u * qpitch, &tmap_q, c0, (int)((N >> 1) + r0), bar);
+                    } else {
+                        tma_load_2d(dst, &tmap_q, c0, (int)row, bar);
+                    }
+                    if (with_sb) copy_sb();
+                    if (++st == nsg) st = 0u, st_wait = true, st_par ^= 1u;
+                }
+                if (++sb == A.nsb) sb = 0u, sb_wait = true, sb_par ^= 1u;
+            }
+        }
+        __syncwarp();
+    }
+
+    // y is one launch's output; ARGMAX: key of the best element this thread has stored
+    unsigned long long my_best = 0ull;
+    const uint32_t world = SHARDED_ ? A.pa.world : 0u;
+    if (warp < WARPS) {
+        // zeros: what lanes of other slots read, and the activations past the end of K
+        const XArea xa = {base + L.x, L.x_pitch, base + L.ms};
+        const uint32_t tid = threadIdx.x;
+        if (tid < ZERO_BYTES / 16u) *reinterpret_cast<uint4*>(smem_raw + L.zeros + 16u * tid) = make_uint4(0u, 0u, 0u, 0u);
+        if (const uint32_t tail = (K + S::SK - 1u) / S::SK * S::SK - K) {
+            for (uint32_t i = tid; i < M * (tail >> 3); i += COMPUTE) {
+                const uint32_t m = i / (tail >> 3), u = i - m * (tail >> 3);
+                *reinterpret_cast<uint4*>(smem_raw + L.x + m * L.x_pitch + 2u * K + 16u * u) = make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+
+        pdl_wait_prior();  // x (and y) belong to the predecessor until here
+
+        if constexpr (NORMED_) {
+            __shared__ float nm_part[4][WARPS];
+            __shared__ float nm_inv[32];
+            stage_x_normed<S>(xa, reinterpret_cast<const float*>(A.x), A.pre.gamma, A.pre.eps, M, K, A.inv_upr, nm_part, nm_inv);
         } else {
-            return __ldg(reinterpret_cast<const uint4*>(x + (size_t)m * K) + u);
+            stage_x<S>(xa, A.x, M, K, A.inv_upr);
         }
-    };
-    bool staged = false;
-    if constexpr (NORMED) staged = K <= 2048u;  // staged above, norm included
-    if constexpr (BITS == 4) {
-        if (staged) {
-        } else if constexpr (MP <= 4) {
-            if (ROOMY || MP <= 2) {
-                stage_x_onepass<BITS, EXACT, MP, PAIR>(xs, xsum, M, K, steps_p, pitch, cpr, ld8);
-                staged = true;
-            }
-        } else if ((ROOMY || MP <= 2) && kslabs == 1u) {
-            stage_x_onepass_wide<BITS, EXACT, MP, PAIR>(xs, xsum, M, K, steps_p, pitch, cpr, ld8);
-            staged = true;
-        }
-    }
-    if (!staged) stage_x_padded<BITS, EXACT, MP, PAIR>(x, xs, xsum, M, K, steps_p, pitch, cpr, x_mul, ld8);
-    for (uint32_t i = threadIdx.x; i < ZERO_BYTES / 16; i += THREADS)
-        zeros[i] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-    TMA_MARK(2);
+        asm volatile("bar.sync 14, %0;" ::"n"(THREADS) : "memory");  // x is staged, the barriers exist
 
-    // per-lane constants, all as 32-bit shared addresses / byte offsets
-    const uint32_t n = lane >> 2;
-    const uint32_t lc0 = wg * 4u + t;                               // first chunk of this lane in a slab
-    const uint32_t ring_a = smem_addr(ring);
-    const uint32_t q_lane = g * qpitch + lc0 * 16u;                 // + i4*256 per step, + 8*qpitch for row g+8
-    const uint32_t sb_lane = Q_BYTES + (g * spitch + ((lc0 * CW) >> gshift)) * 2u;
-    const uint32_t sb_step = ((16u * CW) >> gshift) * 2u;           // groups advance per step (bytes)
-    const uint32_t sb_row8 = 8u * spitch * 2u;
-    uint32_t xb[NT];        // B-fragment base of this lane: k-slab 0, step wg
-    uint32_t xadv[NT];      // advance per k-slab (0 for masked lanes, which read zeros)
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-        const uint32_t m = PAIR ? (n & 3u) : EXACT ? (2u * j + (n & 1u)) : (8u * j + n);
-        const bool active = PAIR ? ((n >> 2) == (t >> 1)) : EXACT ? ((n >> 1) == t) : true;
-        xb[j] = active ? smem_addr(xs + (size_t)m * pitch + x_unit(wg, t, 0)) : smem_addr(zeros);
-        xadv[j] = active ? (uint32_t)SLAB_X_BYTES * kpar : 0u;  // groups sharing a tile stride kpar slabs
-    }
-    const uint32_t xs_adv = 256u * kpar;                            // chunk sums per k-slab stride (bytes)
-    const uint32_t xs_row = cpr * 4u;
-    // chunk (ks*16 + i4*4 + wg)*4 + t of row 0 (PAIR: of the lane's first row, 0 or 2)
-    uint32_t xsp = smem_addr(xsum) + lc0 * 4u + (PAIR ? (t & 1u) * 2u * xs_row : 0u);
-    float* gred = red + (size_t)grp * Red<MP>::GROUP_FLOATS;
-
-    float acc[NT][4];
-#pragma unroll
-    for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
-
-    // `ok` turns false for good once a wait expires; the warp then skips waits and math but
-    // still takes part in every group barrier so that no other warp is left waiting.
-    bool ok = true;
-    uint32_t tile_it = 0;
-    uint32_t c_kmod = 0, c_par = 0;  // this group's slab counter k: k % nsg and (k / nsg) & 1
-    if (producer) {
-        // keep the rings fed until every slab has been issued (bounded: gives up with the CTA)
-        const long long t0 = clock64();
-        while (issued < total && !abort_flag) {
-            try_refill(total);
-            if (clock64() - t0 > 4 * WAIT_LIMIT_CYCLES) {
-                abort_flag = 1u;
-                device_error(0x6E14u, blockIdx.x, issued);
-            }
-        }
-    }
-    for (uint32_t set0 = 0; warp < WARPS && set0 < ntiles; set0 += ngrp) {
-        const uint32_t nt = min(ngrp, ntiles - set0);
-        if (grp >= nt) break;
-        const uint32_t vt = set0 + grp;
-        const uint32_t kp = vt & (kpar - 1u);
-        const uint32_t tile = blockIdx.x + (vt >> kshift) * gridDim.x;
-        // start at this group's first k-slab of the row
-        if (kpar > 1u) {
-#pragma unroll
-            for (int j = 0; j < NT; ++j) xb[j] += kp * (xadv[j] >> kshift);
-            xsp += kp * 256u;
-        }
-        for (uint32_t ks = 0; ks < kslabs_v; ++ks) {
-            const uint32_t stage = grp * nsg + c_kmod, parity = c_par;
-            if (++c_kmod == nsg) { c_kmod = 0; c_par ^= 1u; }
-#ifdef MIORI_TMA_TRACE
-            if (tile_it == 0 && ks == 0) TMA_MARK(7);
-#endif
-            if (ok) {
-                ok = mbar_wait(smem_addr(&full_bars[stage]), parity, &abort_flag, 0x10);
-                ok = __all_sync(0xFFFFFFFFu, ok);
-            }
-#ifdef MIORI_TMA_TRACE
-            if (tile_it == 0 && ks == 0) TMA_MARK(4);
-#endif
-            if (ok) {
-                const uint32_t st = ring_a + stage * (uint32_t)STAGE_BYTES;
-                uint32_t qa = st + q_lane, sa = st + sb_lane, lc = lc0;
-                uint32_t xa[NT];
-#pragma unroll
-                for (int j = 0; j < NT; ++j) xa[j] = xb[j];
-                uint32_t xsa = xsp;
-#pragma unroll 1
-                for (uint32_t i4 = 0; i4 < 4u; ++i4) {
-                    const uint4 q0 = lds128(qa);
-                    const uint4 q1 = lds128(qa + 8u * qpitch);
-                    uint32_t s0 = lds16(sa), b0 = lds16(sa + SB_BYTES);
-                    uint32_t s1 = lds16(sa + sb_row8), b1 = lds16(sa + sb_row8 + SB_BYTES);
-                    // past the end of K (linear mode with a short K only; tiled TMA zero-fills):
-                    // a zero scale and bias against zero-staged x contribute exactly 0
-                    if (ktail && lc >= chunks) s0 = b0 = s1 = b1 = 0u;
-                    const uint32_t w0[4] = {q0.x, q0.y, q0.z, q0.w};
-                    const uint32_t w1[4] = {q1.x, q1.y, q1.z, q1.w};
-                    // two independent accumulation chains (even / odd words), each started by
-                    // an MMA with a zero accumulator input
-                    float d0[NT][4], d1[NT][4];
-                    uint32_t s2a = 0, b2a = 0, s2b = 0, b2b = 0;
-                    if (!EXACT) {
-                        s2a = s0 | (s0 << 16); b2a = b0 | (b0 << 16);
-                        s2b = s1 | (s1 << 16); b2b = b1 | (b1 << 16);
-                    }
-                    if constexpr (BITS == 8) {
-                        // bytes (b0,b2) and (b1,b3) of a word become two fp16 pairs 1024 + code:
-                        // two masks and one shift per word, one MMA per word
-                        constexpr uint32_t BMASK = 0x00FF00FFu, HMAGIC = 0x64006400u;
-#pragma unroll
-                        for (int wd = 0; wd < 4; ++wd) {
-                            const uint32_t a0 = lop3_and_or(w0[wd], BMASK, HMAGIC);
-                            const uint32_t a1 = lop3_and_or(w0[wd] >> 8, BMASK, HMAGIC);
-                            const uint32_t c0 = lop3_and_or(w1[wd], BMASK, HMAGIC);
-                            const uint32_t c1 = lop3_and_or(w1[wd] >> 8, BMASK, HMAGIC);
-#pragma unroll
-                            for (int j = 0; j < NT; ++j) {
-                                const uint2 xu = lds64(xa[j] + wd * 16);
-                                if (wd == 0) mma_f16_z(d0[j], a0, c0, a1, c1, xu.x, xu.y);
-                                else if (wd == 1) mma_f16_z(d1[j], a0, c0, a1, c1, xu.x, xu.y);
-                                else if (wd == 2) mma_f16(d0[j], a0, c0, a1, c1, xu.x, xu.y);
-                                else mma_f16(d1[j], a0, c0, a1, c1, xu.x, xu.y);
-                            }
-                        }
-                    } else {
-#pragma unroll
-                    for (int wd = 0; wd < 4; ++wd) {
-                        uint32_t a[4], c[4];  // pairs (n0,n4),(n1,n5),(n2,n6),(n3,n7), rows g, g+8
-#pragma unroll
-                        for (int p = 0; p < 4; ++p) {
-                            a[p] = lop3_and_or(w0[wd] >> (4 * p), MASK, MAGIC);
-                            c[p] = lop3_and_or(w1[wd] >> (4 * p), MASK, MAGIC);
-                            if (!EXACT) {
-                                a[p] = bf16x2_fma(bf16x2_sub(a[p], MAGIC), s2a, b2a);
-                                c[p] = bf16x2_fma(bf16x2_sub(c[p], MAGIC), s2b, b2b);
-                            }
-                        }
-#pragma unroll
-                        for (int j = 0; j < NT; ++j) {
-                            const uint4 xu = lds128(xa[j] + wd * 16);
-                            if (wd == 0) mma_bf16_z(d0[j], a[0], c[0], a[1], c[1], xu.x, xu.y);
-                            else if (wd == 1) mma_bf16_z(d1[j], a[0], c[0], a[1], c[1], xu.x, xu.y);
-                            else if (wd & 1) mma_bf16(d1[j], a[0], c[0], a[1], c[1], xu.x, xu.y);
-                            else mma_bf16(d0[j], a[0], c[0], a[1], c[1], xu.x, xu.y);
-                            if (wd & 1) mma_bf16(d1[j], a[2], c[2], a[3], c[3], xu.z, xu.w);
-                            else mma_bf16(d0[j], a[2], c[2], a[3], c[3], xu.z, xu.w);
-                        }
-                    }
-                    }
-                    if (EXACT) {
-                        const float sc0 = __uint_as_float(s0 << 16);
-                        const float bt0 = __fmaf_rn(-OFF, sc0, __uint_as_float(b0 << 16));
-                        const float sc1 = __uint_as_float(s1 << 16);
-                        const float bt1 = __fmaf_rn(-OFF, sc1, __uint_as_float(b1 << 16));
-#pragma unroll
-                        for (int j = 0; j < NT; ++j) {
-                            const float xs0 = ldsf32(xsa + (2 * j) * xs_row);
-                            acc[j][0] = __fmaf_rn(sc0, d0[j][0] + d1[j][0], __fmaf_rn(bt0, xs0, acc[j][0]));
-                            acc[j][2] = __fmaf_rn(sc1, d0[j][2] + d1[j][2], __fmaf_rn(bt1, xs0, acc[j][2]));
-                            if (PAIR || 2u * j + 1u < M) {  // CTA-uniform: the odd activation row exists
-                                const float xs1 = ldsf32(xsa + (2 * j + 1) * xs_row);
-                                acc[j][1] = __fmaf_rn(sc0, d0[j][1] + d1[j][1], __fmaf_rn(bt0, xs1, acc[j][1]));
-                                acc[j][3] = __fmaf_rn(sc1, d0[j][3] + d1[j][3], __fmaf_rn(bt1, xs1, acc[j][3]));
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < NT; ++j)
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) acc[j][e] += d0[j][e] + d1[j][e];
-                    }
-                    // next step of this warp: 4 steps (16 chunks) further along the row
-                    qa += 256u;
-                    sa += sb_step;
-                    lc += 16u;
-                    xsa += 64u;
-#pragma unroll
-                    for (int j = 0; j < NT; ++j) xa[j] += 4u * STEP_UNITS * 16u;
+        // N-sharded launch (pa.world > 1): this rank's rows [row0, row0 + N) of an n_total-row output go
+        // into its own y (at user offset y_off of its arena) and, as {value, launch number} packets, into
+        // every peer's inbox; before the CTA exits it collects its share of the peers' rows (peers.cuh).
+        // SHARDED is a template value rather than a run-time test because the single-GPU instantiation then
+        // compiles exactly as if the peer path did not exist (a run-time branch cost 3-16 %).
+        // one output element: y[m][row0 + row]
+        auto store_out = [&](uint32_t m, uint32_t row, float v) {
+            const size_t idx = (size_t)m * A.n_total + A.row0 + row;
+            const uint32_t bits = A.out_bf16 ? float_to_bf16_bits(v) : __float_as_uint(v);
+            if (A.out_bf16) reinterpret_cast<uint16_t*>(A.y)[idx] = (uint16_t)bits;
+            else reinterpret_cast<uint32_t*>(A.y)[idx] = bits;
+            if constexpr (ARGMAX_) {  // compare what was stored (the rounded value when the output is bf16)
+                if (v == v) {
+                    const unsigned long long key = peer_best_key(A.out_bf16 ? bits << 16 : bits, A.row0 + row);
+                    my_best = key > my_best ? key : my_best;
+                }
+            } else if constexpr (SHARDED_) {
+                if (world > 1u) {
+                    const uint32_t e = peer_epoch(A.pa);
+                    const size_t elem = A.y_off / (A.out_bf16 ? 2u : 4u) + idx;
+                    for (uint32_t p = 0; p < world; ++p)
+                        if (p != A.pa.rank) peer_send(peer_slot(A.pa, peer_arena(A.pa, p), e, elem), bits, e);
                 }
             }
-            if (ok) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_addr(&empty_bars[stage]));  // stage consumed
-            }
-#pragma unroll
-            for (int j = 0; j < NT; ++j) xb[j] += xadv[j];
-            xsp += xs_adv;
-        }
-        // back to k-slab 0 of the row
-#pragma unroll
-        for (int j = 0; j < NT; ++j) xb[j] -= kslabs_v * xadv[j] + kp * (xadv[j] >> kshift);
-        xsp -= kslabs_v * xs_adv + kp * 256u;
+        };
+        // GATED: y[m][row] = bf16(silu(gate) * up) of the N/2-column output, with the arithmetic of the
+        // stand-alone activation kernel (shaders/ops.metal:129-139)
+        auto store_gated = [&](uint32_t m, uint32_t row, float gate, float up) {
+            const float sg = gate / (1.0f + expf(-gate));
+            reinterpret_cast<uint16_t*>(A.y)[(size_t)m * (N >> 1) + row] = (uint16_t)float_to_bf16_bits(sg * up);
+        };
+        (void)store_gated;
 
-#ifdef MIORI_TMA_TRACE
-        if (tile_it == 0) TMA_MARK(5);
-#endif
-        // ---- tile complete: quad sum (EXACT), then 4 partials per output through shared memory
-        constexpr int WS = Red<MP>::WS;
-        float* buf = gred + (size_t)(tile_it & 1u) * 4 * WS;
-        float* mine = buf + (size_t)wg * WS;
-        if (PAIR) {
-            // lanes t and t^2 hold the two chunk pairs of the same two activation rows
+        // ---- this lane's place in the MMAs.  As a B operand it supplies column n = lane / 4 = (slot n / RC,
+        // row n % RC); as an accumulator it holds columns 2 t and 2 t + 1.
+        const uint32_t g = lane >> 2, t = lane & 3u, wg = warp & 3u;
+        const uint32_t sl = S::SLOTTED ? 2u * t / RC : 0u, m_acc = S::SLOTTED ? 2u * t % RC : 2u * t;
+        uint32_t xb[NT];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[0][e] += __shfl_xor_sync(0xFFFFFFFFu, acc[0][e], 2);
-            if (t < 2u) {  // t = 0: rows 0, 1; t = 1: rows 2, 3
-                mine[g * MP + 2 * t] = acc[0][0];
-                mine[g * MP + 2 * t + 1] = acc[0][1];
-                mine[(g + 8) * MP + 2 * t] = acc[0][2];
-                mine[(g + 8) * MP + 2 * t + 1] = acc[0][3];
+        for (int j = 0; j < NT; ++j)  // columns past M repeat the last row: results nobody reads
+            xb[j] = xa.x + min((uint32_t)(8 * j) + g % (uint32_t)RC, M - 1u) * xa.pitch + t * (uint32_t)S::XB;
+        const uint32_t zeros = base + L.zeros;
+        const uint32_t q_lane = g * qpitch + t * (uint32_t)S::W;
+        const uint32_t sb_row = g * ng * 2u, sb_row8 = 8u * ng * 2u;
+        using R = Red<ROWS>;
+        const bool vec_sb = ng % 8u == 0u;  // rows of scales start on 16-byte boundaries
+
+        float acc[S::ACCN][4];
+#pragma unroll
+        for (int j = 0; j < S::ACCN; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+
+        // d: sums of columns 2t, 2t + 1 for tile rows g (first two) and g + 8.  ms: {power of two, sum} of both
+        // columns; s, b: scales and biases of [row][column]
+        auto apply = [&](float (&a)[4], const float (&d)[4], const float4& ms, float s00, float s01, float s10, float s11,
+                         float b00, float b01, float b10, float b11) {
+            a[0] = __fmaf_rn(s00 * ms.x, d[0], __fmaf_rn(b00, ms.y, a[0]));
+            a[1] = __fmaf_rn(s01 * ms.z, d[1], __fmaf_rn(b01, ms.w, a[1]));
+            a[2] = __fmaf_rn(s10 * ms.x, d[2], __fmaf_rn(b10, ms.y, a[2]));
+            a[3] = __fmaf_rn(s11 * ms.z, d[3], __fmaf_rn(b11, ms.w, a[3]));
+        };
+
+        // A run: `steps` steps (four when FULL) of 64 bytes of every row from shared address qa on (row g, this
+        // lane's piece), activations xo bytes into the staged rows, first scale group grp0, scales of row g at sa.
+        auto run_math = [&](auto full, uint32_t qa, uint32_t xo, uint32_t grp0, uint32_t sa, uint32_t steps) {
+            constexpr bool FULL = decltype(full)::value;
+            // FULL: the run's scales and biases by one or two wide loads per row (RC == 1 reads pairs in place)
+            constexpr int SW = 2 * GPS;  // words: 4 GPS bf16 values
+            uint32_t vs0[SW], vb0[SW], vs1[SW], vb1[SW];
+            if constexpr (FULL && RC > 1) {
+                lds_words<4 * SW>(vs0, sa + 2u * grp0);
+                lds_words<4 * SW>(vb0, sa + 2u * grp0 + L.sb_half);
+                lds_words<4 * SW>(vs1, sa + 2u * grp0 + sb_row8);
+                lds_words<4 * SW>(vb1, sa + 2u * grp0 + sb_row8 + L.sb_half);
             }
-        } else if (EXACT) {
+            const uint32_t half = (sl & 1u) ? 0x3244u : 0x1044u;
+            // fp32 value of the run's group c + (SLOTTED: this lane's slot)
+            auto pick = [&](const uint32_t (&v)[SW], int c) -> float {
+                if constexpr (!S::SLOTTED) return c & 1 ? bf16hi(v[c >> 1]) : bf16lo(v[c >> 1]);
+                else if constexpr (S::SLOTS == 4) {
+                    if constexpr (SW > 2) return __uint_as_float(__byte_perm((sl & 2u) ? v[(c >> 1) + 1] : v[c >> 1], 0u, half));
+                    else return __uint_as_float(__byte_perm((sl & 2u) ? v[1] : v[0], 0u, half));
+                } else return __uint_as_float(__byte_perm(v[c >> 1], 0u, half));
+            };
+            // not FULL: groups of steps that are not this run's, or past the end of K, count as zero
+            const uint32_t glim = min(ng, grp0 + steps * GPS);
+            auto one = [&](uint32_t at, uint32_t gi) { return __uint_as_float(gi < glim ? lds16(at + 2u * gi) << 16 : 0u); };
+            // apply the sums d to acc: c = first group of the accumulator relative to the run
+            auto scale = [&](float (&a)[4], const float (&d)[4], int c, int j) {
+                if constexpr (RC == 1) {
+                    // two neighbouring groups, one row; with fewer than eight groups a run the upper lanes have
+                    // no group: their sums are zero, and their biases count as zero
+                    constexpr bool SHORT = 4 * GPS < 8;
+                    const uint32_t p = grp0 + (uint32_t)c + (SHORT ? 2u * (t & 1u) : 2u * t);
+                    if constexpr (FULL) {
+                        const uint32_t s0 = lds32(sa + 2u * p), s1 = lds32(sa + 2u * p + sb_row8);
+                        uint32_t b0 = lds32(sa + 2u * p + L.sb_half), b1 = lds32(sa + 2u * p + sb_row8 + L.sb_half);
+                        if (SHORT && t >= 2u) b0 = b1 = 0u;
+                        apply(a, d, ldsf128(xa.ms + p * 8u), bf16lo(s0), bf16hi(s0), bf16lo(s1), bf16hi(s1), bf16lo(b0),
+                              bf16hi(b0), bf16lo(b1), bf16hi(b1));
+                    } else {
+                        const uint32_t lim = SHORT && t >= 2u ? 0u : 2u;
+                        const uint32_t p0 = lim ? p : glim, p1 = lim ? p + 1u : glim;
+                        float4 ms = ldsf128(xa.ms + (p & ~1u) * 8u);  // (p is even unless the run starts on an odd group)
+                        if (p & 1u) {
+                            const float4 nx = ldsf128(xa.ms + (p + 1u) * 8u);
+                            ms = make_float4(ms.z, ms.w, nx.x, nx.y);
+                        }
+                        if (p0 >= glim) ms.x = ms.y = 0.0f;
+                        if (p1 >= glim) ms.z = ms.w = 0.0f;
+                        apply(a, d, ms, one(sa, p0), one(sa, p1), one(sa + sb_row8, p0), one(sa + sb_row8, p1),
+                              one(sa + L.sb_half, p0), one(sa + L.sb_half, p1), one(sa + sb_row8 + L.sb_half, p0),
+                              one(sa + sb_row8 + L.sb_half, p1));
+                    }
+                } else {
+                    const uint32_t gi = grp0 + (uint32_t)c + sl;
+                    float4 ms = ldsf128(xa.ms + (gi * ROWS + (uint32_t)(8 * j) + m_acc) * 8u);
+                    float s0, s1, b0, b1;
+                    if constexpr (FULL) {
+                        s0 = pick(vs0, c), s1 = pick(vs1, c), b0 = pick(vb0, c), b1 = pick(vb1, c);
+                    } else {
+                        s0 = one(sa, gi), s1 = one(sa + sb_row8, gi), b0 = one(sa + L.sb_half, gi), b1 = one(sa + sb_row8 + L.sb_half, gi);
+                        if (gi >= glim) ms = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    }
+                    apply(a, d, ms, s0, s0, s1, s1, b0, b0, b1, b1);
+                }
+            };
+            using AF = AFrag<BITS, S::NW>;
+            if constexpr (S::SLOTTED) {
 #pragma unroll
-            for (int j = 0; j < NT; ++j)
+                for (int p = 0; p < 4 / S::SPA; ++p) {
+                    if (!FULL && (uint32_t)(p * S::SPA) >= steps) break;
+                    float d[S::SETS][2][4];  // two chains each
+#pragma unroll
+                    for (int i = 0; i < S::SPA; ++i) {
+                        const int step = p * S::SPA + i;
+                        if (!FULL && (uint32_t)step >= steps) break;
+                        uint32_t q0[4], q1[4];
+                        lds_words<16>(q0, qa + (uint32_t)step * STEP_BYTES);
+                        lds_words<16>(q1, qa + (uint32_t)step * STEP_BYTES + 8u * qpitch);
+                        AF a;
+                        a.unpack(q0, q1);
+#pragma unroll
+                        for (int j = 0; j < S::SETS; ++j) {
+                            // this lane's codes belong to slot i GPS + t GPS / 4 of the pass
+                            const bool active = g / (uint32_t)RC + (uint32_t)(j * S::SLOTS) == (uint32_t)(i * GPS) + t * (uint32_t)GPS / 4u;
+                            const uint32_t x_at = active ? xb[0] + xo + (uint32_t)step * 2u * S::SK : zeros;
+#pragma unroll
+                            for (int k = 0; k < AF::MMAS; k += 2) {
+                                const uint4 b = lds128(x_at + 8u * k);
+                                a.mma(i == 0 && k == 0, k, d[j][0], b.x, b.y);
+                                a.mma(i == 0 && k == 0, k + 1, d[j][1], b.z, b.w);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < S::SETS; ++j) {
+                        const float sum[4] = {d[j][0][0] + d[j][1][0], d[j][0][1] + d[j][1][1], d[j][0][2] + d[j][1][2], d[j][0][3] + d[j][1][3]};
+                        scale(acc[(p * S::SETS + j) % S::ACCN], sum, p * S::SPA * GPS + j * S::SLOTS, 0);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int step = 0; step < 4; ++step) {
+                    if (!FULL && (uint32_t)step >= steps) break;
+#pragma unroll
+                    for (int c = 0; c < S::CH; ++c) {
+                        uint32_t q0[S::NW], q1[S::NW];
+                        lds_words<S::W>(q0, qa + (uint32_t)step * STEP_BYTES + (uint32_t)(c * 4 * S::W));
+                        lds_words<S::W>(q1, qa + (uint32_t)step * STEP_BYTES + (uint32_t)(c * 4 * S::W) + 8u * qpitch);
+                        AF a;
+                        a.unpack(q0, q1);
+#pragma unroll
+                        for (int j = 0; j < NT; ++j) {
+                            float d[4];
+#pragma unroll
+                            for (int k = 0; k < AF::MMAS; k += 2) {
+                                const uint4 b = lds128(xb[j] + xo + (uint32_t)step * 2u * S::SK + (uint32_t)(c * 4 * S::XB) + 8u * k);
+                                a.mma(k == 0, k, d, b.x, b.y);
+                                a.mma(false, k + 1, d, b.z, b.w);
+                            }
+                            scale(acc[j], d, step * GPS + c, j);
+                        }
+                    }
+                }
+            }
+        };
+
+        // `ok` turns false for good once a wait expires; the warp then skips waits and math but still takes
+        // part in every group barrier so that no other warp is left waiting.
+        bool ok = true;
+        uint32_t tile_it = 0, st = 0, st_par = 0, sb = 0, sb_par = 0;
+        auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t where) {
+            if (!ok) return;
+            if (__all_sync(0xFFFFFFFFu, mbar_try_long(smem_addr(bar), parity))) return;
+            ok = mbar_wait(smem_addr(bar), parity, &abort_flag, where);
+            ok = __all_sync(0xFFFFFFFFu, ok);
+        };
+        const uint32_t gt = wg * 32u + lane;  // thread index inside the group
+        for (uint32_t vt = grp; grp < ngrp && vt < vtiles; vt += ngrp) {
+            const uint32_t sa = base + L.sb + (sb0 + sb) * 2u * L.sb_half + sb_row;
+            if (kpar > 1u) wait(&sb_full[sb0 + sb], sb_par, 0x12);
+            for (uint32_t ks = kp; ks < kslabs; ks += kpar) {
+                wait(&full_bars[bar0 + st], st_par, 0x10);
+                if (ok) {
+                    // steps of this slab, dealt to the warps in runs: four each in a full slab
+                    const uint32_t left = row_bytes - ks * SLAB_ROW;
+                    const uint32_t qa = base + (bar0 + st) * L.stage_bytes + q_lane;
+                    if (vec_sb && left >= SLAB_ROW) {
+                        run_math(std::true_type(), qa + wg * 4u * STEP_BYTES, 2u * (ks * S::KC + wg * 4u * S::SK),
+                                 ks * (S::KC / S::GROUP) + wg * 4u * GPS, sa, 4u);
+                    } else {
+                        const uint32_t nsteps = (min(left, SLAB_ROW) + STEP_BYTES - 1u) / STEP_BYTES;
+                        const uint32_t run = (nsteps + 3u) >> 2, step0 = wg * run;
+                        if (step0 < nsteps)
+                            run_math(std::false_type(), qa + step0 * STEP_BYTES, 2u * (ks * S::KC + step0 * S::SK),
+                                     ks * (S::KC / S::GROUP) + step0 * GPS, sa, min(run, nsteps - step0));
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_addr(&empty_bars[bar0 + st]));  // stage consumed
+                }
+                if (++st == nsg) st = 0u, st_par ^= 1u;
+            }
+            if (kpar > 1u && ok && lane == 0) mbar_arrive(smem_addr(&sb_empty[sb0 + sb]));
+            if (++sb == A.nsb) sb = 0u, sb_par ^= 1u;
+
+            // ---- tile complete: the classes of groups in a fixed tree, then the warps' partials (and those of
+            // the groups that share the tile) through shared memory
+            const uint32_t red0 = base + L.red + (R::BUFS == 2 ? (tile_it & 1u) * (uint32_t)(GROUPS * R::FLOATS * 4) : 0u);
+            const uint32_t mine = red0 + grp * (uint32_t)(R::FLOATS * 4) + wg * 4u;  // + 16 * (m * 16 + tile row)
+            auto put = [&](uint32_t m, uint32_t r, float v) {
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(mine + (m * 16u + r) * 16u), "f"(v) : "memory");
+            };
+            auto xor_add = [](float v, int o) { return v + __shfl_xor_sync(0xFFFFFFFFu, v, o); };
+            if constexpr (RC == 1) {
+                const float v0 = xor_add(xor_add(acc[0][0] + acc[0][1], 1), 2), v1 = xor_add(xor_add(acc[0][2] + acc[0][3], 1), 2);
+                if (t < 2u) put(0u, g + 8u * t, t ? v1 : v0);
+            } else if constexpr (S::SLOTTED) {
+                float r[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    float v = acc[j][e];
-                    v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
-                    v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
-                    acc[j][e] = v;
-                }
-            if (t == 0) {
+                    float v[S::ACCN];
 #pragma unroll
-                for (int j = 0; j < NT; ++j) {
-                    mine[g * MP + 2 * j] = acc[j][0];
-                    mine[g * MP + 2 * j + 1] = acc[j][1];
-                    mine[(g + 8) * MP + 2 * j] = acc[j][2];
-                    mine[(g + 8) * MP + 2 * j + 1] = acc[j][3];
+                    for (int a = 0; a < S::ACCN; ++a) {
+                        v[a] = acc[a][e];
+                        if constexpr (RC == 2) v[a] = xor_add(v[a], 1);
+                        v[a] = xor_add(v[a], 2);
+                    }
+                    r[e] = v[0];
+                    if constexpr (S::ACCN == 2) r[e] = v[0] + v[1];
+                    if constexpr (S::ACCN == 4) r[e] = (v[0] + v[1]) + (v[2] + v[3]);
                 }
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                mine[g * MP + 8 * j + 2 * t] = acc[j][0];
-                mine[g * MP + 8 * j + 2 * t + 1] = acc[j][1];
-                mine[(g + 8) * MP + 8 * j + 2 * t] = acc[j][2];
-                mine[(g + 8) * MP + 8 * j + 2 * t + 1] = acc[j][3];
-            }
-        }
-        named_barrier(1u + grp, 128u);
-        const uint32_t gt = wg * 32u + lane;  // thread index inside the group
-#pragma unroll
-        for (uint32_t base = 0; base < 16u * MP * 4u; base += 128u) {
-            const uint32_t idx = base + gt;
-            const uint32_t o = idx >> 2, w = idx & 3u;  // output o = m*16 + r, partial of warp w
-            // GATED enumerates the outputs as o = (m*8 + r')*2 + half, tile row r = r' + 8 half:
-            // gate and up of an output sit in neighbouring quads (neighbouring threads below)
-            const uint32_t r = GATED ? ((o >> 1) & 7u) + ((o & 1u) << 3) : o & 15u, m = o >> 4;
-            float v = buf[(size_t)w * WS + r * MP + m];
-            v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
-            v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
-            const uint32_t row = tile * 16u + r;
-            if constexpr (GATED) {
-                const float up = __shfl_down_sync(0xFFFFFFFFu, v, 4);
-                if (kpar > 1u) {
-                    if (w == 0) kred[((size_t)(tile_it & 1u) * GROUPS + grp) * (16 * MP) + o] = v;
-                } else if (w == 0 && (o & 1u) == 0u && m < M && ok) {
-                    store_gated(m, tile * 8u + r, v, up);
+                if constexpr (RC == 2) {  // every lane of the quad has all four: each stores one
+                    put(t & 1u, g + 8u * (t >> 1), t == 0u ? r[0] : t == 1u ? r[1] : t == 2u ? r[2] : r[3]);
+                } else {                  // lanes t and t ^ 2 have the same four: two each
+                    const bool up = t >= 2u;
+                    put(m_acc, g + (up ? 8u : 0u), up ? r[2] : r[0]);
+                    put(m_acc + 1u, g + (up ? 8u : 0u), up ? r[3] : r[1]);
                 }
-            } else if (kpar > 1u) {
-                if (w == 0) kred[((size_t)(tile_it & 1u) * GROUPS + grp) * (16 * MP) + o] = v;
-            } else if (w == 0 && m < M && row < N && ok) {
-                store_out(m, row, v);
+            } else {
+#pragma unroll
+                for (int j = 0; j < NT; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) put(8u * j + m_acc + (e & 1), g + 8u * (e >> 1), acc[j][e]);
             }
-        }
-        if (kpar > 1u) {
-            // the kpar groups of this tile meet; the first of them sums the partials in order
-            named_barrier(5u + (grp >> kshift), kpar * 128u);
-            if (kp == 0u) {
-                const float* kr = kred + ((size_t)(tile_it & 1u) * GROUPS + grp) * (16 * MP);
-                for (uint32_t o = gt; o < 16u * MP; o += 128u) {
-                    float v = kr[o];
-                    for (uint32_t j = 1; j < kpar; ++j) v += kr[(size_t)j * (16 * MP) + o];
-                    if constexpr (GATED) {  // 16 MP is a multiple of 32: whole warps run this loop
-                        const float up = __shfl_down_sync(0xFFFFFFFFu, v, 1);
-                        const uint32_t m = o >> 4;
-                        if ((o & 1u) == 0u && m < M && ok) store_gated(m, tile * 8u + ((o >> 1) & 7u), v, up);
-                    } else {
-                        const uint32_t r = o & 15u, m = o >> 4, row = tile * 16u + r;
-                        if (m < M && row < N && ok) store_out(m, row, v);
+#pragma unroll
+            for (int j = 0; j < S::ACCN; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+            named_barrier(1u + (grp >> kshift), kpar * 128u);
+            // output o = m * 16 + r of the tile: warps first, then groups, in order
+            auto total = [&](uint32_t o) {
+                float v = 0.0f;
+                for (uint32_t j = 0; j < kpar; ++j) {
+                    const float4 p = ldsf128(red0 + (grp + j) * (uint32_t)(R::FLOATS * 4) + o * 16u);
+                    const float w = (p.x + p.y) + (p.z + p.w);
+                    v = j == 0u ? w : v + w;
+                }
+                return v * UNSCALE;
+            };
+            const uint32_t tile = blockIdx.x + (vt >> kshift) * gridDim.x;
+            if (kp == 0u && ok) {
+                if constexpr (GATED_) {  // tile rows 0 .. 7 are gates, 8 .. 15 the same outputs' up rows
+                    for (uint32_t i = gt; i < 8u * M; i += 128u) {
+                        const uint32_t m = i >> 3, r = i & 7u;
+                        store_gated(m, tile * 8u + r, total(m * 16u + r), total(m * 16u + r + 8u));
+                    }
+                } else {
+                    for (uint32_t o = gt; o < 16u * M; o += 128u) {
+                        const uint32_t row = tile * 16u + (o & 15u);
+                        const float v = total(o);
+                        if (row < N) store_out(o >> 4, row, v);
                     }
                 }
             }
+            if constexpr (R::BUFS == 1) named_barrier(1u + (grp >> kshift), kpar * 128u);
+            ++tile_it;
         }
-#ifdef MIORI_TMA_TRACE
-        if (tile_it == 0) TMA_MARK(6);
-#endif
-        ++tile_it;
-#pragma unroll
-        for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
     }
 
-    TMA_MARK(3);
+    if constexpr (POSTNORM_ || ARGMAX_ || SHARDED_) __syncthreads();  // the producers are done too
     if (abort_flag) {  // let copies still in flight land before the CTA's memory is released
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000LL) __nanosleep(1000);
     }
-    if constexpr (POSTNORM) {  // every thread of the CTA gets here: no early exits above
+    if constexpr (POSTNORM_) {  // every thread of the CTA gets here: no early exits above
         __shared__ float pn_part[neighbors::NORM_THREADS / 32];
         __shared__ uint32_t pn_last;
         __threadfence();  // this thread's rows of v are visible before the CTA reports in
         __syncthreads();
         if (threadIdx.x == 0) {
-            pn_last = atomicAdd(pn.arrivals, 1u) == gridDim.x - 1u ? 1u : 0u;
+            pn_last = atomicAdd(A.post.arrivals, 1u) == gridDim.x - 1u ? 1u : 0u;
             __threadfence();
         }
         __syncthreads();
         if (pn_last && threadIdx.x < (uint32_t)neighbors::NORM_THREADS) {
-            float* out = reinterpret_cast<float*>(y);
+            float* out = reinterpret_cast<float*>(A.y);
             for (uint32_t m = 0; m < M; ++m) {
                 const size_t at = (size_t)m * N;
                 if (N <= 8u * (uint32_t)neighbors::NORM_THREADS)
-                    neighbors::post_norm_add_row_regs<9, true, 8>(pn.residual + at, out + at, pn.gamma, out + at, N,
-                                                                  pn.eps, pn_part);
+                    neighbors::post_norm_add_row_regs<9, true, 8>(A.post.residual + at, out + at, A.post.gamma, out + at, N,
+                                                                  A.post.eps, pn_part);
                 else
-                    neighbors::post_norm_add_row<9, true>(pn.residual + at, out + at, pn.gamma, out + at, N, pn.eps,
-                                                          pn_part);
+                    neighbors::post_norm_add_row<9, true>(A.post.residual + at, out + at, A.post.gamma, out + at, N,
+                                                          A.post.eps, pn_part);
                 neighbors::norm_sync<9>();  // pn_part is reused by the next row
             }
-            if (threadIdx.x == 0) *pn.arrivals = 0u;  // ready for the next launch
+            if (threadIdx.x == 0) *A.post.arrivals = 0u;  // ready for the next launch
         }
-    } else if constexpr (ARGMAX) {  // every thread of the CTA gets here: no early exits above
+    } else if constexpr (ARGMAX_) {  // every thread of the CTA gets here: no early exits above
         unsigned long long k = my_best;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const unsigned long long other = __shfl_xor_sync(0xFFFFFFFFu, k, o);
             k = other > k ? other : k;
         }
-        __shared__ unsigned long long warp_keys[WARPS + 1];
+        __shared__ unsigned long long warp_keys[THREADS / 32];
         if (lane == 0) warp_keys[warp] = k;
         __syncthreads();
         if (threadIdx.x == 0) {
-            for (uint32_t w = 1; w <= (uint32_t)WARPS; ++w) k = warp_keys[w] > k ? warp_keys[w] : k;
-            if (k != 0ull) atomicMax(best, k);  // one candidate per CTA
-            unsigned int* arrived = reinterpret_cast<unsigned int*>(best + 1);
+            for (uint32_t w = 1; w < (uint32_t)WARPS; ++w) k = warp_keys[w] > k ? warp_keys[w] : k;
+            if (k != 0ull) atomicMax(A.best, k);  // one candidate per CTA
+            unsigned int* arrived = reinterpret_cast<unsigned int*>(A.best + 1);
             __threadfence();
             if (atomicAdd(arrived, 1u) == gridDim.x - 1u) {  // the last CTA: every candidate is in
                 __threadfence();
-                const unsigned long long win = atomicExch(best, 0ull);  // read, and reset for the next launch
+                const unsigned long long win = atomicExch(A.best, 0ull);  // read, and reset for the next launch
                 *arrived = 0u;
-                uint32_t* pairs = reinterpret_cast<uint32_t*>(best) + 4;
-                const size_t base = (size_t)(reinterpret_cast<uint8_t*>(pairs) - (pa.local + PEER_CTL_BYTES)) / 4u;
-                peer_argmax_exchange(pa, pairs, base, peer_best_from_key(win));
+                uint32_t* pairs = reinterpret_cast<uint32_t*>(A.best) + 4;
+                const size_t at = (size_t)(reinterpret_cast<uint8_t*>(pairs) - (A.pa.local + PEER_CTL_BYTES)) / 4u;
+                peer_argmax_exchange(A.pa, pairs, at, peer_best_from_key(win));
             }
         }
-    } else if constexpr (SHARDED) {
+    } else if constexpr (SHARDED_) {
         if (world > 1u) {  // every thread of the CTA gets here: no early exits above
-            const uint32_t e = peer_epoch(pa);
+            const uint32_t e = peer_epoch(A.pa);
             __syncthreads();
-            peer_collect<OUT_BF16>(pa, e, y_off, M, n_total, row0, N);
+            if (A.out_bf16) peer_collect<true>(A.pa, e, A.y_off, M, A.n_total, A.row0, N);
+            else peer_collect<false>(A.pa, e, A.y_off, M, A.n_total, A.row0, N);
             __syncthreads();
-            if (threadIdx.x == 0) peer_finish(pa, e);
-            TMA_MARK(7);  // tracing build: the peers' rows are in y
+            if (threadIdx.x == 0) peer_finish(A.pa, e);
         }
     }
 }
 
-template <int BITS, bool EXACT, int NT, bool PAIR>
-size_t fixed_smem(uint32_t K) {
-    constexpr int KC = 16 * 4 * (128 / BITS);
-    constexpr int MP = EXACT ? (PAIR ? 4 : 2 * NT) : 8 * NT;
-    const uint32_t kslabs = (K + KC - 1) / KC, steps_p = kslabs * 16;
-    size_t bytes = (size_t)MP * (steps_p * STEP_UNITS + 1) * 16 + ZERO_BYTES;
-    if (EXACT) bytes += (size_t)MP * steps_p * 4 * 4;
-    bytes += (size_t)GROUPS * Red<MP>::GROUP_FLOATS * 4;
-    bytes += (size_t)2 * GROUPS * 16 * MP * 4;  // partial outputs of groups that share a tile
-    return bytes;
-}
-
-// Placement of an N-sharded launch's output: peers (world <= 1: none, y is a plain pointer),
-// rows of the whole output, this rank's first row, and the offset of y inside every arena.
+// Placement of an N-sharded launch's output and the fused neighbours of a launch: peers (world <= 1:
+// none, y is a plain pointer), rows of the whole output, this rank's first row, and the offset of y
+// inside every arena.
 struct Shard {
     PeerArgs pa = {};
     uint32_t n_total = 0, row0 = 0;
@@ -1059,178 +996,140 @@ struct Shard {
     bool gated = false;
     // post-norm epilogue (4-bit weights, fp32 out, up to four rows, one GPU); residual null: off
     PostNorm post;
-    // norm prologue (4-bit weights, up to four rows, one GPU; fp32 out or the gated epilogue): x is
-    // fp32; gamma null: off
+    // norm prologue (one GPU): x is fp32; gamma null: off
     PreNorm pre;
 };
 
-// Launch plan: CTAs, active groups and stages per group; ngrp == 0 means the TMA path cannot
-// take the problem.
+// Launch plan: CTAs, active groups, stages per group, scale buffers; ngrp == 0: the activations do not fit.
 struct Plan {
-    uint32_t grid, ngrp, nsg, kpar;
-    bool pad = false;  // raise the shared-memory request above half an SM (see plan_stages)
-    bool roomy;  // one CTA per SM and few tiles: use the instantiation with the larger register budget
+    uint32_t grid = 0, ngrp = 0, nsg = 0, nsb = 0, kpar = 1, slab_row = 0;
+    size_t smem = 0;
 };
-template <int BITS, bool EXACT, int NT, bool PAIR>
-Plan plan_stages(uint32_t N, uint32_t K, uint32_t group) {
-    constexpr int KC = 16 * 4 * (128 / BITS);
-    Plan p = {0, 0, 0, 1, false, false};
-    if ((K / group) % 8 != 0) return p;  // scale rows must have a 16-byte pitch for TMA
-    const size_t fixed = fixed_smem<BITS, EXACT, NT, PAIR>(K);
-    const uint32_t tiles = (N + 15) / 16, kslabs = (K + KC - 1) / KC;
-    const uint32_t sms = (uint32_t)sm_count();
-    // Long streams (many tiles per SM) launch two CTAs per SM, each sized for half an SM, for
-    // latency hiding.  Everything else launches at most one CTA per SM, and the one- and two-row
-    // kernels then also claim more than half of the SM's shared memory, so that no second CTA of
-    // any kernel of this family can join it.  Sharing an SM with the successor of a
-    // dependent-launch chain looks attractive (it prefetches while this one computes) and is
-    // 5-10 % faster while every launch has the same footprint, but the placement is not stable:
-    // after a launch with another footprint the successor's CTAs double up on the SMs that were
-    // free and leave others without one, every later launch inherits the skew, and a 24-layer
-    // chain of four shapes ran 17 % slower than the sum of its parts.  With the SM to itself a CTA
-    // starts as its predecessor's CTA exits, fills a ring of up to 200 KB during the ~1.5 us
-    // hand-over between the grids, and the placement is one CTA per SM whatever ran before.
-    const size_t half = 112 * 1024, hard = 208 * 1024;
-    const bool fits_half = fixed + 4 * STAGE_BYTES <= half;
-    if (!fits_half && fixed + 2 * STAGE_BYTES > hard) return p;
-    const bool two_per_sm = fits_half && NT == 1 && tiles * kslabs > 6 * sms;
-    const bool alone = !two_per_sm && EXACT && NT == 1 && !PAIR;
-    const bool whole = !fits_half || alone;
-    const uint32_t st = (uint32_t)(((whole ? hard : half) - fixed) / STAGE_BYTES);
-    p.grid = std::min<uint32_t>(tiles, two_per_sm ? 2 * sms : sms);
-    p.roomy = !two_per_sm && (tiles <= 2 * sms || alone);
-    p.pad = alone;
-    const uint32_t tiles_cta = (tiles + p.grid - 1) / p.grid;  // tiles of the busiest CTA
-    // few tiles per CTA and a long K: let 2 or 4 groups share a tile, each taking every
-    // kpar-th k-slab
-    while (p.kpar * 2 <= (uint32_t)GROUPS && tiles_cta * p.kpar * 2 <= (uint32_t)GROUPS &&
-           kslabs % (p.kpar * 2) == 0 && st >= p.kpar * 2)
-        p.kpar *= 2;
-    const uint32_t vtiles = tiles_cta * p.kpar;
-    p.ngrp = std::min<uint32_t>(std::min<uint32_t>(GROUPS, st), vtiles);
-    p.ngrp -= p.ngrp % p.kpar;
-    const uint32_t sets = (vtiles + p.ngrp - 1) / p.ngrp;
-    p.nsg = std::min<uint32_t>(st / p.ngrp, sets * (kslabs / p.kpar));  // no more than a group needs
-    if (p.ngrp * p.nsg > (uint32_t)MAX_STAGES) p.nsg = MAX_STAGES / p.ngrp;
+// One CTA per SM, which also claims more than half of the SM's shared memory, so that no second CTA of
+// any kernel of this family can join it.  Sharing an SM with the successor of a dependent-launch chain
+// looks attractive (it prefetches while this one computes) but the placement is not stable: after a
+// launch with another footprint the successor's CTAs double up on the SMs that were free and leave
+// others without one, every later launch inherits the skew, and a 24-layer chain of four shapes ran
+// 17 % slower than the sum of its parts.  With the SM to itself a CTA starts as its predecessor's CTA
+// exits, fills its ring during the hand-over between the grids, and the placement is one CTA per SM
+// whatever ran before.
+template <class S>
+Plan plan_launch(uint32_t N, uint32_t K, uint32_t M) {
+    constexpr size_t LIMIT = 222 * 1024;
+    Plan p;
+    const uint32_t row_bytes = K * S::BITS / 8u;
+    const uint32_t tiles = (N + 15u) / 16u, kslabs = (row_bytes + SLAB_ROW - 1u) / SLAB_ROW;
+    p.slab_row = row_bytes >= SLAB_ROW ? SLAB_ROW : (row_bytes + 127u) / 128u * 128u;
+    p.grid = std::min<uint32_t>(tiles, (uint32_t)sm_count());
+    const uint32_t tiles_cta = (tiles + p.grid - 1u) / p.grid;  // tiles of the busiest CTA
+    // few tiles per CTA and a long K: let 2 or 4 groups share a tile, each taking every kpar-th slab
+    while (p.kpar * 2u <= (uint32_t)GROUPS && tiles_cta * p.kpar * 2u <= (uint32_t)GROUPS && kslabs % (p.kpar * 2u) == 0u)
+        p.kpar *= 2u;
+    for (; p.kpar >= 1u; p.kpar >>= 1) {
+        const uint32_t vtiles = tiles_cta * p.kpar, own = kslabs / p.kpar;  // slabs of a tile per group
+        uint32_t most = std::min<uint32_t>(GROUPS, vtiles);
+        most -= most % p.kpar;
+        for (uint32_t ngrp = most; ngrp >= p.kpar; ngrp -= p.kpar) {
+            const uint32_t each = (vtiles + ngrp - 1u) / ngrp;  // tiles of the busiest group
+            for (uint32_t nsg = std::min<uint32_t>(MAX_NSG, each * own); nsg >= 1u; --nsg) {
+                // scales of every tile the code stages reach into: when the stage of a tile's first slab is
+                // free, so is the buffer of the tile nsb before it
+                const uint32_t nsb = std::min(each, (nsg - 1u + own - 1u) / own + 1u);
+                const size_t bytes = layout<S>(K, M, ngrp * nsg, ngrp / p.kpar * nsb, p.slab_row).total;
+                if (bytes > LIMIT) continue;
+                p.ngrp = ngrp, p.nsg = nsg, p.nsb = nsb;
+                p.smem = std::max<size_t>(bytes, 120 * 1024);
+                return p;
+            }
+        }
+    }
+    p.kpar = 1u;
     return p;
 }
 
-template <int BITS, bool EXACT, int NT, bool PAIR>
-int launch_one(Plan plan, const void* q, const void* s, const void* b, const void* x, void* y,
-               uint32_t N, uint32_t K, uint32_t M, uint32_t group, uint32_t flags,
-               cudaStream_t stream, const Shard& sh) {
-    constexpr int KC = 16 * 4 * (128 / BITS);
-    const size_t smem = fixed_smem<BITS, EXACT, NT, PAIR>(K) + (size_t)plan.ngrp * plan.nsg * STAGE_BYTES;
-    const uint32_t grid = plan.grid;
-    const bool pdl = (flags & MIORI_LAUNCH_PDL) != 0;
-    const uint32_t gshift = group == 32 ? 5u : 6u;
-    // K within one slab: plain bulk copies (rows of a tile are contiguous); else tiled TMA
-    const bool linear = K <= (uint32_t)KC && !(flags & MIORI_TUNE_GEMV_TILED);
-    CUtensorMap tq, ts, tb;
-    const uint32_t box_rows = sh.gated ? 8 : 16;  // gated: a tile is two boxes, one from each half
-    int rc = make_tmap_2d(&tq, q, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, (uint64_t)K * BITS / 32, N,
-                          ROW_BYTES / 4, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
+template <class S, Fuse F>
+int launch_one(const Plan& plan, const void* q, Args& a, bool pdl, cudaStream_t stream) {
+    constexpr bool gated = F == GATED || F == NORMED_GATED;
+    CUtensorMap tq;
+    // rows as 64-bit words, so that the box can be wider than 256 words of 32 bits; gated: a tile is two
+    // boxes, one from each half
+    const int rc = make_tmap_2d(&tq, q, CU_TENSOR_MAP_DATA_TYPE_UINT64, 8, (uint64_t)a.K * S::BITS / 64, a.N,
+                                (plan.slab_row + S::QPAD) / 8, gated ? 8 : 16, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
-    rc = make_tmap_2d(&ts, s, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, K / group, N, KC / group, box_rows,
-                      CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc) return rc;
-    rc = make_tmap_2d(&tb, b, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, K / group, N, KC / group, box_rows,
-                      CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc) return rc;
-    const uint8_t* ql = linear ? reinterpret_cast<const uint8_t*>(q) : nullptr;
-    cudaError_t e = cudaSuccess;
-#define MIORI_TMA_LAUNCH(OB, SH, AM, GT, PN) MIORI_TMA_LAUNCH_N(OB, SH, AM, GT, PN, false)
-#define MIORI_TMA_LAUNCH_N(OB, SH, AM, GT, PN, NM)                                               \
-    do {                                                                                         \
-        auto kern = roomy ? gemv_tma_kernel<BITS, EXACT, NT, OB, SH, NT == 1, PAIR, AM, GT, PN, NM>  \
-                          : gemv_tma_kernel<BITS, EXACT, NT, OB, SH, false, PAIR, AM, GT, PN, NM>;   \
-        e = cudaSuccess;                                                                         \
-        if (smem_l > 48 * 1024)                                                                  \
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_l); \
-        if (e == cudaSuccess)                                                                    \
-            e = launch(kern, dim3(grid), dim3(THREADS), smem_l, stream, pdl, tq, ts, tb, ql,     \
-                       reinterpret_cast<const uint16_t*>(s), reinterpret_cast<const uint16_t*>(b), \
-                       reinterpret_cast<const uint16_t*>(x), y, N, K, M, gshift, plan.ngrp, plan.nsg, plan.kpar, \
-                       sh.pa, placed ? sh.n_total : N, placed ? sh.row0 : 0u, sh.y_off, sh.best, sh.post, sh.pre); \
-    } while (0)
-    const bool sharded = sh.pa.world > 1;
-    constexpr bool can_argmax = EXACT && NT == 1 && !PAIR;  // the one- and two-row kernels
-    const bool argmax = sh.best != nullptr;
-    if (argmax && (!can_argmax || M != 1))
-        return fail(MIORI_E_INVALID, "the arg-max epilogue takes one activation row");
-    const bool placed = sharded || argmax;  // y is a slice of an n_total-row output
-    const bool roomy = NT == 1 && plan.roomy;
-    const size_t smem_l = plan.pad ? std::max<size_t>(smem, 120 * 1024) : smem;
-    if (sh.gated && (BITS != 4 || sharded || argmax || N % 16 != 0))
-        return fail(MIORI_E_INVALID, "the gated epilogue takes 4-bit weights with N a multiple of 16 on one GPU");
-    const bool postnorm = sh.post.residual != nullptr;
-    if (postnorm && (BITS != 4 || !EXACT || sharded || argmax || sh.gated || (flags & MIORI_OUT_BF16)))
-        return fail(MIORI_E_INVALID, "the post-norm epilogue takes 4-bit weights, up to four rows, fp32 out, one GPU");
-    if constexpr (can_argmax) {
-        if (argmax) {
-            if (flags & MIORI_OUT_BF16) MIORI_TMA_LAUNCH(true, true, true, false, false);
-            else MIORI_TMA_LAUNCH(false, true, true, false, false);
-        }
-    }
-    const bool normed = sh.pre.gamma != nullptr;
-    if (normed && (BITS != 4 || !EXACT || sharded || argmax || postnorm || (!sh.gated && (flags & MIORI_OUT_BF16))))
-        return fail(MIORI_E_INVALID, "the norm prologue takes 4-bit weights, up to four rows, one GPU, fp32 out "
-                                     "or the gated epilogue");
-    if constexpr (BITS == 4 && EXACT) {
-        if (normed) {
-            if (sh.gated) MIORI_TMA_LAUNCH_N(true, false, false, true, false, true);
-            else MIORI_TMA_LAUNCH_N(false, false, false, false, false, true);
-        }
-    }
-    if constexpr (BITS == 4) {
-        if (sh.gated && !normed) MIORI_TMA_LAUNCH(true, false, false, true, false);
-    }
-    if constexpr (BITS == 4 && EXACT) {
-        if (postnorm) MIORI_TMA_LAUNCH(false, false, false, false, true);
-    }
-    if (!argmax && !sh.gated && !postnorm && !normed) {
-        if (flags & MIORI_OUT_BF16) {
-            if (sharded) MIORI_TMA_LAUNCH(true, true, false, false, false);
-            else MIORI_TMA_LAUNCH(true, false, false, false, false);
-        } else {
-            if (sharded) MIORI_TMA_LAUNCH(false, true, false, false, false);
-            else MIORI_TMA_LAUNCH(false, false, false, false, false);
-        }
-    }
-#undef MIORI_TMA_LAUNCH
-#undef MIORI_TMA_LAUNCH_N
+    auto kern = gemv_tma_kernel<S, F>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
+    if (e == cudaSuccess) e = launch(kern, dim3(plan.grid), dim3(THREADS), plan.smem, stream, pdl, tq, a);
     if (e != cudaSuccess) return cuda_fail(e, "gemv_tma launch");
     return MIORI_OK;
 }
 
-// Try the TMA path; returns 1 if this problem is not eligible (nothing launched).
+template <class S>
+int launch_shape(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t M,
+                 uint32_t flags, cudaStream_t stream, const Shard& sh) {
+    const Plan plan = plan_launch<S>(N, K, M);
+    if (plan.ngrp == 0) return 1;
+    constexpr bool FEW = S::ROWS <= 4 || (S::ROWS == 8 && S::GROUP == 64);  // shapes that up to four rows run on
+    const bool sharded = sh.pa.world > 1, argmax = sh.best != nullptr;
+    const bool postnorm = sh.post.residual != nullptr, normed = sh.pre.gamma != nullptr;
+    const bool placed = sharded || argmax;  // y is a slice of an n_total-row output
+    Args a;
+    a.s = static_cast<const uint16_t*>(s);
+    a.b = static_cast<const uint16_t*>(b);
+    a.x = static_cast<const uint16_t*>(x);
+    a.y = y;
+    a.N = N, a.K = K, a.M = M;
+    a.ngrp = plan.ngrp, a.nsg = plan.nsg, a.nsb = plan.nsb, a.kpar = plan.kpar, a.slab_row = plan.slab_row;
+    a.inv_upr = (uint32_t)((0x100000000ull + K / 8u - 1u) / (K / 8u));
+    a.out_bf16 = flags & MIORI_OUT_BF16 ? 1u : 0u;
+    a.n_total = placed ? sh.n_total : N, a.row0 = placed ? sh.row0 : 0u, a.y_off = sh.y_off;
+    a.best = sh.best, a.pa = sh.pa, a.post = sh.post, a.pre = sh.pre;
+    const bool pdl = (flags & MIORI_LAUNCH_PDL) != 0;
+    if ((int)argmax + (int)postnorm + (int)(sharded && !argmax) + (int)(sh.gated || normed) > 1)
+        return fail(MIORI_E_INVALID, "gemv: this combination of fused neighbours does not exist");
+    if (argmax) {
+        if constexpr (S::ROWS == 1) return launch_one<S, ARGMAX>(plan, q, a, pdl, stream);
+        return fail(MIORI_E_INVALID, "the arg-max epilogue takes one activation row");
+    }
+    if (postnorm) {
+        if constexpr (S::BITS == 4 && FEW)
+            if (!a.out_bf16 && M <= 4) return launch_one<S, POSTNORM>(plan, q, a, pdl, stream);
+        return fail(MIORI_E_INVALID, "the post-norm epilogue takes 4-bit weights, up to four rows, fp32 out");
+    }
+    if (sh.gated) {
+        if constexpr (S::BITS == 4 && S::ROWS <= 16) {
+            if (N % 16 == 0 && !normed) return launch_one<S, GATED>(plan, q, a, pdl, stream);
+            if constexpr (FEW)
+                if (N % 16 == 0 && M <= 4) return launch_one<S, NORMED_GATED>(plan, q, a, pdl, stream);
+        }
+        return fail(MIORI_E_INVALID, "the gated epilogue takes 4-bit weights with N a multiple of 16, up to 16 rows "
+                                     "(four with the norm in front)");
+    }
+    if (normed) return launch_one<S, NORMED>(plan, q, a, pdl, stream);
+    if (sharded) return launch_one<S, SHARDED>(plan, q, a, pdl, stream);
+    return launch_one<S, NONE>(plan, q, a, pdl, stream);
+}
+
+// Launch, or return 1 if M rows of K activations do not fit shared memory (nothing launched).
 template <int BITS>
-int try_launch(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N,
-               uint32_t K, uint32_t M, uint32_t group, uint32_t flags, cudaStream_t stream,
-               const Shard& sh = Shard()) {
-    Plan pl;
-#define MIORI_TMA_TRY(EX, NTV, PR)                                                               \
-    do {                                                                                         \
-        pl = plan_stages<BITS, EX, NTV, PR>(N, K, group);                                        \
-        if (pl.ngrp == 0) return 1;                                                              \
-        return launch_one<BITS, EX, NTV, PR>(pl, q, s, b, x, y, N, K, M, group, flags, stream, sh); \
-    } while (0)
-    if (M <= 2) MIORI_TMA_TRY(true, 1, false);
-    if constexpr (BITS == 4) {
-        // three and four rows at group 64: one column set instead of two (13-21 % faster while K
-        // fits one slab; over several slabs the two column sets measured 7-12 % faster); one and
-        // two rows stay on the per-chunk columns, which stage half as much x
-        if (M <= 4 && group == 64 && K <= 2048) MIORI_TMA_TRY(true, 1, true);
-    }
-    if (M <= 4) MIORI_TMA_TRY(true, 2, false);
-    if constexpr (BITS == 8) {
-        return 1;
-    } else {
-        if (M <= 8) MIORI_TMA_TRY(false, 1, false);
-        if (M <= 16) MIORI_TMA_TRY(false, 2, false);
-        MIORI_TMA_TRY(false, 4, false);
-    }
-#undef MIORI_TMA_TRY
+int try_launch(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t M,
+               uint32_t group, uint32_t flags, cudaStream_t stream, const Shard& sh = Shard()) {
+    const bool fused = sh.pa.world > 1 || sh.best || sh.gated || sh.post.residual || sh.pre.gamma;
+    if (fused && (K / group) % 8 != 0) return 1;  // what the fused entries promise to take
+#define MIORI_GEMV(ROWS)                                                                                  \
+    if (M <= ROWS)                                                                                        \
+        return group == 64 ? launch_shape<Shape<BITS, 64, ROWS>>(q, s, b, x, y, N, K, M, flags, stream, sh) \
+                           : launch_shape<Shape<BITS, 32, ROWS>>(q, s, b, x, y, N, K, M, flags, stream, sh)
+    const bool slots = !(flags & MIORI_TUNE_GEMV_ALIGNED);
+    if (slots) MIORI_GEMV(1);
+    if (slots) MIORI_GEMV(2);
+    // three and four rows of 4-bit weights at group 64 gain nothing from slots (two, one step a pass): 16384 x
+    // 2048 takes 8.0 us with them and 7.2 without.  At group 32 one to four rows share an arithmetic order.
+    if (slots && !(BITS == 4 && group == 64)) MIORI_GEMV(4);
+    MIORI_GEMV(8);
+    MIORI_GEMV(16);
+    MIORI_GEMV(32);
+#undef MIORI_GEMV
+    return 1;
 }
 
 }  // namespace gemvtma

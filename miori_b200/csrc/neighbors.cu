@@ -1,7 +1,7 @@
 // The steps either side of a projection in the reference's decode graph (src/engine.cpp:389-413,
 // 484-502): RMSNorm in front of it, SiLU x up or post-norm + residual behind it, and the 8-bit
 // embedding gather that shares its table with the LM head.  Each is a small HBM- or latency-bound
-// kernel; the RMSNorm also exists fused into the GEMV's activation staging (gemv_umma.cuh).
+// kernel; the RMSNorm also exists fused into the GEMV's activation staging (gemv_tma.cuh).
 //   rmsnorm        shaders/ops.metal:86-115   y = bf16(x * rsqrt(mean(x^2) + eps) * w)
 //   silu_mul       shaders/ops.metal:129-139  out = bf16(g / (1 + exp(-g)) * up)
 //   post_norm_add  shaders/ops.metal:605-631  out = x + src * rsqrt(mean(src^2) + eps) * w

@@ -1,10 +1,7 @@
 // C ABI launch entries: argument validation, path selection, enqueue.
 #include "common.cuh"
 #include "dequant.cuh"
-#include "gemv_mma.cuh"
-#include "gemv_simt.cuh"
 #include "gemv_tma.cuh"
-#include "gemv_umma.cuh"
 #include "gemv_cache.cuh"
 
 using namespace miori_b200;
@@ -24,6 +21,27 @@ int check_quant_args(const char* op, const void* q, const void* s, const void* b
     return MIORI_OK;
 }
 
+// The GEMV for M rows, as many of them a launch as its shared memory holds: all 32 at K <= 2816, eight at
+// K = 8192.  A row's value depends on the rows of its launch only through their number's class.
+template <int BITS>
+int gemv_rows(const char* op, const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N,
+              uint32_t K, uint32_t M, uint32_t group, uint32_t flags, void* stream,
+              const gemvtma::Shard& sh = gemvtma::Shard()) {
+    const size_t x_row = (size_t)K * (sh.pre.gamma ? 4 : 2), y_row = (size_t)N * ((flags & MIORI_OUT_BF16) ? 2 : 4);
+    for (uint32_t rows = M;; rows = (rows + 1u) / 2u) {
+        uint32_t m0 = 0;
+        for (; m0 < M; m0 += rows) {
+            const int rc = gemvtma::try_launch<BITS>(q, s, b, static_cast<const uint8_t*>(x) + m0 * x_row,
+                                                     static_cast<uint8_t*>(y) + m0 * y_row, N, K, std::min(rows, M - m0),
+                                                     group, flags, (cudaStream_t)stream, sh);
+            if (rc < 0) return rc;
+            if (rc == 1) break;  // too many rows (the first launch of a size tells for all of them)
+        }
+        if (m0 >= M) return MIORI_OK;
+        if (rows == 1u) return fail(MIORI_E_INVALID, "%s: K=%u too large for the activation staging", op, K);
+    }
+}
+
 template <int BITS>
 int gemv_entry(const char* op, const void* q, const void* s, const void* b, const void* x, void* y,
                uint32_t N, uint32_t K, uint32_t M, uint32_t group, uint32_t flags, void* stream) {
@@ -32,36 +50,7 @@ int gemv_entry(const char* op, const void* q, const void* s, const void* b, cons
     if (!x || !y) return fail(MIORI_E_INVALID, "%s: null activation pointer", op);
     if (M == 0 || M > 32) return fail(MIORI_E_INVALID, "%s: M=%u outside 1..32", op, M);
     if (!aligned16(x)) return fail(MIORI_E_INVALID, "%s: x must be 16-byte aligned", op);
-    const bool force_exact = (flags & MIORI_GEMV_EXACT) != 0;
-    const bool force_simt = (flags & MIORI_TUNE_GEMV_SIMT) != 0;  // tuning override: shape-agnostic SIMT path
-    const bool no_bulk = (flags & MIORI_TUNE_GEMV_LDG) != 0;     // tuning override: register-streaming kernel
-    // The tcgen05 kernel (integer tensor cores, fp32 dequantization with an exact inner sum for
-    // every M).  By default it takes the 8-bit weights from three activation rows up: there the
-    // mma.sync kernel needs a second column set (M = 3, 4) or does not apply at all (M > 4 would
-    // fall to the multi-pass scalar kernel), and any batch wider than four rows when the caller
-    // asks for fp32 dequantization (MIORI_GEMV_EXACT), and long streams of 4-bit weights in groups
-    // of 64 (four 128-row tiles per SM and more, up to four activation rows), where it runs two
-    // CTAs per SM and measured 14-17 % faster (at group 32 it drains twice the accumulator columns
-    // and measured 7-30 % slower, so those stay on the mma.sync kernel).  Elsewhere the mma.sync kernel with its shorter
-    // pipeline measured faster and stays the default; MIORI_TUNE_GEMV_UMMA forces this one.
-    const bool long_stream4 = BITS == 4 && M <= 4 && group == 64 && (N + 127u) / 128u >= 4u * (uint32_t)sm_count();
-    const bool umma_default = (BITS == 8 && M >= 3) || (force_exact && M > 4) || long_stream4;
-    if (!force_simt && !no_bulk && !(flags & MIORI_TUNE_GEMV_MMASYNC) &&
-        (umma_default || (flags & MIORI_TUNE_GEMV_UMMA))) {
-        rc = gemvumma::try_launch<BITS>(q, s, b, x, y, N, K, M, group, flags, (cudaStream_t)stream);
-        if (rc <= 0) return rc;  // launched (0) or failed (<0); 1 = not eligible
-    }
-    if (!force_simt && !(force_exact && M > 4)) {
-        if (!no_bulk) {
-            rc = gemvtma::try_launch<BITS>(q, s, b, x, y, N, K, M, group, flags, (cudaStream_t)stream);
-            if (rc <= 0) return rc;  // launched (0) or failed (<0); 1 = not eligible
-        }
-        if (gemvmma::supported<BITS>(K, M, force_exact))
-            return gemvmma::launch<BITS>(q, s, b, x, y, N, K, M, group, flags, (cudaStream_t)stream);
-    }
-    if ((size_t)K * 2 * 4 > 200 * 1024)
-        return fail(MIORI_E_INVALID, "%s: K=%u too large for the activation staging", op, K);
-    return launch_gemv_simt<BITS>(q, s, b, x, y, N, K, M, group, flags, (cudaStream_t)stream);
+    return gemv_rows<BITS>(op, q, s, b, x, y, N, K, M, group, flags, stream);
 }
 
 }  // namespace
@@ -88,29 +77,13 @@ int gemv_rmsnorm_entry(const char* op, const void* q, const void* s, const void*
     if (!x || !y || !gamma) return fail(MIORI_E_INVALID, "%s: null activation, weight or output pointer", op);
     if (M == 0 || M > 32) return fail(MIORI_E_INVALID, "%s: M=%u outside 1..32", op, M);
     if (!aligned16(x) || !aligned16(gamma)) return fail(MIORI_E_INVALID, "%s: x and gamma must be 16-byte aligned", op);
-    // 4-bit weights, up to four rows, fp32 out, K within one slab: the TMA + mma.sync kernel with the norm
-    // in its staging pass (1.2-1.6 us faster than the pair of kernels; the tcgen05 kernel is slower than
-    // the pair there).  Longer rows and long streams go to the tcgen05 kernel (8192 -> 2048: 8.3 us
-    // against 10.3); the private flags force either.
-    if constexpr (BITS == 4) {
-        const bool long_stream = group == 64 && (N + 127u) / 128u >= 4u * (uint32_t)sm_count();
-        if (M <= 4 && !(flags & (MIORI_OUT_BF16 | MIORI_TUNE_GEMV_UMMA)) &&
-            ((!long_stream && K <= 2048u) || (flags & MIORI_TUNE_GEMV_MMASYNC))) {
-            gemvtma::Shard sh;
-            sh.pre.gamma = static_cast<const uint16_t*>(gamma);
-            sh.pre.eps = eps;
-            rc = gemvtma::try_launch<4>(q, s, b, x, y, N, K, M, group, flags, (cudaStream_t)stream, sh);
-            if (rc <= 0) return rc;  // launched (0) or failed (<0); 1 = not eligible: the tcgen05 kernel may be
-        }
-    }
-    gemvumma::Placement pl;
-    pl.gamma = gamma;
-    pl.eps = eps;
-    rc = gemvumma::try_launch<BITS>(q, s, b, x, y, N, K, M, group, flags, (cudaStream_t)stream, pl);
-    if (rc == 1)
+    if ((K / group) % 8 != 0)
         return fail(MIORI_E_INVALID, "%s: shape N=%u K=%u M=%u group=%u is outside the fused kernel's range "
                     "(run miori_rmsnorm and the plain GEMV instead)", op, N, K, M, group);
-    return rc;
+    gemvtma::Shard sh;
+    sh.pre.gamma = static_cast<const uint16_t*>(gamma);
+    sh.pre.eps = eps;
+    return gemv_rows<BITS>(op, q, s, b, x, y, N, K, M, group, flags, stream, sh);
 }
 }  // namespace
 
@@ -302,25 +275,3 @@ MIORI_API int miori_device_error_poll(void) {
          rec[1], rec[2], rec[3]);
     return (int)rec[0];
 }
-
-#ifdef MIORI_TMA_TRACE
-// Profiling build only: read and reset the TMA GEMV's %globaltimer marks.
-MIORI_API int miori_debug_tma_marks(unsigned long long* out4096) {
-    if (cudaMemcpyFromSymbol(out4096, gemvtma::g_tma_marks, 4096 * sizeof(unsigned long long)) != cudaSuccess) return -1;
-    if (cudaMemcpyFromSymbol(out4096 + 4096, gemvtma::g_tma_pmarks, 2048 * sizeof(unsigned long long)) != cudaSuccess) return -1;
-    const unsigned int zero[4] = {0, 0, 0, 0};
-    return cudaMemcpyToSymbol(gemvtma::g_tma_launch, zero, sizeof(zero)) == cudaSuccess ? 0 : -1;
-}
-#endif
-#ifdef MIORI_UMMA_TRACE
-// Profiling build only: read and clear the tcgen05 GEMV's cycle counters.
-MIORI_API int miori_debug_umma_trace(long long* out32) {
-    long long zero[32] = {};
-    if (cudaMemcpyFromSymbol(out32, gemvumma::g_umma_trace, sizeof(zero)) != cudaSuccess) return -1;
-    cudaMemcpyToSymbol(gemvumma::g_umma_trace, zero, sizeof(zero));
-    return 0;
-}
-MIORI_API int miori_debug_umma_events(unsigned int* out1024) {
-    return cudaMemcpyFromSymbol(out1024, gemvumma::g_umma_ev, 1024 * sizeof(unsigned int)) == cudaSuccess ? 0 : -1;
-}
-#endif

@@ -1,0 +1,73 @@
+"""The weight-streaming GEMV where it can go wrong: ragged rows (scales copied in part by hand), K that
+ends inside a step, a run or a slab, scale rows without a 16-byte pitch, groups that share a tile, every
+number-of-rows shape, more rows than one launch holds."""
+import numpy as np
+import pytest
+import torch
+
+import miori_b200
+from miori_b200 import synth
+from conftest import TOL_EXACT_PATH, assert_close, u16, u32
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+OPS = {4: miori_b200.gemv4, 8: miori_b200.gemv8}
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("N,K,group", [(1, 32, 32), (15, 64, 64), (33, 96, 32), (17, 160, 32), (100, 1440, 32), (70, 2112, 64),
+                                       (2500, 2048, 64), (40, 3456, 64), (31, 4128, 32), (700, 8192, 64), (48, 6144, 32),
+                                       (9473, 320, 64)])
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 9, 17])
+def test_edges(port, bits, N, K, group, M):
+    q, s, b = synth.make_weight(N, K, bits, group, seed=N + K + M)
+    x = synth.make_activation(M, K, seed=M)
+    guard = torch.full((M * N + 64,), 777.0, device=DEV)
+    y = guard[32:32 + M * N].view(M, N)
+    OPS[bits](q.to(DEV), s.to(DEV), b.to(DEV), x.to(DEV), group=group, out=y)
+    torch.cuda.synchronize()
+    want = port.gemv(bits, u32(q), u16(s), u16(b), u16(x), group)
+    assert_close(y.cpu().numpy(), want, rel_max=TOL_EXACT_PATH, what=f"gemv{bits} N={N} K={K} g={group} M={M}")
+    assert (guard[:32] == 777.0).all() and (guard[32 + M * N:] == 777.0).all()
+    assert miori_b200.lib.miori_device_error_poll() == 0
+
+
+@pytest.mark.parametrize("bits,group", [(4, 32), (4, 64), (8, 32), (8, 64)])
+def test_activation_range_per_group(port, bits, group):
+    """Activations are scaled to fp16 by their group's power of two: groups of very different size, zeros,
+    and a group with an outlier next to small values."""
+    N, K = 64, 1024
+    q, s, b = synth.make_weight(N, K, bits, group, seed=3)
+    x = synth.make_activation(2, K, seed=4).float()
+    scale = torch.exp2((torch.arange(K) // group % 5 - 2).float() * 12)
+    x = x * scale
+    x[0, :group] = 0.0
+    x[1, 5] = 3.0e4
+    x = x.to(torch.bfloat16)
+    want = port.gemv(bits, u32(q), u16(s), u16(b), u16(x), group)
+    got = OPS[bits](q.to(DEV), s.to(DEV), b.to(DEV), x.to(DEV), group=group).cpu().numpy()
+    assert_close(got, want, rel_max=TOL_EXACT_PATH, what="groups of different size")
+    for k in (-60, 90):
+        xs = (x.float() * 2.0 ** k).to(torch.bfloat16)
+        assert np.array_equal(OPS[bits](q.to(DEV), s.to(DEV), b.to(DEV), xs.to(DEV), group=group).cpu().numpy(),
+                              got * np.float32(2.0 ** k))
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+def test_rows_of_one_class_are_bit_identical(M):
+    N, K = 96, 4096
+    for bits, group in ((4, 32), (8, 32), (8, 64)):
+        q, s, b = (t.to(DEV) for t in synth.make_weight(N, K, bits, group, seed=bits))
+        x = synth.make_activation(4, K, seed=9, device=DEV)
+        full = OPS[bits](q, s, b, x, group=group)
+        assert torch.equal(OPS[bits](q, s, b, x[:M].contiguous(), group=group), full[:M])
+
+
+@pytest.mark.parametrize("M,K", [(32, 8192), (13, 16384), (5, 24576)])
+def test_more_rows_than_a_launch_holds(port, M, K):
+    N = 40
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=K)
+    x = synth.make_activation(M, K, seed=M)
+    want = port.gemv(4, u32(q), u16(s), u16(b), u16(x), 64)
+    got = miori_b200.gemv4(q.to(DEV), s.to(DEV), b.to(DEV), x.to(DEV), group=64, flags=miori_b200.LAUNCH_PDL).cpu().numpy()
+    assert_close(got, want, rel_max=TOL_EXACT_PATH, what=f"M={M} K={K}")
