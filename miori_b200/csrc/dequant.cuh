@@ -2,52 +2,70 @@
 // exactly as the reference does (src/cpu_ref.h:16-23,33,44): an fp32 multiply, an fp32 add
 // (kept unfused so that overflow behaves identically) and the integer RNE to bf16.
 //
-// HBM-bound: 0.5625-1.125 B read and 2 B written per weight.  One thread converts eight
-// consecutive weights of a row (one or two packed words) and stores them as one 16-byte
-// vector, so every warp reads 128/256 contiguous bytes and writes 512.
+// Bound by HBM: 0.5625-1.125 B read and 2 B written per weight.  Rows follow one another without gaps and
+// hold whole scale groups, so the tensor is one array: unit i is eight weights, its scale is number
+// 8 i / group, and no row or column is ever computed.  A thread takes UNITS units one block width apart:
+// every load and store instruction of a warp covers contiguous memory (128-256 bytes of codes, 512 of
+// output), and all loads are issued before the first use.  (With a 64-bit division per unit and one unit
+// in flight 16384 x 2048 took 28 us: DEQUANT_NOW)
 #pragma once
 #include "common.cuh"
 
 namespace miori_b200 {
 
+// eight weights of one group -> eight bf16
 template <int BITS>
-__global__ void __launch_bounds__(256)
-dequant_rowmajor_kernel(const uint32_t* __restrict__ q, const uint16_t* __restrict__ s,
-                        const uint16_t* __restrict__ b, uint4* __restrict__ out, uint32_t N,
-                        uint32_t K, uint32_t gshift) {
-    const uint64_t units = (uint64_t)N * (K >> 3);  // 8 weights per unit
-    const uint32_t upr = K >> 3;                    // units per row
-    const uint32_t ng = K >> gshift;
+__device__ __forceinline__ uint4 dequant_unit(const uint32_t (&w)[BITS / 4], uint32_t sbits, uint32_t bbits) {
+    const float sc = bf16_bits_to_float(sbits), bi = bf16_bits_to_float(bbits);
+    float f[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        // byte k of a register into the low byte of 2^23: 2^23 + code, exactly
+        const uint32_t by = BITS == 8 ? w[BITS == 8 ? j >> 2 : 0] : (j & 1) ? (w[0] >> 4) & 0x0F0F0F0Fu : w[0] & 0x0F0F0F0Fu;
+        const int k = BITS == 8 ? j & 3 : j >> 1;
+        const float q = __uint_as_float(__byte_perm(by, 0x4B000000u, 0x7440 + k)) - 8388608.0f;
+        f[j] = __fadd_rn(__fmul_rn(q, sc), bi);
+    }
+    uint32_t o[4];
+    if ((sbits & 0x7F80u) != 0x7F80u && (bbits & 0x7F80u) != 0x7F80u) {
+        // finite scale and bias: no NaN can arise, and the conversion instruction rounds by the same rule
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[p]) : "f"(f[2 * p + 1]), "f"(f[2 * p]));
+    } else {
+#pragma unroll
+        for (int p = 0; p < 4; ++p) o[p] = float_to_bf16_bits(f[2 * p]) | (float_to_bf16_bits(f[2 * p + 1]) << 16);
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+constexpr int DEQUANT_THREADS = 256;
+
+template <int BITS, int UNITS>
+__global__ void __launch_bounds__(DEQUANT_THREADS)
+dequant_rowmajor_kernel(const uint32_t* __restrict__ q, const uint16_t* __restrict__ s, const uint16_t* __restrict__ b,
+                        uint4* __restrict__ out, uint64_t units, uint32_t ushift) {
     pdl_launch_dependents();
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < units;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t row = (uint32_t)(i / upr), u = (uint32_t)(i - (uint64_t)row * upr);
-        const uint32_t g = (u << 3) >> gshift;
-        const float sc = bf16_bits_to_float(__ldg(s + (size_t)row * ng + g));
-        const float bi = bf16_bits_to_float(__ldg(b + (size_t)row * ng + g));
-        uint32_t code[8];
-        if (BITS == 4) {
-            const uint32_t w = __ldg(q + i);
+    const uint64_t first = (uint64_t)blockIdx.x * (DEQUANT_THREADS * UNITS) + threadIdx.x;
+    uint32_t w[UNITS][BITS / 4], sc[UNITS], bi[UNITS];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) code[j] = (w >> (4 * j)) & 0xFu;
-        } else {
-            const uint2 w = __ldg(reinterpret_cast<const uint2*>(q) + i);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                code[j] = (w.x >> (8 * j)) & 0xFFu;
-                code[4 + j] = (w.y >> (8 * j)) & 0xFFu;
+    for (int j = 0; j < UNITS; ++j) {
+        const uint64_t i = first + (uint64_t)(j * DEQUANT_THREADS);
+        if (i < units) {
+            if constexpr (BITS == 4) {
+                w[j][0] = __ldcs(q + i);
+            } else {
+                const uint2 v = __ldcs(reinterpret_cast<const uint2*>(q) + i);
+                w[j][0] = v.x, w[j][1] = v.y;
             }
+            sc[j] = __ldg(s + (i >> ushift));
+            bi[j] = __ldg(b + (i >> ushift));
         }
-        uint32_t o[4];
+    }
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const float q0 = __uint_as_float(0x4B000000u | code[2 * p]) - 8388608.0f;
-            const float q1 = __uint_as_float(0x4B000000u | code[2 * p + 1]) - 8388608.0f;
-            const float f0 = __fadd_rn(__fmul_rn(q0, sc), bi);
-            const float f1 = __fadd_rn(__fmul_rn(q1, sc), bi);
-            o[p] = float_to_bf16_bits(f0) | (float_to_bf16_bits(f1) << 16);
-        }
-        out[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    for (int j = 0; j < UNITS; ++j) {
+        const uint64_t i = first + (uint64_t)(j * DEQUANT_THREADS);
+        if (i < units) out[i] = dequant_unit<BITS>(w[j], sc[j], bi[j]);
     }
 }
 
@@ -55,15 +73,15 @@ template <int BITS>
 int launch_dequant_rowmajor(const void* q, const void* s, const void* b, void* out, uint32_t N,
                             uint32_t K, uint32_t group, cudaStream_t stream) {
     const uint64_t units = (uint64_t)N * (K >> 3);
-    uint64_t blocks = (units + 255) / 256;
-    const uint64_t cap = (uint64_t)sm_count() * 32;
-    if (blocks > cap) blocks = cap;
-    if (blocks == 0) blocks = 1;
-    cudaError_t e = launch(dequant_rowmajor_kernel<BITS>, dim3((unsigned)blocks), dim3(256), 0,
-                           stream, false, reinterpret_cast<const uint32_t*>(q),
-                           reinterpret_cast<const uint16_t*>(s),
-                           reinterpret_cast<const uint16_t*>(b), reinterpret_cast<uint4*>(out), N,
-                           K, group == 32 ? 5u : 6u);
+    const uint32_t ushift = group == 32 ? 2u : 3u;  // log2 of the units per scale group
+    // four units per thread, or one while that leaves SMs without a block
+    const bool wide = units >= (uint64_t)sm_count() * DEQUANT_THREADS * 8u;
+    const uint64_t per_block = (uint64_t)DEQUANT_THREADS * (wide ? 4u : 1u), blocks = (units + per_block - 1u) / per_block;
+    if (blocks > 0x7FFFFFFFull) return fail(MIORI_E_INVALID, "dequant: N=%u K=%u is too large", N, K);
+    auto kern = wide ? dequant_rowmajor_kernel<BITS, 4> : dequant_rowmajor_kernel<BITS, 1>;
+    cudaError_t e = launch(kern, dim3((unsigned)blocks), dim3(DEQUANT_THREADS), 0, stream, false,
+                           reinterpret_cast<const uint32_t*>(q), reinterpret_cast<const uint16_t*>(s),
+                           reinterpret_cast<const uint16_t*>(b), reinterpret_cast<uint4*>(out), units, ushift);
     if (e != cudaSuccess) return cuda_fail(e, "dequant_rowmajor launch");
     return MIORI_OK;
 }

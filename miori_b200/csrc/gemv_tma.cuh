@@ -393,6 +393,7 @@ struct PostNorm {
     const uint16_t* gamma = nullptr;   // bf16 [N]
     unsigned int* arrivals = nullptr;  // one zeroed word; the kernel leaves it zero
     float eps = 0.0f;
+    bool vec = false;                  // neighbors::norm_vec
 };
 
 // What the norm prologue needs (null gamma: off): x then points at fp32 activations.
@@ -935,12 +936,8 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             float* out = reinterpret_cast<float*>(A.y);
             for (uint32_t m = 0; m < M; ++m) {
                 const size_t at = (size_t)m * N;
-                if (N <= 8u * (uint32_t)neighbors::NORM_THREADS)
-                    neighbors::post_norm_add_row_regs<9, true, 8>(A.post.residual + at, out + at, A.post.gamma, out + at, N,
-                                                                  A.post.eps, pn_part);
-                else
-                    neighbors::post_norm_add_row<9, true>(A.post.residual + at, out + at, A.post.gamma, out + at, N,
-                                                          A.post.eps, pn_part);
+                neighbors::post_norm_add_any<9, true>(A.post.residual + at, out + at, A.post.gamma, out + at, N, A.post.eps,
+                                                      pn_part, A.post.vec);
                 neighbors::norm_sync<9>();  // pn_part is reused by the next row
             }
             if (threadIdx.x == 0) *A.post.arrivals = 0u;  // ready for the next launch

@@ -8,41 +8,61 @@
 //   embed8         shaders/ops.metal:170-197  out[t][k] = bf16(code * scale + bias) of row tokens[t]
 #include "common.cuh"
 #include "norm.cuh"
+#include "peers.cuh"
 
 namespace miori_b200 {
 namespace neighbors {
 
+// PIECES > 0: rows of at most 4 * NORM_THREADS * PIECES elements in 16-byte pieces, read once (norm.cuh).
+template <int PIECES>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, uint16_t* __restrict__ y,
                uint32_t n, float eps) {
     __shared__ float part[NORM_THREADS / 32];
     pdl_launch_dependents();
-    pdl_wait_prior();
     const float* row = x + (size_t)blockIdx.x * n;
-    const float inv = rsqrtf(row_sum_squares<0, false>(row, n, part) / (float)n + eps);
-    for (uint32_t i = threadIdx.x; i < n; i += NORM_THREADS)
-        y[(size_t)blockIdx.x * n + i] = (uint16_t)float_to_bf16_bits(row[i] * inv * bf16_bits_to_float(w[i]));
+    uint16_t* to = y + (size_t)blockIdx.x * n;
+    if constexpr (PIECES > 0) {
+        rmsnorm_row_vec<PIECES>(row, w, to, n, eps, part);
+    } else {
+        pdl_wait_prior();
+        const float inv = rsqrtf(row_sum_squares<0, false>(row, n, part) / (float)n + eps);
+        for (uint32_t i = threadIdx.x; i < n; i += NORM_THREADS)
+            to[i] = (uint16_t)float_to_bf16_bits(row[i] * inv * bf16_bits_to_float(w[i]));
+    }
 }
 
 __global__ void __launch_bounds__(NORM_THREADS)
 post_norm_add_kernel(const float* __restrict__ x, const float* __restrict__ src,
-                     const uint16_t* __restrict__ w, float* __restrict__ out, uint32_t n, float eps) {
+                     const uint16_t* __restrict__ w, float* __restrict__ out, uint32_t n, float eps, bool vec) {
     __shared__ float part[NORM_THREADS / 32];
     pdl_launch_dependents();
     pdl_wait_prior();
     const size_t at = (size_t)blockIdx.x * n;
-    post_norm_add_row<0, false>(x + at, src + at, w, out + at, n, eps, part);
+    post_norm_add_any<0, false>(x + at, src + at, w, out + at, n, eps, part, vec);
 }
 
+__device__ __forceinline__ uint32_t silu_mul_bits(float g, float u) {
+    const float s = g / (1.0f + expf(-g));
+    return float_to_bf16_bits(s * u);
+}
+// HBM-bound (8 B read, 2 B written per element): four elements per thread and 16-byte loads where the
+// pointers allow it (1024 x 8192: SILU_NOW).
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const float* __restrict__ gate, const float* __restrict__ up, uint16_t* __restrict__ out,
                 size_t n) {
     pdl_launch_dependents();
     pdl_wait_prior();
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float g = gate[i];
-        const float s = g / (1.0f + expf(-g));
-        out[i] = (uint16_t)float_to_bf16_bits(s * up[i]);
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+    if constexpr (VEC) {
+        for (size_t i = first; i < n / 4u; i += stride) {
+            const float4 g = reinterpret_cast<const float4*>(gate)[i], u = reinterpret_cast<const float4*>(up)[i];
+            reinterpret_cast<uint2*>(out)[i] =
+                make_uint2(silu_mul_bits(g.x, u.x) | (silu_mul_bits(g.y, u.y) << 16), silu_mul_bits(g.z, u.z) | (silu_mul_bits(g.w, u.w) << 16));
+        }
+    } else {
+        for (size_t i = first; i < n; i += stride) out[i] = (uint16_t)silu_mul_bits(gate[i], up[i]);
     }
 }
 
@@ -85,13 +105,27 @@ embed8_kernel(const uint4* __restrict__ q, const uint16_t* __restrict__ s, const
 // src/engine.cpp:740-747 finds it).  A thread-block cluster of up to 8 CTAs shares the vector:
 // 16-byte loads, a shuffle and shared-memory reduction per CTA, then every CTA hands its
 // candidate to CTA 0 through distributed shared memory and CTA 0's first thread holds the result.
+//
+// A candidate is one 64-bit key, value above inverted index, in an order that integers compare: one compare
+// per element and one shuffle pair per reduction step.  (What a call costs is latency: the first form had
+// every thread walk the 32 warps' candidates one after the other.)
 struct Best {
     float v;
     uint32_t i;
 };
 constexpr int ARGMAX_THREADS = 1024, ARGMAX_CLUSTER = 8;
-__device__ __forceinline__ Best better(Best a, Best b) {
-    return (b.v > a.v || (b.v == a.v && b.i < a.i)) ? b : a;
+__device__ __forceinline__ unsigned long long best_key(float v, uint32_t i) {
+    return v == v ? peer_best_key(__float_as_uint(v == 0.0f ? 0.0f : v), i) : 0ull;  // the zeros are equal
+}
+__device__ __forceinline__ Best best_of_key(unsigned long long k) {
+    const PeerBest b = peer_best_from_key(k);
+    return Best{b.v, b.i};
+}
+__device__ __forceinline__ unsigned long long key_max(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
+__device__ __forceinline__ unsigned long long warp_key_max(unsigned long long k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) k = key_max(k, __shfl_xor_sync(0xFFFFFFFFu, k, o));
+    return k;
 }
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
@@ -103,85 +137,76 @@ __device__ __forceinline__ uint32_t cluster_nctarank() {
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
     return r;
 }
-// This CTA's best over its slice of v[0, n): elements are compared in index order inside a thread
-// and ties across threads go to the lower index, so the result is the first maximum.
+// This CTA's best over its slice of v[0, n), in thread 0.  Ties go to the lower index.
 template <bool BF16>
-__device__ __forceinline__ Best block_argmax(const void* __restrict__ v, uint32_t n, uint32_t index0,
-                                             Best* warp_best) {
+__device__ __forceinline__ unsigned long long block_argmax(const void* __restrict__ v, uint32_t n, uint32_t index0,
+                                                           unsigned long long* warp_best) {
     constexpr uint32_t PER = BF16 ? 8u : 4u;  // elements per 16-byte load
     const uint32_t nct = cluster_nctarank(), cr = cluster_ctarank();
     // slices of whole 16-byte pieces; the last CTA also takes the ragged tail
     const uint32_t pieces = n / PER, per_cta = (pieces + nct - 1u) / nct;
     const uint32_t p0 = min(cr * per_cta, pieces), p1 = min(p0 + per_cta, pieces);
-    Best me = {-INFINITY, 0xFFFFFFFFu};
+    // a thread compares floats (first of equals, in index order) and makes one key at the end
+    float bv = -INFINITY;
+    uint32_t bi = 0xFFFFFFFFu;
+    auto see = [&](float f, uint32_t i) {
+        if (f > bv || (f == bv && i < bi)) bv = f, bi = i;
+    };
     const bool vec_ok = (reinterpret_cast<uintptr_t>(v) & 15u) == 0;
     if (vec_ok) {
         const uint4* v4 = static_cast<const uint4*>(v);
-        for (uint32_t p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
+#pragma unroll 2
+        for (uint32_t p = p0 + threadIdx.x; p < p1; p += ARGMAX_THREADS) {
             const uint4 w = __ldg(v4 + p);
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
             const uint32_t i0 = index0 + p * PER;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if (BF16) {
-                    me = better(me, Best{bf16lo(ww[k]), i0 + 2u * k});
-                    me = better(me, Best{bf16hi(ww[k]), i0 + 2u * k + 1u});
+                    see(bf16lo(ww[k]), i0 + 2u * k);
+                    see(bf16hi(ww[k]), i0 + 2u * k + 1u);
                 } else {
-                    me = better(me, Best{__uint_as_float(ww[k]), i0 + (uint32_t)k});
+                    see(__uint_as_float(ww[k]), i0 + (uint32_t)k);
                 }
             }
         }
     }
-    // scalar part: everything when v is not 16-byte aligned (CTA 0 of the cluster walks it all),
-    // else the tail past the last whole piece (last CTA)
-    uint32_t s0 = n, s1 = n;
-    if (!vec_ok) { if (cr == 0u) s0 = 0u; }
-    else if (cr == nct - 1u) s0 = pieces * PER;
-    for (uint32_t i = s0 + threadIdx.x; i < s1; i += blockDim.x) {
-        const float f = BF16 ? bf16_bits_to_float(static_cast<const uint16_t*>(v)[i])
-                             : static_cast<const float*>(v)[i];
-        me = better(me, Best{f, index0 + i});
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        Best other;
-        other.v = __shfl_xor_sync(0xFFFFFFFFu, me.v, o);
-        other.i = __shfl_xor_sync(0xFFFFFFFFu, me.i, o);
-        me = better(me, other);
-    }
-    if ((threadIdx.x & 31u) == 0) warp_best[threadIdx.x >> 5] = me;
+    // scalar part: everything when v is not 16-byte aligned (dealt to the CTAs), else the tail past the last
+    // whole piece (last CTA)
+    uint32_t s0 = n, step = ARGMAX_THREADS;
+    if (!vec_ok) s0 = cr * ARGMAX_THREADS + threadIdx.x, step = nct * ARGMAX_THREADS;
+    else if (cr == nct - 1u) s0 = pieces * PER + threadIdx.x;
+    for (uint32_t i = s0; i < n; i += step)
+        see(BF16 ? bf16_bits_to_float(static_cast<const uint16_t*>(v)[i]) : static_cast<const float*>(v)[i], index0 + i);
+    const unsigned long long mine = warp_key_max(bi == 0xFFFFFFFFu ? 0ull : best_key(bv, bi));
+    if ((threadIdx.x & 31u) == 0) warp_best[threadIdx.x >> 5] = mine;
     __syncthreads();
-    Best all = warp_best[0];
-    for (uint32_t w = 1; w < blockDim.x / 32u; ++w) all = better(all, warp_best[w]);
-    return all;
+    return threadIdx.x < 32u ? warp_key_max(warp_best[threadIdx.x]) : 0ull;
 }
 // Cluster-wide result, valid in thread 0 of CTA 0 of the cluster.  Every thread of every CTA of
 // the cluster must call it (it contains cluster barriers).  cta_best: ARGMAX_CLUSTER entries of
 // shared memory, at the same offset in every CTA.
 template <bool BF16>
 __device__ __forceinline__ Best cluster_argmax(const void* __restrict__ v, uint32_t n, uint32_t index0,
-                                               Best* warp_best, Best* cta_best) {
-    const Best mine = block_argmax<BF16>(v, n, index0, warp_best);
+                                               unsigned long long* warp_best, unsigned long long* cta_best) {
+    unsigned long long mine = block_argmax<BF16>(v, n, index0, warp_best);
     const uint32_t nct = cluster_nctarank(), cr = cluster_ctarank();
-    if (nct == 1u) return mine;
+    if (nct == 1u) return best_of_key(mine);
     if (threadIdx.x == 0) {
         uint32_t remote;  // cta_best[cr] in CTA 0's shared memory
         asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(smem_addr(cta_best + cr)));
-        asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(remote), "r"(__float_as_uint(mine.v)), "r"(mine.i)
-                     : "memory");
+        asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(mine) : "memory");
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    Best all = mine;
     if (cr == 0u && threadIdx.x == 0)
-        for (uint32_t c = 1; c < nct; ++c) all = better(all, cta_best[c]);
-    return all;
+        for (uint32_t c = 1; c < nct; ++c) mine = key_max(mine, cta_best[c]);
+    return best_of_key(mine);
 }
 template <bool BF16>
 __global__ void __launch_bounds__(ARGMAX_THREADS)
 argmax_kernel(const void* __restrict__ v, uint32_t n, uint32_t index0, uint32_t* __restrict__ out_index,
               float* __restrict__ out_value) {
-    __shared__ Best warp_best[32];
-    __shared__ __align__(8) Best cta_best[ARGMAX_CLUSTER];
+    __shared__ unsigned long long warp_best[ARGMAX_THREADS / 32], cta_best[ARGMAX_CLUSTER];
     pdl_launch_dependents();
     pdl_wait_prior();
     const Best all = cluster_argmax<BF16>(v, n, index0, warp_best, cta_best);
@@ -229,7 +254,9 @@ MIORI_API int miori_rmsnorm(const void* x, const void* gamma, void* y, uint32_t 
                             uint32_t flags, void* stream) {
     if (!x || !gamma || !y) return fail(MIORI_E_INVALID, "miori_rmsnorm: null pointer");
     if (rows == 0 || n == 0) return fail(MIORI_E_INVALID, "miori_rmsnorm: empty shape rows=%u n=%u", rows, n);
-    const cudaError_t e = launch(neighbors::rmsnorm_kernel, dim3(rows), dim3(neighbors::NORM_THREADS), 0,
+    const bool vec = n % 4u == 0u && aligned16(x) && (reinterpret_cast<uintptr_t>(gamma) & 7u) == 0 && (reinterpret_cast<uintptr_t>(y) & 7u) == 0;
+    auto kern = !vec || n > 8192u ? neighbors::rmsnorm_kernel<0> : n <= 2048u ? neighbors::rmsnorm_kernel<2> : neighbors::rmsnorm_kernel<8>;
+    const cudaError_t e = launch(kern, dim3(rows), dim3(neighbors::NORM_THREADS), 0,
                                  (cudaStream_t)stream, (flags & MIORI_LAUNCH_PDL) != 0,
                                  static_cast<const float*>(x), static_cast<const uint16_t*>(gamma),
                                  static_cast<uint16_t*>(y), n, eps);
@@ -244,7 +271,8 @@ MIORI_API int miori_post_norm_add(const void* x, const void* src, const void* ga
     const cudaError_t e = launch(neighbors::post_norm_add_kernel, dim3(rows), dim3(neighbors::NORM_THREADS), 0,
                                  (cudaStream_t)stream, (flags & MIORI_LAUNCH_PDL) != 0,
                                  static_cast<const float*>(x), static_cast<const float*>(src),
-                                 static_cast<const uint16_t*>(gamma), static_cast<float*>(out), n, eps);
+                                 static_cast<const uint16_t*>(gamma), static_cast<float*>(out), n, eps,
+                                 neighbors::norm_vec(n, x, src, out, gamma));
     if (e != cudaSuccess) return cuda_fail(e, "miori_post_norm_add launch");
     return MIORI_OK;
 }
@@ -252,8 +280,9 @@ MIORI_API int miori_post_norm_add(const void* x, const void* src, const void* ga
 MIORI_API int miori_silu_mul(const void* gate, const void* up, void* out, size_t n, uint32_t flags, void* stream) {
     if (!gate || !up || !out) return fail(MIORI_E_INVALID, "miori_silu_mul: null pointer");
     if (n == 0) return fail(MIORI_E_INVALID, "miori_silu_mul: empty vector");
-    const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 8);
-    const cudaError_t e = launch(neighbors::silu_mul_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream,
+    const bool vec = n % 4u == 0u && aligned16(gate) && aligned16(up) && (reinterpret_cast<uintptr_t>(out) & 7u) == 0;
+    const unsigned blocks = (unsigned)std::min<size_t>((n / (vec ? 4u : 1u) + 255) / 256, (size_t)sm_count() * 16);
+    const cudaError_t e = launch(vec ? neighbors::silu_mul_kernel<true> : neighbors::silu_mul_kernel<false>, dim3(blocks), dim3(256), 0, (cudaStream_t)stream,
                                  (flags & MIORI_LAUNCH_PDL) != 0, static_cast<const float*>(gate),
                                  static_cast<const float*>(up), static_cast<uint16_t*>(out), n);
     if (e != cudaSuccess) return cuda_fail(e, "miori_silu_mul launch");

@@ -146,6 +146,7 @@ MIORI_API int miori_gemv4_post_norm_add(const void* q, const void* s, const void
     sh.post.gamma = static_cast<const uint16_t*>(gamma);
     sh.post.arrivals = static_cast<unsigned int*>(counter);
     sh.post.eps = eps;
+    sh.post.vec = neighbors::norm_vec(N, residual, out, out, gamma);
     rc = gemvtma::try_launch<4>(q, s, b, x, out, N, K, M, group, flags, (cudaStream_t)stream, sh);
     if (rc == 1)
         return fail(MIORI_E_INVALID, "%s: shape N=%u K=%u M=%u group=%u is outside the fused kernel's range "

@@ -64,8 +64,7 @@ template <bool BF16>
 __global__ void __launch_bounds__(1024)
 argmax_allreduce_kernel(const PeerArgs pa, const void* __restrict__ v, uint32_t n_local, uint32_t index0,
                         size_t y_off) {
-    __shared__ neighbors::Best warp_best[32];
-    __shared__ __align__(8) neighbors::Best cta_best[neighbors::ARGMAX_CLUSTER];
+    __shared__ unsigned long long warp_best[neighbors::ARGMAX_THREADS / 32], cta_best[neighbors::ARGMAX_CLUSTER];
     pdl_launch_dependents();
     pdl_wait_prior();
     const neighbors::Best mine = neighbors::cluster_argmax<BF16>(v, n_local, index0, warp_best, cta_best);
