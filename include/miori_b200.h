@@ -147,11 +147,13 @@ int miori_gemm_plan(uint32_t M, uint32_t N, uint32_t K, size_t workspace_bytes, 
                     uint32_t* ctas_per_tile, uint32_t* splits);
 /* Same product with a caller-provided scratch area that lets problems with few output tiles
  * (small M or N, long K) split K across SMs: partial tiles go to `workspace` (fp32) and a
- * second kernel sums them in a fixed order, so results stay reproducible and independent of
- * M.  miori_gemm_workspace_bytes gives the size worth passing (0: the shape does not
- * split); a smaller or NULL workspace only reduces or disables the splitting.  The workspace
- * contents are scratch; two launches in flight at once must not share it.  (The reference
- * has no counterpart: its GEMM is a library call, shaders/gemm_mpp.metal:47-53.) */
+ * second kernel sums them in a fixed order, so results stay reproducible.  (Up to 48 rows the
+ * slices are the CTAs of a cluster, their number depends on N and K only, and the partials meet
+ * on the chip: the workspace is then the permission to split, and is not written.)
+ * miori_gemm_workspace_bytes gives the size worth passing (0: the shape does not split); a
+ * smaller or NULL workspace only reduces or disables the splitting.  The workspace
+ * contents are scratch; two launches in flight at once must not share it.  (The reference has no
+ * counterpart: its GEMM is a library call, shaders/gemm_mpp.metal:47-53.) */
 size_t miori_gemm_workspace_bytes(uint32_t M, uint32_t N, uint32_t K);
 int miori_gemm_bf16_cache_ws(const void* A, const void* cache, void* C, uint32_t M, uint32_t N,
                              uint32_t K, uint32_t flags, void* workspace, size_t workspace_bytes,

@@ -315,7 +315,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty_bar(acc));
         }
-        if (lane == 0) tma_store_wait_all();  // stores complete before shared memory goes away
+        if (lane == 0) tma_store_wait_read<0>();  // shared memory is read; the writes are the grid's to complete
     }
 
     // teardown: on abort give in-flight copies and MMAs time to land before freeing TMEM
@@ -544,7 +544,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
             __syncwarp();
             if (lane == 0) mbar_arrive_leader(tempty_bar(acc));
         }
-        if (lane == 0) tma_store_wait_all();
+        if (lane == 0) tma_store_wait_read<0>();
     }
 
     __syncwarp();
@@ -565,8 +565,9 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
 }  // namespace pair
 
-// Sum the split-K partials in slice order (deterministic) and write C as fp32 or bf16.
-template <bool OUT_BF16>
+// Sum the split-K partials in slice order (deterministic) and write C as fp32 or bf16.  All slices of an
+// element are loaded before the first is added (at most MAX_SPLITS of them): this kernel is one trip to L2.
+template <bool OUT_BF16, int MAX_SPLITS>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float4* __restrict__ ws, void* __restrict__ Cout, size_t quads,
                      uint32_t splits) {
@@ -574,11 +575,14 @@ splitk_reduce_kernel(const float4* __restrict__ ws, void* __restrict__ Cout, siz
     pdl_wait_prior();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < quads;
          i += (size_t)gridDim.x * blockDim.x) {
-        float4 a = ws[i];
-        for (uint32_t s = 1; s < splits; ++s) {
-            const float4 b = ws[(size_t)s * quads + i];
-            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-        }
+        float4 v[MAX_SPLITS];
+#pragma unroll
+        for (uint32_t s = 0; s < (uint32_t)MAX_SPLITS; ++s)
+            if (s < splits) v[s] = __ldcg(ws + (size_t)s * quads + i);
+        float4 a = v[0];
+#pragma unroll
+        for (uint32_t s = 1; s < (uint32_t)MAX_SPLITS; ++s)
+            if (s < splits) a.x += v[s].x, a.y += v[s].y, a.z += v[s].z, a.w += v[s].w;
         if (OUT_BF16) {
             uint2 o;
             o.x = float_to_bf16_bits(a.x) | (float_to_bf16_bits(a.y) << 16);
@@ -616,6 +620,8 @@ static int make_tmap_out(CUtensorMap* map, void* Cm, float* ws, uint32_t M, uint
     return make_tmap_3d(map, Cm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, N, M, 1, 32, 32,
                         CU_TENSOR_MAP_SWIZZLE_128B, ldc);
 }
+
+#include "gemm_skinny.cuh"
 
 // Launch the two-CTA kernel: clusters of 2, one pair per SM pair.
 static int launch_gemm_pair(const void* A, const void* Bc, void* Cm, uint32_t M, uint32_t N,
@@ -666,13 +672,11 @@ static int launch_reduce(void* Cm, uint32_t M, uint32_t N, uint32_t flags, float
     const bool bf16 = (flags & MIORI_OUT_BF16) != 0, pdl = (flags & MIORI_LAUNCH_PDL) != 0;
     const size_t quads = (size_t)M * N / 4;
     const unsigned blocks = (unsigned)std::min<size_t>((quads + 255) / 256, (size_t)sm_count() * 8);
-    cudaError_t e;
-    if (bf16)
-        e = launch(splitk_reduce_kernel<true>, dim3(blocks), dim3(256), 0, stream, pdl,
-                   reinterpret_cast<const float4*>(ws), Cm, quads, splits);
-    else
-        e = launch(splitk_reduce_kernel<false>, dim3(blocks), dim3(256), 0, stream, pdl,
-                   reinterpret_cast<const float4*>(ws), Cm, quads, splits);
+    auto kern = splits <= 2   ? (bf16 ? splitk_reduce_kernel<true, 2> : splitk_reduce_kernel<false, 2>)
+                : splits <= 4 ? (bf16 ? splitk_reduce_kernel<true, 4> : splitk_reduce_kernel<false, 4>)
+                : splits <= 8 ? (bf16 ? splitk_reduce_kernel<true, 8> : splitk_reduce_kernel<false, 8>)
+                              : (bf16 ? splitk_reduce_kernel<true, 16> : splitk_reduce_kernel<false, 16>);
+    const cudaError_t e = launch(kern, dim3(blocks), dim3(256), 0, stream, pdl, reinterpret_cast<const float4*>(ws), Cm, quads, splits);
     if (e != cudaSuccess) return cuda_fail(e, "splitk_reduce launch");
     return MIORI_OK;
 }
@@ -851,6 +855,10 @@ MIORI_API int miori_gemm_bf16_cache_ws(const void* A, const void* cache, void* C
     if (rc) return rc;
     if (workspace && !aligned16(workspace))
         return fail(MIORI_E_INVALID, "miori_gemm_bf16_cache: workspace must be 16-byte aligned");
+    if (!(flags & MIORI_TUNE_GEMM_MASK)) {
+        const uint32_t cs = gemm::skinny::plan(M, N, K, workspace != nullptr);
+        if (cs) return gemm::skinny::launch_skinny(A, cache, Cm, M, N, K, flags, cs, (cudaStream_t)stream);
+    }
     const gemm::GemmPlan p = gemm::plan_gemm(M, N, K, flags, workspace ? workspace_bytes : 0);
     float* ws = reinterpret_cast<float*>(workspace);
     return gemm::run_plan(p, A, cache, Cm, M, N, K, flags, ws, (cudaStream_t)stream);
@@ -874,8 +882,8 @@ MIORI_API int miori_gemm_bf16_strided(const void* A, uint32_t lda, const void* B
     const bool bf16 = (flags & MIORI_OUT_BF16) != 0, pdl = (flags & MIORI_LAUNCH_PDL) != 0;
     const uint32_t csz = bf16 ? 2 : 4;
     // what the TMA descriptors can express: 16-byte aligned bases and row pitches
-    const bool tma_ok = aligned16(A) && aligned16(B) && aligned16(Cm) && lda % 8 == 0 && ldb % 8 == 0 &&
-                        ((size_t)ldc * csz) % 16 == 0;
+    const bool rows_ok = aligned16(A) && aligned16(B) && lda % 8 == 0 && ldb % 8 == 0;
+    const bool tma_ok = rows_ok && aligned16(Cm) && ((size_t)ldc * csz) % 16 == 0;
     // TMA stores clip at 16-byte granularity, so the tensor-core kernels take the columns up to
     // the last multiple of 16 bytes and the plain kernel the few that remain
     uint32_t n_done = 0;
@@ -953,6 +961,10 @@ MIORI_API int miori_gemm_bf16_cache_static(const void* A, const void* cache, voi
                     "without a K split and without scratch (miori_gemm_bf16_cache_ws splits it given a "
                     "caller workspace)",
                     M, N, K, need, want.splits, kStaticScratchBytes);
+    if (!(flags & MIORI_TUNE_GEMM_MASK)) {
+        const uint32_t cs = gemm::skinny::plan(M, N, K, true);
+        if (cs) return gemm::skinny::launch_skinny(A, cache, Cm, M, N, K, flags, cs, (cudaStream_t)stream);
+    }
     float* ws = nullptr;
     if (want.splits > 1) {
         rc = static_scratch_ptr(&ws);

@@ -1,0 +1,38 @@
+"""GEMMs of few rows (a cluster of CTAs per tile, K slices meeting in distributed shared memory), at the
+edges of their tiles, slices and ranges."""
+import pytest
+import torch
+
+import miori_b200
+from conftest import assert_close, u16
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+NARROW = 0x100  # force the tiled kernel with 128 x 128 tiles
+
+
+def _bf16(rows, cols, seed):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(seed)
+    return torch.randn((rows, cols), generator=g, device=DEV).to(torch.bfloat16)
+
+
+# N, K: clusters of 8, 8, 4, 2, 1 and 1 CTAs; ragged last tiles, uneven slices, one k-block
+@pytest.mark.parametrize("N,K", [(8, 4096), (1000, 4160), (2056, 2112), (5000, 1088), (136, 64), (16384, 192)])
+@pytest.mark.parametrize("M", [1, 15, 17, 32, 48])
+def test_few_rows(port, N, K, M):
+    A, B = _bf16(M, K, M + K), _bf16(N, K, N + K)
+    cache = B.view(-1)
+    ws = torch.empty(16, device=DEV)  # its presence allows the split
+    guard = torch.full((M * N + 64,), 777.0, device=DEV)
+    split = guard[32:32 + M * N].view(M, N)
+    miori_b200.gemm_bf16_cache(A, cache, N, out=split, workspace=ws)
+    want = port.gemm_bf16(u16(A), u16(B))
+    assert_close(split.cpu().numpy(), want, rel_max=1e-4, what=f"{M}x{N}x{K}")
+    assert (guard[:32] == 777.0).all() and (guard[32 + M * N:] == 777.0).all()
+    # rows do not depend on M, the bf16 epilogue rounds the fp32 result, unsplit is the tiled kernel's product
+    assert torch.equal(miori_b200.gemm_bf16_cache(A[:(M + 1) // 2], cache, N, workspace=ws), split[:(M + 1) // 2])
+    c16 = miori_b200.gemm_bf16_cache(A, cache, N, flags=miori_b200.OUT_BF16, workspace=ws)
+    assert torch.equal(c16, split.to(torch.bfloat16))
+    assert torch.equal(miori_b200.gemm_bf16_cache(A, cache, N), miori_b200.gemm_bf16_cache(A, cache, N, flags=NARROW))
+    assert miori_b200.lib.miori_device_error_poll() == 0
