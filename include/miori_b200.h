@@ -187,7 +187,8 @@ int miori_gemm_bf16_cache_static(const void* A, const void* cache, void* C, uint
  * apart) x B[N][K]^T (bf16, rows ldb apart), fp32 accumulation; any M, N, K >= 1.  Byte offsets
  * of the reference's signature are folded into the pointers.  Operands whose bases and row
  * pitches are 16-byte multiples (lda % 8 == 0, ldb % 8 == 0, ldc * element size % 16 == 0) run on
- * the tcgen05 kernels of miori_gemm_bf16_cache; anything else runs on a plain fp32-FMA kernel. */
+ * the tcgen05 kernels of miori_gemm_bf16_cache, or for N <= 32 on an mma.sync kernel that reads
+ * them from global memory; anything else runs on a plain fp32-FMA kernel. */
 int miori_gemm_bf16_strided(const void* A, uint32_t lda, const void* B, uint32_t ldb, void* C,
                             uint32_t ldc, uint32_t M, uint32_t N, uint32_t K, uint32_t flags,
                             void* stream);

@@ -621,6 +621,7 @@ static int make_tmap_out(CUtensorMap* map, void* Cm, float* ws, uint32_t M, uint
                         CU_TENSOR_MAP_SWIZZLE_128B, ldc);
 }
 
+#include "gemm_narrow.cuh"
 #include "gemm_skinny.cuh"
 
 // Launch the two-CTA kernel: clusters of 2, one pair per SM pair.
@@ -887,6 +888,8 @@ MIORI_API int miori_gemm_bf16_strided(const void* A, uint32_t lda, const void* B
     // TMA stores clip at 16-byte granularity, so the tensor-core kernels take the columns up to
     // the last multiple of 16 bytes and the plain kernel the few that remain
     uint32_t n_done = 0;
+    if (rows_ok && gemm::narrow::takes(M, N, K) && !(flags & MIORI_TUNE_GEMM_MASK))
+        return gemm::narrow::launch_narrow(A, lda, B, ldb, Cm, ldc, M, N, K, flags, (cudaStream_t)stream);
     if (tma_ok) {
         const uint32_t n_main = N - N % (16u / csz);
         if (n_main) {

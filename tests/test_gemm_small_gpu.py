@@ -1,5 +1,5 @@
-"""GEMMs of few rows (a cluster of CTAs per tile, K slices meeting in distributed shared memory), at the
-edges of their tiles, slices and ranges."""
+"""GEMMs of few rows (a cluster of CTAs per tile, K slices meeting in distributed shared memory) and of
+few columns (operands straight from global memory), at the edges of their tiles, slices and ranges."""
 import pytest
 import torch
 
@@ -36,3 +36,18 @@ def test_few_rows(port, N, K, M):
     assert torch.equal(c16, split.to(torch.bfloat16))
     assert torch.equal(miori_b200.gemm_bf16_cache(A, cache, N), miori_b200.gemm_bf16_cache(A, cache, N, flags=NARROW))
     assert miori_b200.lib.miori_device_error_poll() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (15, 7, 40), (16, 8, 512), (17, 9, 520), (33, 16, 2056), (100, 17, 2048),
+                                   (31, 31, 4104), (5, 32, 4096), (4737, 16, 64), (4800, 5, 1024)])
+def test_few_columns(port, M, N, K):
+    A, B = _bf16(M, K + 8, M + K)[:, :K], _bf16(N, K + 16, N + K)[:, :K]
+    C = torch.full((M + 2, 48), -7.0, device=DEV)
+    miori_b200.gemm_bf16_strided(A, B, out=C[1:M + 1, :N])
+    want = port.gemm_bf16(u16(A.contiguous()), u16(B.contiguous()))
+    assert_close(C[1:M + 1, :N].cpu().numpy(), want, rel_max=1e-4, what=f"{M}x{N}x{K}")
+    assert (C[0] == -7.0).all() and (C[M + 1] == -7.0).all() and (C[1:M + 1, N:] == -7.0).all()
+    assert torch.equal(miori_b200.gemm_bf16_strided(A[:1], B), C[1:2, :N])
+    c16 = torch.zeros((M, 64), dtype=torch.bfloat16, device=DEV)
+    miori_b200.gemm_bf16_strided(A, B, flags=miori_b200.OUT_BF16, out=c16[:, :N])
+    assert torch.equal(c16[:, :N], C[1:M + 1, :N].to(torch.bfloat16))
