@@ -13,10 +13,10 @@
 //     group's largest (the error below that is under 2^-36 of the largest).
 // Every lane of the accumulator then applies the group's fp32 scale and bias: fp32 dequantization, the
 // arithmetic class of the reference's gemv4 / gemv4_b / gemv8, for every M.  (The same product with
-// e4m3 operands, whose subnormals hold a 4-bit code in a byte, needs half the MMAs; mma.sync takes 25
-// cycles for one on sm_100a against 2 for fp16.)
+// e4m3 operands, whose subnormals hold a 4-bit code in a byte, halves the unpacking but takes as many MMAs, for
+// bf16's eight bits need two e4m3 terms: 16384 x 2048 at 8 rows took 14.8 us against 12.4 at the time.)
 //
-// What bounds it: HBM for long 8-bit streams, the issue slots (some 90 warp instructions per KiB of codes)
+// What bounds it: HBM for long 8-bit streams, the issue slots (128 warp instructions per KiB of codes at K = 2048, 109 at 8192)
 // for long 4-bit ones, the hand-over between dependent launches and the trip of x through L2 for short
 // ones.  Measured in chains of dependent launches over weights larger than L2, before (codes as bf16
 // 128 + code, one producer) and now, us: 8-bit head 131072 x 2048 at 1, 4, 16 rows 53.1, 60.3, 93 -> 44.1
@@ -46,10 +46,13 @@
 // groups instead of once per group.  The sums of a row then meet in the same order for one to four rows:
 // lane and register hold the groups of one residue modulo eight, added up in a fixed tree.
 //
-// Optional neighbours of the projection, each a template value so that the plain instantiation is
-// compiled as if they did not exist: NORMED (RMSNorm of fp32 activations inside the staging pass),
-// GATED (SiLU x up behind the fused gate + up rows), POSTNORM (post-norm and residual add by the CTA
-// that finishes last), SHARDED / ARGMAX (exchange with the peer GPUs, greedy pick of a sharded head).
+// Optional neighbours of the projection: the template value FUSED has the RMSNorm of fp32 activations inside
+// the staging pass and SiLU x up behind the fused gate + up rows, POSTNORM the post-norm and residual add by
+// the CTA that finishes last, SHARDED / ARGMAX the exchange with the peer GPUs and the greedy pick of a
+// sharded head.  The plain instantiation is compiled as if they did not exist.  FUSED is one instantiation
+// with run-time switches because a step's kernels evict one another from the instruction cache (code
+// not there costs 70 ns per KiB): with three instantiations instead of two a 24-layer step took 588 us, now
+// 574.  (With the switches in the plain kernel too: 561, but every projection by itself 0.17 us more.)
 #pragma once
 #include "common.cuh"
 #include "norm.cuh"
@@ -409,19 +412,19 @@ struct PreNorm {
 //            candidates meet in a 64-bit atomic maximum, and the CTA that finishes last exchanges this
 //            rank's best with the peers (peers.cuh: peer_argmax_exchange), so the kernel ends with the
 //            winning token on every rank and nothing else has crossed NVLink
-//   GATED:   the weight rows are a gate half [0, N/2) and an up half [N/2, N) (the fused w1/w3
+//   FUSED, gated: the weight rows are a gate half [0, N/2) and an up half [N/2, N) (the fused w1/w3
 //            projection); a tile is eight rows of each, so that after the tile's reduction one thread
 //            pair holds gate and up of the same output, and y is bf16 [M][N/2] of silu(gate) * up
 //   POSTNORM: y = residual + v * rsqrt(mean(v^2) + eps) * gamma over each whole output row v of the GEMV
 //            (shaders/ops.metal:605-631).  Every CTA stores its part of v into y; the CTA that arrives
 //            last then runs the stand-alone kernel's row pass over y in place
-//   NORMED:  x is fp32; bf16(x * rsqrt(mean(x^2) + eps) * gamma) is what is multiplied
-enum Fuse { NONE, SHARDED, ARGMAX, GATED, POSTNORM, NORMED, NORMED_GATED };
+//   FUSED, normed: x is fp32; bf16(x * rsqrt(mean(x^2) + eps) * gamma) is what is multiplied
+enum Fuse { NONE, FUSED, SHARDED, ARGMAX, POSTNORM };
 
 struct Args {
-    const uint16_t *s, *b;  // scales and biases, [N][K / GROUP]
-    const uint16_t* x;      // activations, bf16 [M][K] (fp32 when NORMED)
+    const uint16_t* x;      // activations, bf16 [M][K] (fp32 when normed)
     void* y;
+    PreNorm pre;
     uint32_t N, K, M;
     uint32_t ngrp, nsg;     // active groups of four warps; code stages per group
     uint32_t nsb;           // scale buffers of every set of groups that share a tile
@@ -429,12 +432,13 @@ struct Args {
     uint32_t slab_row;      // bytes of a row in a slab: SLAB_ROW, or a shorter whole row rounded up to 128
     uint32_t inv_upr;       // ceil(2^32 / (K / 8))
     uint32_t out_bf16;
+    uint32_t gated;         // SiLU x up of the two halves
     uint32_t n_total, row0; // the whole output's rows and this launch's first one
+    const uint16_t *s, *b;  // scales and biases, [N][K / GROUP]
+    PostNorm post;
     size_t y_off;
     unsigned long long* best;
     PeerArgs pa;
-    PostNorm post;
-    PreNorm pre;
 };
 
 // The dynamic shared memory, identical on host and device (bytes from a 128-byte aligned base).
@@ -470,7 +474,7 @@ __host__ __device__ inline Layout layout(uint32_t K, uint32_t M, uint32_t stages
 template <class S, Fuse F>
 __global__ void __launch_bounds__(THREADS, 1)
 gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ Args A) {
-    constexpr bool GATED_ = F == GATED || F == NORMED_GATED, NORMED_ = F == NORMED || F == NORMED_GATED;
+    const bool gated = F == FUSED && A.gated != 0u, normed = F == FUSED && A.pre.gamma != nullptr;
     constexpr bool SHARDED_ = F == SHARDED, ARGMAX_ = F == ARGMAX, POSTNORM_ = F == POSTNORM;
     constexpr int BITS = S::BITS, NT = S::NT, ROWS = S::ROWS, GPS = S::GPS, RC = S::RC;
     const uint32_t N = A.N, K = A.K, M = A.M, kpar = A.kpar, nsg = A.nsg, ngrp = A.ngrp;
@@ -541,7 +545,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 const bool shared = kpar > 1u;
                 uint32_t sb_bar = smem_addr(&full_bars[bar0 + st]), extra = 2u * L.sb_half;
                 const uint32_t sdst = base + L.sb + (sb0 + sb) * 2u * L.sb_half;
-                const uint32_t r0 = GATED_ ? row >> 1 : row;  // GATED: N is a multiple of 16, eight whole rows of each half
+                const uint32_t r0 = gated ? row >> 1 : row;  // gated: N is a multiple of 16, eight whole rows of each half
                 const uint8_t* src_s = reinterpret_cast<const uint8_t*>(A.s) + (size_t)r0 * (2u * ng);
                 const uint8_t* src_b = reinterpret_cast<const uint8_t*>(A.b) + (size_t)r0 * (2u * ng);
                 if (row + 16u > N && kp == 0u) {  // a ragged last tile: whole 16-byte pieces by bulk copy ...
@@ -555,7 +559,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                     }
                 }
                 auto copy_sb = [&] {
-                    if (GATED_) {
+                    if (gated) {
                         const uint32_t half = L.sb_half >> 1;
                         const size_t up = (size_t)(N >> 1) * (2u * ng);
                         bulk_g2s(sdst, src_s, half, sb_bar);
@@ -579,7 +583,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                     const int c0 = (int)(ks * (SLAB_ROW / 8u));
                     const bool with_sb = !shared && ks == 0u;
                     mbar_expect_tx(bar, L.stage_bytes + (with_sb ? extra : 0u));
-                    if (GATED_) {  // the tensor map's boxes are eight rows high
+                    if (gated) {  // the tensor map's boxes are eight rows high
                         tma_load_2d(dst, &tmap_q, c0, (int)r0, bar);
                         tma_load_2d(dst + 8u * qpitch, &tmap_q, c0, (int)((N >> 1) + r0), bar);
                     } else {
@@ -611,7 +615,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
         pdl_wait_prior();  // x (and y) belong to the predecessor until here
 
-        if constexpr (NORMED_) {
+        if (normed) {
             __shared__ float nm_part[4][WARPS];
             __shared__ float nm_inv[32];
             stage_x_normed<S>(xa, reinterpret_cast<const float*>(A.x), A.pre.gamma, A.pre.eps, M, K, A.inv_upr, nm_part, nm_inv);
@@ -645,13 +649,12 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 }
             }
         };
-        // GATED: y[m][row] = bf16(silu(gate) * up) of the N/2-column output, with the arithmetic of the
+        // gated: y[m][row] = bf16(silu(gate) * up) of the N/2-column output, with the arithmetic of the
         // stand-alone activation kernel (shaders/ops.metal:129-139)
         auto store_gated = [&](uint32_t m, uint32_t row, float gate, float up) {
             const float sg = gate / (1.0f + expf(-gate));
             reinterpret_cast<uint16_t*>(A.y)[(size_t)m * (N >> 1) + row] = (uint16_t)float_to_bf16_bits(sg * up);
         };
-        (void)store_gated;
 
         // ---- this lane's place in the MMAs.  As a B operand it supplies column n = lane / 4 = (slot n / RC,
         // row n % RC); as an accumulator it holds columns 2 t and 2 t + 1.
@@ -899,7 +902,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             };
             const uint32_t tile = blockIdx.x + (vt >> kshift) * gridDim.x;
             if (kp == 0u && ok) {
-                if constexpr (GATED_) {  // tile rows 0 .. 7 are gates, 8 .. 15 the same outputs' up rows
+                if (gated) {  // tile rows 0 .. 7 are gates, 8 .. 15 the same outputs' up rows
                     for (uint32_t i = gt; i < 8u * M; i += 128u) {
                         const uint32_t m = i >> 3, r = i & 7u;
                         store_gated(m, tile * 8u + r, total(m * 16u + r), total(m * 16u + r + 8u));
@@ -1046,7 +1049,7 @@ Plan plan_launch(uint32_t N, uint32_t K, uint32_t M) {
 
 template <class S, Fuse F>
 int launch_one(const Plan& plan, const void* q, Args& a, bool pdl, cudaStream_t stream) {
-    constexpr bool gated = F == GATED || F == NORMED_GATED;
+    const bool gated = a.gated != 0u;
     CUtensorMap tq;
     // rows as 64-bit words, so that the box can be wider than 256 words of 32 bits; gated: a tile is two
     // boxes, one from each half
@@ -1078,6 +1081,7 @@ int launch_shape(const void* q, const void* s, const void* b, const void* x, voi
     a.ngrp = plan.ngrp, a.nsg = plan.nsg, a.nsb = plan.nsb, a.kpar = plan.kpar, a.slab_row = plan.slab_row;
     a.inv_upr = (uint32_t)((0x100000000ull + K / 8u - 1u) / (K / 8u));
     a.out_bf16 = flags & MIORI_OUT_BF16 ? 1u : 0u;
+    a.gated = sh.gated ? 1u : 0u;
     a.n_total = placed ? sh.n_total : N, a.row0 = placed ? sh.row0 : 0u, a.y_off = sh.y_off;
     a.best = sh.best, a.pa = sh.pa, a.post = sh.post, a.pre = sh.pre;
     const bool pdl = (flags & MIORI_LAUNCH_PDL) != 0;
@@ -1092,16 +1096,10 @@ int launch_shape(const void* q, const void* s, const void* b, const void* x, voi
             if (!a.out_bf16 && M <= 4) return launch_one<S, POSTNORM>(plan, q, a, pdl, stream);
         return fail(MIORI_E_INVALID, "the post-norm epilogue takes 4-bit weights, up to four rows, fp32 out");
     }
-    if (sh.gated) {
-        if constexpr (S::BITS == 4 && S::ROWS <= 16) {
-            if (N % 16 == 0 && !normed) return launch_one<S, GATED>(plan, q, a, pdl, stream);
-            if constexpr (FEW)
-                if (N % 16 == 0 && M <= 4) return launch_one<S, NORMED_GATED>(plan, q, a, pdl, stream);
-        }
+    if (sh.gated && (S::BITS != 4 || N % 16 != 0 || M > (normed ? 4u : 16u)))
         return fail(MIORI_E_INVALID, "the gated epilogue takes 4-bit weights with N a multiple of 16, up to 16 rows "
                                      "(four with the norm in front)");
-    }
-    if (normed) return launch_one<S, NORMED>(plan, q, a, pdl, stream);
+    if (normed || sh.gated) return launch_one<S, FUSED>(plan, q, a, pdl, stream);
     if (sharded) return launch_one<S, SHARDED>(plan, q, a, pdl, stream);
     return launch_one<S, NONE>(plan, q, a, pdl, stream);
 }

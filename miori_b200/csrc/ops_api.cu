@@ -21,7 +21,7 @@ int check_quant_args(const char* op, const void* q, const void* s, const void* b
     return MIORI_OK;
 }
 
-// The GEMV for M rows, as many of them a launch as its shared memory holds: all 32 at K <= 2816, eight at
+// The GEMV for M rows, as many of them a launch as its shared memory holds: all 32 at K <= 2304, eight at
 // K = 8192.  A row's value depends on the rows of its launch only through their number's class.
 template <int BITS>
 int gemv_rows(const char* op, const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N,
