@@ -45,6 +45,8 @@ template <int BITS, int UNITS>
 __global__ void __launch_bounds__(DEQUANT_THREADS)
 dequant_rowmajor_kernel(const uint32_t* __restrict__ q, const uint16_t* __restrict__ s, const uint16_t* __restrict__ b,
                         uint4* __restrict__ out, uint64_t units, uint32_t ushift) {
+    // a programmatic launch, which costs the host less, that waits and only then lets dependents start early
+    pdl_wait_prior();
     pdl_launch_dependents();
     const uint64_t first = (uint64_t)blockIdx.x * (DEQUANT_THREADS * UNITS) + threadIdx.x;
     uint32_t w[UNITS][BITS / 4], sc[UNITS], bi[UNITS];
@@ -79,7 +81,7 @@ int launch_dequant_rowmajor(const void* q, const void* s, const void* b, void* o
     const uint64_t per_block = (uint64_t)DEQUANT_THREADS * (wide ? 4u : 1u), blocks = (units + per_block - 1u) / per_block;
     if (blocks > 0x7FFFFFFFull) return fail(MIORI_E_INVALID, "dequant: N=%u K=%u is too large", N, K);
     auto kern = wide ? dequant_rowmajor_kernel<BITS, 4> : dequant_rowmajor_kernel<BITS, 1>;
-    cudaError_t e = launch(kern, dim3((unsigned)blocks), dim3(DEQUANT_THREADS), 0, stream, false,
+    cudaError_t e = launch(kern, dim3((unsigned)blocks), dim3(DEQUANT_THREADS), 0, stream, true,
                            reinterpret_cast<const uint32_t*>(q), reinterpret_cast<const uint16_t*>(s),
                            reinterpret_cast<const uint16_t*>(b), reinterpret_cast<uint4*>(out), units, ushift);
     if (e != cudaSuccess) return cuda_fail(e, "dequant_rowmajor launch");
