@@ -139,9 +139,10 @@ int miori_gemm_bf16_cache(const void* A, const void* cache, void* C, uint32_t M,
                           uint32_t K, uint32_t flags, void* stream);
 
 /* Host-only: what the planner would launch for this shape with `workspace_bytes` of workspace --
- * the tile's width in output columns (128 or 256; a tile is 128 rows, 256 when two CTAs share it),
+ * the tile's width in output columns (128, 192 or 256; a tile is 128 rows, 256 when two CTAs share it),
  * the CTAs per tile (1, or 2 for the cta_group::2 kernel) and the number of K slices (1 = no
- * split).  For tests and for hosts that want to log the choice; no device is touched beyond the
+ * split).  (Up to 48 rows a kernel with tiles of its own may take the product instead, see below.)
+ * For tests and for hosts that want to log the choice; no device is touched beyond the
  * SM count. */
 int miori_gemm_plan(uint32_t M, uint32_t N, uint32_t K, size_t workspace_bytes, uint32_t* tile_n,
                     uint32_t* ctas_per_tile, uint32_t* splits);

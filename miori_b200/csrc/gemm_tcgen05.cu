@@ -335,7 +335,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 }
 
 // ---------------------------------------------------------------------------------------
-// Two-CTA variant: a cluster of two CTAs (one SM pair) computes a 256 x 256 tile with
+// Two-CTA variant: a cluster of two CTAs (one SM pair) computes a 256 x 256 (or x 192) tile with
 // tcgen05.mma.cta_group::2.  CTA r of the pair owns rows [128r, 128r+128) of the tile (its A
 // tile and its TMEM accumulator) and loads only rows [128r, 128r+128) of the B tile; the MMA,
 // issued by CTA 0, reads both halves of B out of the two CTAs' shared memory.  Per k-block
@@ -345,13 +345,16 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 // accumulators to both CTAs with tcgen05.commit ... multicast::cluster.
 namespace pair {
 
-constexpr int BN = 256;
-constexpr int STAGES = 6;
-constexpr int A_BYTES = BM * BK * 2;         // 16 KB: this CTA's 128 rows of A
-constexpr int B_BYTES = (BN / 2) * BK * 2;   // 16 KB: this CTA's 128 rows of B
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int TMEM_COLS = 2 * BN;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_STAGE_BYTES + 1024 + 256;
+// BN: columns of a tile, 192 or 256
+template <int BN>
+struct Cfg {
+    static constexpr int STAGES = 6;
+    static constexpr int A_BYTES = BM * BK * 2;         // this CTA's 128 rows of A
+    static constexpr int B_BYTES = (BN / 2) * BK * 2;   // this CTA's half of the rows of B
+    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int TMEM_COLS = 512;               // two accumulators, a power of two
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + OUT_STAGE_BYTES + 1024 + 256;
+};
 constexpr uint32_t PEER_MASK = 0xFEFFFFFFu;  // clears the CTA-rank bit of a shared::cluster address
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -399,12 +402,14 @@ __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar_local) {
         : "memory");
 }
 
-template <bool OUT_BF16>
+template <int BN, bool OUT_BF16>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
                               const __grid_constant__ CUtensorMap tmap_b,
                               const __grid_constant__ CUtensorMap tmap_c, uint32_t splits,
                               uint32_t M, uint32_t N, uint32_t K) {
+    using C = Cfg<BN>;
+    constexpr int STAGES = C::STAGES, A_BYTES = C::A_BYTES, STAGE_BYTES = C::STAGE_BYTES, TMEM_COLS = C::TMEM_COLS;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint32_t tmem_base_slot;
     __shared__ volatile uint32_t abort_flag;
@@ -625,24 +630,25 @@ static int make_tmap_out(CUtensorMap* map, void* Cm, float* ws, uint32_t M, uint
 #include "gemm_skinny.cuh"
 
 // Launch the two-CTA kernel: clusters of 2, one pair per SM pair.
+template <int BN>
 static int launch_gemm_pair(const void* A, const void* Bc, void* Cm, uint32_t M, uint32_t N,
                             uint32_t K, uint32_t flags, float* ws, uint32_t splits,
                             cudaStream_t stream, const Ld& ld) {
     CUtensorMap ta, tb, tc;
     int rc = make_tmap(&ta, A, M, K, BM, ld.a);
     if (rc) return rc;
-    rc = make_tmap(&tb, Bc, N, K, pair::BN / 2, ld.b);
+    rc = make_tmap(&tb, Bc, N, K, BN / 2, ld.b);
     if (rc) return rc;
     rc = make_tmap_out(&tc, Cm, ws, M, N, splits, (flags & MIORI_OUT_BF16) != 0, ld.c);
     if (rc) return rc;
-    const uint32_t tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + pair::BN - 1) / pair::BN) * splits;
+    const uint32_t tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * splits;
     uint32_t pairs = (uint32_t)sm_count() / 2;
     if (pairs > tiles) pairs = tiles;
     const bool bf16 = (flags & MIORI_OUT_BF16) != 0, pdl = (flags & MIORI_LAUNCH_PDL) != 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = pair::SMEM_BYTES;
+    cfg.dynamicSmemBytes = pair::Cfg<BN>::SMEM_BYTES;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -655,12 +661,12 @@ static int launch_gemm_pair(const void* A, const void* Bc, void* Cm, uint32_t M,
     cfg.numAttrs = pdl ? 2 : 1;
     cudaError_t e;
     if (bf16) {
-        auto kern = pair::gemm_bf16_tcgen05_pair_kernel<true>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::SMEM_BYTES);
+        auto kern = pair::gemm_bf16_tcgen05_pair_kernel<BN, true>;
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::Cfg<BN>::SMEM_BYTES);
         if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, splits, M, N, K);
     } else {
-        auto kern = pair::gemm_bf16_tcgen05_pair_kernel<false>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::SMEM_BYTES);
+        auto kern = pair::gemm_bf16_tcgen05_pair_kernel<BN, false>;
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::Cfg<BN>::SMEM_BYTES);
         if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, splits, M, N, K);
     }
     if (e != cudaSuccess) return cuda_fail(e, "gemm_bf16_tcgen05_pair launch");
@@ -733,11 +739,12 @@ static int check_gemm_args(const char* op, const void* A, const void* cache, con
 // Tile shape and split count for a problem (workspace of ws_bytes available, 0 = none).
 struct GemmPlan {
     bool wide;   // 128 x 256 tiles instead of 128 x 128 (single-CTA kernel)
-    bool pair;   // 256 x 256 tiles on SM pairs (two-CTA kernel)
+    bool pair;   // 256-row tiles on SM pairs (two-CTA kernel)
     uint32_t splits;
+    uint32_t pair_n;  // their columns: 192 or 256
 };
 
-// The plan is the cheapest of {128x128, 128x256, 256x256-on-pairs} x {1..16 K-splits} under a
+// The plan is the cheapest of {128x128, 128x256, 256x256- and 256x192-on-pairs} x {1..16 K-splits} under a
 // small cost model (microseconds):
 //   main loop  = waves x k-blocks per work item x time per k-block of that tile shape, where
 //                waves = ceil(work items / SMs or SM pairs) -- but never less than the time
@@ -745,7 +752,11 @@ struct GemmPlan {
 //   split cost = a second (reduction) kernel plus (splits + 1) passes over M x N fp32.
 // The per-k-block times are what the kernels sustain on a B200 when L2 feeds them (bigger tiles
 // need fewer bytes per flop): 0.31 us for 128x128, 0.375 us for 128x256, 0.315 us for a
-// 256x256 pair tile.  Splitting K therefore happens when the tiles alone would leave most SMs
+// 256x256 pair tile.  A 256x192 one measures 0.24 (a shorter k-block is not served faster: 256x128 also took
+// 0.24), but pays a pair's longer prologue and epilogue; 0.304 sends a single wave that 128x128 tiles fill
+// as well to those (1024 x 2048, K = 2048: 12.7 us against 14.1) and everything to it where its waves are
+// as few as the 256-wide ones' (1024 x 3072: 16.6 -> 14.4, 768 x 8192: 26.5 -> 23.6, 2048 x 3072: 26.0 ->
+// 23.3, 1536 x 2048 at K = 8192: 45.0 -> 40.4).  Splitting K therefore happens when the tiles alone would leave most SMs
 // idle and K is long enough to pay for the reduction, never below 4 k-blocks per split.
 static GemmPlan plan_gemm(uint32_t M, uint32_t N, uint32_t K, uint32_t flags, size_t ws_bytes) {
     const uint32_t sms = (uint32_t)sm_count();
@@ -755,22 +766,25 @@ static GemmPlan plan_gemm(uint32_t M, uint32_t N, uint32_t K, uint32_t flags, si
         bool wide, pair, allowed;
         uint32_t tiles, units;
         double t_kb;
+        uint32_t pair_n;
     };
     const uint32_t m128 = (M + 127) / 128, m256 = (M + 255) / 256;
     const uint32_t n128 = (N + 127) / 128, n256 = (N + 255) / 256;
     const bool force_narrow = flags & MIORI_TUNE_GEMM_NARROW, force_wide = flags & MIORI_TUNE_GEMM_WIDE;
     const bool force_pair = flags & MIORI_TUNE_GEMM_PAIR, no_pair = flags & MIORI_TUNE_GEMM_NOPAIR;
     const bool forced = force_narrow || force_wide || force_pair;
-    Shape shapes[3] = {
-        {false, false, !forced || force_narrow, m128 * n128, sms, 0.31},
-        {true, false, !forced || force_wide, m128 * n256, sms, 0.375},
-        {false, true, ((!forced && M > 128) || force_pair) && !no_pair, m256 * n256, sms / 2, 0.315},
+    const bool pair_ok = ((!forced && M > 128) || force_pair) && !no_pair;
+    Shape shapes[4] = {
+        {false, false, !forced || force_narrow, m128 * n128, sms, 0.31, 0},
+        {true, false, !forced || force_wide, m128 * n256, sms, 0.375, 0},
+        {false, true, pair_ok, m256 * n256, sms / 2, 0.315, 256},
+        {false, true, pair_ok && !force_pair, m256 * ((N + 191) / 192), sms / 2, 0.304, 192},
     };
     const double t_hbm = ((double)N * K * 2 + (double)M * K * 2) / 6.5e6;  // us at 6.5 TB/s
     uint32_t max_s = std::min<uint32_t>(16, std::max<uint32_t>(1, k_blocks / 4));
     if (!ws_bytes) max_s = 1;
     else if (mn) max_s = (uint32_t)std::min<size_t>(max_s, std::max<size_t>(1, ws_bytes / (mn * 4)));
-    GemmPlan best = {false, false, 1};
+    GemmPlan best = {false, false, 1, 0};
     double best_t = 1e30;
     const uint32_t force_split = (flags >> MIORI_TUNE_GEMM_SPLIT_SHIFT) & 15u;
     for (const Shape& sh : shapes) {
@@ -783,7 +797,7 @@ static GemmPlan plan_gemm(uint32_t M, uint32_t N, uint32_t K, uint32_t flags, si
             if (sp > 1) t += 2.0 + (double)(sp + 1) * mn * 4 / 5e6;
             if (t < best_t * 0.97) {  // a later candidate must win by 3 %: prefers fewer splits
                 best_t = t;
-                best = {sh.wide, sh.pair, sp};
+                best = {sh.wide, sh.pair, sp, sh.pair_n};
             }
         }
     }
@@ -794,7 +808,8 @@ static int run_plan(const GemmPlan& p, const void* A, const void* cache, void* C
                     uint32_t N, uint32_t K, uint32_t flags, float* ws, cudaStream_t stream,
                     const Ld& ld = Ld()) {
     if (p.pair) {
-        int rc = launch_gemm_pair(A, cache, Cm, M, N, K, flags, ws, p.splits, stream, ld);
+        auto run = p.pair_n == 192u ? launch_gemm_pair<192> : launch_gemm_pair<256>;
+        int rc = run(A, cache, Cm, M, N, K, flags, ws, p.splits, stream, ld);
         if (rc == MIORI_OK && p.splits > 1) rc = launch_reduce(Cm, M, N, flags, ws, p.splits, stream);
         return rc;
     }
@@ -982,7 +997,7 @@ MIORI_API int miori_gemm_plan(uint32_t M, uint32_t N, uint32_t K, size_t workspa
                               uint32_t* ctas_per_tile, uint32_t* splits) {
     if (M == 0 || N == 0 || K == 0) return fail(MIORI_E_INVALID, "miori_gemm_plan: empty shape");
     const gemm::GemmPlan p = gemm::plan_gemm(M, N, K, 0, workspace_bytes);
-    if (tile_n) *tile_n = (p.wide || p.pair) ? 256u : 128u;
+    if (tile_n) *tile_n = p.pair ? p.pair_n : p.wide ? 256u : 128u;
     if (ctas_per_tile) *ctas_per_tile = p.pair ? 2u : 1u;
     if (splits) *splits = p.splits;
     return MIORI_OK;

@@ -1,5 +1,8 @@
 """GEMMs of few rows (a cluster of CTAs per tile, K slices meeting in distributed shared memory) and of
-few columns (operands straight from global memory), at the edges of their tiles, slices and ranges."""
+few columns (operands straight from global memory), at the edges of their tiles, slices and ranges; tiles
+of 192 columns on SM pairs."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -51,3 +54,19 @@ def test_few_columns(port, M, N, K):
     c16 = torch.zeros((M, 64), dtype=torch.bfloat16, device=DEV)
     miori_b200.gemm_bf16_strided(A, B, flags=miori_b200.OUT_BF16, out=c16[:, :N])
     assert torch.equal(c16[:, :N], C[1:M + 1, :N].to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("M,N,K", [(1024, 3072, 128), (1500, 2056, 192), (2047, 3080, 64), (600, 8192, 320)])
+def test_pair_tiles_of_192_columns(port, M, N, K):
+    tile, ctas, splits = C.c_uint32(), C.c_uint32(), C.c_uint32()
+    assert miori_b200.lib.miori_gemm_plan(M, N, K, 0, C.byref(tile), C.byref(ctas), C.byref(splits)) == 0
+    assert (tile.value, ctas.value) == (192, 2), "the planner changed: pick shapes that run on these tiles"
+    A, B = _bf16(M, K, M + K), _bf16(N, K, N + K)
+    guard = torch.full((M + 2, N), 777.0, device=DEV)
+    miori_b200.gemm_bf16_cache(A, B.view(-1), N, out=guard[1:M + 1])
+    assert_close(guard[1:M + 1].cpu().numpy(), port.gemm_bf16(u16(A), u16(B)), rel_max=1e-4, what=f"{M}x{N}x{K}")
+    assert (guard[0] == 777.0).all() and (guard[M + 1] == 777.0).all()
+    assert torch.equal(miori_b200.gemm_bf16_cache(A, B.view(-1), N, flags=NARROW), guard[1:M + 1])
+    c16 = miori_b200.gemm_bf16_cache(A, B.view(-1), N, flags=miori_b200.OUT_BF16)
+    assert torch.equal(c16, guard[1:M + 1].to(torch.bfloat16))
+    assert miori_b200.lib.miori_device_error_poll() == 0
