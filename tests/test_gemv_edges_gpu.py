@@ -71,3 +71,24 @@ def test_more_rows_than_a_launch_holds(port, M, K):
     want = port.gemv(4, u32(q), u16(s), u16(b), u16(x), 64)
     got = miori_b200.gemv4(q.to(DEV), s.to(DEV), b.to(DEV), x.to(DEV), group=64, flags=miori_b200.LAUNCH_PDL).cpu().numpy()
     assert_close(got, want, rel_max=TOL_EXACT_PATH, what=f"M={M} K={K}")
+
+
+@pytest.mark.parametrize("N,K", [(40, 256), (2048, 2048), (5000, 2048)])
+def test_plain_launch_reads_what_the_launch_before_it_wrote(N, K):
+    """Without the early-start flag a launch may have its weights, its cache or its activations written by
+    whatever precedes it on the stream, kernels that let their dependents start early included."""
+    ws = [synth.make_weight(N, K, 4, 64, seed=i, device=DEV) for i in range(3)]
+    x = synth.make_activation(1, K, seed=9, device=DEV)
+    want = [miori_b200.gemv4(*w, x, group=64) for w in ws]
+    caches = [miori_b200.dequant4_cache(*w, group=64) for w in ws]
+    torch.cuda.synchronize()
+    live = [t.clone() for t in ws[0]]
+    warm = torch.empty((1, N), device=DEV)
+    for it in range(30):
+        i = it % 3
+        miori_b200.gemv4(*ws[i], x, group=64, flags=miori_b200.LAUNCH_PDL, out=warm)
+        for t, src in zip(live, ws[i]):
+            t.copy_(src)
+        got = miori_b200.gemv4(*live, x, group=64)
+        again = miori_b200.dequant4_cache(*live, group=64)
+        assert torch.equal(got, want[i]) and torch.equal(again, caches[i]), it
