@@ -3,11 +3,15 @@
 //   y[m][n] = sum_g ( s[n][g] * sum_{k in g} code[n][k] * x[m][k]  +  b[n][g] * sum_{k in g} x[m][k] )
 //
 // The inner sum runs on mma.sync.m16n8k16 with fp16 operands and fp32 accumulators:
-//   * a code in the low bits of a 16-bit half IS an fp16 value: the subnormal code * 2^-24.  So a word
-//     of eight 4-bit codes becomes its four A registers with one shift and four ANDs, the codes in bits
-//     4 .. 7 of a half counting 16 times (their activations are staged divided by 16), a word of four
-//     8-bit codes becomes two registers with one shift and two ANDs.  No offset is added to the codes, so
-//     none has to be subtracted from the sums;
+//   * a code in the mantissa bits of a 16-bit half IS an fp16 value, the subnormal code * 2^-24 times its
+//     place.  So a word of eight 4-bit codes becomes its four A registers with two shifts and four ANDs, the
+//     codes in bits 2 .. 5 of a half or in bits 6 .. 9, where they count 16 times as much (their activations
+//     are staged divided by 16); a word of four 8-bit codes becomes two registers with one shift and two
+//     ANDs.  No offset is added to the codes, so none has to be subtracted from the sums.  (The place matters:
+//     the tensor core aligns its products by the operands' exponents, and a subnormal's is that of 2^-14, so
+//     what a code leaves empty above itself is cut off the sum.  With codes in bits 0 .. 7, one shift fewer,
+//     the error against 64-bit sums was 1.9e-7, 5.6e-7, 5.2e-7 of the result at 1, 4, 8 rows of 2048 x 2048, now
+//     0.7e-7, 1.3e-7, 1.2e-7, for 1 % of the time; every code in bits 6 .. 9: 0.7e-7, 1.0e-7, 1.1e-7, for 3-5 %.)
 //   * a scale group's activations are multiplied by the power of two that puts the largest into
 //     [2^15, 2^16): bf16's eight bits are exact in fp16 for every activation of at least 2^-28 of the
 //     group's largest (the error below that is under 2^-36 of the largest).
@@ -188,11 +192,12 @@ struct AFrag {
     __device__ __forceinline__ void unpack(const uint32_t (&q0)[NW], const uint32_t (&q1)[NW]) {
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
-            const uint32_t h0 = q0[w] >> 8, h1 = q1[w] >> 8;
             if constexpr (BITS == 4) {
-                r0[w][0] = q0[w] & 0x000F000Fu, r0[w][1] = q0[w] & 0x00F000F0u, r0[w][2] = h0 & 0x000F000Fu, r0[w][3] = h0 & 0x00F000F0u;
-                r1[w][0] = q1[w] & 0x000F000Fu, r1[w][1] = q1[w] & 0x00F000F0u, r1[w][2] = h1 & 0x000F000Fu, r1[w][3] = h1 & 0x00F000F0u;
+                const uint32_t l0 = q0[w] << 2, h0 = q0[w] >> 6, l1 = q1[w] << 2, h1 = q1[w] >> 6;
+                r0[w][0] = l0 & 0x003C003Cu, r0[w][1] = l0 & 0x03C003C0u, r0[w][2] = h0 & 0x003C003Cu, r0[w][3] = h0 & 0x03C003C0u;
+                r1[w][0] = l1 & 0x003C003Cu, r1[w][1] = l1 & 0x03C003C0u, r1[w][2] = h1 & 0x003C003Cu, r1[w][3] = h1 & 0x03C003C0u;
             } else {
+                const uint32_t h0 = q0[w] >> 8, h1 = q1[w] >> 8;
                 r0[w][0] = q0[w] & 0x00FF00FFu, r0[w][1] = h0 & 0x00FF00FFu;
                 r1[w][0] = q1[w] & 0x00FF00FFu, r1[w][1] = h1 & 0x00FF00FFu;
             }
@@ -217,10 +222,11 @@ __device__ __forceinline__ uint32_t f16x2_bits(float lo, float hi) {
 
 // Stage one unit -- eight consecutive activations of a row as bf16 -- for the MMA B operand: scaled fp16
 // pairs in the order of the A registers and, by the first lane of each scale group, the group's {power
-// of two that undoes the scaling, sum of x} / 512 (so that the power of two stays finite for every
+// of two that undoes the scaling, sum of x} / UNSCALE (so that the power of two stays finite for every
 // input; the outputs are multiplied at the end).  The GROUP / 8 lanes of a group hold neighbouring
-// units; every lane of the warp calls.
-constexpr float UNSCALE = 512.0f;
+// units; every lane of the warp calls.  512 for codes that count from bit 0 of a half, 128 from bit 2.
+template <int BITS>
+constexpr float UNSCALE = BITS == 4 ? 128.0f : 512.0f;
 template <int BITS, int GROUP>
 __device__ __forceinline__ void stage_unit(const uint4& v, bool live, uint32_t x_addr, bool first, uint32_t ms_addr) {
     const uint32_t a = v.x & 0x7FFF7FFFu, b = v.y & 0x7FFF7FFFu, c = v.z & 0x7FFF7FFFu, d = v.w & 0x7FFF7FFFu;
@@ -247,7 +253,7 @@ __device__ __forceinline__ void stage_unit(const uint4& v, bool live, uint32_t x
     if (live) {
         asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(x_addr), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
         if (first)
-            asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ms_addr), "f"(__uint_as_float(e << 23)), "f"(sum * (1.0f / UNSCALE)) : "memory");
+            asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(ms_addr), "f"(__uint_as_float(e << 23)), "f"(sum * (1.0f / UNSCALE<BITS>)) : "memory");
     }
 }
 
@@ -902,7 +908,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                     const float w = (p.x + p.y) + (p.z + p.w);
                     v = j == 0u ? w : v + w;
                 }
-                return v * UNSCALE;
+                return v * UNSCALE<BITS>;
             };
             const uint32_t tile = blockIdx.x + (vt >> kshift) * gridDim.x;
             if (kp == 0u && ok) {

@@ -92,3 +92,24 @@ def test_plain_launch_reads_what_the_launch_before_it_wrote(N, K):
         got = miori_b200.gemv4(*live, x, group=64)
         again = miori_b200.dequant4_cache(*live, group=64)
         assert torch.equal(got, want[i]) and torch.equal(again, caches[i]), it
+
+
+def _weights64(q, s, b, bits, group):
+    shift = torch.arange(32 // bits, device=q.device, dtype=torch.int64) * bits
+    codes = ((q.to(torch.int64).unsqueeze(-1) >> shift) & (2 ** bits - 1)).reshape(q.shape[0], -1)
+    return codes.double() * s.double().repeat_interleave(group, 1) + b.double().repeat_interleave(group, 1)
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("group", [32, 64])
+@pytest.mark.parametrize("N,K", [(2048, 2048), (256, 8192)])
+@pytest.mark.parametrize("M", [1, 2, 4, 8, 16, 32])
+def test_error_is_that_of_fp32_sums(bits, group, N, K, M):
+    """Against 64-bit sums, 2-norm over 2-norm.  Products are exact; a group's sum and its bias term, each about
+    1.5 times the result, and the sum over groups take a rounding of 2^-24 each, and the result one: under 4 of
+    them.  (Whatever the tensor core cuts off has to stay below that.)"""
+    q, s, b = synth.make_weight(N, K, bits, group, seed=N + K, device=DEV)
+    x = synth.make_activation(M, K, seed=M, device=DEV)
+    want = x.double() @ _weights64(q, s, b, bits, group).T
+    got = OPS[bits](q, s, b, x, group=group).double()
+    assert float((got - want).norm() / want.norm()) < 4 * 2.0 ** -24
