@@ -454,7 +454,8 @@ struct Layout {
     uint32_t sb, x, ms, zeros, red, total;
 };
 template <class S>
-__host__ __device__ inline Layout layout(uint32_t K, uint32_t M, uint32_t stages, uint32_t sb_bufs, uint32_t slab_row) {
+__host__ __device__ inline Layout layout(uint32_t K, uint32_t M, uint32_t stages, uint32_t sb_bufs, uint32_t slab_row,
+                                         uint32_t red_bufs = Red<S::ROWS>::BUFS) {
     Layout L;
     L.qpitch = slab_row + S::QPAD;
     L.stage_bytes = 16u * L.qpitch;
@@ -473,7 +474,7 @@ __host__ __device__ inline Layout layout(uint32_t K, uint32_t M, uint32_t stages
     L.zeros = at;
     at += ZERO_BYTES;
     L.red = at;  // 16-byte aligned
-    at += GROUPS * Red<S::ROWS>::BUFS * Red<S::ROWS>::FLOATS * 4u;
+    at += GROUPS * red_bufs * Red<S::ROWS>::FLOATS * 4u;  // last: nothing else lies by their number
     L.total = at;
     return L;
 }
@@ -1010,7 +1011,7 @@ struct Shard {
     PreNorm pre;
 };
 
-// Launch plan: CTAs, active groups, stages per group, scale buffers; ngrp == 0: the activations do not fit.
+// Launch plan: CTAs, active groups, stages per group, scale buffers.
 struct Plan {
     uint32_t grid = 0, ngrp = 0, nsg = 0, nsb = 0, kpar = 1, slab_row = 0;
     size_t smem = 0;
@@ -1023,37 +1024,64 @@ struct Plan {
 // 17 % slower than the sum of its parts.  With the SM to itself a CTA starts as its predecessor's CTA
 // exits, fills its ring during the hand-over between the grids, and the placement is one CTA per SM
 // whatever ran before.
+constexpr size_t SMEM_LIMIT = 222 * 1024;
+
+// What a launch's size is made of: 16-row tiles of the busiest CTA, slabs of a row.
+struct Extent {
+    uint32_t tiles, grid, tiles_cta, kslabs, slab_row;
+};
 template <class S>
-Plan plan_launch(uint32_t N, uint32_t K, uint32_t M) {
-    constexpr size_t LIMIT = 222 * 1024;
-    Plan p;
+Extent extent(uint32_t N, uint32_t K) {
+    Extent e;
     const uint32_t row_bytes = K * S::BITS / 8u;
-    const uint32_t tiles = (N + 15u) / 16u, kslabs = (row_bytes + SLAB_ROW - 1u) / SLAB_ROW;
-    p.slab_row = row_bytes >= SLAB_ROW ? SLAB_ROW : (row_bytes + 127u) / 128u * 128u;
-    p.grid = std::min<uint32_t>(tiles, (uint32_t)sm_count());
-    const uint32_t tiles_cta = (tiles + p.grid - 1u) / p.grid;  // tiles of the busiest CTA
-    // few tiles per CTA and a long K: let 2 or 4 groups share a tile, each taking every kpar-th slab
-    while (p.kpar * 2u <= (uint32_t)GROUPS && tiles_cta * p.kpar * 2u <= (uint32_t)GROUPS && kslabs % (p.kpar * 2u) == 0u)
-        p.kpar *= 2u;
-    for (; p.kpar >= 1u; p.kpar >>= 1) {
-        const uint32_t vtiles = tiles_cta * p.kpar, own = kslabs / p.kpar;  // slabs of a tile per group
-        uint32_t most = std::min<uint32_t>(GROUPS, vtiles);
-        most -= most % p.kpar;
-        for (uint32_t ngrp = most; ngrp >= p.kpar; ngrp -= p.kpar) {
-            const uint32_t each = (vtiles + ngrp - 1u) / ngrp;  // tiles of the busiest group
-            for (uint32_t nsg = std::min<uint32_t>(MAX_NSG, each * own); nsg >= 1u; --nsg) {
-                // scales of every tile the code stages reach into: when the stage of a tile's first slab is
-                // free, so is the buffer of the tile nsb before it
-                const uint32_t nsb = std::min(each, (nsg - 1u + own - 1u) / own + 1u);
-                const size_t bytes = layout<S>(K, M, ngrp * nsg, ngrp / p.kpar * nsb, p.slab_row).total;
-                if (bytes > LIMIT) continue;
-                p.ngrp = ngrp, p.nsg = nsg, p.nsb = nsb;
-                p.smem = std::max<size_t>(bytes, 120 * 1024);
-                return p;
-            }
+    e.tiles = (N + 15u) / 16u;
+    e.grid = std::min<uint32_t>(e.tiles, (uint32_t)sm_count());
+    e.tiles_cta = (e.tiles + e.grid - 1u) / e.grid;
+    e.kslabs = (row_bytes + SLAB_ROW - 1u) / SLAB_ROW;
+    e.slab_row = row_bytes >= SLAB_ROW ? SLAB_ROW : (row_bytes + 127u) / 128u * 128u;
+    return e;
+}
+// Shared memory of a launch whose busiest group has `each` tiles (one reduction buffer is enough for one).
+template <class S>
+size_t smem_bytes(const Extent& e, uint32_t K, uint32_t M, uint32_t ngrp, uint32_t nsg, uint32_t nsb, uint32_t kpar, uint32_t each) {
+    return layout<S>(K, M, ngrp * nsg, ngrp / kpar * nsb, e.slab_row, each == 1u ? 1u : (uint32_t)Red<S::ROWS>::BUFS).total;
+}
+
+// How many groups share a tile: with few tiles per CTA and a long K two or four, each taking every kpar-th slab,
+// as far as M rows of activations leave room for a stage each.  0: M rows do not fit.
+template <class S>
+uint32_t choose_kpar(uint32_t N, uint32_t K, uint32_t M) {
+    if (K > (1u << 20)) return 0u;  // (the sums below stay inside 32 bits)
+    const Extent e = extent<S>(N, K);
+    uint32_t kpar = 1u;
+    while (kpar * 2u <= (uint32_t)GROUPS && e.tiles_cta * kpar * 2u <= (uint32_t)GROUPS && e.kslabs % (kpar * 2u) == 0u) kpar *= 2u;
+    for (; kpar >= 1u; kpar >>= 1)
+        if (smem_bytes<S>(e, K, M, kpar, 1u, 1u, kpar, e.tiles_cta) <= SMEM_LIMIT) return kpar;
+    return 0u;
+}
+
+// The plan for M rows with kpar groups to a tile, which fit.
+template <class S>
+Plan plan_launch(uint32_t N, uint32_t K, uint32_t M, uint32_t kpar) {
+    Plan p;
+    const Extent e = extent<S>(N, K);
+    p.grid = e.grid, p.kpar = kpar, p.slab_row = e.slab_row;
+    const uint32_t vtiles = e.tiles_cta * kpar, own = e.kslabs / kpar;  // slabs of a tile per group
+    uint32_t most = std::min<uint32_t>(GROUPS, vtiles);
+    most -= most % kpar;
+    for (uint32_t ngrp = most; ngrp >= kpar; ngrp -= kpar) {
+        const uint32_t each = (vtiles + ngrp - 1u) / ngrp;  // tiles of the busiest group
+        for (uint32_t nsg = std::min<uint32_t>(MAX_NSG, each * own); nsg >= 1u; --nsg) {
+            // scales of every tile the code stages reach into: when the stage of a tile's first slab is
+            // free, so is the buffer of the tile nsb before it
+            const uint32_t nsb = std::min(each, (nsg - 1u + own - 1u) / own + 1u);
+            const size_t bytes = smem_bytes<S>(e, K, M, ngrp, nsg, nsb, kpar, each);
+            if (bytes > SMEM_LIMIT) continue;
+            p.ngrp = ngrp, p.nsg = nsg, p.nsb = nsb;
+            p.smem = std::max<size_t>(bytes, 120 * 1024);
+            return p;
         }
     }
-    p.kpar = 1u;
     return p;
 }
 
@@ -1076,10 +1104,10 @@ int launch_one(const Plan& plan, const void* q, const Args& a, cudaStream_t stre
 
 template <class S>
 int launch_shape(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t M,
-                 uint32_t flags, cudaStream_t stream, const Shard& sh) {
-    const Plan plan = plan_launch<S>(N, K, M);
-    if (plan.ngrp == 0) return 1;
-    constexpr bool FEW = S::ROWS <= 4 || (S::ROWS == 8 && S::GROUP == 64);  // shapes that up to four rows run on
+                 uint32_t flags, cudaStream_t stream, const Shard& sh, uint32_t kpar) {
+    const Plan plan = plan_launch<S>(N, K, M, kpar);
+    if (plan.ngrp == 0) return fail(MIORI_E_INVALID, "gemv: no plan for N=%u K=%u M=%u", N, K, M);
+    constexpr bool FEW = S::ROWS <= 4 || (S::ROWS == 8 && S::GROUP == 64);  // shapes that up to four 4-bit rows run on
     const bool sharded = sh.pa.world > 1, argmax = sh.best != nullptr;
     const bool postnorm = sh.post.residual != nullptr, normed = sh.pre.gamma != nullptr;
     const bool placed = sharded || argmax;  // y is a slice of an n_total-row output
@@ -1115,27 +1143,70 @@ int launch_shape(const void* q, const void* s, const void* b, const void* x, voi
     return launch_one<S, NONE>(plan, q, a, stream);
 }
 
-// Launch, or return 1 if M rows of K activations do not fit shared memory (nothing launched).
+// ---- batches
+//
+// A row's bits must not depend on how many rows are in flight beside it, so everything that decides the order of
+// its sums -- the shape and how many groups share a tile -- is chosen by a class of batch sizes and not by M:
+// the class's largest batch has to fit, and where it does not, every batch of the class is dealt to launches of
+// the next smaller class.  Classes: 1..4 rows (4-bit weights in groups of 64: 1..2, see below), up to 8, 16, 32.
+template <int BITS, int GROUP>
+struct Batch {
+    // Three and four rows of 4-bit weights at group 64 gain nothing from slots (two, one step a pass): 16384 x
+    // 2048 takes 8.0 us with them and 7.2 without; they run as eight do.
+    static constexpr bool WIDE3 = BITS == 4 && GROUP == 64;
+    static constexpr uint32_t class_of(uint32_t M) { return M <= 2u ? (WIDE3 ? 2u : 4u) : M <= 4u ? (WIDE3 ? 8u : 4u) : M <= 8u ? 8u : M <= 16u ? 16u : 32u; }
+    static uint32_t kpar_of(uint32_t cls, uint32_t N, uint32_t K) {
+        switch (cls) {
+        case 1: return choose_kpar<Shape<BITS, GROUP, 1>>(N, K, 1);
+        case 2: return choose_kpar<Shape<BITS, GROUP, 2>>(N, K, 2);
+        case 4: return choose_kpar<Shape<BITS, GROUP, WIDE3 ? 8 : 4>>(N, K, 4);
+        case 8: return choose_kpar<Shape<BITS, GROUP, 8>>(N, K, 8);
+        case 16: return choose_kpar<Shape<BITS, GROUP, 16>>(N, K, 16);
+        default: return choose_kpar<Shape<BITS, GROUP, 32>>(N, K, 32);
+        }
+    }
+    // One launch of up to cls rows.  Below eight the shapes of fewer rows sum in the same order.
+    static int launch(uint32_t cls, uint32_t kpar, const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N,
+                      uint32_t K, uint32_t M, uint32_t flags, cudaStream_t stream, const Shard& sh) {
+#define MIORI_GEMV(ROWS) return launch_shape<Shape<BITS, GROUP, ROWS>>(q, s, b, x, y, N, K, M, flags, stream, sh, kpar)
+        if (cls > 16u) MIORI_GEMV(32);
+        if (cls > 8u) MIORI_GEMV(16);
+        if (cls > 4u || (WIDE3 && cls > 2u)) MIORI_GEMV(8);
+        if (M == 1u) MIORI_GEMV(1);
+        if (M == 2u) MIORI_GEMV(2);
+        if constexpr (!WIDE3) MIORI_GEMV(4);
+#undef MIORI_GEMV
+        return fail(MIORI_E_INVALID, "gemv: %u rows are not of the class of %u", M, cls);
+    }
+    static int run(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t M,
+                   uint32_t flags, cudaStream_t stream, Shard sh) {
+        uint32_t cls = class_of(M), kpar = 0;
+        if (flags & MIORI_TUNE_GEMV_ALIGNED) cls = std::max(cls, 8u);
+        while (cls && (kpar = kpar_of(cls, N, K)) == 0u) cls >>= 1;
+        if (!cls) return 1;
+        const uint32_t launches = (M + cls - 1u) / cls, rows = (M + launches - 1u) / launches;
+        const uint32_t n_out = sh.gated ? N / 2u : sh.pa.world > 1 || sh.best ? sh.n_total : N;
+        const size_t x_row = (size_t)K * (sh.pre.gamma ? 4 : 2), y_row = (size_t)n_out * ((flags & MIORI_OUT_BF16) ? 2 : 4);
+        for (uint32_t m0 = 0; m0 < M; m0 += rows) {
+            const int rc = launch(cls, kpar, q, s, b, static_cast<const uint8_t*>(x) + m0 * x_row, static_cast<uint8_t*>(y) + m0 * y_row,
+                                  N, K, std::min(rows, M - m0), flags, stream, sh);
+            if (rc) return rc;
+            sh.y_off += rows * y_row;
+            if (sh.post.residual) sh.post.residual += (size_t)rows * N;
+        }
+        return MIORI_OK;
+    }
+};
+
+// Launch, or return 1 if not even one row of K activations fits shared memory, or a fused form does not take the
+// shape (nothing launched).
 template <int BITS>
 int try_launch(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t M,
                uint32_t group, uint32_t flags, cudaStream_t stream, const Shard& sh = Shard()) {
     const bool fused = sh.pa.world > 1 || sh.best || sh.gated || sh.post.residual || sh.pre.gamma;
     if (fused && (K / group) % 8 != 0) return 1;  // what the fused entries promise to take
-#define MIORI_GEMV(ROWS)                                                                                  \
-    if (M <= ROWS)                                                                                        \
-        return group == 64 ? launch_shape<Shape<BITS, 64, ROWS>>(q, s, b, x, y, N, K, M, flags, stream, sh) \
-                           : launch_shape<Shape<BITS, 32, ROWS>>(q, s, b, x, y, N, K, M, flags, stream, sh)
-    const bool slots = !(flags & MIORI_TUNE_GEMV_ALIGNED);
-    if (slots) MIORI_GEMV(1);
-    if (slots) MIORI_GEMV(2);
-    // three and four rows of 4-bit weights at group 64 gain nothing from slots (two, one step a pass): 16384 x
-    // 2048 takes 8.0 us with them and 7.2 without.  At group 32 one to four rows share an arithmetic order.
-    if (slots && !(BITS == 4 && group == 64)) MIORI_GEMV(4);
-    MIORI_GEMV(8);
-    MIORI_GEMV(16);
-    MIORI_GEMV(32);
-#undef MIORI_GEMV
-    return 1;
+    return group == 64 ? Batch<BITS, 64>::run(q, s, b, x, y, N, K, M, flags, stream, sh)
+                       : Batch<BITS, 32>::run(q, s, b, x, y, N, K, M, flags, stream, sh);
 }
 
 }  // namespace gemvtma

@@ -21,27 +21,6 @@ int check_quant_args(const char* op, const void* q, const void* s, const void* b
     return MIORI_OK;
 }
 
-// The GEMV for M rows, as many of them a launch as its shared memory holds: all 32 at K <= 2304, eight at
-// K = 8192.  A row's value depends on the rows of its launch only through their number's class.
-template <int BITS>
-int gemv_rows(const char* op, const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N,
-              uint32_t K, uint32_t M, uint32_t group, uint32_t flags, void* stream,
-              const gemvtma::Shard& sh = gemvtma::Shard()) {
-    const size_t x_row = (size_t)K * (sh.pre.gamma ? 4 : 2), y_row = (size_t)N * ((flags & MIORI_OUT_BF16) ? 2 : 4);
-    for (uint32_t rows = M;; rows = (rows + 1u) / 2u) {
-        uint32_t m0 = 0;
-        for (; m0 < M; m0 += rows) {
-            const int rc = gemvtma::try_launch<BITS>(q, s, b, static_cast<const uint8_t*>(x) + m0 * x_row,
-                                                     static_cast<uint8_t*>(y) + m0 * y_row, N, K, std::min(rows, M - m0),
-                                                     group, flags, (cudaStream_t)stream, sh);
-            if (rc < 0) return rc;
-            if (rc == 1) break;  // too many rows (the first launch of a size tells for all of them)
-        }
-        if (m0 >= M) return MIORI_OK;
-        if (rows == 1u) return fail(MIORI_E_INVALID, "%s: K=%u too large for the activation staging", op, K);
-    }
-}
-
 template <int BITS>
 int gemv_entry(const char* op, const void* q, const void* s, const void* b, const void* x, void* y,
                uint32_t N, uint32_t K, uint32_t M, uint32_t group, uint32_t flags, void* stream) {
@@ -50,7 +29,8 @@ int gemv_entry(const char* op, const void* q, const void* s, const void* b, cons
     if (!x || !y) return fail(MIORI_E_INVALID, "%s: null activation pointer", op);
     if (M == 0 || M > 32) return fail(MIORI_E_INVALID, "%s: M=%u outside 1..32", op, M);
     if (!aligned16(x)) return fail(MIORI_E_INVALID, "%s: x must be 16-byte aligned", op);
-    return gemv_rows<BITS>(op, q, s, b, x, y, N, K, M, group, flags, stream);
+    rc = gemvtma::try_launch<BITS>(q, s, b, x, y, N, K, M, group, flags, (cudaStream_t)stream);
+    return rc == 1 ? fail(MIORI_E_INVALID, "%s: K=%u too large for the activation staging", op, K) : rc;
 }
 
 }  // namespace
@@ -83,7 +63,8 @@ int gemv_rmsnorm_entry(const char* op, const void* q, const void* s, const void*
     gemvtma::Shard sh;
     sh.pre.gamma = static_cast<const uint16_t*>(gamma);
     sh.pre.eps = eps;
-    return gemv_rows<BITS>(op, q, s, b, x, y, N, K, M, group, flags, stream, sh);
+    rc = gemvtma::try_launch<BITS>(q, s, b, x, y, N, K, M, group, flags, (cudaStream_t)stream, sh);
+    return rc == 1 ? fail(MIORI_E_INVALID, "%s: K=%u too large for the activation staging", op, K) : rc;
 }
 }  // namespace
 
@@ -93,7 +74,6 @@ MIORI_API int miori_gemv4_silu(const void* q, const void* s, const void* b, cons
     int rc = check_quant_args(op, q, s, b, N, K, group);
     if (rc) return rc;
     if (!x || !y) return fail(MIORI_E_INVALID, "%s: null activation pointer", op);
-    // 17..32 staged rows do not fit the kernel's shared memory at any K
     if (M == 0 || M > 16) return fail(MIORI_E_INVALID, "%s: M=%u outside 1..16", op, M);
     if (!aligned16(x)) return fail(MIORI_E_INVALID, "%s: x must be 16-byte aligned", op);
     if (N % 16 != 0)

@@ -113,3 +113,35 @@ def test_error_is_that_of_fp32_sums(bits, group, N, K, M):
     want = x.double() @ _weights64(q, s, b, bits, group).T
     got = OPS[bits](q, s, b, x, group=group).double()
     assert float((got - want).norm() / want.norm()) < 4 * 2.0 ** -24
+
+
+# shapes where the number of groups that share a tile, or of launches that a batch is dealt to, would change inside the class
+@pytest.mark.parametrize("bits,group,N,K,lo,hi", [
+    (4, 64, 2048, 8192, 3, 8), (4, 64, 256, 8192, 9, 16), (4, 32, 256, 8192, 5, 8), (4, 64, 1024, 16384, 3, 8), (4, 64, 1024, 16384, 1, 2),
+    (8, 64, 2048, 4096, 9, 16), (8, 32, 64, 16384, 1, 4), (4, 64, 256, 3072, 17, 32), (4, 32, 48, 6144, 9, 16), (8, 64, 48, 8192, 17, 32)])
+def test_a_row_does_not_depend_on_the_batch_of_its_class(bits, group, N, K, lo, hi):
+    q, s, b = synth.make_weight(N, K, bits, group, seed=K, device=DEV)
+    x = synth.make_activation(hi, K, seed=9, device=DEV)
+    full = OPS[bits](q, s, b, x, group=group)
+    for M in range(lo, hi):
+        assert torch.equal(OPS[bits](q, s, b, x[:M].contiguous(), group=group), full[:M]), M
+
+
+@pytest.mark.parametrize("group,K,M", [(32, 32768, 2), (64, 8192, 9), (64, 16384, 4)])
+def test_fused_forms_of_batches_dealt_to_several_launches(group, K, M):
+    """Bit for bit the unfused pair, also where a launch does not hold the batch."""
+    N = 64
+    q, s, b = synth.make_weight(N, K, 4, group, seed=K, device=DEV)
+    x = synth.make_activation(M, K, seed=M, device=DEV)
+    v = miori_b200.gemv4(q, s, b, x, group=group)
+    want = miori_b200.silu_mul(v[:, :N // 2].contiguous(), v[:, N // 2:].contiguous())
+    assert torch.equal(miori_b200.gemv4_silu(q, s, b, x, group=group), want)
+    if M <= 4:
+        res, w = torch.randn((M, N), device=DEV), synth.make_activation(1, N, seed=1, device=DEV).reshape(-1)
+        counter = torch.zeros(1, dtype=torch.int32, device=DEV)
+        got = miori_b200.gemv4_post_norm_add(q, s, b, x, res, w, 1e-5, counter, group=group)
+        assert torch.equal(got, miori_b200.post_norm_add(res, v, w, 1e-5)) and int(counter) == 0
+        xf, g = x.float() * 3.0, synth.make_activation(1, K, seed=2, device=DEV).reshape(-1)
+        y = miori_b200.gemv4_rmsnorm(q, s, b, xf, g, 1e-5, group=group)
+        z = miori_b200.silu_mul(y[:, :N // 2].contiguous(), y[:, N // 2:].contiguous())
+        assert torch.equal(miori_b200.gemv4_rmsnorm_silu(q, s, b, xf, g, 1e-5, group=group), z)
