@@ -12,6 +12,7 @@
 
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <dlfcn.h>
@@ -83,8 +84,11 @@ struct Args {
         return (uint32_t)r;
     }
     float f32(int i) const {
-        const double d = PyFloat_AsDouble(v[i]);
-        if (d == -1.0 && PyErr_Occurred()) throw Failed();
+        if (PyFloat_CheckExact(v[i])) return (float)PyFloat_AS_DOUBLE(v[i]);
+        PyObject* f = PyNumber_Float(v[i]);  // whatever float() takes
+        if (!f) throw Failed();
+        const double d = PyFloat_AS_DOUBLE(f);
+        Py_DECREF(f);
         return (float)d;
     }
 };
@@ -111,27 +115,35 @@ struct Out {
         return THPVariable_Wrap(std::move(made));
     }
 };
-template <class F>
-Out output(const Args& a, int i, F make) {
+// Memory of the caller's that a kernel writes: on a GPU or pinned, contiguous, large enough.
+void need_room(const at::Tensor& t, const char* what, size_t bytes) {
+    if (!t.is_cuda() && !t.is_pinned()) raise(PyExc_ValueError, "%s: a CUDA tensor is expected", what);
+    if (!t.is_contiguous()) raise(PyExc_ValueError, "%s: a contiguous tensor is expected", what);
+    if ((size_t)t.numel() * t.element_size() < bytes)
+        raise(PyExc_ValueError, "%s: %zu bytes needed, the tensor has %zu", what, bytes, (size_t)t.numel() * t.element_size());
+}
+// `need`: what the kernel writes, where that is not the type of a new tensor.
+Out output(const Args& a, int i, at::IntArrayRef shape, at::ScalarType dt, const at::Tensor& like,
+           at::ScalarType need = at::ScalarType::Undefined) {
     Out o;
     if (a.given(i)) {
-        a.tensor(i);
+        size_t bytes = c10::elementSize(need == at::ScalarType::Undefined ? dt : need);
+        for (const int64_t n : shape) bytes *= (size_t)n;
+        need_room(a.tensor(i), "out", bytes);
         o.given = a.v[i];
     } else {
-        o.made = make();
+        o.made = empty(shape, dt, like);
     }
     return o;
 }
 
-// Call into the library without the interpreter lock (a launch may block on a full queue).
-template <class F>
-void call(F f) {
-    int rc;
-    {
-        PyThreadState* ts = PyEval_SaveThread();
-        rc = f();
-        PyEval_RestoreThread(ts);
-    }
+// Call into the library without the interpreter lock (a launch may block on a full queue).  The arguments
+// are evaluated before, under the lock: reading a tensor's pointer may throw.
+template <class... P, class... A>
+void call(int (*fn)(P...), A... args) {
+    PyThreadState* ts = PyEval_SaveThread();
+    const int rc = fn(static_cast<P>(args)...);
+    PyEval_RestoreThread(ts);
     if (rc != MIORI_OK) {
         PyObject* exc = PyObject_CallFunction(g_error, "is", rc, abi.last_error());
         if (exc) {
@@ -147,8 +159,8 @@ PyObject* guarded(F body) {
     try {
         return body();
     } catch (const Failed&) {
-    } catch (const std::exception& e) {  // torch's allocator: out of memory
-        PyErr_SetString(PyExc_RuntimeError, e.what());
+    } catch (...) {  // torch's own, as its operators raise them: out of memory, no storage, a missing dimension
+        torch::translate_exception_to_python(std::current_exception());
     }
     return nullptr;
 }
@@ -186,10 +198,8 @@ PyObject* gemv(const Args& a, decltype(abi.gemv4) fn, int64_t per_word) {
     check_words(q, per_word, K);
     const int64_t N = q.size(0);
     const uint32_t group = a.u32(4, 32), flags = a.u32(5, 0);
-    Out y = output(a, 6, [&] { return empty({M, N}, out_type(flags), x); });
-    call([&] {
-        return fn(q.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), y.ptr(), N, K, M, group, flags, stream());
-    });
+    Out y = output(a, 6, {M, N}, out_type(flags), x);
+    call(fn, q.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), y.ptr(), N, K, M, group, flags, stream());
     return y.result();
 }
 OP(gemv4, 4, "q", "s", "b", "x", "group", "flags", "out") { return gemv(a, abi.gemv4, 8); }
@@ -200,11 +210,9 @@ PyObject* dequant(const Args& a, decltype(abi.dequant4_rowmajor) fn, int64_t per
     need_cuda({&q, &s, &b});
     const int64_t N = q.size(0), K = q.size(1) * per_word;
     const uint32_t group = a.u32(3, 32);
-    Out o = output(a, 4, [&] {
-        if (flat) return empty({(int64_t)(abi.cache_bytes(N, K) / 2)}, at::kBFloat16, q);
-        return empty({N, K}, at::kBFloat16, q);
-    });
-    call([&] { return fn(q.data_ptr(), s.data_ptr(), b.data_ptr(), o.ptr(), N, K, group, stream()); });
+    const int64_t flat_shape[1] = {(int64_t)(abi.cache_bytes(N, K) / 2)}, shape[2] = {N, K};
+    Out o = output(a, 4, flat ? at::IntArrayRef(flat_shape) : at::IntArrayRef(shape), at::kBFloat16, q);
+    call(fn, q.data_ptr(), s.data_ptr(), b.data_ptr(), o.ptr(), N, K, group, stream());
     return o.result();
 }
 OP(dequant4_rowmajor, 3, "q", "s", "b", "group", "out") { return dequant(a, abi.dequant4_rowmajor, 8, false); }
@@ -216,6 +224,7 @@ void workspace(const Args& a, int i, void*& p, size_t& bytes) {
     p = nullptr, bytes = 0;
     if (!a.given(i)) return;
     const at::Tensor& w = a.tensor(i);
+    need_room(w, "workspace", 0);
     p = w.data_ptr();
     bytes = (size_t)w.numel() * w.element_size();
 }
@@ -226,13 +235,11 @@ OP(gemm_bf16_cache, 3, "A", "cache", "N", "flags", "out", "workspace") {
     if (A.dim() != 2) raise(PyExc_ValueError, "gemm_bf16_cache: A [M][K] expected");
     const int64_t M = A.size(0), K = A.size(1), N = a.u32(2, 0);
     const uint32_t flags = a.u32(3, 0);
-    Out c = output(a, 4, [&] { return empty({M, N}, out_type(flags), A); });
+    Out c = output(a, 4, {M, N}, out_type(flags), A);
     void* wp;
     size_t wb;
     workspace(a, 5, wp, wb);
-    call([&] {
-        return abi.gemm_bf16_cache_ws(A.data_ptr(), cache.data_ptr(), c.ptr(), M, N, K, flags, wp, wb, stream());
-    });
+    call(abi.gemm_bf16_cache_ws, A.data_ptr(), cache.data_ptr(), c.ptr(), M, N, K, flags, wp, wb, stream());
     return c.result();
 }
 
@@ -246,14 +253,15 @@ OP(gemm_bf16_strided, 2, "A", "B", "flags", "out") {
     const int64_t M = A.size(0), K = A.size(1), N = B.size(0);
     const uint32_t flags = a.u32(2, 0);
     const at::ScalarType dt = out_type(flags);
-    Out o = output(a, 3, [&] { return empty({M, N}, dt, A); });
+    Out o;  // rows of a caller's output may lie apart
+    if (a.given(3)) a.tensor(3), o.given = a.v[3];
+    else o.made = empty({M, N}, dt, A);
     const at::Tensor& c = o.given ? THPVariable_Unpack(o.given) : o.made;
+    if (!c.is_cuda() && !c.is_pinned()) raise(PyExc_ValueError, "out: a CUDA tensor is expected");
     if (c.scalar_type() != dt || c.dim() != 2 || c.size(0) != M || c.size(1) != N || c.stride(1) != 1)
         raise(PyExc_ValueError, "gemm_bf16_strided: bad output tensor");
-    call([&] {
-        return abi.gemm_bf16_strided(A.data_ptr(), A.stride(0), B.data_ptr(), B.stride(0), c.data_ptr(), c.stride(0), M, N,
-                                     K, flags, stream());
-    });
+    call(abi.gemm_bf16_strided, A.data_ptr(), A.stride(0), B.data_ptr(), B.stride(0), c.data_ptr(), c.stride(0), M, N,
+         K, flags, stream());
     return o.result();
 }
 
@@ -263,8 +271,8 @@ OP(gemv_bf16_cache, 3, "x", "cache", "N", "flags", "out") {
     if (x.dim() != 2) raise(PyExc_ValueError, "gemv_bf16_cache: x [M][K] expected");
     const int64_t M = x.size(0), K = x.size(1), N = a.u32(2, 0);
     const uint32_t flags = a.u32(3, 0);
-    Out y = output(a, 4, [&] { return empty({M, N}, out_type(flags), x); });
-    call([&] { return abi.gemv_bf16_cache(x.data_ptr(), cache.data_ptr(), y.ptr(), M, N, K, flags, stream()); });
+    Out y = output(a, 4, {M, N}, out_type(flags), x);
+    call(abi.gemv_bf16_cache, x.data_ptr(), cache.data_ptr(), y.ptr(), M, N, K, flags, stream());
     return y.result();
 }
 
@@ -275,14 +283,12 @@ OP(linear4, 5, "q", "s", "b", "cache", "x", "group", "flags", "out", "workspace"
     const int64_t M = x.size(0), K = x.size(1), N = q.size(0);
     const void* cache = a.given(3) ? a.tensor(3).data_ptr() : nullptr;
     const uint32_t group = a.u32(5, 32), flags = a.u32(6, 0);
-    Out y = output(a, 7, [&] { return empty({M, N}, at::kFloat, x); });
+    Out y = output(a, 7, {M, N}, at::kFloat, x, out_type(flags));
     void* wp;
     size_t wb;
     workspace(a, 8, wp, wb);
-    call([&] {
-        return abi.linear4(q.data_ptr(), s.data_ptr(), b.data_ptr(), cache, x.data_ptr(), y.ptr(), N, K, M, group, flags,
-                           wp, wb, stream());
-    });
+    call(abi.linear4, q.data_ptr(), s.data_ptr(), b.data_ptr(), cache, x.data_ptr(), y.ptr(), N, K, M, group, flags,
+         wp, wb, stream());
     return y.result();
 }
 
@@ -293,8 +299,8 @@ OP(rmsnorm, 3, "x", "gamma", "eps", "flags", "out") {
     const int64_t rows = x.size(0), n = x.size(1);
     const float eps = a.f32(2);
     const uint32_t flags = a.u32(3, 0);
-    Out y = output(a, 4, [&] { return empty({rows, n}, at::kBFloat16, x); });
-    call([&] { return abi.rmsnorm(x.data_ptr(), gamma.data_ptr(), y.ptr(), rows, n, eps, flags, stream()); });
+    Out y = output(a, 4, {rows, n}, at::kBFloat16, x);
+    call(abi.rmsnorm, x.data_ptr(), gamma.data_ptr(), y.ptr(), rows, n, eps, flags, stream());
     return y.result();
 }
 
@@ -305,10 +311,8 @@ OP(post_norm_add, 4, "x", "src", "gamma", "eps", "flags", "out") {
     const int64_t rows = x.size(0), n = x.size(1);
     const float eps = a.f32(3);
     const uint32_t flags = a.u32(4, 0);
-    Out o = output(a, 5, [&] { return empty(x.sizes(), x.scalar_type(), x); });
-    call([&] {
-        return abi.post_norm_add(x.data_ptr(), src.data_ptr(), gamma.data_ptr(), o.ptr(), rows, n, eps, flags, stream());
-    });
+    Out o = output(a, 5, {rows, n}, x.scalar_type(), x, at::kFloat);
+    call(abi.post_norm_add, x.data_ptr(), src.data_ptr(), gamma.data_ptr(), o.ptr(), rows, n, eps, flags, stream());
     return o.result();
 }
 
@@ -316,8 +320,8 @@ OP(silu_mul, 2, "gate", "up", "flags", "out") {
     const at::Tensor &gate = a.tensor(0), &up = a.tensor(1);
     need_cuda({&gate, &up});
     const uint32_t flags = a.u32(2, 0);
-    Out o = output(a, 3, [&] { return empty(gate.sizes(), at::kBFloat16, gate); });
-    call([&] { return abi.silu_mul(gate.data_ptr(), up.data_ptr(), o.ptr(), gate.numel(), flags, stream()); });
+    Out o = output(a, 3, gate.sizes(), at::kBFloat16, gate);
+    call(abi.silu_mul, gate.data_ptr(), up.data_ptr(), o.ptr(), gate.numel(), flags, stream());
     return o.result();
 }
 
@@ -326,11 +330,9 @@ OP(embed8, 4, "q", "s", "b", "tokens", "group", "flags", "out") {
     need_cuda({&q, &s, &b, &tokens});
     const int64_t rows = q.size(0), K = q.size(1) * 4, T = tokens.numel();
     const uint32_t group = a.u32(4, 32), flags = a.u32(5, 0);
-    Out o = output(a, 6, [&] { return empty({T, K}, at::kBFloat16, q); });
-    call([&] {
-        return abi.embed8(q.data_ptr(), s.data_ptr(), b.data_ptr(), tokens.data_ptr(), o.ptr(), T, rows, K, group, flags,
-                          stream());
-    });
+    Out o = output(a, 6, {T, K}, at::kBFloat16, q);
+    call(abi.embed8, q.data_ptr(), s.data_ptr(), b.data_ptr(), tokens.data_ptr(), o.ptr(), T, rows, K, group, flags,
+         stream());
     return o.result();
 }
 
@@ -339,7 +341,7 @@ OP(argmax, 1, "v", "flags") {
     need_cuda({&v});
     const uint32_t flags = a.u32(1, 0) | (v.scalar_type() == at::kBFloat16 ? MIORI_OUT_BF16 : 0u);
     at::Tensor idx = empty({1}, at::kInt, v), val = empty({1}, at::kFloat, v);
-    call([&] { return abi.argmax(v.data_ptr(), v.numel(), flags, idx.data_ptr(), val.data_ptr(), stream()); });
+    call(abi.argmax, v.data_ptr(), v.numel(), flags, idx.data_ptr(), val.data_ptr(), stream());
     PyObject* pair = PyTuple_New(2);
     if (!pair) throw Failed();
     PyTuple_SET_ITEM(pair, 0, THPVariable_Wrap(std::move(idx)));
@@ -359,11 +361,9 @@ PyObject* gemv_rmsnorm(const Args& a, decltype(abi.gemv4_rmsnorm) fn) {
     const int64_t N = q.size(0);
     const float eps = a.f32(5);
     const uint32_t group = a.u32(6, 32), flags = a.u32(7, 0);
-    Out y = output(a, 8, [&] { return empty({M, N}, out_type(flags), x); });
-    call([&] {
-        return fn(q.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), gamma.data_ptr(), eps, y.ptr(), N, K, M, group,
-                  flags, stream());
-    });
+    Out y = output(a, 8, {M, N}, out_type(flags), x);
+    call(fn, q.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), gamma.data_ptr(), eps, y.ptr(), N, K, M, group,
+         flags, stream());
     return y.result();
 }
 OP(gemv4_rmsnorm, 6, "q", "s", "b", "x", "gamma", "eps", "group", "flags", "out") { return gemv_rmsnorm(a, abi.gemv4_rmsnorm); }
@@ -377,11 +377,9 @@ OP(gemv4_silu, 4, "q", "s", "b", "x", "group", "flags", "out") {
     check_words(q, 8, K);
     const int64_t N = q.size(0);
     const uint32_t group = a.u32(4, 32), flags = a.u32(5, 0);
-    Out y = output(a, 6, [&] { return empty({M, N / 2}, at::kBFloat16, x); });
-    call([&] {
-        return abi.gemv4_silu(q.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), y.ptr(), N, K, M, group, flags,
-                              stream());
-    });
+    Out y = output(a, 6, {M, N / 2}, at::kBFloat16, x);
+    call(abi.gemv4_silu, q.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), y.ptr(), N, K, M, group, flags,
+         stream());
     return y.result();
 }
 
@@ -397,11 +395,9 @@ OP(gemv4_post_norm_add, 8, "q", "s", "b", "x", "residual", "gamma", "eps", "coun
         raise(PyExc_ValueError, "residual: fp32 [M][N] expected");
     const float eps = a.f32(6);
     const uint32_t group = a.u32(8, 32), flags = a.u32(9, 0);
-    Out o = output(a, 10, [&] { return empty({M, N}, at::kFloat, x); });
-    call([&] {
-        return abi.gemv4_post_norm_add(q.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), residual.data_ptr(),
-                                       gamma.data_ptr(), eps, counter.data_ptr(), o.ptr(), N, K, M, group, flags, stream());
-    });
+    Out o = output(a, 10, {M, N}, at::kFloat, x);
+    call(abi.gemv4_post_norm_add, q.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), residual.data_ptr(),
+         gamma.data_ptr(), eps, counter.data_ptr(), o.ptr(), N, K, M, group, flags, stream());
     return o.result();
 }
 
@@ -414,11 +410,9 @@ OP(gemv4_rmsnorm_silu, 6, "q", "s", "b", "x", "gamma", "eps", "group", "flags", 
     const int64_t N = q.size(0);
     const float eps = a.f32(5);
     const uint32_t group = a.u32(6, 32), flags = a.u32(7, 0);
-    Out y = output(a, 8, [&] { return empty({M, N / 2}, at::kBFloat16, x); });
-    call([&] {
-        return abi.gemv4_rmsnorm_silu(q.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), gamma.data_ptr(), eps,
-                                      y.ptr(), N, K, M, group, flags, stream());
-    });
+    Out y = output(a, 8, {M, N / 2}, at::kBFloat16, x);
+    call(abi.gemv4_rmsnorm_silu, q.data_ptr(), s.data_ptr(), b.data_ptr(), x.data_ptr(), gamma.data_ptr(), eps,
+         y.ptr(), N, K, M, group, flags, stream());
     return y.result();
 }
 

@@ -36,6 +36,54 @@ def test_no_operator_takes_cpu_tensors(name):
         getattr(ops, name)(*args)
 
 
+def _fakes():
+    """CUDA tensors without memory."""
+    from torch._subclasses import FakeTensorMode
+    with FakeTensorMode():
+        return {"q": torch.empty((16, 8), dtype=torch.int32, device="cuda"), "s": torch.empty((16, 2), dtype=torch.bfloat16, device="cuda"),
+                "x": torch.empty((1, 64), dtype=torch.bfloat16, device="cuda"), "y": torch.empty((1, 16), device="cuda"),
+                "strided": torch.empty((4, 32), device="cuda")[:, :16], "f": torch.empty((1, 64), device="cuda")}
+
+
+def test_tensors_without_storage_raise():
+    """Reading such a tensor's pointer throws inside the C function: an exception as from torch's own operators."""
+    f = _fakes()
+    for call in (lambda: ops.gemv4(f["q"], f["s"], f["s"], f["x"], group=32, out=f["y"]),
+                 lambda: ops.gemm_bf16_cache(f["x"], f["x"], 16, out=f["y"]),
+                 lambda: ops.gemm_bf16_cache(f["x"], f["x"], 16, out=f["y"], workspace=f["y"]),
+                 lambda: ops.silu_mul(f["f"], f["f"], out=f["f"]), lambda: ops.post_norm_add(f["f"], f["f"], f["x"], 1e-5, out=f["f"]),
+                 lambda: ops.rmsnorm(f["f"], f["x"], "1e-5", out=f["f"])):
+        with pytest.raises(RuntimeError):
+            call()
+    with pytest.raises(IndexError):
+        ops.gemv4(f["q"][0], f["s"], f["s"], f["x"], out=f["y"])
+
+
+def test_outputs_and_workspaces_are_checked():
+    f = _fakes()
+    host = torch.zeros((1, 16))
+    args = (f["q"], f["s"], f["s"], f["x"])
+    with pytest.raises(ValueError, match="out: a CUDA tensor"):
+        ops.gemv4(*args, out=host)
+    with pytest.raises(ValueError, match="out: a CUDA tensor"):
+        ops.gemm_bf16_strided(f["x"], f["x"], out=torch.zeros((1, 1)))
+    with pytest.raises(ValueError, match="out: 64 bytes needed, the tensor has 32"):
+        ops.gemv4(*args, out=f["y"][:, :8])
+    with pytest.raises(ValueError, match="out: a contiguous tensor"):
+        ops.gemv4(f["q"], f["s"], f["s"], f["x"].expand(4, 64).clone(), out=f["strided"])
+    with pytest.raises(ValueError, match="out: 128 bytes needed"):
+        ops.rmsnorm(f["f"], f["x"], 1e-5, out=f["y"])
+    with pytest.raises(ValueError, match="workspace: a CUDA tensor"):
+        ops.gemm_bf16_cache(f["x"], f["x"], 16, out=f["y"], workspace=host)
+
+
+@pytest.mark.gpu
+def test_out_of_memory_is_torchs():
+    A = torch.zeros((64, 64), dtype=torch.bfloat16, device="cuda:0")
+    with pytest.raises(torch.OutOfMemoryError):
+        ops.gemm_bf16_cache(A, A, 2 ** 32 - 8)  # an output of a terabyte
+
+
 @pytest.mark.gpu
 def test_given_and_allocated_outputs():
     dev = "cuda:0"
