@@ -120,7 +120,8 @@ int miori_dequant8_rowmajor(const void* q, const void* s, const void* b, void* o
  * miori_cache_bytes gives its size and miori_cache_to_rowmajor undoes the layout.  One promise
  * is public: weight rows are stored one after the other, so bytes [miori_cache_bytes(r0, K),
  * miori_cache_bytes(r0 + n, K)) of a cache are the cache of its rows r0 .. r0 + n - 1, and a
- * row shard of a projection needs no copy. */
+ * row shard of a projection needs no copy.  A launch with MIORI_LAUNCH_PDL may follow a build on its
+ * stream: the build lets nothing start before its weights are written. */
 size_t miori_cache_bytes(uint32_t N, uint32_t K);
 int miori_dequant4_cache(const void* q, const void* s, const void* b, void* cache,
                          uint32_t N, uint32_t K, uint32_t group, void* stream);

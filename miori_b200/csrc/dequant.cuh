@@ -7,7 +7,7 @@
 // 8 i / group, and no row or column is ever computed.  A thread takes UNITS units one block width apart:
 // every load and store instruction of a warp covers contiguous memory (128-256 bytes of codes, 512 of
 // output), and all loads are issued before the first use.  Chained launches of 16384 x 2048: 25.7 us with
-// a 64-bit division per unit and one unit in flight, 17.0 now (5.05 TB/s); 8-bit 25.7 and 18.7 (5.6 TB/s).
+// a 64-bit division per unit and one unit in flight, 17.3 now (5.0 TB/s).
 #pragma once
 #include "common.cuh"
 
@@ -45,9 +45,7 @@ template <int BITS, int UNITS>
 __global__ void __launch_bounds__(DEQUANT_THREADS)
 dequant_rowmajor_kernel(const uint32_t* __restrict__ q, const uint16_t* __restrict__ s, const uint16_t* __restrict__ b,
                         uint4* __restrict__ out, uint64_t units, uint32_t ushift) {
-    // a programmatic launch, which costs the host less, that waits and only then lets dependents start early
-    pdl_wait_prior();
-    pdl_launch_dependents();
+    pdl_wait_prior();  // a programmatic launch, which costs the host less
     const uint64_t first = (uint64_t)blockIdx.x * (DEQUANT_THREADS * UNITS) + threadIdx.x;
     uint32_t w[UNITS][BITS / 4], sc[UNITS], bi[UNITS];
 #pragma unroll
@@ -69,6 +67,12 @@ dequant_rowmajor_kernel(const uint32_t* __restrict__ q, const uint16_t* __restri
         const uint64_t i = first + (uint64_t)(j * DEQUANT_THREADS);
         if (i < units) out[i] = dequant_unit<BITS>(w[j], sc[j], bi[j]);
     }
+    // No early trigger: dependents start when every CTA has exited, and a CTA exits with its weights written.
+    // A product launched early fetches its first tiles of a cache ahead of its wait for the kernel before it, and
+    // that may be the cache's build.  (Built and multiplied in turn in a graph, 2048 x 2048 gave wrong products with
+    // the trigger at the top.  The fence costs 0.6 us: 16384 x 2048 16.6 -> 17.3; without it the writes of a CTA
+    // that has exited may still be under way, though no product has come out wrong then.)
+    __threadfence();
 }
 
 template <int BITS>

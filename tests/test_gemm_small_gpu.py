@@ -7,6 +7,7 @@ import pytest
 import torch
 
 import miori_b200
+from miori_b200 import synth
 from conftest import assert_close, u16
 
 pytestmark = pytest.mark.gpu
@@ -70,3 +71,31 @@ def test_pair_tiles_of_192_columns(port, M, N, K):
     c16 = miori_b200.gemm_bf16_cache(A, B.view(-1), N, flags=miori_b200.OUT_BF16)
     assert torch.equal(c16, guard[1:M + 1].to(torch.bfloat16))
     assert miori_b200.lib.miori_device_error_poll() == 0
+
+
+@pytest.mark.parametrize("N,K", [(512, 2048), (2048, 2048), (16384, 2048)])
+@pytest.mark.parametrize("M", [8, 32, 77, 256])
+def test_early_launch_reads_the_cache_built_before_it(N, K, M):
+    """A product launched early right behind the build of its cache, or with another early launch between, reads
+    what the build wrote.  Replayed as a graph, so that nothing but the device orders them."""
+    ws = [synth.make_weight(N, K, 4, 64, seed=i, device=DEV) for i in (1, 2)]
+    x = synth.make_activation(M, K, seed=3, device=DEV)
+    cache = torch.empty(N * K, dtype=torch.bfloat16, device=DEV)
+    xf, g = torch.randn((1, 2048), device=DEV), torch.ones(2048, dtype=torch.bfloat16, device=DEV)
+    product = miori_b200.gemv_bf16_cache if M == 8 else miori_b200.gemm_bf16_cache
+    want = []
+    for w in ws:
+        miori_b200.dequant4_cache(*w, group=64, out=cache)
+        torch.cuda.synchronize()
+        want.append(product(x, cache, N))
+    graph, got = torch.cuda.CUDAGraph(), []
+    with torch.cuda.graph(graph):
+        for i in range(16):
+            miori_b200.dequant4_cache(*ws[i % 2], group=64, out=cache)
+            if i % 4 >= 2:
+                miori_b200.rmsnorm(xf, g, 1e-5, flags=miori_b200.LAUNCH_PDL)
+            got.append(product(x, cache, N, flags=miori_b200.LAUNCH_PDL))
+    for _ in range(3):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert [i for i, y in enumerate(got) if not torch.equal(y, want[i % 2])] == []
