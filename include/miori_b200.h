@@ -151,7 +151,8 @@ int miori_gemm_plan(uint32_t M, uint32_t N, uint32_t K, size_t workspace_bytes, 
  * (small M or N, long K) split K across SMs: partial tiles go to `workspace` (fp32) and a
  * second kernel sums them in a fixed order, so results stay reproducible.  (Up to 48 rows the
  * slices are the CTAs of a cluster, their number depends on N and K only, and the partials meet
- * on the chip: the workspace is then the permission to split, and is not written.)
+ * on the chip: a workspace of any size is then the permission to split, and is not written; one of no
+ * bytes is none.)
  * miori_gemm_workspace_bytes gives the size worth passing (0: the shape does not split); a
  * smaller or NULL workspace only reduces or disables the splitting.  The workspace
  * contents are scratch; two launches in flight at once must not share it.  (The reference has no

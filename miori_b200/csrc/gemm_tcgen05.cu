@@ -871,11 +871,12 @@ MIORI_API int miori_gemm_bf16_cache_ws(const void* A, const void* cache, void* C
     if (rc) return rc;
     if (workspace && !aligned16(workspace))
         return fail(MIORI_E_INVALID, "miori_gemm_bf16_cache: workspace must be 16-byte aligned");
+    if (!workspace) workspace_bytes = 0;
     if (!(flags & MIORI_TUNE_GEMM_MASK)) {
-        const uint32_t cs = gemm::skinny::plan(M, N, K, workspace != nullptr);
+        const uint32_t cs = gemm::skinny::plan(M, N, K, workspace_bytes != 0);
         if (cs) return gemm::skinny::launch_skinny(A, cache, Cm, M, N, K, flags, cs, (cudaStream_t)stream);
     }
-    const gemm::GemmPlan p = gemm::plan_gemm(M, N, K, flags, workspace ? workspace_bytes : 0);
+    const gemm::GemmPlan p = gemm::plan_gemm(M, N, K, flags, workspace_bytes);
     float* ws = reinterpret_cast<float*>(workspace);
     return gemm::run_plan(p, A, cache, Cm, M, N, K, flags, ws, (cudaStream_t)stream);
 }

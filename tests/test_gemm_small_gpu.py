@@ -21,6 +21,20 @@ def _bf16(rows, cols, seed):
     return torch.randn((rows, cols), generator=g, device=DEV).to(torch.bfloat16)
 
 
+def test_a_workspace_of_no_bytes_is_none():
+    M, N, K = 32, 512, 4096
+    A, B, ws = _bf16(M, K, 1), _bf16(N, K, 2), torch.empty(1 << 20, device=DEV)
+
+    def product(nbytes):
+        c = torch.empty((M, N), device=DEV)
+        rc = miori_b200.lib.miori_gemm_bf16_cache_ws(A.data_ptr(), B.data_ptr(), c.data_ptr(), M, N, K, 0, ws.data_ptr(), nbytes,
+                                                     torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        return c
+    unsplit = miori_b200.gemm_bf16_cache(A, B.view(-1), N)
+    assert torch.equal(product(0), unsplit) and not torch.equal(product(4 << 20), unsplit)
+
+
 # N, K: clusters of 8, 8, 4, 2, 1 and 1 CTAs; ragged last tiles, uneven slices, one k-block
 @pytest.mark.parametrize("N,K", [(8, 4096), (1000, 4160), (2056, 2112), (5000, 1088), (136, 64), (16384, 192)])
 @pytest.mark.parametrize("M", [1, 15, 17, 32, 48])
