@@ -758,7 +758,7 @@ struct GemmPlan {
 // as few as the 256-wide ones' (1024 x 3072: 16.6 -> 14.4, 768 x 8192: 26.5 -> 23.6, 2048 x 3072: 26.0 ->
 // 23.3, 1536 x 2048 at K = 8192: 45.0 -> 40.4).  Splitting K therefore happens when the tiles alone would leave most SMs
 // idle and K is long enough to pay for the reduction, never below 4 k-blocks per split.
-static GemmPlan plan_gemm(uint32_t M, uint32_t N, uint32_t K, uint32_t flags, size_t ws_bytes) {
+static GemmPlan plan_gemm(uint32_t M, uint32_t N, uint32_t K, uint32_t flags, size_t ws_bytes, bool with_192 = true) {
     const uint32_t sms = (uint32_t)sm_count();
     const uint32_t k_blocks = (K + BK - 1) / BK;
     const size_t mn = (size_t)M * N;
@@ -778,7 +778,7 @@ static GemmPlan plan_gemm(uint32_t M, uint32_t N, uint32_t K, uint32_t flags, si
         {false, false, !forced || force_narrow, m128 * n128, sms, 0.31, 0},
         {true, false, !forced || force_wide, m128 * n256, sms, 0.375, 0},
         {false, true, pair_ok, m256 * n256, sms / 2, 0.315, 256},
-        {false, true, pair_ok && !force_pair, m256 * ((N + 191) / 192), sms / 2, 0.304, 192},
+        {false, true, pair_ok && with_192 && !force_pair, m256 * ((N + 191) / 192), sms / 2, 0.304, 192},
     };
     const double t_hbm = ((double)N * K * 2 + (double)M * K * 2) / 6.5e6;  // us at 6.5 TB/s
     uint32_t max_s = std::min<uint32_t>(16, std::max<uint32_t>(1, k_blocks / 4));
@@ -970,20 +970,23 @@ MIORI_API int miori_gemm_bf16_cache_static(const void* A, const void* cache, voi
                                            uint32_t N, uint32_t K, uint32_t flags, void* stream) {
     int rc = gemm::check_gemm_args("miori_gemm_bf16_cache_static", A, cache, Cm, M, N, K);
     if (rc) return rc;
-    // the split count the shape wants with unlimited scratch decides whether it fits
-    const gemm::GemmPlan want = gemm::plan_gemm(M, N, K, flags, ~(size_t)0 >> 1);
-    const size_t need = want.splits > 1 ? (size_t)want.splits * M * N * sizeof(float) : 0;
+    // The split count the shape wants with unlimited scratch decides whether it fits, that of the 128- and 256-wide
+    // tiles: what is taken here is a promise, which another tile shape in the planner must not move (with the
+    // 192-wide ones 3436 x 312 at K = 6528 would want five slices for two, and be refused).
+    const gemm::GemmPlan limit = gemm::plan_gemm(M, N, K, flags, ~(size_t)0 >> 1, false);
+    const size_t need = limit.splits > 1 ? (size_t)limit.splits * M * N * sizeof(float) : 0;
     if (need > kStaticScratchBytes)
         return fail(MIORI_E_INVALID,
                     "miori_gemm_bf16_cache_static: M=%u N=%u K=%u needs %zu bytes of scratch (%u "
                     "K-splits), the built-in scratch holds %zu; miori_gemm_bf16_cache runs the shape "
                     "without a K split and without scratch (miori_gemm_bf16_cache_ws splits it given a "
                     "caller workspace)",
-                    M, N, K, need, want.splits, kStaticScratchBytes);
+                    M, N, K, need, limit.splits, kStaticScratchBytes);
     if (!(flags & MIORI_TUNE_GEMM_MASK)) {
         const uint32_t cs = gemm::skinny::plan(M, N, K, true);
         if (cs) return gemm::skinny::launch_skinny(A, cache, Cm, M, N, K, flags, cs, (cudaStream_t)stream);
     }
+    const gemm::GemmPlan want = gemm::plan_gemm(M, N, K, flags, kStaticScratchBytes);
     float* ws = nullptr;
     if (want.splits > 1) {
         rc = static_scratch_ptr(&ws);

@@ -90,3 +90,13 @@ def test_static_entry_allocates_nothing():
     torch.cuda.synchronize()
     free1, _ = torch.cuda.mem_get_info()
     assert free1 == free0, f"free device memory changed by {free0 - free1} bytes across the calls"
+
+
+@pytest.mark.parametrize("M,N,K", [(5129, 264, 7040), (3436, 312, 6528), (2120, 568, 7104), (2366, 272, 11392)])
+def test_shapes_that_fit_with_wide_tiles_are_taken(M, N, K):
+    """Two or three slices of 256-wide tiles fit the built-in scratch; that other tiles would want five does not matter."""
+    A = synth.make_activation(M, K, seed=1, device=DEV)
+    cache = synth.make_activation(N, K, seed=2, device=DEV).reshape(-1)
+    got = _static(A, cache, N)
+    assert_close(got.cpu().numpy(), miori_b200.gemm_bf16_cache(A, cache, N).cpu().numpy(), rel_max=1e-4, what=f"{M}x{N}x{K}")
+    assert lib.miori_device_error_poll() == 0
