@@ -183,6 +183,13 @@ __device__ __forceinline__ unsigned long long block_argmax(const void* __restric
     __syncthreads();
     return threadIdx.x < 32u ? warp_key_max(warp_best[threadIdx.x]) : 0ull;
 }
+// A candidate's value with the sign that its zero has in v (keys know one zero).
+template <bool BF16>
+__device__ __forceinline__ Best signed_zero(Best b, const void* __restrict__ v, uint32_t index0) {
+    if (b.v == 0.0f)
+        b.v = BF16 ? bf16_bits_to_float(static_cast<const uint16_t*>(v)[b.i - index0]) : static_cast<const float*>(v)[b.i - index0];
+    return b;
+}
 // Cluster-wide result, valid in thread 0 of CTA 0 of the cluster.  Every thread of every CTA of
 // the cluster must call it (it contains cluster barriers).  cta_best: ARGMAX_CLUSTER entries of
 // shared memory, at the same offset in every CTA.
@@ -191,7 +198,7 @@ __device__ __forceinline__ Best cluster_argmax(const void* __restrict__ v, uint3
                                                unsigned long long* warp_best, unsigned long long* cta_best) {
     unsigned long long mine = block_argmax<BF16>(v, n, index0, warp_best);
     const uint32_t nct = cluster_nctarank(), cr = cluster_ctarank();
-    if (nct == 1u) return best_of_key(mine);
+    if (nct == 1u) return signed_zero<BF16>(best_of_key(mine), v, index0);
     if (threadIdx.x == 0) {
         uint32_t remote;  // cta_best[cr] in CTA 0's shared memory
         asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(smem_addr(cta_best + cr)));
@@ -200,7 +207,7 @@ __device__ __forceinline__ Best cluster_argmax(const void* __restrict__ v, uint3
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (cr == 0u && threadIdx.x == 0)
         for (uint32_t c = 1; c < nct; ++c) mine = key_max(mine, cta_best[c]);
-    return best_of_key(mine);
+    return cr == 0u ? signed_zero<BF16>(best_of_key(mine), v, index0) : best_of_key(mine);
 }
 template <bool BF16>
 __global__ void __launch_bounds__(ARGMAX_THREADS)

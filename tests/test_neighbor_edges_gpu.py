@@ -63,6 +63,16 @@ def test_argmax_special_values(dtype):
         assert int(idx) == 3 and float(val) == -1.0
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [5, 9000])
+def test_argmax_zeros_tie_and_keep_their_sign(dtype, n):
+    for zeros in ((-0.0, 0.0), (0.0, -0.0)):
+        v = torch.full((n,), -2.0, dtype=dtype, device=DEV)
+        v[n - 3], v[n - 1] = zeros
+        idx, val = miori_b200.argmax(v)
+        assert int(idx) == n - 3 and float(val).hex() == zeros[0].hex()
+
+
 @pytest.mark.parametrize("bits", [4, 8])
 @pytest.mark.parametrize("N,K,group", [(1, 32, 32), (3, 96, 32), (7, 2048, 64), (149, 1440, 32), (20000, 320, 64), (33, 8192, 64)])
 def test_cache_build(port, bits, N, K, group):
