@@ -29,6 +29,12 @@ constexpr int TILE = 128;                     // weight rows per CTA
 constexpr int W_BYTES = TILE * BK * 2;        // 16 KiB per k-block
 constexpr int MAX_M = 48;
 constexpr int MAX_STAGES = 10;
+// Accumulators of a K slice, a share of its k-blocks each, which are added in fp32: the tensor core cuts its running
+// sum off instead of rounding it, and the error grows with the chain, by about 2^-24 of the result a k-block.
+// (Four and eight slices of eight k-blocks, 3072 x 2048 and 512 x 4096, against 64-bit sums: 4.7e-7 of the result
+// with one, 2.3e-7 with two, 1.3e-7 with four; the split tiled kernel has 3.2e-7 and 2.4e-7.  16 rows of 3072 x 2048
+// take 5.8, 5.9 and 6.2 us.)  One where K is not split: the bits are then the tiled kernels'.
+constexpr int ACCS = 2;
 
 struct Geo {
     uint32_t M, N, K;
@@ -109,17 +115,21 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         if (lane == 0) {
             // D = f32, A = B = bf16, both K-major, shape 128 x mp
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((g.mp >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
-            uint32_t s = 0, parity = 0u;
-            for (uint32_t i = 0; i < nkb && ok; ++i) {
-                if (!(ok = mbar_wait(smem_addr(&full_bars[s]), parity, &abort_flag, 0x32))) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t wdesc = umma_desc_sw128(ring + s * stage_bytes);
-                const uint64_t xdesc = umma_desc_sw128(ring + s * stage_bytes + W_BYTES);
+            const uint32_t accs = g.cs > 1u ? (uint32_t)ACCS : 1u;
+            uint32_t s = 0, parity = 0u, i = 0;
+            for (uint32_t a = 0; a < accs; ++a) {
+                const uint32_t acc = tmem + a * g.mp, i0 = i, i1 = (a + 1u) * nkb / accs;
+                for (; i < i1 && ok; ++i) {
+                    if (!(ok = mbar_wait(smem_addr(&full_bars[s]), parity, &abort_flag, 0x32))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t wdesc = umma_desc_sw128(ring + s * stage_bytes);
+                    const uint64_t xdesc = umma_desc_sw128(ring + s * stage_bytes + W_BYTES);
 #pragma unroll
-                for (uint32_t k = 0; k < BK / UMMA_K; ++k)
-                    umma_f16(tmem, wdesc + 2u * k, xdesc + 2u * k, idesc, (i | k) != 0u);
-                umma_commit(smem_addr(&empty_bars[s]));
-                if (++s == g.stages) s = 0u, parity ^= 1u;
+                    for (uint32_t k = 0; k < BK / UMMA_K; ++k)
+                        umma_f16(acc, wdesc + 2u * k, xdesc + 2u * k, idesc, ((i - i0) | k) != 0u);
+                    umma_commit(smem_addr(&empty_bars[s]));
+                    if (++s == g.stages) s = 0u, parity ^= 1u;
+                }
             }
             if (ok) umma_commit(smem_addr(&done_bar));
         }
@@ -156,9 +166,14 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         if (warp >= 2u) {
             uint32_t owner = 0, cg = 0, to = 0;
             for (uint32_t c = 0; c < g.mp; c += 16u) {
-                uint32_t r[16];
-                tmem_ld16(tmem + ((quad * 32u) << 16) + c, r);
+                uint32_t part[ACCS][16], (&r)[16] = part[0];
+#pragma unroll
+                for (uint32_t a = 0; a < (uint32_t)ACCS; ++a) tmem_ld16(tmem + ((quad * 32u) << 16) + a * g.mp + c, part[a]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (uint32_t a = 1; a < (uint32_t)ACCS; ++a)
+#pragma unroll
+                    for (uint32_t j = 0; j < 16u; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(part[a][j]));
 #pragma unroll
                 for (uint32_t j = 0; j < 16u; j += 4u) {
                     if (cg == 0u)
@@ -224,7 +239,8 @@ static int launch_skinny(const void* A, const void* Bc, void* Cm, uint32_t M, ui
     g.M = M, g.N = N, g.K = K, g.cs = cs;
     const uint32_t pad = std::max(16u, 4u * cs);  // whole groups of four columns for every CTA of a cluster
     g.mp = (M + pad - 1u) / pad * pad;
-    g.tmem_cols = g.mp <= 32u ? 32u : 64u;
+    g.tmem_cols = 32u;  // of the 512 of an SM, which shared memory lets at most three of these CTAs share
+    while (g.tmem_cols < g.mp * (cs > 1u ? (uint32_t)ACCS : 1u)) g.tmem_cols *= 2u;
     g.out_bf16 = flags & MIORI_OUT_BF16 ? 1u : 0u;
     const uint32_t stage_bytes = W_BYTES + g.mp * BK * 2u, k_blocks = (K + BK - 1) / BK;
     // clusters of eight find a place on half SMs only (33 of them against 15 on whole ones)

@@ -21,6 +21,15 @@ def _bf16(rows, cols, seed):
     return torch.randn((rows, cols), generator=g, device=DEV).to(torch.bfloat16)
 
 
+@pytest.mark.parametrize("M,N,K", [(16, 3072, 2048), (48, 512, 4096), (1, 512, 4096)])
+def test_split_sums_are_as_exact_as_the_tiled_kernels(M, N, K):
+    """Chains of four k-blocks, each of which costs about 2^-24 of the result (2-norm over 2-norm, against 64 bits)."""
+    A, B, ws = _bf16(M, K, 1), _bf16(N, K, 2), torch.empty(16, device=DEV)
+    want = A.double() @ B.double().T
+    got = miori_b200.gemm_bf16_cache(A, B.view(-1), N, workspace=ws).double()
+    assert float((got - want).norm() / want.norm()) < 5 * 2.0 ** -24
+
+
 def test_a_workspace_of_no_bytes_is_none():
     M, N, K = 32, 512, 4096
     A, B, ws = _bf16(M, K, 1), _bf16(N, K, 2), torch.empty(1 << 20, device=DEV)
