@@ -425,7 +425,9 @@ struct PreNorm {
 //            (shaders/ops.metal:605-631).  Every CTA stores its part of v into y; the CTA that arrives
 //            last then runs the stand-alone kernel's row pass over y in place
 //   FUSED, normed: x is fp32; bf16(x * rsqrt(mean(x^2) + eps) * gamma) is what is multiplied
-enum Fuse { NONE, FUSED, SHARDED, ARGMAX, POSTNORM };
+//   LONG: one row of a K whose scales do not fit beside it: they are read from global memory as they are needed.
+//            Plain or normed
+enum Fuse { NONE, FUSED, SHARDED, ARGMAX, POSTNORM, LONG };
 
 struct Args {
     const uint16_t* x;      // activations, bf16 [M][K] (fp32 when normed)
@@ -482,7 +484,8 @@ __host__ __device__ inline Layout layout(uint32_t K, uint32_t M, uint32_t stages
 template <class S, Fuse F>
 __global__ void __launch_bounds__(THREADS, 1)
 gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ Args A) {
-    const bool gated = F == FUSED && A.gated != 0u, normed = F == FUSED && A.pre.gamma != nullptr;
+    constexpr bool LONG_ = F == LONG;
+    const bool gated = F == FUSED && A.gated != 0u, normed = (F == FUSED || LONG_) && A.pre.gamma != nullptr;
     constexpr bool SHARDED_ = F == SHARDED, ARGMAX_ = F == ARGMAX, POSTNORM_ = F == POSTNORM;
     constexpr int BITS = S::BITS, NT = S::NT, ROWS = S::ROWS, GPS = S::GPS, RC = S::RC;
     const uint32_t N = A.N, K = A.K, M = A.M, kpar = A.kpar, nsg = A.nsg, ngrp = A.ngrp;
@@ -559,7 +562,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 const uint32_t r0 = gated ? row >> 1 : row;  // gated: N is a multiple of 16, eight whole rows of each half
                 const uint8_t* src_s = reinterpret_cast<const uint8_t*>(A.s) + (size_t)r0 * (2u * ng);
                 const uint8_t* src_b = reinterpret_cast<const uint8_t*>(A.b) + (size_t)r0 * (2u * ng);
-                if (row + 16u > N && kp == 0u) {  // a ragged last tile: whole 16-byte pieces by bulk copy ...
+                if (!LONG_ && row + 16u > N && kp == 0u) {  // a ragged last tile: whole 16-byte pieces by bulk copy ...
                     if (!shared && st_wait && !reuse(&empty_bars[bar0 + st], st_par, 0x16)) break;
                     if (shared && sb_wait && !reuse(&sb_empty[sb0 + sb], sb_par, 0x15)) break;
                     const uint32_t n = (N - row) * ng;
@@ -582,7 +585,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                         bulk_g2s(sdst + L.sb_half, src_b, extra >> 1, sb_bar);
                     }
                 };
-                if (shared && kp == 0u) {
+                if (!LONG_ && shared && kp == 0u) {
                     sb_bar = smem_addr(&sb_full[sb0 + sb]);
                     if (sb_wait && !reuse(&sb_empty[sb0 + sb], sb_par, 0x15)) break;
                     mbar_expect_tx(sb_bar, extra);
@@ -592,7 +595,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                     const uint32_t bar = smem_addr(&full_bars[bar0 + st]), dst = base + (bar0 + st) * L.stage_bytes;
                     if (st_wait && !reuse(&empty_bars[bar0 + st], st_par, 0x14)) break;
                     const int c0 = (int)(ks * (SLAB_ROW / 8u));
-                    const bool with_sb = !shared && ks == 0u;
+                    const bool with_sb = !LONG_ && !shared && ks == 0u;
                     mbar_expect_tx(bar, L.stage_bytes + (with_sb ? extra : 0u));
                     if (gated) {  // the tensor map's boxes are eight rows high
                         tma_load_2d(dst, &tmap_q, c0, (int)r0, bar);
@@ -677,7 +680,9 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             xb[j] = xa.x + min((uint32_t)(8 * j) + g % (uint32_t)RC, M - 1u) * xa.pitch + t * (uint32_t)S::XB;
         const uint32_t zeros = base + L.zeros;
         const uint32_t q_lane = g * qpitch + t * (uint32_t)S::W;
-        const uint32_t sb_row = g * ng * 2u, sb_row8 = 8u * ng * 2u;
+        // where scales and biases lie from row g's scales; LONG: bits of the number that stands for their address
+        const uint32_t sb_row = LONG_ ? 0u : g * ng * 2u, sb_row8 = LONG_ ? 1u : 8u * ng * 2u, sb_half = LONG_ ? 2u : L.sb_half;
+        uint32_t long_row = 0;  // LONG: this lane's first row of the tile
         using R = Red<ROWS>;
         const bool vec_sb = ng % 8u == 0u;  // rows of scales start on 16-byte boundaries
 
@@ -704,9 +709,9 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             uint32_t vs0[SW], vb0[SW], vs1[SW], vb1[SW];
             if constexpr (FULL && RC > 1) {
                 lds_words<4 * SW>(vs0, sa + 2u * grp0);
-                lds_words<4 * SW>(vb0, sa + 2u * grp0 + L.sb_half);
+                lds_words<4 * SW>(vb0, sa + 2u * grp0 + sb_half);
                 lds_words<4 * SW>(vs1, sa + 2u * grp0 + sb_row8);
-                lds_words<4 * SW>(vb1, sa + 2u * grp0 + sb_row8 + L.sb_half);
+                lds_words<4 * SW>(vb1, sa + 2u * grp0 + sb_row8 + sb_half);
             }
             const uint32_t half = (sl & 1u) ? 0x3244u : 0x1044u;
             // fp32 value of the run's group c + (SLOTTED: this lane's slot)
@@ -719,7 +724,14 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             };
             // not FULL: groups of steps that are not this run's, or past the end of K, count as zero
             const uint32_t glim = min(ng, grp0 + steps * GPS);
-            auto one = [&](uint32_t at, uint32_t gi) { return __uint_as_float(gi < glim ? lds16(at + 2u * gi) << 16 : 0u); };
+            auto one = [&](uint32_t at, uint32_t gi) {
+                if constexpr (LONG_) {
+                    const uint16_t* p = (at & 2u ? A.b : A.s) + (size_t)min(long_row + 8u * (at & 1u), N - 1u) * ng;
+                    return __uint_as_float(gi < glim ? (uint32_t)__ldg(p + gi) << 16 : 0u);
+                } else {
+                    return __uint_as_float(gi < glim ? lds16(at + 2u * gi) << 16 : 0u);
+                }
+            };
             // apply the sums d to acc: c = first group of the accumulator relative to the run
             auto scale = [&](float (&a)[4], const float (&d)[4], int c, int j) {
                 if constexpr (RC == 1) {
@@ -729,7 +741,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                     const uint32_t p = grp0 + (uint32_t)c + (SHORT ? 2u * (t & 1u) : 2u * t);
                     if constexpr (FULL) {
                         const uint32_t s0 = lds32(sa + 2u * p), s1 = lds32(sa + 2u * p + sb_row8);
-                        uint32_t b0 = lds32(sa + 2u * p + L.sb_half), b1 = lds32(sa + 2u * p + sb_row8 + L.sb_half);
+                        uint32_t b0 = lds32(sa + 2u * p + sb_half), b1 = lds32(sa + 2u * p + sb_row8 + sb_half);
                         if (SHORT && t >= 2u) b0 = b1 = 0u;
                         apply(a, d, ldsf128(xa.ms + p * 8u), bf16lo(s0), bf16hi(s0), bf16lo(s1), bf16hi(s1), bf16lo(b0),
                               bf16hi(b0), bf16lo(b1), bf16hi(b1));
@@ -744,8 +756,8 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                         if (p0 >= glim) ms.x = ms.y = 0.0f;
                         if (p1 >= glim) ms.z = ms.w = 0.0f;
                         apply(a, d, ms, one(sa, p0), one(sa, p1), one(sa + sb_row8, p0), one(sa + sb_row8, p1),
-                              one(sa + L.sb_half, p0), one(sa + L.sb_half, p1), one(sa + sb_row8 + L.sb_half, p0),
-                              one(sa + sb_row8 + L.sb_half, p1));
+                              one(sa + sb_half, p0), one(sa + sb_half, p1), one(sa + sb_row8 + sb_half, p0),
+                              one(sa + sb_row8 + sb_half, p1));
                     }
                 } else {
                     const uint32_t gi = grp0 + (uint32_t)c + sl;
@@ -754,7 +766,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                     if constexpr (FULL) {
                         s0 = pick(vs0, c), s1 = pick(vs1, c), b0 = pick(vb0, c), b1 = pick(vb1, c);
                     } else {
-                        s0 = one(sa, gi), s1 = one(sa + sb_row8, gi), b0 = one(sa + L.sb_half, gi), b1 = one(sa + sb_row8 + L.sb_half, gi);
+                        s0 = one(sa, gi), s1 = one(sa + sb_row8, gi), b0 = one(sa + sb_half, gi), b1 = one(sa + sb_row8 + sb_half, gi);
                         if (gi >= glim) ms = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
                     apply(a, d, ms, s0, s0, s1, s1, b0, b0, b1, b1);
@@ -833,15 +845,16 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         };
         const uint32_t gt = wg * 32u + lane;  // thread index inside the group
         for (uint32_t vt = grp; grp < ngrp && vt < vtiles; vt += ngrp) {
-            const uint32_t sa = base + L.sb + (sb0 + sb) * 2u * L.sb_half + sb_row;
-            if (kpar > 1u) wait(&sb_full[sb0 + sb], sb_par, 0x12);
+            const uint32_t sa = LONG_ ? 0u : base + L.sb + (sb0 + sb) * 2u * L.sb_half + sb_row;
+            if (LONG_) long_row = (blockIdx.x + (vt >> kshift) * gridDim.x) * 16u + g;
+            else if (kpar > 1u) wait(&sb_full[sb0 + sb], sb_par, 0x12);
             for (uint32_t ks = kp; ks < kslabs; ks += kpar) {
                 wait(&full_bars[bar0 + st], st_par, 0x10);
                 if (ok) {
                     // steps of this slab, dealt to the warps in runs: four each in a full slab
                     const uint32_t left = row_bytes - ks * SLAB_ROW;
                     const uint32_t qa = base + (bar0 + st) * L.stage_bytes + q_lane;
-                    if (vec_sb && left >= SLAB_ROW) {
+                    if (!LONG_ && vec_sb && left >= SLAB_ROW) {
                         run_math(std::true_type(), qa + wg * 4u * STEP_BYTES, 2u * (ks * S::KC + wg * 4u * S::SK),
                                  ks * (S::KC / S::GROUP) + wg * 4u * GPS, sa, 4u);
                     } else {
@@ -856,7 +869,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 }
                 if (++st == nsg) st = 0u, st_par ^= 1u;
             }
-            if (kpar > 1u && ok && lane == 0) mbar_arrive(smem_addr(&sb_empty[sb0 + sb]));
+            if (!LONG_ && kpar > 1u && ok && lane == 0) mbar_arrive(smem_addr(&sb_empty[sb0 + sb]));
             if (++sb == A.nsb) sb = 0u, sb_par ^= 1u;
 
             // ---- tile complete: the classes of groups in a fixed tree, then the warps' partials (and those of
@@ -1048,21 +1061,21 @@ size_t smem_bytes(const Extent& e, uint32_t K, uint32_t M, uint32_t ngrp, uint32
 }
 
 // How many groups share a tile: with few tiles per CTA and a long K two or four, each taking every kpar-th slab,
-// as far as M rows of activations leave room for a stage each.  0: M rows do not fit.
+// as far as M rows of activations, and a tile's scales, leave room for a stage each.  0: M rows do not fit.
 template <class S>
-uint32_t choose_kpar(uint32_t N, uint32_t K, uint32_t M) {
+uint32_t choose_kpar(uint32_t N, uint32_t K, uint32_t M, bool scales = true) {
     if (K > (1u << 20)) return 0u;  // (the sums below stay inside 32 bits)
     const Extent e = extent<S>(N, K);
     uint32_t kpar = 1u;
     while (kpar * 2u <= (uint32_t)GROUPS && e.tiles_cta * kpar * 2u <= (uint32_t)GROUPS && e.kslabs % (kpar * 2u) == 0u) kpar *= 2u;
     for (; kpar >= 1u; kpar >>= 1)
-        if (smem_bytes<S>(e, K, M, kpar, 1u, 1u, kpar, e.tiles_cta) <= SMEM_LIMIT) return kpar;
+        if (smem_bytes<S>(e, K, M, kpar, 1u, scales ? 1u : 0u, kpar, e.tiles_cta) <= SMEM_LIMIT) return kpar;
     return 0u;
 }
 
 // The plan for M rows with kpar groups to a tile, which fit.
 template <class S>
-Plan plan_launch(uint32_t N, uint32_t K, uint32_t M, uint32_t kpar) {
+Plan plan_launch(uint32_t N, uint32_t K, uint32_t M, uint32_t kpar, bool scales = true) {
     Plan p;
     const Extent e = extent<S>(N, K);
     p.grid = e.grid, p.kpar = kpar, p.slab_row = e.slab_row;
@@ -1074,7 +1087,7 @@ Plan plan_launch(uint32_t N, uint32_t K, uint32_t M, uint32_t kpar) {
         for (uint32_t nsg = std::min<uint32_t>(MAX_NSG, each * own); nsg >= 1u; --nsg) {
             // scales of every tile the code stages reach into: when the stage of a tile's first slab is
             // free, so is the buffer of the tile nsb before it
-            const uint32_t nsb = std::min(each, (nsg - 1u + own - 1u) / own + 1u);
+            const uint32_t nsb = scales ? std::min(each, (nsg - 1u + own - 1u) / own + 1u) : 0u;
             const size_t bytes = smem_bytes<S>(e, K, M, ngrp, nsg, nsb, kpar, each);
             if (bytes > SMEM_LIMIT) continue;
             p.ngrp = ngrp, p.nsg = nsg, p.nsb = nsb;
@@ -1104,8 +1117,8 @@ int launch_one(const Plan& plan, const void* q, const Args& a, cudaStream_t stre
 
 template <class S>
 int launch_shape(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t M,
-                 uint32_t flags, cudaStream_t stream, const Shard& sh, uint32_t kpar) {
-    const Plan plan = plan_launch<S>(N, K, M, kpar);
+                 uint32_t flags, cudaStream_t stream, const Shard& sh, uint32_t kpar, bool wide_k = false) {
+    const Plan plan = plan_launch<S>(N, K, M, kpar, !wide_k);
     if (plan.ngrp == 0) return fail(MIORI_E_INVALID, "gemv: no plan for N=%u K=%u M=%u", N, K, M);
     constexpr bool FEW = S::ROWS <= 4 || (S::ROWS == 8 && S::GROUP == 64);  // shapes that up to four 4-bit rows run on
     const bool sharded = sh.pa.world > 1, argmax = sh.best != nullptr;
@@ -1138,6 +1151,8 @@ int launch_shape(const void* q, const void* s, const void* b, const void* x, voi
     if (sh.gated && (S::BITS != 4 || N % 16 != 0 || M > (normed ? 4u : 16u)))
         return fail(MIORI_E_INVALID, "the gated epilogue takes 4-bit weights with N a multiple of 16, up to 16 rows "
                                      "(four with the norm in front)");
+    if constexpr (S::ROWS == 1)
+        if (wide_k) return launch_one<S, LONG>(plan, q, a, stream);
     if (normed || sh.gated) return launch_one<S, FUSED>(plan, q, a, stream);
     if (sharded) return launch_one<S, SHARDED>(plan, q, a, stream);
     return launch_one<S, NONE>(plan, q, a, stream);
@@ -1167,8 +1182,8 @@ struct Batch {
     }
     // One launch of up to cls rows.  Below eight the shapes of fewer rows sum in the same order.
     static int launch(uint32_t cls, uint32_t kpar, const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N,
-                      uint32_t K, uint32_t M, uint32_t flags, cudaStream_t stream, const Shard& sh) {
-#define MIORI_GEMV(ROWS) return launch_shape<Shape<BITS, GROUP, ROWS>>(q, s, b, x, y, N, K, M, flags, stream, sh, kpar)
+                      uint32_t K, uint32_t M, uint32_t flags, cudaStream_t stream, const Shard& sh, bool wide_k) {
+#define MIORI_GEMV(ROWS) return launch_shape<Shape<BITS, GROUP, ROWS>>(q, s, b, x, y, N, K, M, flags, stream, sh, kpar, wide_k)
         if (cls > 16u) MIORI_GEMV(32);
         if (cls > 8u) MIORI_GEMV(16);
         if (cls > 4u || (WIDE3 && cls > 2u)) MIORI_GEMV(8);
@@ -1183,13 +1198,18 @@ struct Batch {
         uint32_t cls = class_of(M), kpar = 0;
         if (flags & MIORI_TUNE_GEMV_ALIGNED) cls = std::max(cls, 8u);
         while (cls && (kpar = kpar_of(cls, N, K)) == 0u) cls >>= 1;
-        if (!cls) return 1;
+        const bool wide_k = cls == 0u;  // not even one row and its scales fit
+        if (wide_k) {
+            if (sh.gated || sh.post.residual || sh.best || sh.pa.world > 1) return 1;
+            cls = 1u, kpar = choose_kpar<Shape<BITS, GROUP, 1>>(N, K, 1u, false);
+            if (!kpar) return 1;
+        }
         const uint32_t launches = (M + cls - 1u) / cls, rows = (M + launches - 1u) / launches;
         const uint32_t n_out = sh.gated ? N / 2u : sh.pa.world > 1 || sh.best ? sh.n_total : N;
         const size_t x_row = (size_t)K * (sh.pre.gamma ? 4 : 2), y_row = (size_t)n_out * ((flags & MIORI_OUT_BF16) ? 2 : 4);
         for (uint32_t m0 = 0; m0 < M; m0 += rows) {
             const int rc = launch(cls, kpar, q, s, b, static_cast<const uint8_t*>(x) + m0 * x_row, static_cast<uint8_t*>(y) + m0 * y_row,
-                                  N, K, std::min(rows, M - m0), flags, stream, sh);
+                                  N, K, std::min(rows, M - m0), flags, stream, sh, wide_k);
             if (rc) return rc;
             sh.y_off += rows * y_row;
             if (sh.post.residual) sh.post.residual += (size_t)rows * N;

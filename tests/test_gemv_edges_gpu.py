@@ -145,3 +145,25 @@ def test_fused_forms_of_batches_dealt_to_several_launches(group, K, M):
         y = miori_b200.gemv4_rmsnorm(q, s, b, xf, g, 1e-5, group=group)
         z = miori_b200.silu_mul(y[:, :N // 2].contiguous(), y[:, N // 2:].contiguous())
         assert torch.equal(miori_b200.gemv4_rmsnorm_silu(q, s, b, xf, g, 1e-5, group=group), z)
+
+
+@pytest.mark.parametrize("bits,group,K", [(4, 32, 51200), (8, 32, 56320), (4, 64, 75776), (8, 64, 74752), (8, 32, 50432)])
+@pytest.mark.parametrize("N,M", [(24, 1), (2500, 1), (40, 3)])
+def test_rows_whose_scales_do_not_fit_beside_them(bits, group, K, N, M):
+    q, s, b = synth.make_weight(N, K, bits, group, seed=K, device=DEV)
+    w = _weights64(q, s, b, bits, group)
+    x = synth.make_activation(M, K, seed=M, device=DEV)
+    guard = torch.full((M * N + 64,), 777.0, device=DEV)
+    y = guard[32:32 + M * N].view(M, N)
+    OPS[bits](q, s, b, x, group=group, out=y)
+    want = x.double() @ w.T
+    assert float((y.double() - want).norm() / want.norm()) < 8 * 2.0 ** -24  # as above, and four times as many groups
+    assert (guard[:32] == 777.0).all() and (guard[32 + M * N:] == 777.0).all()
+    if K // group % 8 == 0:
+        g = synth.make_activation(1, K, seed=2, device=DEV).reshape(-1)
+        xf = x.float() * 3.0
+        xn = (xf.double() * (xf.double().pow(2).mean(1, keepdim=True) + 1e-5).rsqrt() * g.double()).to(torch.bfloat16)
+        got = (miori_b200.gemv4_rmsnorm if bits == 4 else miori_b200.gemv8_rmsnorm)(q, s, b, xf, g, 1e-5, group=group).double()
+        want = xn.double() @ w.T
+        assert float((got - want).norm() / want.norm()) < 1e-4  # single roundings of the normalised activations may tip over
+    assert miori_b200.lib.miori_device_error_poll() == 0
