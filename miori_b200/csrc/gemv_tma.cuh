@@ -1069,7 +1069,8 @@ uint32_t choose_kpar(uint32_t N, uint32_t K, uint32_t M, bool scales = true) {
     uint32_t kpar = 1u;
     while (kpar * 2u <= (uint32_t)GROUPS && e.tiles_cta * kpar * 2u <= (uint32_t)GROUPS && e.kslabs % (kpar * 2u) == 0u) kpar *= 2u;
     for (; kpar >= 1u; kpar >>= 1)
-        if (smem_bytes<S>(e, K, M, kpar, 1u, scales ? 1u : 0u, kpar, e.tiles_cta) <= SMEM_LIMIT) return kpar;
+        // (whether M rows fit at all must not depend on N: ranks with shards of different heights launch alike)
+        if (smem_bytes<S>(e, K, M, kpar, 1u, scales ? 1u : 0u, kpar, kpar == 1u ? 2u : e.tiles_cta) <= SMEM_LIMIT) return kpar;
     return 0u;
 }
 
