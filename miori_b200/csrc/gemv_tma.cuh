@@ -485,7 +485,7 @@ template <class S, Fuse F>
 __global__ void __launch_bounds__(THREADS, 1)
 gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ Args A) {
     constexpr bool LONG_ = F == LONG;
-    const bool gated = F == FUSED && A.gated != 0u, normed = (F == FUSED || LONG_) && A.pre.gamma != nullptr;
+    const bool gated = F == FUSED && S::BITS == 4 && S::ROWS <= 16 && A.gated != 0u, normed = (F == FUSED || LONG_) && A.pre.gamma != nullptr;
     constexpr bool SHARDED_ = F == SHARDED, ARGMAX_ = F == ARGMAX, POSTNORM_ = F == POSTNORM;
     constexpr int BITS = S::BITS, NT = S::NT, ROWS = S::ROWS, GPS = S::GPS, RC = S::RC;
     const uint32_t N = A.N, K = A.K, M = A.M, kpar = A.kpar, nsg = A.nsg, ngrp = A.ngrp;
@@ -1197,7 +1197,6 @@ struct Batch {
     static int run(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t M,
                    uint32_t flags, cudaStream_t stream, Shard sh) {
         uint32_t cls = class_of(M), kpar = 0;
-        if (flags & MIORI_TUNE_GEMV_ALIGNED) cls = std::max(cls, 8u);
         while (cls && (kpar = kpar_of(cls, N, K)) == 0u) cls >>= 1;
         const bool wide_k = cls == 0u;  // not even one row and its scales fit
         if (wide_k) {

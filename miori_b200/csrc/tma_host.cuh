@@ -93,10 +93,6 @@ template <int N>
 __device__ __forceinline__ void tma_store_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
-// wait until every bulk group of this thread has completed (its writes are performed)
-__device__ __forceinline__ void tma_store_wait_all() {
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-}
 #endif
 
 }  // namespace miori_b200

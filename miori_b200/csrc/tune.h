@@ -8,4 +8,3 @@
 #define MIORI_TUNE_GEMM_NOPAIR 0x8000u  // GEMM: never the two-CTA kernel
 #define MIORI_TUNE_GEMM_SPLIT_SHIFT 16  // GEMM: bits 16..19 = forced K split count (1..15; needs the workspace for it)
 #define MIORI_TUNE_GEMM_MASK 0xFC300u       // GEMM: any of the above
-#define MIORI_TUNE_GEMV_ALIGNED 0x100000u  // GEMV: activation rows as MMA columns for every M (no slots)

@@ -28,9 +28,9 @@ for (N, K) in [(3072, 2048), (2048, 2048), (16384, 2048), (2048, 8192)]:
     for i in range(npool):
         q, s, b = synth.make_weight(N, K, 4, G, seed=N + K + i, device=dev)
         pool.append(miori_b200.dequant4_cache(q, s, b, group=G)); del q, s, b
-    for M in (16, 32, 1024):
+    for M in (64, 128, 1024):
         A = synth.make_activation(M, K, seed=3, device=dev)
-        obf = M >= 128
+        obf = M > 128
         Cm = torch.empty((M, N), device=dev, dtype=torch.bfloat16 if obf else torch.float32)
         ws = torch.empty(16 * M * N, dtype=torch.float32, device=dev)
         t, c, sp = C.c_uint32(), C.c_uint32(), C.c_uint32()

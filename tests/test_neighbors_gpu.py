@@ -106,17 +106,15 @@ def test_argmax_sizes_and_alignment(n, dtype):
 @pytest.mark.parametrize("bits,N,K,M,group", [(4, 2048, 2048, 1, 64), (4, 3072, 2048, 4, 32), (4, 640, 2048, 8, 64),
                                               (8, 1024, 2048, 2, 64), (4, 2048, 8192, 1, 64), (4, 1536, 2048, 32, 64),
                                               (4, 16384, 2048, 2, 64), (4, 1000, 4096, 3, 64), (4, 48, 512, 3, 32)])
-@pytest.mark.parametrize("force", [0, 0x100000, 0x1000], ids=["default", "tcgen05", "mma.sync"])
-def test_gemv_with_fused_rmsnorm(port, bits, N, K, M, group, force):
-    """y = W * bf16(rmsnorm(x)): the fused kernels (by default the TMA + mma.sync one for 4-bit weights,
-    up to four rows and K <= 2048, the tcgen05 one otherwise; either when forced, where it applies)
-    against the oracle's norm followed by its GEMV, and against this library's own unfused pair."""
+def test_gemv_with_fused_rmsnorm(port, bits, N, K, M, group):
+    """y = W * bf16(rmsnorm(x)): the norm in the kernel's activation staging, against the oracle's norm
+    followed by its GEMV, and against this library's own unfused pair."""
     q, s, b = synth.make_weight(N, K, bits, group, seed=N + K + M)
     g = torch.Generator().manual_seed(M)
     x = torch.randn((M, K), generator=g) * 2.5
     w = (torch.randn(K, generator=g) * 0.2 + 1.0).to(torch.bfloat16)
     fused = (miori_b200.gemv4_rmsnorm if bits == 4 else miori_b200.gemv8_rmsnorm)(
-        q.to(DEV), s.to(DEV), b.to(DEV), x.to(DEV), w.to(DEV), 1e-5, group=group, flags=force).cpu().numpy()
+        q.to(DEV), s.to(DEV), b.to(DEV), x.to(DEV), w.to(DEV), 1e-5, group=group).cpu().numpy()
     xn = port.rmsnorm(x.numpy(), u16(w), 1e-5)
     want = port.gemv(bits, u32(q), u16(s), u16(b), xn, group)
     # a bf16 rounding of a normalised activation may tip differently than in the oracle (fp32 order
@@ -124,29 +122,27 @@ def test_gemv_with_fused_rmsnorm(port, bits, N, K, M, group, force):
     assert_close(fused, want, rel_max=1e-3, what=f"fused norm gemv{bits} M={M}")
     xn_dev = miori_b200.rmsnorm(x.to(DEV), w.to(DEV), 1e-5)
     unfused = (miori_b200.gemv4 if bits == 4 else miori_b200.gemv8)(
-        q.to(DEV), s.to(DEV), b.to(DEV), xn_dev, group=group, flags=0x100000).cpu().numpy()
+        q.to(DEV), s.to(DEV), b.to(DEV), xn_dev, group=group).cpu().numpy()
     assert_close(fused, unfused, rel_max=1e-3, what="fused vs unfused")
 
 
-TILED = 0x2000    # tuning flag: tiled TMA even where one slab of K fits the linear copies
-MMASYNC = 0x1000  # tuning flag: keep the unfused GEMV on the kernel the fused entry runs on
+EARLY = miori_b200.LAUNCH_PDL
 
 
 @pytest.mark.parametrize("N,K,M,group,flags", [
     (16384, 2048, 1, 64, 0), (16384, 2048, 2, 64, 0), (12288, 2048, 3, 64, 0), (4096, 2048, 4, 32, 0),
     (2048, 2048, 8, 64, 0), (3072, 2048, 16, 64, 0), (1024, 1024, 16, 32, 0), (4096, 4096, 1, 64, 0),
-    (512, 8192, 2, 64, 0), (2048, 2048, 1, 64, TILED), (1024, 2048, 6, 32, TILED), (4096, 1024, 5, 32, 0),
+    (512, 8192, 2, 64, 0), (2048, 2048, 1, 64, EARLY), (1024, 2048, 6, 32, EARLY), (4096, 1024, 5, 32, 0),
     (32, 2048, 1, 64, 0), (16, 512, 7, 64, 0), (6000 * 2, 1536, 4, 64, 0)])
 def test_gemv_with_silu_epilogue(port, N, K, M, group, flags):
     """bf16(silu(gate) * up) out of the fused gate + up projection: bit for bit the unfused pair of
-    this library, and the oracle's GEMV followed by its silu_mul within one bf16 step (M <= 4, the
-    fp32-dequantization kernels) resp. the batched GEMV's tolerance."""
+    this library, and the oracle's GEMV followed by its silu_mul within one bf16 step."""
     q, s, b = synth.make_weight(N, K, 4, group, seed=N + K + M)
     x = synth.make_activation(M, K, seed=M)
     dq, ds, db, dx = q.to(DEV), s.to(DEV), b.to(DEV), x.to(DEV)
     fused = miori_b200.gemv4_silu(dq, ds, db, dx, group=group, flags=flags)
     assert fused.shape == (M, N // 2) and fused.dtype == torch.bfloat16
-    y = miori_b200.gemv4(dq, ds, db, dx, group=group, flags=flags | MMASYNC)
+    y = miori_b200.gemv4(dq, ds, db, dx, group=group, flags=flags)
     h = N // 2
     unfused = miori_b200.silu_mul(y[:, :h].contiguous(), y[:, h:].contiguous())
     assert torch.equal(fused.view(torch.int16), unfused.view(torch.int16)), "fused and unfused differ"
@@ -154,13 +150,10 @@ def test_gemv_with_silu_epilogue(port, N, K, M, group, flags):
     want = port.silu_mul(np.ascontiguousarray(want_y[:, :h]), np.ascontiguousarray(want_y[:, h:]))
     got = fused.float().cpu().numpy()
     ref = (want.astype(np.uint32) << 16).view(np.float32).reshape(got.shape)
-    if M <= 4:
-        # one bf16 step plus what the GEMV's fp32 sums (within 2e-5 of the largest output) may move a
-        # small product by; nearly all outputs equal bit for bit
-        assert (np.abs(got - ref) <= np.abs(ref) * 2.0 ** -7 + 1e-3).all()
-        assert (u16(fused).reshape(-1) != want.reshape(-1)).mean() < 0.01
-    else:
-        assert_close(got, ref, rel_max=2e-2, what=f"gated gemv4 M={M}")
+    # one bf16 step plus what the GEMV's fp32 sums (within 2e-5 of the largest output) may move a
+    # small product by; nearly all outputs equal bit for bit
+    assert (np.abs(got - ref) <= np.abs(ref) * 2.0 ** -7 + 1e-3).all()
+    assert (u16(fused).reshape(-1) != want.reshape(-1)).mean() < 0.01
     assert miori_b200.lib.miori_device_error_poll() == 0
 
 
@@ -170,12 +163,12 @@ def test_gemv_with_silu_epilogue_refuses_what_it_cannot_take():
     with pytest.raises(miori_b200.MioriError, match="multiple of 16"):
         miori_b200.gemv4_silu(q[:40].contiguous().to(DEV), s[:40].contiguous().to(DEV), b[:40].contiguous().to(DEV), x,
                               group=64)
-    # scale rows of 96 / 32 = 3 groups have no 16-byte pitch: outside the TMA kernel's range
+    # scale rows of 96 / 32 = 3 groups have no 16-byte pitch
     q2, s2, b2 = synth.make_weight(32, 96, 4, 32, seed=2)
     x2 = synth.make_activation(1, 96, seed=2).to(DEV)
     with pytest.raises(miori_b200.MioriError, match="outside the fused kernel's range"):
         miori_b200.gemv4_silu(q2.to(DEV), s2.to(DEV), b2.to(DEV), x2, group=32)
-    # more than 16 activation rows do not fit the kernel's staging area
+    # the entry takes up to 16 activation rows
     x3 = synth.make_activation(17, 2048, seed=3).to(DEV)
     with pytest.raises(miori_b200.MioriError, match="outside 1..16"):
         miori_b200.gemv4_silu(q.to(DEV), s.to(DEV), b.to(DEV), x3, group=64)
@@ -183,7 +176,7 @@ def test_gemv_with_silu_epilogue_refuses_what_it_cannot_take():
 
 @pytest.mark.parametrize("N,K,M,group,flags", [
     (2048, 2048, 1, 64, 0), (2048, 8192, 1, 64, 0), (2048, 2048, 2, 32, 0), (2048, 2048, 3, 64, 0),
-    (2048, 8192, 4, 64, 0), (1000, 2048, 4, 32, 0), (2048, 2048, 1, 64, TILED), (16, 512, 2, 64, 0),
+    (2048, 8192, 4, 64, 0), (1000, 2048, 4, 32, 0), (2048, 2048, 1, 64, EARLY), (16, 512, 2, 64, 0),
     (5120, 4096, 1, 64, 0)])
 def test_gemv_with_post_norm_add_epilogue(port, N, K, M, group, flags):
     """residual + v * rsqrt(mean(v^2) + eps) * gamma with v the GEMV's output row: bit for bit the
@@ -199,7 +192,7 @@ def test_gemv_with_post_norm_add_epilogue(port, N, K, M, group, flags):
     fused = miori_b200.gemv4_post_norm_add(dq, ds, db, dx, dres, dw, 1e-5, counter, group=group, flags=flags)
     again = miori_b200.gemv4_post_norm_add(dq, ds, db, dx, dres, dw, 1e-5, counter, group=group, flags=flags)
     assert int(counter.item()) == 0
-    v = miori_b200.gemv4(dq, ds, db, dx, group=group, flags=flags | MMASYNC)
+    v = miori_b200.gemv4(dq, ds, db, dx, group=group, flags=flags)
     unfused = miori_b200.post_norm_add(dres, v, dw, 1e-5)
     assert torch.equal(fused, unfused), "fused and unfused differ"
     assert torch.equal(fused, again), "second launch differs"
@@ -223,7 +216,7 @@ def test_gemv_with_post_norm_add_epilogue_refuses_what_it_cannot_take():
 
 
 @pytest.mark.parametrize("N,K,M,group,flags", [(16384, 2048, 1, 64, 0), (4096, 2048, 2, 32, 0), (12288, 2048, 3, 64, 0),
-                                               (2048, 4096, 4, 64, 0), (1024, 2048, 1, 64, TILED), (32, 512, 4, 64, 0)])
+                                               (2048, 4096, 4, 64, 0), (1024, 2048, 1, 64, EARLY), (32, 512, 4, 64, 0)])
 def test_gate_up_projection_with_both_neighbours(port, N, K, M, group, flags):
     """rmsnorm, w1, w3 and silu_mul in one launch, against this library's own chain (norm kernel, then
     the gated GEMV) and against the oracle's."""
