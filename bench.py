@@ -582,7 +582,8 @@ def main():
                 continue
             rows = N // world if split[M][i] else N
             if route(M, rows, K) == 2:
-                n += 2 if lib.miori_gemm_workspace_bytes(M, rows, K) else 1   # GEMM (+ K-split sum)
+                # a cluster's K slices meet in the GEMM's own launch up to 48 rows, in a second kernel above
+                n += 2 if M > 48 and lib.miori_gemm_workspace_bytes(M, rows, K) else 1
             else:
                 n += 1
             n += 1 if (grp is not None and split[M][i]) else 0            # peer all-gather
@@ -688,7 +689,7 @@ def main():
     # weights a launch streams
     DRAM_PER_ALGO_BYTE = 1.003
     roofline = {
-        "kernel": "gemv_tma_kernel<4,exact,1> (M=1 pass of the stack, 96 launches per pass)",
+        "kernel": "gemv_tma_kernel, one row of 4-bit weights (M=1 pass of the stack, 96 launches per pass)",
         "bound": "hbm", "achieved": m1["gbs"] / world, "peak": peaks["hbm_gbs"], "unit": "GB/s",
         "frac": m1["gbs"] / world / peaks["hbm_gbs"], "peak_kind": peak_kind,
         "bytes_per_launch": bytes_pass / launches_pass / world,

@@ -43,6 +43,19 @@ def _sources(root: str, exts: tuple[str, ...]) -> list[str]:
     return out
 
 
+def _torch_tag() -> str:
+    """What a binding carries to say which torch's headers it was compiled against."""
+    from importlib import metadata
+    return f"built against torch {metadata.version('torch')};"
+
+
+def _binding_stale(sources: list[str]) -> bool:
+    if _stale(BINDING, sources):
+        return True
+    with open(BINDING, "rb") as f:
+        return _torch_tag().encode() not in f.read()
+
+
 def _build_binding() -> None:
     """The operators' native call path: a CPython extension against torch's C++ headers."""
     import sysconfig
@@ -50,7 +63,7 @@ def _build_binding() -> None:
     import torch
     from torch.utils import cpp_extension
     cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DMIORI_TORCH_TAG="{_torch_tag()}"',
            "-I", sysconfig.get_paths()["include"]]
     for d in [*cpp_extension.include_paths(), os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]:
         cmd += ["-isystem", d]
@@ -80,7 +93,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             raise RuntimeError("nvcc failed:\n" + r.stdout + r.stderr)
     header = os.path.join(HERE, "..", "include", "miori_b200.h")
-    if force or _stale(BINDING, [os.path.join(CSRC, "binding.cpp"), header]):
+    if force or _binding_stale([os.path.join(CSRC, "binding.cpp"), header]):
         _build_binding()
     shim_dir = os.path.join(HERE, "shim")
     shim_srcs = _sources(shim_dir, (".cpp", ".h", ".hpp"))

@@ -478,7 +478,7 @@ PyMethodDef methods[] = {
          "x fp32 [M][K], M <= 4: one launch for the norm, both projections and the activation."),
     {nullptr, nullptr, 0, nullptr}};
 
-PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Native call path of the operators.", -1, methods,
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Native call path of the operators, " MIORI_TORCH_TAG, -1, methods,
                       nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -105,3 +105,10 @@ def test_given_and_allocated_outputs():
         ops.gemv4(q, s, b, x, group=48)
     with pytest.raises(ValueError, match="words per row"):
         ops.gemv8(q, s, b, x, group=64)
+
+
+def test_a_binding_of_another_torch_is_rebuilt(monkeypatch):
+    from miori_b200 import build
+    assert not build._binding_stale([])
+    monkeypatch.setattr(build, "_torch_tag", lambda: "built against torch 0.0;")
+    assert build._binding_stale([])
