@@ -1,7 +1,9 @@
 // Up to 48 rows of activations against the bf16 cache: C[M][N] = A[M][K] * Bc[N][K]^T.
 //
-// What bounds such a product is the cache's trip from HBM into the SMs (55 bytes per cycle and SM) and, below
-// some 20 MB of it, the launch: the tiled GEMM's 128 x 128 tiles of C leave most SMs without one, so K is
+// What bounds such a product: a wide one, one tile a CTA, the cache's trip from HBM (16384 x 2048: 4.8 TB/s); a
+// short one the launch and a chain of k-blocks, each of which takes 0.23 us whatever its bytes -- the one thread
+// that waits, issues four MMAs and commits is what they queue for (one computed address more in its loop
+// cost 25 ns a block).  The tiled GEMM's 128 x 128 tiles of C leave most SMs without one, so K is
 // split, the partials travel through a workspace and a second kernel sums them, and each of the two pays
 // the hand-over to the next.  Here one kernel does it: a CTA owns 128 weight rows and a slice of K, the
 // slices of a tile are the CTAs of one cluster, and the partial sums meet in distributed shared memory.
@@ -18,8 +20,8 @@
 // Every wait is bounded; the cluster barriers are reached by every thread whatever its waits returned.
 //
 // Measured in chains of dependent launches over caches larger than L2, the split tiled GEMM and this, us:
-// 32 rows, N x K: 2048 x 2048 6.9 -> 5.1, 3072 x 2048 8.2 -> 6.5, 8192 x 2048 12.2 -> 10.7, 16384 x 2048 (one
-// slice) 15.5 -> 14.5 (4.6 TB/s), 2048 x 8192 11.8 -> 9.9, 8192 x 8192 31.9 -> 28.8 (4.7 TB/s).  The exchange
+// 32 rows, N x K: 2048 x 2048 8.1 -> 5.4, 3072 x 2048 8.9 -> 6.5, 8192 x 2048 12.4 -> 10.5, 16384 x 2048 (one
+// slice) 15.8 -> 13.9, 2048 x 8192 12.9 -> 9.7, 8192 x 8192 29.5 -> 25.7 (5.2 TB/s).  The exchange
 // grows with the rows: even at 64 (6.9 and 6.7 at 2048 x 2048, 10.8 and 11.3 at 6144 x 2048), behind at 77.
 #pragma once
 

@@ -2,11 +2,11 @@
 //
 // What the reference's wide-batch path multiplies (its bf16 cache, shaders/gemm_mpp.metal:36-73,
 // reached through BatchEngine::linear, src/batch.cpp:223-230) for the batch sizes of a decode
-// step.  The tcgen05 GEMM serves these shapes badly: a 128-row tile of A is three quarters empty,
-// a projection of 2048 outputs has 16 tiles for 148 SMs, so K has to be split and summed by a
-// second kernel, and the launch pays TMEM allocation and a long pipeline fill.  Here the cache is
-// streamed once in 16-row tiles, exactly like the packed weights of the decode GEMV -- there are
-// 128 tiles where the GEMM had 16 -- with no unpack at all: 16 bytes of a cache row ARE an A
+// step.  The tcgen05 kernel for few rows (gemm_skinny.cuh) has 16 tiles of 128 weight rows for a
+// projection of 2048 outputs, splits K over a cluster to fill the SMs, and pays TMEM allocation, a
+// pipeline fill and the exchange: 5.3 us where the cache streams in 1.3.  Here the cache is
+// streamed once in 16-row tiles, exactly like the packed weights of the decode GEMV -- 128 of
+// them, 3.1-4.2 us -- with no unpack at all: 16 bytes of a cache row ARE an A
 // fragment of mma.sync.m16n8k16 (under the fixed k permutation "slot 2t, 2t+1, 2t+8, 2t+9 of lane
 // t = elements 8t .. 8t+3"), and the same 16 bytes of an activation row are the matching B
 // fragment, so x needs no permutation either.
@@ -236,7 +236,7 @@ inline int try_launch(const void* x, const void* cache, void* y, uint32_t M, uin
     const uint32_t nstage =
         std::min<uint32_t>(MAX_STAGES, std::max<uint32_t>(2u, ((tiles + grid - 1) / grid) * slabs_t));
     // more than half of an SM's shared memory, so that no second CTA of a neighbouring launch joins
-    // this one (see the placement note in gemv_tma.cuh: plan_stages)
+    // this one (see the placement note at Plan in gemv_tma.cuh)
     const size_t need = nt == 1 ? smem_bytes<1>(nstage) : nt == 2 ? smem_bytes<2>(nstage) : smem_bytes<4>(nstage);
     const size_t smem = std::max<size_t>(need, 120 * 1024);
     CUtensorMap tw;

@@ -20,12 +20,13 @@
 // e4m3 operands, whose subnormals hold a 4-bit code in a byte, halves the unpacking but takes as many MMAs, for
 // bf16's eight bits need two e4m3 terms: 16384 x 2048 at 8 rows took 14.8 us against 12.4 at the time.)
 //
-// What bounds it: HBM for long 8-bit streams, the issue slots (128 warp instructions per KiB of codes at K = 2048, 109 at 8192)
+// What bounds it: HBM for long 8-bit streams, the issue slots (some 136 warp instructions per KiB of codes at K = 2048)
 // for long 4-bit ones, the hand-over between dependent launches and the trip of x through L2 for short
-// ones.  Measured in chains of dependent launches over weights larger than L2, before (codes as bf16
-// 128 + code, one producer) and now, us: 8-bit head 131072 x 2048 at 1, 4, 16 rows 53.1, 60.3, 93 -> 44.1
-// (6.46 TB/s, 0.99 of a plain copy), 45.2, 75; 4-bit 16384 x 2048 at 1, 4, 8 rows 7.44, 8.80, 10.2 ->
-// 6.54, 7.14, 7.75; 2048 x 8192 at 1, 4 rows 6.58, 9.56 -> 4.62, 6.15; 2048 x 2048 at 1 row 2.64 -> 2.40.
+// ones.  Measured in chains of dependent launches over weights larger than L2, with codes as bf16 128 + code
+// and one producer, and now, us: 8-bit head 131072 x 2048 at 1, 4, 16 rows 53.1, 60.3, 93 -> 42.7
+// (6.7 TB/s, what a plain copy does), 44.2, 72.5; 4-bit 16384 x 2048 at 1, 4, 8 rows 7.44, 8.80, 10.2 ->
+// 6.56, 7.19, 7.72; 2048 x 8192 at 1, 4 rows 6.58, 9.56 -> 4.63, 6.27.  2048 x 2048 at 1 row is no faster: 2.68
+// and 2.76 (2.71 with less exact sums, see above).
 //
 // One CTA per SM owns every gridDim-th 16-row tile.  A slab -- 16 rows x up to 1 KiB of codes -- is one
 // 2-D TMA copy into a shared-memory ring; a tile's scales and biases (contiguous in memory) are two

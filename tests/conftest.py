@@ -12,7 +12,7 @@ GOLDEN = os.path.join(ROOT, "tests", "golden")
 
 # Tolerances of the quantized-matmul path against the CPU oracle.
 #   Contract: max|d| <= 1e-2 * max|ref| and cosine >= 0.9999 for every GEMV / GEMM output.
-#   The fp32-dequant GEMV (M <= 4) is additionally held to 2e-5 * max|ref|, the order of the
+#   The GEMV, fp32 dequantization at every M, is additionally held to 2e-5 * max|ref|, the order of the
 #   reference's own recorded error (max_rel 8.35e-05 on real weights).
 TOL_REL_MAX = 1e-2
 TOL_COS = 0.9999
