@@ -31,11 +31,41 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // Number of SMs of the current device (cached per device ordinal).
 int sm_count();
 
+// What a kernel is set to before its first launch on a device: as much dynamic shared memory as there is beside its
+// static and, for the kernels of a decode step of few rows, the largest shared-memory share of an SM's memory.  They
+// all ask for the same share, because a change of it waits until the SM is empty, and none could start beside one
+// that wants another (four projections of a decode layer 24 us instead of 18).  The others leave it to the
+// driver: the largest share is the smallest L1 (a cache build of 8-bit weights 7.6 us, 11.3 with it).  The settings are
+// the same whoever makes them; what a thread has made it remembers (as launch attributes the share costs 1.4 us of host
+// time a launch, and each call here 0.1).
+enum class Split { DRIVERS, SHARED };
+inline cudaError_t set_up_kernel(const void* kernel, Split split) {
+    constexpr uint32_t SLOTS = 128;
+    static thread_local struct { const void* kernel; int device; } made[SLOTS];
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    auto& m = made[(reinterpret_cast<uintptr_t>(kernel) >> 4) % SLOTS];
+    if (m.kernel == kernel && m.device == device) return cudaSuccess;
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, kernel);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes);
+    if (e == cudaSuccess && split == Split::SHARED)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) m = {kernel, device};
+    return e;
+}
+
 // Launch helper: grid/block/smem on `stream`, optionally with the programmatic
 // dependent launch attribute so that the kernel may begin before its predecessor ends.
-template <class... KArgs, class... Args>
+template <Split SPLIT = Split::DRIVERS, class... KArgs, class... Args>
 inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                           cudaStream_t stream, bool pdl, Args... args) {
+    if (SPLIT == Split::SHARED || smem > 0) {
+        const cudaError_t e = set_up_kernel(reinterpret_cast<const void*>(kernel), SPLIT);
+        if (e != cudaSuccess) return e;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -91,6 +121,18 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// One look, which never sleeps.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
         : "r"(bar), "r"(parity)

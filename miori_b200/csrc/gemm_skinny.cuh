@@ -254,7 +254,7 @@ static int launch_skinny(const void* A, const void* Bc, void* Cm, uint32_t M, ui
     if (rc) return rc;
     rc = make_tmap(&tx, A, M, K, g.mp, 0);
     if (rc) return rc;
-    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = set_up_kernel(reinterpret_cast<const void*>(gemm_skinny_kernel), Split::DRIVERS);
     if (e == cudaSuccess) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((N + TILE - 1) / TILE * cs);

@@ -662,11 +662,11 @@ static int launch_gemm_pair(const void* A, const void* Bc, void* Cm, uint32_t M,
     cudaError_t e;
     if (bf16) {
         auto kern = pair::gemm_bf16_tcgen05_pair_kernel<BN, true>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::Cfg<BN>::SMEM_BYTES);
+        e = set_up_kernel(reinterpret_cast<const void*>(kern), Split::DRIVERS);
         if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, splits, M, N, K);
     } else {
         auto kern = pair::gemm_bf16_tcgen05_pair_kernel<BN, false>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::Cfg<BN>::SMEM_BYTES);
+        e = set_up_kernel(reinterpret_cast<const void*>(kern), Split::DRIVERS);
         if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, splits, M, N, K);
     }
     if (e != cudaSuccess) return cuda_fail(e, "gemm_bf16_tcgen05_pair launch");
@@ -707,16 +707,10 @@ static int launch_gemm(const void* A, const void* Bc, void* Cm, uint32_t M, uint
     cudaError_t e;
     if (bf16) {
         auto kern = gemm_bf16_tcgen05_kernel<BN, true>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-        if (e == cudaSuccess)
-            e = launch(kern, dim3(grid), dim3(THREADS), (size_t)C::SMEM_BYTES, stream, pdl, ta, tb,
-                       tc, splits, M, N, K, a_box);
+        e = launch(kern, dim3(grid), dim3(THREADS), (size_t)C::SMEM_BYTES, stream, pdl, ta, tb, tc, splits, M, N, K, a_box);
     } else {
         auto kern = gemm_bf16_tcgen05_kernel<BN, false>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-        if (e == cudaSuccess)
-            e = launch(kern, dim3(grid), dim3(THREADS), (size_t)C::SMEM_BYTES, stream, pdl, ta, tb,
-                       tc, splits, M, N, K, a_box);
+        e = launch(kern, dim3(grid), dim3(THREADS), (size_t)C::SMEM_BYTES, stream, pdl, ta, tb, tc, splits, M, N, K, a_box);
     }
     if (e != cudaSuccess) return cuda_fail(e, "gemm_bf16_tcgen05 launch");
     if (splits > 1) return launch_reduce(Cm, M, N, flags, ws, splits, stream);

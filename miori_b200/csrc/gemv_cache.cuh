@@ -249,19 +249,13 @@ inline int try_launch(const void* x, const void* cache, void* y, uint32_t M, uin
 #define MIORI_CACHE_LAUNCH(NTV, SL, OB)                                                           \
     do {                                                                                          \
         auto kern = gemv_cache_kernel<NTV, SL, OB>;                                               \
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
-        if (e == cudaSuccess)                                                                     \
-            e = launch(kern, dim3(grid), dim3(THREADS), smem, stream_, pdl, tw,                   \
-                       static_cast<const uint16_t*>(x), y, N, K, M, nstage);                      \
+        e = launch(kern, dim3(grid), dim3(THREADS), smem, stream_, pdl, tw, static_cast<const uint16_t*>(x), y, N, K, M, nstage); \
     } while (0)
 #define MIORI_CACHE_SL(NTV, SL) do { if (bf16) MIORI_CACHE_LAUNCH(NTV, SL, true); else MIORI_CACHE_LAUNCH(NTV, SL, false); } while (0)
 #define MIORI_CACHE_STREAM(NTV, SL)                                                               \
     do {                                                                                          \
         auto kern = bf16 ? gemv_cache_kernel<NTV, SL, true, true> : gemv_cache_kernel<NTV, SL, false, true>; \
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
-        if (e == cudaSuccess)                                                                     \
-            e = launch(kern, dim3(grid), dim3(THREADS), smem, stream_, pdl, tw,                   \
-                       static_cast<const uint16_t*>(x), y, N, K, M, nstage);                      \
+        e = launch(kern, dim3(grid), dim3(THREADS), smem, stream_, pdl, tw, static_cast<const uint16_t*>(x), y, N, K, M, nstage); \
     } while (0)
     if (stream) {
         if (nt == 2) MIORI_CACHE_STREAM(2, 16);

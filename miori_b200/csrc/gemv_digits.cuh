@@ -1,0 +1,682 @@
+// The decode GEMV for one and two activation rows on 4-bit weights in groups of 64, K a multiple of 256 up to 8192.
+//
+//   y[m][n] = sum_g ( s[n][g] * sum_{k in g} code[n][k] * x[m][k]  +  b[n][g] * sum_{k in g} x[m][k] )
+//
+// The inner sum runs on mma.sync.m16n8k32 with 8-bit integers, and exactly:
+//   * a word of eight 4-bit codes becomes two A registers with two ANDs and no shift: the low nibbles as they
+//     are, the high ones where they stand, counting sixteen times as much;
+//   * an activation is an integer below 2^26 -- its group's largest decides the power of two; bf16's eight bits
+//     are exact for everything of at least 2^-17 of the largest, the rest is rounded by less than 2^-25 of it
+//     -- times sixteen for the codes in low nibbles, cut into four digits of -128 .. 127, a column of the MMA
+//     each.  With one row the eight columns are the digits of two groups, with two rows those of one.
+// A row's sums are int32, then fp32 per group: its bits depend neither on the other row nor on N or the grid.
+// (The fp16 operands of gemv_tma.cuh take twice the MMAs and three times the ALU work for the unpacking, which
+// are worth it only where the columns are full of rows.)
+//
+// What bounds it: in a chain of dependent launches the steps that follow one another -- the hand-over from grid
+// to grid (0.7 us), the trip of x through L2 (0.35), its conversion (0.3; 0.25 a slab beyond), each piece of weights
+// (0.33) -- and not HBM: with the weights in L2 the four projections of a layer take 13.4 instead of 13.8.  So nothing else is on that path:
+//   * TWO CTAs of 256 threads fit an SM, one of this launch and one of the next, which fetches its weights
+//     while this one works.  Every launch is one CTA per SM, those without rows included: a launch of
+//     fewer would let the next one's double up, and every later launch would inherit the skew;
+//   * a 1-KiB slab of a row is cut into eight positions of 128 bytes, and warp w owns position w of every tile
+//     of the CTA: it fetches its own pieces (16 rows x 128 bytes by TMA, 128-byte swizzle, and their scales by
+//     cp.async) into its own ring, and converts the activations of its own position.  Warps meet once per
+//     batch of tiles, when the eight partial sums of an output are added in a fixed tree.  (With the
+//     activations staged by the whole CTA behind a barrier a layer took 4 % more.)
+//   * K <= 2048: the activations stay in registers from tile to tile;
+//   * the first piece is read while x is on its way.
+// After its first pieces a CTA holds the others back for 800 cycles: it starts when its predecessor fetches
+// x, whose loads would queue up behind them (four projections of a layer 15.2 us when all are fetched at once, 14.5 so).
+//
+// Measured in chains over weights larger than L2, the kernel of gemv_tma.cuh and this one, us, one row:
+// 2048 x 2048 2.50 -> 2.16, 3072 x 2048 2.92 -> 2.41, 16384 x 2048 6.51 -> 4.74, 2048 x 8192 4.64 -> 4.46, the four
+// together 16.6 -> 13.4; a layer of them with its norms and activation (six launches) 21.1 -> 18.3.  Two rows: 2.56 -> 2.43,
+// 2.93 -> 2.84, 6.99 -> 5.83, 17.4 -> 17.2 together; behind from K = 3072 on, where the conversion of two rows (2.2
+// times the instructions of fp16's) is most of the time: 2048 x 4096 3.52 -> 3.97, 2048 x 8192 4.89 -> 6.34.  A row's bits
+// must not depend on the other row, and one row is what this is for.
+#pragma once
+#include "gemv_tma.cuh"
+
+namespace miori_b200 {
+namespace gemvdigits {
+
+using gemvtma::cmax;
+using gemvtma::Fuse;
+using gemvtma::lds128;
+using gemvtma::lds16;
+using gemvtma::lds_words;
+
+constexpr int WARPS = 8, THREADS = 32 * WARPS;
+constexpr int MAX_STAGES = 8;
+constexpr uint32_t GROUP = 64;
+constexpr uint32_t SLAB = 1024, PIECE = 128, PIECE_BYTES = 16 * PIECE;  // bytes of a row; 16 rows
+constexpr uint32_t PK = 2 * PIECE;          // codes of a row in a piece
+constexpr uint32_t NG = PK / GROUP;         // its scale groups
+constexpr uint32_t XPAD = 64;               // between digit planes: their 64-byte reads fall into different banks
+constexpr uint32_t MAX_K = 8192;
+constexpr int HEAD_PIECES = 2;              // fetched at once; the others after HOLD_CYCLES
+constexpr long long HOLD_CYCLES = 800, LINGER_CYCLES = 3500;
+// Two of these fit the 228 KB of an SM, three do not (and more than 77 KB keep other kernels' CTAs from taking
+// the successor's place).
+constexpr size_t SMEM_LIMIT = 112 * 1024, SMEM_FLOOR = 78 * 1024;
+
+template <int ROWS_>
+struct Shape {
+    static constexpr int ROWS = ROWS_;
+    static constexpr int GS = 2 / ROWS;               // scale groups side by side in the eight columns
+    static constexpr int NU = 2 * GS;                 // MMAs of a chain = units of eight activations per lane
+    static constexpr int CH = (int)NG / GS;           // chains of a piece
+    static constexpr int QW = NU;                     // words of a row per chain and lane
+    static constexpr uint32_t BATCH = 8 / ROWS;       // tiles of a warp between two meetings of the CTA
+};
+
+struct Args {
+    const uint16_t* x;      // activations, bf16 [M][K] (fp32 when normed)
+    void* y;
+    const uint16_t *s, *b;  // scales and biases, [N][K / 64]
+    const uint8_t* q;
+    gemvtma::PreNorm pre;
+    gemvtma::PostNorm post;
+    uint32_t N, K, M, stages, out_bf16, gated, early;
+    uint32_t n_total, row0;
+    size_t y_off;
+    unsigned long long* best;
+    PeerArgs pa;
+};
+
+// Dynamic shared memory, from a 1024-byte aligned base.
+struct Layout {
+    uint32_t pitch, sc, x, ms, zeros, part, total;
+};
+constexpr uint32_t SC_ROW = 4u * NG, SC_BYTES = 16u * SC_ROW;  // scales and biases of a row of a piece, and of a piece
+template <class S>
+__host__ __device__ inline Layout layout(uint32_t K, uint32_t M, uint32_t stages, uint32_t parts) {
+    Layout L;
+    const uint32_t nslab = (K / 2u + SLAB - 1u) / SLAB;
+    L.pitch = nslab * PK + XPAD;  // of a digit plane of one warp
+    uint32_t at = WARPS * stages * PIECE_BYTES;
+    L.sc = at;
+    at += WARPS * stages * SC_BYTES;
+    L.x = at;
+    at += WARPS * M * 4u * L.pitch;
+    L.ms = at;
+    at += WARPS * nslab * NG * S::ROWS * 16u;
+    L.zeros = at;
+    at += WARPS * 16u;
+    L.part = at;
+    at += parts * S::ROWS * 128u;  // partial sums of a tile's positions
+    L.total = at + 1024u;
+    return L;
+}
+
+// D += A B, 16 x 8 x 32, codes x digits.
+__device__ __forceinline__ void mma_s32(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_s32_z(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {  // D = A B
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// Largest magnitudes of two pairs of bf16 (signs to be masked; NaN is the largest).
+__device__ __forceinline__ uint32_t max_abs2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+// Rows that digits do not hold, by their largest magnitude (bf16 bits): not all finite, or all below 2^-98, where
+// digits that end at 2^-122 would be too few.
+__device__ __forceinline__ bool no_digits(uint32_t largest) { return largest >= 0x7F80u || (largest != 0u && largest < (29u << 7)); }
+
+// Eight consecutive activations (bf16) -> four digit planes, the even ones times sixteen; the first lane of a
+// scale group (eight neighbouring lanes) stores {r, sum of x, 256 r, 0}: r r undoes the scaling for the digits
+// 0 and 1, (256 r)^2 for 2 and 3.  (As a square, so that neither a scale nor a sum leaves fp32's range when it
+// meets half of it.)  Every lane of the warp calls.  Returns the group's largest magnitude.
+__device__ __forceinline__ uint32_t stage_unit(const uint4& v, bool live, uint32_t at, uint32_t pitch, bool first, uint32_t ms_at) {
+    const uint32_t mx2 = max_abs2(max_abs2(v.x, v.y), max_abs2(v.z, v.w)) & 0x7FFF7FFFu;
+    uint32_t mx = max(mx2 & 0xFFFFu, mx2 >> 16);
+    const float f[8] = {bf16lo(v.x), bf16hi(v.x), bf16lo(v.y), bf16hi(v.y), bf16lo(v.z), bf16hi(v.z), bf16lo(v.w), bf16hi(v.w)};
+    float sum = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+#pragma unroll
+    for (int o = 1; o < (int)GROUP / 8; o <<= 1) {
+        mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    }
+    // half of the largest's exponent field, rounded up: |x| < 2^(2 e - 126); 2^(156 - 2 e) is to stay finite
+    const uint32_t e = max((mx >> 7) + 1u, 30u) >> 1;
+    const float up = __uint_as_float((279u - 2u * e) << 23), up16 = 16.0f * up;  // 2^(152 - 2 e): |x up| < 2^26
+    uint32_t q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)  // the bytes of (q + 0x80808080) are the digits + 128
+        q[i] = (uint32_t)(__float2int_rn(f[i] * (i & 1 ? up : up16)) + (int)0x80808080) ^ 0x80808080u;
+    uint32_t p[2][4];  // byte l of the even (odd) ones
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t l01 = __byte_perm(q[h], q[2 + h], 0x5140), h01 = __byte_perm(q[h], q[2 + h], 0x7362);
+        const uint32_t l23 = __byte_perm(q[4 + h], q[6 + h], 0x5140), h23 = __byte_perm(q[4 + h], q[6 + h], 0x7362);
+        p[h][0] = __byte_perm(l01, l23, 0x5410), p[h][1] = __byte_perm(l01, l23, 0x7632);
+        p[h][2] = __byte_perm(h01, h23, 0x5410), p[h][3] = __byte_perm(h01, h23, 0x7632);
+    }
+    if (live) {
+#pragma unroll
+        for (int l = 0; l < 4; ++l)
+            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + (uint32_t)l * pitch), "r"(p[0][l]), "r"(p[1][l]) : "memory");
+        if (first) {
+            const float r = __uint_as_float((49u + e) << 23);  // 2^(e - 78)
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ms_at), "f"(r), "f"(sum), "f"(r * 256.0f), "f"(0.0f) : "memory");
+        }
+    }
+    return mx;
+}
+
+// The slow side of a wait on a barrier, out of the way of the code that runs.
+__device__ __noinline__ bool wait_on(uint32_t bar, uint32_t parity, volatile uint32_t* abort, uint32_t where) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort, where));
+}
+
+// One output of a row of activations that are not all finite, or all next to nothing, in fp32: they have no digits.
+template <bool NORMED>
+__device__ __noinline__ float plain_dot(const Args& A, uint32_t n, uint32_t m, float inv) {
+    const uint32_t ng = A.K / GROUP;
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(A.q) + (size_t)n * (A.K / 8u);
+    float y = 0.0f;
+    for (uint32_t g = 0; g < ng; ++g) {
+        float cx = 0.0f, sx = 0.0f;
+        for (uint32_t w = 0; w < GROUP / 8u; ++w) {
+            const uint32_t codes = q[g * (GROUP / 8u) + w];
+            for (uint32_t i = 0; i < 8u; ++i) {
+                const size_t k = (size_t)g * GROUP + w * 8u + i, at = (size_t)m * A.K + k;
+                const float x = NORMED ? bf16_bits_to_float(float_to_bf16_bits(reinterpret_cast<const float*>(A.x)[at] * inv *
+                                                                               bf16_bits_to_float(A.pre.gamma[k])))
+                                       : bf16_bits_to_float(A.x[at]);
+                cx = __fmaf_rn((float)((codes >> (4u * i)) & 15u), x, cx);
+                sx += x;
+            }
+        }
+        y = __fmaf_rn(bf16_bits_to_float(A.s[(size_t)n * ng + g]), cx, __fmaf_rn(bf16_bits_to_float(A.b[(size_t)n * ng + g]), sx, y));
+    }
+    return y;
+}
+
+// RES: K <= 2048, one slab: the activations of a warp's position stay in registers.
+template <class S, Fuse F, bool RES>
+__global__ void __launch_bounds__(THREADS, 2)
+gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ Args A) {
+    constexpr int ROWS = S::ROWS, CH = S::CH, NU = S::NU, GS = S::GS;
+    constexpr bool SHARDED_ = F == gemvtma::SHARDED, ARGMAX_ = F == gemvtma::ARGMAX, POSTNORM_ = F == gemvtma::POSTNORM;
+    const bool gated = F == gemvtma::FUSED && A.gated != 0u, normed = F == gemvtma::FUSED && A.pre.gamma != nullptr;
+    const uint32_t N = A.N, K = A.K, M = A.M, stages = A.stages;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t tiles = (N + 15u) >> 4, row_bytes = K / 2u, ng = K / GROUP;
+    const uint32_t full_slabs = row_bytes / SLAB, rest = row_bytes % SLAB, nslab = (row_bytes + SLAB - 1u) / SLAB;
+    // short rows have fewer positions, and the warps of a position share the tiles
+    const uint32_t P = full_slabs ? 8u : (rest + PIECE - 1u) / PIECE;
+    const uint32_t pshift = P > 4u ? 3u : P > 2u ? 2u : P - 1u, TG = 8u >> pshift;
+    const uint32_t pos = warp & ((1u << pshift) - 1u), tg = warp >> pshift;
+    const uint32_t slabs = full_slabs + (pos * PIECE < rest ? 1u : 0u);
+
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t bars[WARPS * MAX_STAGES];
+    __shared__ volatile uint32_t abort_flag;
+    __shared__ uint32_t largest[WARPS][ROWS];  // magnitudes, in what each warp has seen of a row
+
+    // A launch that may not start early waits here, and lets its dependents start only when its predecessor is
+    // complete: they prefetch what that may have written.
+    const long long born = clock64();
+    if (A.early == 0u) pdl_wait_prior();
+    pdl_launch_dependents();
+
+    const uint32_t my_tiles = (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x;
+    const uint32_t batch = TG * S::BATCH;
+    const uint32_t wt = my_tiles > tg ? (my_tiles - tg + TG - 1u) / TG : 0u;  // tiles of this warp
+    const uint32_t pieces = wt * slabs;
+    const Layout L = layout<S>(K, M, stages, (my_tiles > batch ? 2u * batch : my_tiles) << pshift);
+    const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
+    const uint32_t ring = base + warp * stages * PIECE_BYTES, bar0 = smem_addr(&bars[warp * MAX_STAGES]);
+    const uint32_t sc_ring = base + L.sc + warp * stages * SC_BYTES;
+    auto tile_of = [&](uint32_t j) { return blockIdx.x + j * gridDim.x; };
+
+    // ---- fetching: tile after tile, slab after slab.  gated: a tile is eight gate rows and the up rows of the same outputs
+    auto row_of = [&](uint32_t tile, uint32_t r) {
+        return gated ? tile * 8u + (r & 7u) + (r >= 8u ? N >> 1 : 0u) : min(tile * 16u + r, N - 1u);
+    };
+    uint32_t issued = 0, itile = tile_of(tg), ic0 = pos * (PIECE / 8u);
+    const uint16_t* const sc_src = lane < 16u ? A.s : A.b;
+    size_t ie = (size_t)row_of(itile, lane & 15u) * ng + pos * NG;
+    const uint32_t sc_dst = sc_ring + (lane & 15u) * SC_ROW + (lane >> 4) * (SC_ROW / 2u);
+    auto issue = [&](uint32_t st) {
+        const uint32_t bar = bar0 + st * 8u;
+        if (lane == 0) {
+            const uint32_t dst = ring + st * PIECE_BYTES;
+            if (issued >= stages) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // behind the reads of what lay there
+            mbar_expect_tx(bar, PIECE_BYTES);
+            if (gated) {  // the tensor map's boxes are eight rows high
+                tma_load_2d(dst, &tmap_q, (int)ic0, (int)(itile * 8u), bar);
+                tma_load_2d(dst + 8u * PIECE, &tmap_q, (int)ic0, (int)((N >> 1) + itile * 8u), bar);
+            } else {
+                tma_load_2d(dst, &tmap_q, (int)ic0, (int)(itile * 16u), bar);
+            }
+        }
+        cp_async8(sc_dst + st * SC_BYTES, sc_src + ie);
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+        ++issued;
+        ic0 += SLAB / 8u, ie += 8u * NG;
+        if (RES || ic0 * 8u >= row_bytes) {
+            ic0 = pos * (PIECE / 8u);
+            itile += TG * gridDim.x;
+            ie = (size_t)row_of(itile, lane & 15u) * ng + pos * NG;
+        }
+    };
+    if (lane == 0) {
+        abort_flag = 0u;
+        for (uint32_t i = 0; i < stages; ++i) mbar_init(bar0 + 8u * i, 33);  // the copy's issuer and every lane's scales
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(base + L.zeros + 16u * warp), "r"(0u) : "memory");
+    }
+    __syncwarp();
+    {
+        const uint32_t n = min(stages, pieces);
+        uint32_t i = 0;
+        for (; i < min(n, (uint32_t)HEAD_PIECES); ++i) issue(i);
+        if (i < n && A.early) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < HOLD_CYCLES) __nanosleep(40);
+        }
+        for (; i < n; ++i) issue(i);
+    }
+
+    // ---- this lane's place in the MMAs: tile rows prow and prow + 8 (in an order that spreads the swizzled rows which
+    // a quarter- or half-warp reads over all banks); as a B operand column lane / 4 = (slot or row, digit)
+    const uint32_t g = lane >> 2, t = lane & 3u;
+    const uint32_t prow = ROWS == 1 ? ((g & 1u) << 2) | (g >> 1) : ((g & 3u) << 1) | (g >> 2);
+    const uint32_t xw = base + L.x + warp * M * 4u * L.pitch, msw = base + L.ms + warp * nslab * (NG * ROWS * 16u);
+    const bool mine = ROWS > 1 || (g >> 2) == (t >> 1);  // one row: the codes of this lane belong to its column's group
+    const uint32_t xb = mine ? xw + ((ROWS == 1 ? 0u : min(g >> 2, M - 1u)) * 4u + (g & 3u)) * L.pitch + t * (uint32_t)(NU * 8)
+                             : base + L.zeros + 16u * warp;
+    const uint32_t xstep = mine ? 1u : 0u;
+    const uint32_t ms0 = msw + (t >> 1) * 16u + (t & 1u) * 8u;  // one row: of group t / 2; two: of row t / 2
+    const uint32_t sel = ROWS == 1 && t >= 2u ? 0x3244u : 0x1044u;
+    const uint32_t q_lane = ring + prow * PIECE, s_lane = sc_ring + prow * SC_ROW;
+    const uint32_t q_at0 = (t * (uint32_t)(4 * S::QW)) ^ (prow << 4);
+
+    bool ok = true;  // turns false for good once a wait expires; the warp then goes on without waiting, to meet the others
+    // a look at a barrier costs 100 cycles: it is made ahead of the work that hides them, and used behind it
+    auto test_stage = [&](uint32_t st, uint32_t parity) { return mbar_test(bar0 + st * 8u, parity); };
+    auto settle = [&](bool there, uint32_t st, uint32_t parity) {
+        if (!__all_sync(0xFFFFFFFFu, there) && ok) ok = wait_on(bar0 + st * 8u, parity, &abort_flag, 0x10);
+    };
+    struct Codes { uint32_t a[CH * NU][4]; };
+    struct Packed { uint32_t q0[CH * NU], q1[CH * NU]; };
+    auto load_q = [&](uint32_t stage, Packed& p) {
+        const uint32_t qa = q_lane + stage * PIECE_BYTES;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            uint32_t v0[NU], v1[NU];
+            const uint32_t at = qa + (q_at0 ^ (uint32_t)(c * 16 * S::QW));
+            lds_words<4 * NU>(v0, at);
+            lds_words<4 * NU>(v1, at + 8u * PIECE);
+#pragma unroll
+            for (int i = 0; i < NU; ++i) p.q0[c * NU + i] = v0[i], p.q1[c * NU + i] = v1[i];
+        }
+    };
+    auto unpack = [&](const Packed& p, Codes& o) {
+#pragma unroll
+        for (int i = 0; i < CH * NU; ++i) {
+            o.a[i][0] = p.q0[i] & 0x0F0F0F0Fu, o.a[i][1] = p.q1[i] & 0x0F0F0F0Fu;
+            o.a[i][2] = p.q0[i] & 0xF0F0F0F0u, o.a[i][3] = p.q1[i] & 0xF0F0F0F0u;
+        }
+    };
+    constexpr int SW = (int)NG / 2;
+    struct Scales { uint32_t s0[SW], b0[SW], s1[SW], b1[SW]; };
+    auto load_s = [&](uint32_t stage, Scales& v) {
+        uint32_t r0[2 * SW], r1[2 * SW];
+        lds_words<8 * SW>(r0, s_lane + stage * SC_BYTES);
+        lds_words<8 * SW>(r1, s_lane + stage * SC_BYTES + 8u * SC_ROW);
+#pragma unroll
+        for (int i = 0; i < SW; ++i) v.s0[i] = r0[i], v.b0[i] = r0[SW + i], v.s1[i] = r1[i], v.b1[i] = r1[SW + i];
+    };
+    struct Acts { uint32_t b[CH * NU][2]; float r[CH], sum[CH]; };
+    auto load_x = [&](uint32_t slab, Acts& a) {
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            const uint32_t at = xb + xstep * (slab * PK + (uint32_t)c * (GS * GROUP));
+#pragma unroll
+            for (int i = 0; i < NU; i += 2) {
+                const uint4 v = lds128(at + xstep * 8u * i);
+                a.b[c * NU + i][0] = v.x, a.b[c * NU + i][1] = v.y, a.b[c * NU + i + 1][0] = v.z, a.b[c * NU + i + 1][1] = v.w;
+            }
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a.r[c]), "=f"(a.sum[c])
+                         : "r"(ms0 + (slab * NG + (uint32_t)(c * GS)) * (ROWS * 16u)));
+        }
+    };
+    struct Sums { int d[CH][4]; };
+    auto multiply = [&](const Codes& q, const Acts& x, Sums& o) {
+#pragma unroll
+        for (int i = 0; i < NU; ++i)
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                if (i == 0) mma_s32_z(o.d[c], q.a[c * NU], x.b[c * NU][0], x.b[c * NU][1]);
+                else mma_s32(o.d[c], q.a[c * NU + i], x.b[c * NU + i][0], x.b[c * NU + i][1]);
+            }
+    };
+    // sums of tile rows prow and prow + 8: of two digits, and with one row of every other group; with two rows even and
+    // odd groups apart, so that a row's sums meet in the same order
+    constexpr int PAR = ROWS;
+    float acc[PAR][2];
+    auto apply = [&](const Sums& o, const Scales& sc, const Acts& x) {
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            auto pick = [&](const uint32_t (&w)[SW]) {
+                if constexpr (GS == 2) return __uint_as_float(__byte_perm(w[c], 0u, sel));
+                else return c & 1 ? bf16hi(w[c >> 1]) : bf16lo(w[c >> 1]);
+            };
+            const float r = x.r[c];
+            const float v0 = (float)(o.d[c][1] * 256 + o.d[c][0]) * r, v1 = (float)(o.d[c][3] * 256 + o.d[c][2]) * r;
+            float (&a)[2] = acc[c & (PAR - 1)];
+            a[0] = __fmaf_rn(pick(sc.s0) * r, v0, __fmaf_rn(pick(sc.b0), x.sum[c], a[0]));
+            a[1] = __fmaf_rn(pick(sc.s1) * r, v1, __fmaf_rn(pick(sc.b1), x.sum[c], a[1]));
+        }
+    };
+
+    // the next piece: its codes and scales into registers, and its stage to the copies
+    uint32_t st = 0, par = 0;
+    Packed q;
+    Scales sc;
+    auto take = [&](bool there) {
+        settle(there, st, par);
+        load_q(st, q);
+        load_s(st, sc);
+        __syncwarp();
+        if (issued != pieces) issue(st);
+    };
+    auto first_piece = [&] {
+        if (pieces) take(test_stage(0u, 0u));
+    };
+
+    pdl_wait_prior();  // x (and y) belong to the predecessor until here
+
+    // A CTA without rows keeps its place until the next launch has taken its own: at the head of a chain it would be gone
+    // first, and leave its SM to two of the next launch's
+    if (my_tiles == 0u && A.early)
+        while (clock64() - born < LINGER_CYCLES) __nanosleep(100);
+
+    // ---- the activations of this warp's position: one unit of every row and slab a lane
+    __shared__ float nm_part[ROWS][WARPS], nm_inv[ROWS];
+    if (my_tiles && (pieces || normed)) {
+        const uint32_t upr = K >> 3, sets = M * slabs;
+        auto place = [&](uint32_t r, uint32_t& m, uint32_t& sl) {
+            m = ROWS > 1 && r >= slabs ? 1u : 0u;
+            sl = r - m * slabs;
+            return (sl * 8u + pos) * 32u + lane;
+        };
+        // normed: the squares first (of tg 0: every unit once), warps in order.  One slab's stay in registers, more are read
+        // again (from L2)
+        constexpr bool KEEP = RES;
+        float4 xa4[ROWS], xc4[ROWS];
+        uint4 gm = make_uint4(0u, 0u, 0u, 0u);
+        float inv[ROWS];
+        if (normed) {
+            const float4* x4 = reinterpret_cast<const float4*>(A.x);
+            auto squares = [](const float4& a, const float4& c, float ss) {
+                ss = __fmaf_rn(a.x, a.x, ss), ss = __fmaf_rn(a.y, a.y, ss), ss = __fmaf_rn(a.z, a.z, ss), ss = __fmaf_rn(a.w, a.w, ss);
+                ss = __fmaf_rn(c.x, c.x, ss), ss = __fmaf_rn(c.y, c.y, ss), ss = __fmaf_rn(c.z, c.z, ss);
+                return __fmaf_rn(c.w, c.w, ss);
+            };
+            auto add_up = [&](uint32_t m, float ss) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+                if (lane == 0) nm_part[m][warp] = tg == 0u ? ss : 0.0f;
+            };
+            if constexpr (KEEP) {
+                const uint32_t u = pos * 32u + lane;
+#pragma unroll
+                for (int m = 0; m < ROWS; ++m) {
+                    xa4[m] = xc4[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (slabs && u < upr) xa4[m] = __ldg(x4 + (m * upr + u) * 2u), xc4[m] = __ldg(x4 + (m * upr + u) * 2u + 1u);
+                }
+                if (slabs && u < upr) gm = __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + u);
+                first_piece();
+#pragma unroll
+                for (int m = 0; m < ROWS; ++m) add_up((uint32_t)m, squares(xa4[m], xc4[m], 0.0f));
+            } else {
+                for (uint32_t m = 0; m < M; ++m) {
+                    float ss = 0.0f;
+                    for (uint32_t s = 0; s < slabs; ++s) {
+                        const uint32_t u = (s * 8u + pos) * 32u + lane;
+                        if (u < upr) ss = squares(__ldg(x4 + ((size_t)m * upr + u) * 2u), __ldg(x4 + ((size_t)m * upr + u) * 2u + 1u), ss);
+                    }
+                    add_up(m, ss);
+                }
+                first_piece();
+            }
+            __syncthreads();
+#pragma unroll
+            for (int m = 0; m < ROWS; ++m) {
+                float tot = 0.0f;
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) tot += nm_part[m][w];
+                inv[m] = rsqrtf(tot / (float)K + A.pre.eps);
+                if (threadIdx.x == 0) nm_inv[m] = inv[m];
+            }
+        }
+        auto load = [&](uint32_t r) {
+            uint32_t m, sl;
+            const uint32_t u = place(r, m, sl);
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (r < sets && u < upr) {
+                const size_t i = (size_t)m * upr + u;
+                if (KEEP && normed) {
+                    v = ROWS == 1 || m == 0u ? gemvtma::normed8(xa4[0], xc4[0], inv[0], gm) : gemvtma::normed8(xa4[ROWS - 1], xc4[ROWS - 1], inv[ROWS - 1], gm);
+                } else if (normed) {
+                    const float4* x4 = reinterpret_cast<const float4*>(A.x) + 2u * i;
+                    v = gemvtma::normed8(__ldg(x4), __ldg(x4 + 1), ROWS == 1 || m == 0u ? inv[0] : inv[ROWS - 1],
+                                         __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + u));
+                } else {
+                    v = __ldg(reinterpret_cast<const uint4*>(A.x) + i);
+                }
+            }
+            return v;
+        };
+        auto stage = [&](uint32_t r, const uint4& v) {
+            uint32_t m, sl;
+            place(r, m, sl);
+            return stage_unit(v, r < sets, xw + m * 4u * L.pitch + sl * PK + lane * 8u, L.pitch, (lane & 7u) == 0u,
+                              msw + ((sl * NG + (lane >> 3)) * ROWS + m) * 16u);
+        };
+        uint32_t top[ROWS];
+#pragma unroll
+        for (int m = 0; m < ROWS; ++m) top[m] = 0u;
+        if constexpr (RES && ROWS == 1) {
+            const uint4 v = load(0u);
+            if (!normed) first_piece();
+            top[0] = stage(0u, v);
+        } else {  // AHEAD loads in flight, PAIR units at a time (more would be straight code, which costs its fetches)
+            constexpr int AHEAD = RES ? 2 : 4, PAIR = 2;
+            uint4 v[AHEAD];
+#pragma unroll
+            for (int h = 0; h < AHEAD; ++h) v[h] = load((uint32_t)h);
+            if (!normed) first_piece();
+#pragma unroll 1
+            for (uint32_t r = 0; r < sets; r += PAIR) {
+                uint4 w[PAIR];
+#pragma unroll
+                for (int h = 0; h < PAIR; ++h) w[h] = RES ? v[h] : load(r + (uint32_t)(AHEAD + h));
+                const uint32_t t0 = stage(r, v[0]), t1 = stage(r + 1u, v[1]);
+                if (ROWS == 1 || r < slabs) top[0] = max(top[0], t0);
+                else top[ROWS - 1] = max(top[ROWS - 1], t0);
+                if (ROWS == 1 || r + 1u < slabs) top[0] = max(top[0], t1);
+                else top[ROWS - 1] = max(top[ROWS - 1], t1);
+#pragma unroll
+                for (int h = 0; h + PAIR < AHEAD; ++h) v[h] = v[h + PAIR];
+#pragma unroll
+                for (int h = 0; h < PAIR; ++h) v[AHEAD - PAIR + h] = w[h];
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < ROWS; ++m) {
+            const uint32_t all = __reduce_max_sync(0xFFFFFFFFu, top[m]);
+            if (lane == 0) largest[warp][m] = all;
+        }
+    } else if (lane == 0) {
+#pragma unroll
+        for (int m = 0; m < ROWS; ++m) largest[warp][m] = 0u;
+    }
+    __syncwarp();
+    Acts xa;
+    if constexpr (RES) {
+        if (pieces) load_x(0u, xa);
+    }
+
+    // y is one launch's output; ARGMAX: key of the best element this thread has stored
+    unsigned long long my_best = 0ull;
+    auto store_out = [&](uint32_t m, uint32_t row, float v) { gemvtma::store_out<F>(A, m, row, v, my_best); };
+    uint32_t j = tg, left = pieces;
+    for (uint32_t j0 = 0; j0 < my_tiles; j0 += batch) {
+        const uint32_t jend = min(my_tiles, j0 + batch), buf = (j0 / batch) & 1u ? batch : 0u;  // two buffers: one meeting a batch
+        uint32_t at = base + L.part + (((buf + j - j0) << pshift) + pos) * (ROWS * 128u) + lane * (ROWS * 4u);
+#pragma unroll 1
+        for (; j < jend && slabs; j += TG, at += 8u * (ROWS * 128u)) {
+#pragma unroll
+            for (int p = 0; p < PAR; ++p) acc[p][0] = acc[p][1] = 0.0f;
+#pragma unroll 1
+            for (uint32_t s = 0; s < (RES ? 1u : slabs); ++s) {
+                if constexpr (!RES) load_x(s, xa);
+                Codes cur;
+                Sums sums;
+                if (++st == stages) st = 0u, par ^= 1u;
+                const bool there = test_stage(st, par);
+                unpack(q, cur);
+                multiply(cur, xa, sums);
+                const Scales now = sc;
+                if (--left) take(there);
+                apply(sums, now, xa);
+            }
+            // the digits' sums; lanes of even t go on with row prow, the others with row prow + 8
+#pragma unroll
+            for (int p = 0; p < PAR; ++p) {
+                const float send = t & 1u ? acc[p][0] : acc[p][1], keep = t & 1u ? acc[p][1] : acc[p][0];
+                const float v = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 1);
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (uint32_t)p * 4u), "f"(v) : "memory");
+            }
+        }
+        __syncthreads();
+        uint32_t top = 0u;  // of this lane's row
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) top = max(top, largest[w][ROWS == 1 ? 0u : t >> 1]);
+        for (uint32_t jj = j0 + warp; jj < jend; jj += WARPS) {  // a tile a warp: positions in a fixed tree, even and odd groups last
+            const uint32_t from = base + L.part + ((buf + jj - j0) << pshift) * (ROWS * 128u) + lane * (ROWS * 4u);
+            float v[PAR];
+#pragma unroll
+            for (int p = 0; p < PAR; ++p) {
+                float h[8];
+#pragma unroll
+                for (uint32_t i = 0; i < 8u; ++i) {
+                    h[i] = 0.0f;
+                    if (i < P) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(h[i]) : "r"(from + i * (ROWS * 128u) + (uint32_t)p * 4u));
+                }
+                v[p] = ((h[0] + h[1]) + (h[2] + h[3])) + ((h[4] + h[5]) + (h[6] + h[7]));
+            }
+            float y = ROWS == 1 ? v[0] + __shfl_xor_sync(0xFFFFFFFFu, v[0], 2) : v[0] + v[PAR - 1];
+            const uint32_t m = ROWS == 1 ? 0u : t >> 1, r = prow + 8u * (t & 1u), tile = tile_of(jj);
+            const bool live = m < M && (ROWS > 1 || t < 2u) && (gated || tile * 16u + r < N);
+            if (no_digits(top) && live) {
+                if (normed) y = plain_dot<true>(A, row_of(tile, r), m, nm_inv[m]);
+                else y = plain_dot<false>(A, row_of(tile, r), m, 0.0f);
+            }
+            if (gated) {  // even t: gate of output prow, odd t: its up
+                __syncwarp();
+                const float up = __shfl_xor_sync(0xFFFFFFFFu, y, 1);
+                if (live && ok && (t & 1u) == 0u) gemvtma::store_gated(A, m, tile * 8u + prow, y, up);
+            } else if (live && ok) {
+                store_out(m, tile * 16u + r, y);
+            }
+        }
+    }
+
+    if constexpr (POSTNORM_ || ARGMAX_ || SHARDED_) __syncthreads();
+    if (abort_flag) {  // let copies still in flight land before the CTA's memory is released
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000LL) __nanosleep(1000);
+    }
+    gemvtma::close_launch<F, WARPS, WARPS>(A, my_best);
+}
+
+// Launch plan: stages of a warp's ring (0: does not fit) and shared memory.
+struct Plan {
+    uint32_t grid, stages;
+    size_t smem;
+};
+template <class S>
+Plan plan_launch(uint32_t N, uint32_t K, uint32_t M, bool normed) {
+    Plan p;
+    // One CTA per SM, but for the SM that the norm kernel before a normed projection is on: its CTAs take the room
+    // of one of ours there, and ours would join another SM's (a layer with its two norms at one row 21.7 us so, 18.3
+    // with one CTA fewer, at two rows 24.2, and 26.1 with two fewer; a chain of plain projections needs them all).
+    p.grid = std::max(1u, (uint32_t)sm_count() - (normed ? 1u : 0u));
+    const uint32_t tiles = (N + 15u) / 16u, tc = (tiles + p.grid - 1u) / p.grid, row_bytes = K / 2u;
+    const uint32_t P = row_bytes >= SLAB ? 8u : (row_bytes + PIECE - 1u) / PIECE, TG = P > 4u ? 1u : P > 2u ? 2u : P > 1u ? 4u : 8u;
+    const uint32_t slabs = (row_bytes + SLAB - 1u) / SLAB, batch = TG * S::BATCH, part = (tc > batch ? 2u * batch : tc) * (8u / TG);
+    for (p.stages = std::min<uint32_t>(MAX_STAGES, (tc + TG - 1u) / TG * slabs); p.stages > 0u; --p.stages) {
+        p.smem = layout<S>(K, M, p.stages, part).total;
+        if (p.smem <= SMEM_LIMIT) break;  // two rows of 8192 and several batches of tiles leave room for one
+    }
+    p.smem = std::max(p.smem, SMEM_FLOOR);
+    return p;
+}
+
+template <class S, Fuse F, bool RES>
+int launch_one(const void* q, Args a, cudaStream_t stream) {
+    const Plan p = plan_launch<S>(a.N, a.K, a.M, a.pre.gamma != nullptr);
+    if (!p.stages) return fail(MIORI_E_INVALID, "gemv: no plan for N=%u K=%u M=%u", a.N, a.K, a.M);
+    a.stages = p.stages;
+    CUtensorMap tq;
+    const int rc = make_tmap_2d(&tq, q, CU_TENSOR_MAP_DATA_TYPE_UINT64, 8, (uint64_t)a.K / 16, a.N, PIECE / 8, a.gated ? 8 : 16,
+                                CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    const cudaError_t e = launch<Split::SHARED>(gemv_digits_kernel<S, F, RES>, dim3(p.grid), dim3(THREADS), p.smem, stream, true, tq, a);
+    if (e != cudaSuccess) return cuda_fail(e, "gemv_digits launch");
+    return MIORI_OK;
+}
+
+template <class S, Fuse F>
+int launch_k(const void* q, const Args& a, cudaStream_t stream) {
+    return a.K / 2u <= SLAB ? launch_one<S, F, true>(q, a, stream) : launch_one<S, F, false>(q, a, stream);
+}
+
+// K that this kernel takes: whole pieces (a row of 6208 codes, with its last groups picked out one by one, took 11.3 us at
+// 5967 rows, 7.6 in gemv_tma.cuh), up to where its launches still pay.
+inline bool takes(uint32_t K) { return K % PK == 0u && K <= MAX_K; }
+
+// One or two rows, of a K that is taken.
+template <int ROWS>
+int launch_rows(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t flags,
+                cudaStream_t stream, const gemvtma::Shard& sh) {
+    using S = Shape<ROWS>;
+    const bool placed = sh.pa.world > 1 || sh.best;  // y is a slice of an n_total-row output
+    Args a;
+    a.x = static_cast<const uint16_t*>(x), a.y = y;
+    a.q = static_cast<const uint8_t*>(q), a.s = static_cast<const uint16_t*>(s), a.b = static_cast<const uint16_t*>(b);
+    a.pre = sh.pre, a.post = sh.post;
+    a.N = N, a.K = K, a.M = ROWS, a.stages = 0u;
+    a.out_bf16 = flags & MIORI_OUT_BF16 ? 1u : 0u, a.gated = sh.gated ? 1u : 0u, a.early = flags & MIORI_LAUNCH_PDL ? 1u : 0u;
+    a.n_total = placed ? sh.n_total : N, a.row0 = placed ? sh.row0 : 0u, a.y_off = sh.y_off, a.best = sh.best, a.pa = sh.pa;
+    const int rc = gemvtma::check_fuse(sh, 4, N, ROWS, a.out_bf16 != 0u);
+    if (rc) return rc;
+    if (sh.best) {
+        if constexpr (ROWS == 1) return launch_k<S, gemvtma::ARGMAX>(q, a, stream);
+    }
+    if (sh.pa.world > 1) return launch_k<S, gemvtma::SHARDED>(q, a, stream);
+    if (sh.post.residual) return launch_k<S, gemvtma::POSTNORM>(q, a, stream);
+    if (sh.gated || sh.pre.gamma) return launch_k<S, gemvtma::FUSED>(q, a, stream);
+    return launch_k<S, gemvtma::NONE>(q, a, stream);
+}
+
+}  // namespace gemvdigits
+}  // namespace miori_b200

@@ -1,4 +1,5 @@
-// Weight-streaming GEMV for 1 <= M <= 32 activation rows on the packed 4- or 8-bit weights.
+// Weight-streaming GEMV for 1 <= M <= 32 activation rows on the packed 4- or 8-bit weights.  (One and two rows of 4-bit
+// weights in groups of 64 come here only where gemv_digits.cuh does not take K: gemv.cuh.)
 //
 //   y[m][n] = sum_g ( s[n][g] * sum_{k in g} code[n][k] * x[m][k]  +  b[n][g] * sum_{k in g} x[m][k] )
 //
@@ -482,6 +483,101 @@ __host__ __device__ inline Layout layout(uint32_t K, uint32_t M, uint32_t stages
     return L;
 }
 
+// ---- epilogues, shared by the kernels of the decode GEMV
+
+// One output element: y[m][row0 + row].  N-sharded launch (pa.world > 1): this rank's rows [row0, row0 + N) of an
+// n_total-row output go into its own y (at user offset y_off of its arena) and, as {value, launch number} packets,
+// into every peer's inbox; before the CTA exits it collects its share of the peers' rows (peers.cuh).
+// SHARDED is a template value rather than a run-time test because the single-GPU instantiation then compiles
+// exactly as if the peer path did not exist (a run-time branch cost 3-16 %).
+template <Fuse F, class A_>
+__device__ __forceinline__ void store_out(const A_& A, uint32_t m, uint32_t row, float v, unsigned long long& my_best) {
+    const size_t idx = (size_t)m * A.n_total + A.row0 + row;
+    const uint32_t bits = A.out_bf16 ? float_to_bf16_bits(v) : __float_as_uint(v);
+    if (A.out_bf16) reinterpret_cast<uint16_t*>(A.y)[idx] = (uint16_t)bits;
+    else reinterpret_cast<uint32_t*>(A.y)[idx] = bits;
+    if constexpr (F == ARGMAX) {  // compare what was stored (the rounded value when the output is bf16)
+        if (v == v) {
+            const unsigned long long key = peer_best_key(A.out_bf16 ? bits << 16 : bits, A.row0 + row);
+            my_best = key > my_best ? key : my_best;
+        }
+    } else if constexpr (F == SHARDED) {
+        if (A.pa.world > 1u) {
+            const uint32_t e = peer_epoch(A.pa);
+            const size_t elem = A.y_off / (A.out_bf16 ? 2u : 4u) + idx;
+            for (uint32_t p = 0; p < A.pa.world; ++p)
+                if (p != A.pa.rank) peer_send(peer_slot(A.pa, peer_arena(A.pa, p), e, elem), bits, e);
+        }
+    }
+}
+// gated: y[m][row] = bf16(silu(gate) * up) of the N/2-column output, with the arithmetic of the stand-alone
+// activation kernel (shaders/ops.metal:129-139)
+template <class A_>
+__device__ __forceinline__ void store_gated(const A_& A, uint32_t m, uint32_t row, float gate, float up) {
+    const float sg = gate / (1.0f + expf(-gate));
+    reinterpret_cast<uint16_t*>(A.y)[(size_t)m * (A.N >> 1) + row] = (uint16_t)float_to_bf16_bits(sg * up);
+}
+// What the grid does together once its rows are stored.  Every thread of every CTA gets here, behind a CTA-wide
+// barrier for all but the plain launch; WORK of the CTA's ALL warps have stored outputs.
+template <Fuse F, int WORK, int ALL, class A_>
+__device__ __forceinline__ void close_launch(const A_& A, unsigned long long my_best) {
+    if constexpr (F == POSTNORM) {
+        __shared__ float pn_part[neighbors::NORM_THREADS / 32];
+        __shared__ uint32_t pn_last;
+        __threadfence();  // this thread's rows of v are visible before the CTA reports in
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            pn_last = atomicAdd(A.post.arrivals, 1u) == gridDim.x - 1u ? 1u : 0u;
+            __threadfence();
+        }
+        __syncthreads();
+        if (pn_last && threadIdx.x < (uint32_t)neighbors::NORM_THREADS) {
+            float* out = reinterpret_cast<float*>(A.y);
+            for (uint32_t m = 0; m < A.M; ++m) {
+                const size_t at = (size_t)m * A.N;
+                neighbors::post_norm_add_any<9, true>(A.post.residual + at, out + at, A.post.gamma, out + at, A.N, A.post.eps,
+                                                      pn_part, A.post.vec);
+                neighbors::norm_sync<9>();  // pn_part is reused by the next row
+            }
+            if (threadIdx.x == 0) *A.post.arrivals = 0u;  // ready for the next launch
+        }
+    } else if constexpr (F == ARGMAX) {
+        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+        unsigned long long k = my_best;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xFFFFFFFFu, k, o);
+            k = other > k ? other : k;
+        }
+        __shared__ unsigned long long warp_keys[ALL];
+        if (lane == 0) warp_keys[warp] = k;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (uint32_t w = 1; w < (uint32_t)WORK; ++w) k = warp_keys[w] > k ? warp_keys[w] : k;
+            if (k != 0ull) atomicMax(A.best, k);  // one candidate per CTA
+            unsigned int* arrived = reinterpret_cast<unsigned int*>(A.best + 1);
+            __threadfence();
+            if (atomicAdd(arrived, 1u) == gridDim.x - 1u) {  // the last CTA: every candidate is in
+                __threadfence();
+                const unsigned long long win = atomicExch(A.best, 0ull);  // read, and reset for the next launch
+                *arrived = 0u;
+                uint32_t* pairs = reinterpret_cast<uint32_t*>(A.best) + 4;
+                const size_t at = (size_t)(reinterpret_cast<uint8_t*>(pairs) - (A.pa.local + PEER_CTL_BYTES)) / 4u;
+                peer_argmax_exchange(A.pa, pairs, at, peer_best_from_key(win));
+            }
+        }
+    } else if constexpr (F == SHARDED) {
+        if (A.pa.world > 1u) {
+            const uint32_t e = peer_epoch(A.pa);
+            __syncthreads();
+            if (A.out_bf16) peer_collect<true>(A.pa, e, A.y_off, A.M, A.n_total, A.row0, A.N);
+            else peer_collect<false>(A.pa, e, A.y_off, A.M, A.n_total, A.row0, A.N);
+            __syncthreads();
+            if (threadIdx.x == 0) peer_finish(A.pa, e);
+        }
+    }
+}
+
 template <class S, Fuse F>
 __global__ void __launch_bounds__(THREADS, 1)
 gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ Args A) {
@@ -615,7 +711,6 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
     // y is one launch's output; ARGMAX: key of the best element this thread has stored
     unsigned long long my_best = 0ull;
-    const uint32_t world = SHARDED_ ? A.pa.world : 0u;
     if (warp < WARPS) {
         // zeros: what lanes of other slots read, and the activations past the end of K
         const XArea xa = {base + L.x, L.x_pitch, base + L.ms};
@@ -639,37 +734,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         asm volatile("bar.sync 14, %0;" ::"n"(THREADS) : "memory");  // x is staged, the barriers exist
 
-        // N-sharded launch (pa.world > 1): this rank's rows [row0, row0 + N) of an n_total-row output go
-        // into its own y (at user offset y_off of its arena) and, as {value, launch number} packets, into
-        // every peer's inbox; before the CTA exits it collects its share of the peers' rows (peers.cuh).
-        // SHARDED is a template value rather than a run-time test because the single-GPU instantiation then
-        // compiles exactly as if the peer path did not exist (a run-time branch cost 3-16 %).
-        // one output element: y[m][row0 + row]
-        auto store_out = [&](uint32_t m, uint32_t row, float v) {
-            const size_t idx = (size_t)m * A.n_total + A.row0 + row;
-            const uint32_t bits = A.out_bf16 ? float_to_bf16_bits(v) : __float_as_uint(v);
-            if (A.out_bf16) reinterpret_cast<uint16_t*>(A.y)[idx] = (uint16_t)bits;
-            else reinterpret_cast<uint32_t*>(A.y)[idx] = bits;
-            if constexpr (ARGMAX_) {  // compare what was stored (the rounded value when the output is bf16)
-                if (v == v) {
-                    const unsigned long long key = peer_best_key(A.out_bf16 ? bits << 16 : bits, A.row0 + row);
-                    my_best = key > my_best ? key : my_best;
-                }
-            } else if constexpr (SHARDED_) {
-                if (world > 1u) {
-                    const uint32_t e = peer_epoch(A.pa);
-                    const size_t elem = A.y_off / (A.out_bf16 ? 2u : 4u) + idx;
-                    for (uint32_t p = 0; p < world; ++p)
-                        if (p != A.pa.rank) peer_send(peer_slot(A.pa, peer_arena(A.pa, p), e, elem), bits, e);
-                }
-            }
-        };
-        // gated: y[m][row] = bf16(silu(gate) * up) of the N/2-column output, with the arithmetic of the
-        // stand-alone activation kernel (shaders/ops.metal:129-139)
-        auto store_gated = [&](uint32_t m, uint32_t row, float gate, float up) {
-            const float sg = gate / (1.0f + expf(-gate));
-            reinterpret_cast<uint16_t*>(A.y)[(size_t)m * (N >> 1) + row] = (uint16_t)float_to_bf16_bits(sg * up);
-        };
+        auto store_out = [&](uint32_t m, uint32_t row, float v) { gemvtma::store_out<F>(A, m, row, v, my_best); };
 
         // ---- this lane's place in the MMAs.  As a B operand it supplies column n = lane / 4 = (slot n / RC,
         // row n % RC); as an accumulator it holds columns 2 t and 2 t + 1.
@@ -930,7 +995,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 if (gated) {  // tile rows 0 .. 7 are gates, 8 .. 15 the same outputs' up rows
                     for (uint32_t i = gt; i < 8u * M; i += 128u) {
                         const uint32_t m = i >> 3, r = i & 7u;
-                        store_gated(m, tile * 8u + r, total(m * 16u + r), total(m * 16u + r + 8u));
+                        store_gated(A, m, tile * 8u + r, total(m * 16u + r), total(m * 16u + r + 8u));
                     }
                 } else {
                     for (uint32_t o = gt; o < 16u * M; o += 128u) {
@@ -950,60 +1015,7 @@ gemv_tma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000LL) __nanosleep(1000);
     }
-    if constexpr (POSTNORM_) {  // every thread of the CTA gets here: no early exits above
-        __shared__ float pn_part[neighbors::NORM_THREADS / 32];
-        __shared__ uint32_t pn_last;
-        __threadfence();  // this thread's rows of v are visible before the CTA reports in
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            pn_last = atomicAdd(A.post.arrivals, 1u) == gridDim.x - 1u ? 1u : 0u;
-            __threadfence();
-        }
-        __syncthreads();
-        if (pn_last && threadIdx.x < (uint32_t)neighbors::NORM_THREADS) {
-            float* out = reinterpret_cast<float*>(A.y);
-            for (uint32_t m = 0; m < M; ++m) {
-                const size_t at = (size_t)m * N;
-                neighbors::post_norm_add_any<9, true>(A.post.residual + at, out + at, A.post.gamma, out + at, N, A.post.eps,
-                                                      pn_part, A.post.vec);
-                neighbors::norm_sync<9>();  // pn_part is reused by the next row
-            }
-            if (threadIdx.x == 0) *A.post.arrivals = 0u;  // ready for the next launch
-        }
-    } else if constexpr (ARGMAX_) {  // every thread of the CTA gets here: no early exits above
-        unsigned long long k = my_best;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long other = __shfl_xor_sync(0xFFFFFFFFu, k, o);
-            k = other > k ? other : k;
-        }
-        __shared__ unsigned long long warp_keys[THREADS / 32];
-        if (lane == 0) warp_keys[warp] = k;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (uint32_t w = 1; w < (uint32_t)WARPS; ++w) k = warp_keys[w] > k ? warp_keys[w] : k;
-            if (k != 0ull) atomicMax(A.best, k);  // one candidate per CTA
-            unsigned int* arrived = reinterpret_cast<unsigned int*>(A.best + 1);
-            __threadfence();
-            if (atomicAdd(arrived, 1u) == gridDim.x - 1u) {  // the last CTA: every candidate is in
-                __threadfence();
-                const unsigned long long win = atomicExch(A.best, 0ull);  // read, and reset for the next launch
-                *arrived = 0u;
-                uint32_t* pairs = reinterpret_cast<uint32_t*>(A.best) + 4;
-                const size_t at = (size_t)(reinterpret_cast<uint8_t*>(pairs) - (A.pa.local + PEER_CTL_BYTES)) / 4u;
-                peer_argmax_exchange(A.pa, pairs, at, peer_best_from_key(win));
-            }
-        }
-    } else if constexpr (SHARDED_) {
-        if (world > 1u) {  // every thread of the CTA gets here: no early exits above
-            const uint32_t e = peer_epoch(A.pa);
-            __syncthreads();
-            if (A.out_bf16) peer_collect<true>(A.pa, e, A.y_off, M, A.n_total, A.row0, N);
-            else peer_collect<false>(A.pa, e, A.y_off, M, A.n_total, A.row0, N);
-            __syncthreads();
-            if (threadIdx.x == 0) peer_finish(A.pa, e);
-        }
-    }
+    close_launch<F, WARPS, THREADS / 32>(A, my_best);
 }
 
 // Placement of an N-sharded launch's output and the fused neighbours of a launch: peers (world <= 1:
@@ -1024,6 +1036,20 @@ struct Shard {
     // norm prologue (one GPU): x is fp32; gamma null: off
     PreNorm pre;
 };
+
+// Whether a form of M rows exists.
+inline int check_fuse(const Shard& sh, int bits, uint32_t N, uint32_t M, bool out_bf16) {
+    const bool sharded = sh.pa.world > 1, argmax = sh.best != nullptr, postnorm = sh.post.residual != nullptr, normed = sh.pre.gamma != nullptr;
+    if ((int)argmax + (int)postnorm + (int)(sharded && !argmax) + (int)(sh.gated || normed) > 1)
+        return fail(MIORI_E_INVALID, "gemv: this combination of fused neighbours does not exist");
+    if (argmax && M != 1u) return fail(MIORI_E_INVALID, "the arg-max epilogue takes one activation row");
+    if (postnorm && (bits != 4 || out_bf16 || M > 4u))
+        return fail(MIORI_E_INVALID, "the post-norm epilogue takes 4-bit weights, up to four rows, fp32 out");
+    if (sh.gated && (bits != 4 || N % 16 != 0 || M > (normed ? 4u : 16u)))
+        return fail(MIORI_E_INVALID, "the gated epilogue takes 4-bit weights with N a multiple of 16, up to 16 rows "
+                                     "(four with the norm in front)");
+    return MIORI_OK;
+}
 
 // Launch plan: CTAs, active groups, stages per group, scale buffers.
 struct Plan {
@@ -1109,10 +1135,8 @@ int launch_one(const Plan& plan, const void* q, const Args& a, cudaStream_t stre
     const int rc = make_tmap_2d(&tq, q, CU_TENSOR_MAP_DATA_TYPE_UINT64, 8, (uint64_t)a.K * S::BITS / 64, a.N,
                                 (plan.slab_row + S::QPAD) / 8, gated ? 8 : 16, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
-    auto kern = gemv_tma_kernel<S, F>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
     // always with the programmatic attribute (the kernel knows when to wait): 2.0 us of host time against 2.5
-    if (e == cudaSuccess) e = launch(kern, dim3(plan.grid), dim3(THREADS), plan.smem, stream, true, tq, a);
+    const cudaError_t e = launch<Split::SHARED>(gemv_tma_kernel<S, F>, dim3(plan.grid), dim3(THREADS), plan.smem, stream, true, tq, a);
     if (e != cudaSuccess) return cuda_fail(e, "gemv_tma launch");
     return MIORI_OK;
 }
@@ -1139,95 +1163,19 @@ int launch_shape(const void* q, const void* s, const void* b, const void* x, voi
     a.n_total = placed ? sh.n_total : N, a.row0 = placed ? sh.row0 : 0u, a.y_off = sh.y_off;
     a.best = sh.best, a.pa = sh.pa, a.post = sh.post, a.pre = sh.pre;
     a.early = (flags & MIORI_LAUNCH_PDL) != 0 ? 1u : 0u;
-    if ((int)argmax + (int)postnorm + (int)(sharded && !argmax) + (int)(sh.gated || normed) > 1)
-        return fail(MIORI_E_INVALID, "gemv: this combination of fused neighbours does not exist");
+    const int rc = check_fuse(sh, S::BITS, N, M, a.out_bf16 != 0u);
+    if (rc) return rc;
     if (argmax) {
         if constexpr (S::ROWS == 1) return launch_one<S, ARGMAX>(plan, q, a, stream);
-        return fail(MIORI_E_INVALID, "the arg-max epilogue takes one activation row");
     }
     if (postnorm) {
-        if constexpr (S::BITS == 4 && FEW)
-            if (!a.out_bf16 && M <= 4) return launch_one<S, POSTNORM>(plan, q, a, stream);
-        return fail(MIORI_E_INVALID, "the post-norm epilogue takes 4-bit weights, up to four rows, fp32 out");
+        if constexpr (S::BITS == 4 && FEW) return launch_one<S, POSTNORM>(plan, q, a, stream);
     }
-    if (sh.gated && (S::BITS != 4 || N % 16 != 0 || M > (normed ? 4u : 16u)))
-        return fail(MIORI_E_INVALID, "the gated epilogue takes 4-bit weights with N a multiple of 16, up to 16 rows "
-                                     "(four with the norm in front)");
     if constexpr (S::ROWS == 1)
         if (wide_k) return launch_one<S, LONG>(plan, q, a, stream);
     if (normed || sh.gated) return launch_one<S, FUSED>(plan, q, a, stream);
     if (sharded) return launch_one<S, SHARDED>(plan, q, a, stream);
     return launch_one<S, NONE>(plan, q, a, stream);
-}
-
-// ---- batches
-//
-// A row's bits must not depend on how many rows are in flight beside it, so everything that decides the order of
-// its sums -- the shape and how many groups share a tile -- is chosen by a class of batch sizes and not by M:
-// the class's largest batch has to fit, and where it does not, every batch of the class is dealt to launches of
-// the next smaller class.  Classes: 1..4 rows (4-bit weights in groups of 64: 1..2, see below), up to 8, 16, 32.
-template <int BITS, int GROUP>
-struct Batch {
-    // Three and four rows of 4-bit weights at group 64 gain nothing from slots (two, one step a pass): 16384 x
-    // 2048 takes 8.0 us with them and 7.2 without; they run as eight do.
-    static constexpr bool WIDE3 = BITS == 4 && GROUP == 64;
-    static constexpr uint32_t class_of(uint32_t M) { return M <= 2u ? (WIDE3 ? 2u : 4u) : M <= 4u ? (WIDE3 ? 8u : 4u) : M <= 8u ? 8u : M <= 16u ? 16u : 32u; }
-    static uint32_t kpar_of(uint32_t cls, uint32_t N, uint32_t K) {
-        switch (cls) {
-        case 1: return choose_kpar<Shape<BITS, GROUP, 1>>(N, K, 1);
-        case 2: return choose_kpar<Shape<BITS, GROUP, 2>>(N, K, 2);
-        case 4: return choose_kpar<Shape<BITS, GROUP, WIDE3 ? 8 : 4>>(N, K, 4);
-        case 8: return choose_kpar<Shape<BITS, GROUP, 8>>(N, K, 8);
-        case 16: return choose_kpar<Shape<BITS, GROUP, 16>>(N, K, 16);
-        default: return choose_kpar<Shape<BITS, GROUP, 32>>(N, K, 32);
-        }
-    }
-    // One launch of up to cls rows.  Below eight the shapes of fewer rows sum in the same order.
-    static int launch(uint32_t cls, uint32_t kpar, const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N,
-                      uint32_t K, uint32_t M, uint32_t flags, cudaStream_t stream, const Shard& sh, bool wide_k) {
-#define MIORI_GEMV(ROWS) return launch_shape<Shape<BITS, GROUP, ROWS>>(q, s, b, x, y, N, K, M, flags, stream, sh, kpar, wide_k)
-        if (cls > 16u) MIORI_GEMV(32);
-        if (cls > 8u) MIORI_GEMV(16);
-        if (cls > 4u || (WIDE3 && cls > 2u)) MIORI_GEMV(8);
-        if (M == 1u) MIORI_GEMV(1);
-        if (M == 2u) MIORI_GEMV(2);
-        if constexpr (!WIDE3) MIORI_GEMV(4);
-#undef MIORI_GEMV
-        return fail(MIORI_E_INVALID, "gemv: %u rows are not of the class of %u", M, cls);
-    }
-    static int run(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t M,
-                   uint32_t flags, cudaStream_t stream, Shard sh) {
-        uint32_t cls = class_of(M), kpar = 0;
-        while (cls && (kpar = kpar_of(cls, N, K)) == 0u) cls >>= 1;
-        const bool wide_k = cls == 0u;  // not even one row and its scales fit
-        if (wide_k) {
-            if (sh.gated || sh.post.residual || sh.best || sh.pa.world > 1) return 1;
-            cls = 1u, kpar = choose_kpar<Shape<BITS, GROUP, 1>>(N, K, 1u, false);
-            if (!kpar) return 1;
-        }
-        const uint32_t launches = (M + cls - 1u) / cls, rows = (M + launches - 1u) / launches;
-        const uint32_t n_out = sh.gated ? N / 2u : sh.pa.world > 1 || sh.best ? sh.n_total : N;
-        const size_t x_row = (size_t)K * (sh.pre.gamma ? 4 : 2), y_row = (size_t)n_out * ((flags & MIORI_OUT_BF16) ? 2 : 4);
-        for (uint32_t m0 = 0; m0 < M; m0 += rows) {
-            const int rc = launch(cls, kpar, q, s, b, static_cast<const uint8_t*>(x) + m0 * x_row, static_cast<uint8_t*>(y) + m0 * y_row,
-                                  N, K, std::min(rows, M - m0), flags, stream, sh, wide_k);
-            if (rc) return rc;
-            sh.y_off += rows * y_row;
-            if (sh.post.residual) sh.post.residual += (size_t)rows * N;
-        }
-        return MIORI_OK;
-    }
-};
-
-// Launch, or return 1 if not even one row of K activations fits shared memory, or a fused form does not take the
-// shape (nothing launched).
-template <int BITS>
-int try_launch(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t M,
-               uint32_t group, uint32_t flags, cudaStream_t stream, const Shard& sh = Shard()) {
-    const bool fused = sh.pa.world > 1 || sh.best || sh.gated || sh.post.residual || sh.pre.gamma;
-    if (fused && (K / group) % 8 != 0) return 1;  // what the fused entries promise to take
-    return group == 64 ? Batch<BITS, 64>::run(q, s, b, x, y, N, K, M, flags, stream, sh)
-                       : Batch<BITS, 32>::run(q, s, b, x, y, N, K, M, flags, stream, sh);
 }
 
 }  // namespace gemvtma

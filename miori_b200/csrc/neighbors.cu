@@ -14,7 +14,8 @@ namespace miori_b200 {
 namespace neighbors {
 
 // PIECES > 0: rows of at most 4 * NORM_THREADS * PIECES elements in 16-byte pieces, read once (norm.cuh).
-template <int PIECES>
+// SPLIT: copies of the norm kernels for a few rows between the projections of a decode step (common.cuh: set_up_kernel).
+template <int PIECES, Split SPLIT>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, uint16_t* __restrict__ y,
                uint32_t n, float eps) {
@@ -32,6 +33,7 @@ rmsnorm_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, uint
     }
 }
 
+template <Split SPLIT>
 __global__ void __launch_bounds__(NORM_THREADS)
 post_norm_add_kernel(const float* __restrict__ x, const float* __restrict__ src,
                      const uint16_t* __restrict__ w, float* __restrict__ out, uint32_t n, float eps, bool vec) {
@@ -262,11 +264,13 @@ MIORI_API int miori_rmsnorm(const void* x, const void* gamma, void* y, uint32_t 
     if (!x || !gamma || !y) return fail(MIORI_E_INVALID, "miori_rmsnorm: null pointer");
     if (rows == 0 || n == 0) return fail(MIORI_E_INVALID, "miori_rmsnorm: empty shape rows=%u n=%u", rows, n);
     const bool vec = n % 4u == 0u && aligned16(x) && (reinterpret_cast<uintptr_t>(gamma) & 7u) == 0 && (reinterpret_cast<uintptr_t>(y) & 7u) == 0;
-    auto kern = !vec || n > 8192u ? neighbors::rmsnorm_kernel<0> : n <= 2048u ? neighbors::rmsnorm_kernel<2> : neighbors::rmsnorm_kernel<8>;
-    const cudaError_t e = launch(kern, dim3(rows), dim3(neighbors::NORM_THREADS), 0,
-                                 (cudaStream_t)stream, (flags & MIORI_LAUNCH_PDL) != 0,
-                                 static_cast<const float*>(x), static_cast<const uint16_t*>(gamma),
-                                 static_cast<uint16_t*>(y), n, eps);
+    auto run = [&](auto split) {
+        constexpr Split S = decltype(split)::value;
+        auto kern = !vec || n > 8192u ? neighbors::rmsnorm_kernel<0, S> : n <= 2048u ? neighbors::rmsnorm_kernel<2, S> : neighbors::rmsnorm_kernel<8, S>;
+        return launch<S>(kern, dim3(rows), dim3(neighbors::NORM_THREADS), 0, (cudaStream_t)stream, (flags & MIORI_LAUNCH_PDL) != 0,
+                         static_cast<const float*>(x), static_cast<const uint16_t*>(gamma), static_cast<uint16_t*>(y), n, eps);
+    };
+    const cudaError_t e = rows <= 4u ? run(std::integral_constant<Split, Split::SHARED>()) : run(std::integral_constant<Split, Split::DRIVERS>());
     if (e != cudaSuccess) return cuda_fail(e, "miori_rmsnorm launch");
     return MIORI_OK;
 }
@@ -275,11 +279,13 @@ MIORI_API int miori_post_norm_add(const void* x, const void* src, const void* ga
                                   uint32_t n, float eps, uint32_t flags, void* stream) {
     if (!x || !src || !gamma || !out) return fail(MIORI_E_INVALID, "miori_post_norm_add: null pointer");
     if (rows == 0 || n == 0) return fail(MIORI_E_INVALID, "miori_post_norm_add: empty shape rows=%u n=%u", rows, n);
-    const cudaError_t e = launch(neighbors::post_norm_add_kernel, dim3(rows), dim3(neighbors::NORM_THREADS), 0,
-                                 (cudaStream_t)stream, (flags & MIORI_LAUNCH_PDL) != 0,
-                                 static_cast<const float*>(x), static_cast<const float*>(src),
-                                 static_cast<const uint16_t*>(gamma), static_cast<float*>(out), n, eps,
-                                 neighbors::norm_vec(n, x, src, out, gamma));
+    auto run = [&](auto split) {
+        constexpr Split S = decltype(split)::value;
+        return launch<S>(neighbors::post_norm_add_kernel<S>, dim3(rows), dim3(neighbors::NORM_THREADS), 0, (cudaStream_t)stream,
+                         (flags & MIORI_LAUNCH_PDL) != 0, static_cast<const float*>(x), static_cast<const float*>(src),
+                         static_cast<const uint16_t*>(gamma), static_cast<float*>(out), n, eps, neighbors::norm_vec(n, x, src, out, gamma));
+    };
+    const cudaError_t e = rows <= 4u ? run(std::integral_constant<Split, Split::SHARED>()) : run(std::integral_constant<Split, Split::DRIVERS>());
     if (e != cudaSuccess) return cuda_fail(e, "miori_post_norm_add launch");
     return MIORI_OK;
 }

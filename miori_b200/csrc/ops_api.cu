@@ -1,7 +1,7 @@
 // C ABI launch entries: argument validation, path selection, enqueue.
 #include "common.cuh"
 #include "dequant.cuh"
-#include "gemv_tma.cuh"
+#include "gemv.cuh"
 #include "gemv_cache.cuh"
 
 using namespace miori_b200;

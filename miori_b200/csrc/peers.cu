@@ -2,7 +2,7 @@
 // entries whose epilogue is the all-gather (peers.cuh), and a stand-alone all-gather kernel for
 // outputs produced by another kernel (the cache GEMM).
 #include "common.cuh"
-#include "gemv_tma.cuh"
+#include "gemv.cuh"
 #include "peers.cuh"
 
 #include <cstring>

@@ -167,3 +167,83 @@ def test_rows_whose_scales_do_not_fit_beside_them(bits, group, K, N, M):
         want = xn.double() @ w.T
         assert float((got - want).norm() / want.norm()) < 1e-4  # single roundings of the normalised activations may tip over
     assert miori_b200.lib.miori_device_error_poll() == 0
+
+
+# one and two rows of 4-bit weights in groups of 64: rows of one to eight 128-byte pieces and of several slabs, whole and not, one
+# tile, as many as CTAs, one more, and several batches of a CTA's tiles
+@pytest.mark.parametrize("K", [256, 512, 768, 1024, 1280, 1792, 2048, 2304, 3840, 4096, 7936, 8192])
+@pytest.mark.parametrize("N", [1, 17, 2368, 2371, 40000])
+def test_integer_sums_of_one_and_two_rows(K, N):
+    if N * K > 1 << 27:
+        pytest.skip("covered by shorter rows")
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=N + K, device=DEV)
+    x = synth.make_activation(2, K, seed=K, device=DEV)
+    x[1, K // 2:] *= 2.0 ** -9   # groups of different size
+    guard = torch.full((2 * N + 64,), 777.0, device=DEV)
+    y = guard[32:32 + 2 * N].view(2, N)
+    miori_b200.gemv4(q, s, b, x, group=64, flags=miori_b200.LAUNCH_PDL, out=y)
+    groups = x.double().view(2, -1, 64)
+    parts = torch.einsum("mgk,ngk->mng", groups, _weights64(q, s, b, 4, 64).view(N, -1, 64))
+    bias = torch.einsum("mg,ng->mng", groups.sum(-1), b.double())
+    want, size = parts.sum(-1), (parts.abs() + 2 * bias.abs()).square().sum(-1).sqrt()
+    # a group's sum is exact; that of its codes and its bias term (which cancel), and the sum over groups, round by 2^-24 of
+    # what they come to, some three times a group and at random
+    for m in (0, 1):
+        assert float((y[m].double() - want[m]).norm() / size[m].norm()) < 4 * 2.0 ** -24
+        assert torch.equal(miori_b200.gemv4(q, s, b, x[m:m + 1].contiguous(), group=64), y[m:m + 1])
+    assert (guard[:32] == 777.0).all() and (guard[32 + 2 * N:] == 777.0).all()
+    assert torch.equal(miori_b200.gemv4(q, s, b, x, group=64, flags=miori_b200.OUT_BF16), y.to(torch.bfloat16))
+    assert miori_b200.lib.miori_device_error_poll() == 0
+
+
+@pytest.mark.parametrize("K", [256, 2048, 8192])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_rows_with_values_that_are_not_finite(K, bad):
+    N = 100
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=K, device=DEV)
+    x = synth.make_activation(2, K, seed=K, device=DEV)
+    want = miori_b200.gemv4(q, s, b, x, group=64)
+    x[1, K - 3] = bad
+    got = miori_b200.gemv4(q, s, b, x, group=64)
+    assert torch.equal(got[0], want[0]) and not torch.isfinite(got[1]).any()
+    assert not torch.isfinite(miori_b200.gemv4(q, s, b, x[1:].contiguous(), group=64)).any()
+
+
+@pytest.mark.parametrize("K", [256, 2048, 4096])
+@pytest.mark.parametrize("shift", [-118, -100, -96, 100, 118])
+def test_rows_next_to_nothing_and_huge_ones(K, shift):
+    """bf16 goes down to 2^-126 with all its bits, and up to 2^127: what the weights make of that is in fp32's range."""
+    N = 64
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=K, device=DEV)
+    x = synth.make_activation(2, K, seed=K, device=DEV).clamp(-4.0, 4.0)
+    x = torch.where(x.abs() < 2.0 ** -7, torch.full_like(x, 2.0 ** -7), x)  # no subnormals after the shift
+    x[1] = x[1] * (2.0 if shift < 0 else 0.5)
+    want = x.double() @ _weights64(q, s, b, 4, 64).T
+    got = miori_b200.gemv4(q, s, b, (x.float() * 2.0 ** shift).to(torch.bfloat16), group=64).double() * 2.0 ** -shift
+    # sums of a whole row in order at worst: K roundings, growing as their square root
+    assert float((got - want).norm() / want.norm()) < 2.0 ** -24 * 4 * K ** 0.5
+
+
+def test_rows_of_zeros_and_groups_of_zeros():
+    N, K = 48, 1024
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=1, device=DEV)
+    x = synth.make_activation(2, K, seed=2, device=DEV)
+    x[0] = 0.0
+    x[1, 64:960] = 0.0
+    got = miori_b200.gemv4(q, s, b, x, group=64)
+    want = x.double() @ _weights64(q, s, b, 4, 64).T
+    assert (got[0] == 0).all() and float((got[1].double() - want[1]).norm() / want[1].norm()) < 4 * 2.0 ** -24
+
+
+def test_fused_forms_of_activations_that_are_not_finite():
+    N, K = 64, 2048
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=3, device=DEV)
+    x = synth.make_activation(2, K, seed=4, device=DEV).float()
+    x[1, 7] = float("nan")
+    g = synth.make_activation(1, K, seed=2, device=DEV).reshape(-1)
+    y = miori_b200.gemv4_rmsnorm(q, s, b, x, g, 1e-5, group=64)
+    pair = miori_b200.gemv4(q, s, b, miori_b200.rmsnorm(x, g, 1e-5), group=64)
+    assert torch.isfinite(y[0]).all() and torch.equal(y[1], pair[1])  # the norm's rounding to bf16 is for finite values
+    z = miori_b200.gemv4_silu(q, s, b, x.to(torch.bfloat16), group=64)
+    v = miori_b200.gemv4(q, s, b, x.to(torch.bfloat16), group=64)
+    assert torch.equal(z[0], miori_b200.silu_mul(v[:, :N // 2].contiguous(), v[:, N // 2:].contiguous())[0])
