@@ -4,12 +4,17 @@
 //
 // Bound by HBM: 0.5625-1.125 B read and 2 B written per weight.  Rows follow one another without gaps and
 // hold whole scale groups, so the tensor is one array: unit i is eight weights, its scale is number
-// 8 i / group, and no row or column is ever computed.  A thread takes UNITS units one block width apart:
-// every load and store instruction of a warp covers contiguous memory (128-256 bytes of codes, 512 of
-// output), and all loads are issued before the first use.  Chained launches of 16384 x 2048: 25.7 us with
-// a 64-bit division per unit and one unit in flight, 17.3 now (5.0 TB/s).
+// 8 i / group, and no row or column is ever computed.
+//
+// Large tensors (dequant_wide_kernel): a grid that is resident at once, a thread per 32 weights, its next ones read before
+// it works on these, 32-byte stores.  Chains of launches, the kernel of four units a thread and this, us: 4-bit
+// 16384 x 2048 17.2 -> 15.4 (5.6 TB/s), over one buffer 14.3 -> 12.2, 2048 x 2048 3.5 -> 3.15, 1024 x 8192 5.4 -> 4.5; 8-bit
+// 8192 x 2048 11.0 -> 8.8.  (16 weights a thread 15.7; two iterations ahead 16.9; blocks of four units without a loop
+// are 3.5 waves, and each of their 4096 CTAs ends with a fence.)
 #pragma once
 #include "common.cuh"
+
+#include <algorithm>
 
 namespace miori_b200 {
 
@@ -75,15 +80,64 @@ dequant_rowmajor_kernel(const uint32_t* __restrict__ q, const uint16_t* __restri
     __threadfence();
 }
 
+// The same by a resident grid, 32 weights -- four units of one scale group -- a thread and step.  out: 32-byte aligned.
+constexpr uint32_t WIDE_UNITS = 4, WIDE_CTAS = 6;  // a step; CTAs of an SM
+template <int BITS>
+__global__ void __launch_bounds__(DEQUANT_THREADS)
+dequant_wide_kernel(const uint4* __restrict__ q, const uint16_t* __restrict__ s, const uint16_t* __restrict__ b,
+                    uint4* __restrict__ out, uint64_t steps, uint32_t sshift) {
+    constexpr int WORDS = BITS, PER = BITS / 4;  // of a step, of a unit
+    struct Step { uint32_t w[WORDS], sc, bi; };
+    pdl_wait_prior();  // a programmatic launch, which costs the host less
+    const uint64_t stride = (uint64_t)gridDim.x * DEQUANT_THREADS;
+    auto load = [&](uint64_t i, Step& l) {
+        if (i >= steps) return;
+#pragma unroll
+        for (int k = 0; k < WORDS / 4; ++k) {
+            const uint4 v = __ldcs(q + i * (WORDS / 4) + k);
+            l.w[4 * k] = v.x, l.w[4 * k + 1] = v.y, l.w[4 * k + 2] = v.z, l.w[4 * k + 3] = v.w;
+        }
+        l.sc = __ldg(s + (i >> sshift));
+        l.bi = __ldg(b + (i >> sshift));
+    };
+    uint64_t i = (uint64_t)blockIdx.x * DEQUANT_THREADS + threadIdx.x;
+    Step cur, next;
+    load(i, cur);
+    for (; i < steps; i += stride) {
+        load(i + stride, next);
+#pragma unroll
+        for (int u = 0; u < (int)WIDE_UNITS; u += 2) {
+            uint32_t w0[PER], w1[PER];
+#pragma unroll
+            for (int k = 0; k < PER; ++k) w0[k] = cur.w[u * PER + k], w1[k] = cur.w[(u + 1) * PER + k];
+            const uint4 lo = dequant_unit<BITS>(w0, cur.sc, cur.bi), hi = dequant_unit<BITS>(w1, cur.sc, cur.bi);
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                         ::"l"(out + i * WIDE_UNITS + u), "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w)
+                         : "memory");
+        }
+        cur = next;
+    }
+    __threadfence();  // no early trigger: as above
+}
+
 template <int BITS>
 int launch_dequant_rowmajor(const void* q, const void* s, const void* b, void* out, uint32_t N,
                             uint32_t K, uint32_t group, cudaStream_t stream) {
     const uint64_t units = (uint64_t)N * (K >> 3);
     const uint32_t ushift = group == 32 ? 2u : 3u;  // log2 of the units per scale group
-    // four units per thread, or one while that leaves SMs without a block
+    // one unit per thread while four leave SMs without a block (256 x 2048: 1.94 us, 2.04 on the resident grid)
     const bool wide = units >= (uint64_t)sm_count() * DEQUANT_THREADS * 8u;
     const uint64_t per_block = (uint64_t)DEQUANT_THREADS * (wide ? 4u : 1u), blocks = (units + per_block - 1u) / per_block;
     if (blocks > 0x7FFFFFFFull) return fail(MIORI_E_INVALID, "dequant: N=%u K=%u is too large", N, K);
+    if (wide && (reinterpret_cast<uintptr_t>(out) & 31u) == 0) {  // (a row is a multiple of 32 weights)
+        const uint64_t steps = units / WIDE_UNITS, fill = (steps + DEQUANT_THREADS - 1u) / DEQUANT_THREADS;
+        const cudaError_t e = launch(dequant_wide_kernel<BITS>, dim3((unsigned)std::min<uint64_t>((uint64_t)sm_count() * WIDE_CTAS, fill)),
+                                     dim3(DEQUANT_THREADS), 0, stream, true, reinterpret_cast<const uint4*>(q),
+                                     reinterpret_cast<const uint16_t*>(s), reinterpret_cast<const uint16_t*>(b),
+                                     reinterpret_cast<uint4*>(out), steps, ushift - 2u);
+        if (e != cudaSuccess) return cuda_fail(e, "dequant_wide launch");
+        return MIORI_OK;
+    }
     auto kern = wide ? dequant_rowmajor_kernel<BITS, 4> : dequant_rowmajor_kernel<BITS, 1>;
     cudaError_t e = launch(kern, dim3((unsigned)blocks), dim3(DEQUANT_THREADS), 0, stream, true,
                            reinterpret_cast<const uint32_t*>(q), reinterpret_cast<const uint16_t*>(s),

@@ -61,3 +61,19 @@ def test_full_size_cache_checksum(port):
                                           b[i:i + 4096].contiguous(), group=64)
              for i in range(0, N, 4096)]
     assert torch.equal(torch.cat(parts), out)
+
+
+@pytest.mark.parametrize("bits,N,K,group", [(4, 9471, 256, 32), (4, 9472, 256, 64), (4, 4736, 544, 32), (8, 2369, 1024, 64), (8, 4735, 512, 32),
+                                            (4, 37889, 64, 64), (8, 20001, 160, 32)])
+@pytest.mark.parametrize("shift", [0, 8])
+def test_resident_grid_where_it_begins_and_ends(port, bits, N, K, group, shift):
+    """About as many weights as the resident grid starts at, a last step of some threads only, and an output that
+    its 32-byte stores do not fit."""
+    q, s, b = synth.make_weight(N, K, bits, group, seed=N, device=DEV)
+    buf = torch.full((N * K + 64,), 777.0, dtype=torch.bfloat16, device=DEV)
+    out = buf[16 + shift:16 + shift + N * K].view(N, K)
+    fn = miori_b200.dequant4_rowmajor if bits == 4 else miori_b200.dequant8_rowmajor
+    fn(q, s, b, group=group, out=out)
+    want = port.dequant_rowmajor(bits, u32(q), u16(s), u16(b), group)
+    assert np.array_equal(u16(out), want)
+    assert (buf[:16 + shift] == 777.0).all() and (buf[16 + shift + N * K:] == 777.0).all()
