@@ -45,7 +45,7 @@ struct Batch {
                    uint32_t flags, cudaStream_t stream, Shard sh) {
         if constexpr (BITS == 4 && GROUP == 64) {
             // the class of one and two rows: exact integer sums (gemv_digits.cuh)
-            if (M <= 2u && gemvdigits::takes(K))
+            if (M <= 2u && gemvdigits::takes(N, K))
                 return M == 1u ? gemvdigits::launch_rows<1>(q, s, b, x, y, N, K, flags, stream, sh)
                                : gemvdigits::launch_rows<2>(q, s, b, x, y, N, K, flags, stream, sh);
         }

@@ -15,7 +15,9 @@
 //
 // What bounds it: in a chain of dependent launches the steps that follow one another -- the hand-over from grid
 // to grid (0.7 us), the trip of x through L2 (0.35), its conversion (0.3; 0.25 a slab beyond), each piece of weights
-// (0.33) -- and not HBM: with the weights in L2 the four projections of a layer take 13.4 instead of 13.8.  So nothing else is on that path:
+// (0.33) -- and
+// not HBM: with the weights in L2 the four projections of a layer took 13.4 instead of 13.8.  So nothing else is on that
+// path:
 //   * TWO CTAs of 256 threads fit an SM, one of this launch and one of the next, which fetches its weights
 //     while this one works.  Every launch is one CTA per SM, those without rows included: a launch of
 //     fewer would let the next one's double up, and every later launch would inherit the skew;
@@ -29,22 +31,22 @@
 // After its first pieces a CTA holds the others back for 800 cycles: it starts when its predecessor fetches
 // x, whose loads would queue up behind them (four projections of a layer 15.2 us when all are fetched at once, 14.5 so).
 //
-// Measured in chains over weights larger than L2, the kernel of gemv_tma.cuh and this one, us, one row:
-// 2048 x 2048 2.50 -> 2.16, 3072 x 2048 2.92 -> 2.41, 16384 x 2048 6.51 -> 4.74, 2048 x 8192 4.64 -> 4.46, the four
-// together 16.6 -> 13.4; a layer of them with its norms and activation (six launches) 21.1 -> 18.3.  Two rows: 2.56 -> 2.43,
-// 2.93 -> 2.84, 6.99 -> 5.83, 17.4 -> 17.2 together; behind from K = 3072 on, where the conversion of two rows (2.2
-// times the instructions of fp16's) is most of the time: 2048 x 4096 3.52 -> 3.97, 2048 x 8192 4.89 -> 6.34.  A row's bits
-// must not depend on the other row, and one row is what this is for.
+// Measured in chains over weights larger than L2, the kernel of gemv_tma.cuh and this one, us, one row: 2048 x 2048
+// 2.45 -> 2.16, 3072 x 2048 2.92 -> 2.43, 16384 x 2048 6.57 -> 4.86, 32768 x 512 6.55 -> 3.43, 2048 x 8192 4.63 -> 4.38, the four
+// projections of a layer 16.6 -> 13.4, with its norms and activation (six launches) 21.1 -> 17.8; launches that wait for the
+// one before, 2048 x 2048 2.86 -> 2.76, 16384 x 2048 7.69 -> 6.94.  Two rows 2.50 -> 2.44, 2.93 -> 2.85, 7.03 -> 5.88.
+// Behind, because converting a row takes 2.2 times the instructions of fp16's and is most of the time there: two rows
+// beyond one slab (2048 x 4096 3.46 -> 3.89, 2048 x 8192 4.89 -> 6.26), and launches that wait of such rows (one row 4.12 ->
+// 4.49 and 5.61 -> 6.93) or of two short ones (2048 x 2048 2.93 -> 3.19).  A row's bits must depend neither on the other row
+// nor on how it is launched, and a chain of dependent launches at one row is what this is for.
 #pragma once
 #include "gemv_tma.cuh"
 
 namespace miori_b200 {
 namespace gemvdigits {
 
-using gemvtma::cmax;
 using gemvtma::Fuse;
 using gemvtma::lds128;
-using gemvtma::lds16;
 using gemvtma::lds_words;
 
 constexpr int WARPS = 8, THREADS = 32 * WARPS;
@@ -136,7 +138,7 @@ __device__ __forceinline__ uint32_t max_abs2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ bool no_digits(uint32_t largest) { return largest >= 0x7F80u || (largest != 0u && largest < (29u << 7)); }
 
 // Eight consecutive activations (bf16) -> four digit planes, the even ones times sixteen; the first lane of a
-// scale group (eight neighbouring lanes) stores {r, sum of x, 256 r, 0}: r r undoes the scaling for the digits
+// scale group (eight neighbouring lanes) stores {r, sum of x, 256 r, sum of x}: r r undoes the scaling for the digits
 // 0 and 1, (256 r)^2 for 2 and 3.  (As a square, so that neither a scale nor a sum leaves fp32's range when it
 // meets half of it.)  Every lane of the warp calls.  Returns the group's largest magnitude.
 __device__ __forceinline__ uint32_t stage_unit(const uint4& v, bool live, uint32_t at, uint32_t pitch, bool first, uint32_t ms_at) {
@@ -170,7 +172,7 @@ __device__ __forceinline__ uint32_t stage_unit(const uint4& v, bool live, uint32
             asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + (uint32_t)l * pitch), "r"(p[0][l]), "r"(p[1][l]) : "memory");
         if (first) {
             const float r = __uint_as_float((49u + e) << 23);  // 2^(e - 78)
-            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ms_at), "f"(r), "f"(sum), "f"(r * 256.0f), "f"(0.0f) : "memory");
+            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ms_at), "f"(r), "f"(sum), "f"(r * 256.0f), "f"(sum) : "memory");
         }
     }
     return mx;
@@ -227,11 +229,8 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     __shared__ volatile uint32_t abort_flag;
     __shared__ uint32_t largest[WARPS][ROWS];  // magnitudes, in what each warp has seen of a row
 
-    // A launch that may not start early waits here, and lets its dependents start only when its predecessor is
-    // complete: they prefetch what that may have written.
     const long long born = clock64();
-    if (A.early == 0u) pdl_wait_prior();
-    pdl_launch_dependents();
+    if (A.early) pdl_launch_dependents();
 
     const uint32_t my_tiles = (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x;
     const uint32_t batch = TG * S::BATCH;
@@ -281,15 +280,22 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(base + L.zeros + 16u * warp), "r"(0u) : "memory");
     }
     __syncwarp();
+    // A launch that may not start early waits here, and lets its dependents start only when its predecessor is
+    // complete: they prefetch what that may have written.
+    if (A.early == 0u) {
+        pdl_wait_prior();
+        pdl_launch_dependents();
+    }
     {
         const uint32_t n = min(stages, pieces);
-        uint32_t i = 0;
-        for (; i < min(n, (uint32_t)HEAD_PIECES); ++i) issue(i);
-        if (i < n && A.early) {
-            const long long t0 = clock64();
-            while (clock64() - t0 < HOLD_CYCLES) __nanosleep(40);
+#pragma unroll 1  // one copy of the code: three copies of it cost a layer with its norms 0.5 to 1.6 us
+        for (uint32_t i = 0; i < n; ++i) {
+            if (i == (uint32_t)HEAD_PIECES && A.early) {
+                const long long t0 = clock64();
+                while (clock64() - t0 < HOLD_CYCLES) __nanosleep(40);
+            }
+            issue(i);
         }
-        for (; i < n; ++i) issue(i);
     }
 
     // ---- this lane's place in the MMAs: tile rows prow and prow + 8 (in an order that spreads the swizzled rows which
@@ -380,8 +386,15 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             const float r = x.r[c];
             const float v0 = (float)(o.d[c][1] * 256 + o.d[c][0]) * r, v1 = (float)(o.d[c][3] * 256 + o.d[c][2]) * r;
             float (&a)[2] = acc[c & (PAR - 1)];
-            a[0] = __fmaf_rn(pick(sc.s0) * r, v0, __fmaf_rn(pick(sc.b0), x.sum[c], a[0]));
-            a[1] = __fmaf_rn(pick(sc.s1) * r, v1, __fmaf_rn(pick(sc.b1), x.sum[c], a[1]));
+            // the bias term goes with the high digits, where it cancels most of them, and what its rounding leaves with the
+            // low ones (error against 64-bit sums at 2048 x 2048 0.68e-7 of the result, 0.89e-7 without the latter, 1.4e-7 with the
+            // term among the low ones; fp16 operands: 0.74e-7, 11e-7 with outliers among the activations against 0.9e-7 here)
+            auto bias = [&](float b) {
+                const float p = b * x.sum[c];
+                return t & 1u ? p : __fmaf_rn(b, x.sum[c], -p);
+            };
+            a[0] += __fmaf_rn(pick(sc.s0) * r, v0, bias(pick(sc.b0)));
+            a[1] += __fmaf_rn(pick(sc.s1) * r, v1, bias(pick(sc.b1)));
         }
     };
 
@@ -396,7 +409,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         __syncwarp();
         if (issued != pieces) issue(st);
     };
-    auto first_piece = [&] {
+    auto first_piece = [&] {  // once the loads of x are on their way
         if (pieces) take(test_stage(0u, 0u));
     };
 
@@ -652,7 +665,12 @@ int launch_k(const void* q, const Args& a, cudaStream_t stream) {
 
 // K that this kernel takes: whole pieces (a row of 6208 codes, with its last groups picked out one by one, took 11.3 us at
 // 5967 rows, 7.6 in gemv_tma.cuh), up to where its launches still pay.
-inline bool takes(uint32_t K) { return K % PK == 0u && K <= MAX_K; }
+// Beyond one slab as long as there is one tile a CTA: what a layer's last projection is, which the
+// others of a chain start beside; with more, the conversion of x and the pieces take longer than there (8192 x 8192 at one
+// row 11.5 us, 10.1).
+inline bool takes(uint32_t N, uint32_t K) {
+    return K % PK == 0u && (K <= 2u * SLAB || (K <= MAX_K && (N + 15u) / 16u <= (uint32_t)sm_count()));
+}
 
 // One or two rows, of a K that is taken.
 template <int ROWS>

@@ -1136,7 +1136,7 @@ int launch_one(const Plan& plan, const void* q, const Args& a, cudaStream_t stre
                                 (plan.slab_row + S::QPAD) / 8, gated ? 8 : 16, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
     // always with the programmatic attribute (the kernel knows when to wait): 2.0 us of host time against 2.5
-    const cudaError_t e = launch<Split::SHARED>(gemv_tma_kernel<S, F>, dim3(plan.grid), dim3(THREADS), plan.smem, stream, true, tq, a);
+    const cudaError_t e = launch(gemv_tma_kernel<S, F>, dim3(plan.grid), dim3(THREADS), plan.smem, stream, true, tq, a);
     if (e != cudaSuccess) return cuda_fail(e, "gemv_tma launch");
     return MIORI_OK;
 }
