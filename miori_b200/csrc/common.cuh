@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <cstring>
 
 #include "../../include/miori_b200.h"
 #include "tune.h"
@@ -98,6 +99,36 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 }
 __device__ __forceinline__ void pdl_wait_prior() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// A read of what the launch before this one may have written, after pdl_wait_prior.  Not __ldg, nor a plain read through a
+// const __restrict__ pointer: both say that nobody writes the data while this grid lives, whereas its producer may run
+// beside this grid's prologue, and the compiler may then move the read in front of the wait.
+template <class T, bool STREAM = false>  // STREAM: read once, evicted first
+__device__ __forceinline__ T ld_fresh(const T* p) {
+    static_assert(sizeof(T) == 2 || sizeof(T) == 4 || sizeof(T) == 8 || sizeof(T) == 16, "one access");
+    T v;
+    if constexpr (sizeof(T) == 2) {
+        uint16_t w;
+        asm volatile("ld.global.u16 %0, [%1];" : "=h"(w) : "l"(p));
+        memcpy(&v, &w, sizeof(T));
+    } else if constexpr (sizeof(T) == 4) {
+        uint32_t w;
+        if constexpr (STREAM) asm volatile("ld.global.cs.u32 %0, [%1];" : "=r"(w) : "l"(p));
+        else asm volatile("ld.global.u32 %0, [%1];" : "=r"(w) : "l"(p));
+        memcpy(&v, &w, sizeof(T));
+    } else if constexpr (sizeof(T) == 8) {
+        uint2 w;
+        if constexpr (STREAM) asm volatile("ld.global.cs.v2.u32 {%0, %1}, [%2];" : "=r"(w.x), "=r"(w.y) : "l"(p));
+        else asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(w.x), "=r"(w.y) : "l"(p));
+        memcpy(&v, &w, sizeof(T));
+    } else {
+        uint4 w;
+        if constexpr (STREAM) asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "l"(p));
+        else asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "l"(p));
+        memcpy(&v, &w, sizeof(T));
+    }
+    return v;
 }
 
 // ---- shared-memory barriers (mbarrier) and bounded waits -------------------------------

@@ -58,13 +58,13 @@ dequant_rowmajor_kernel(const uint32_t* __restrict__ q, const uint16_t* __restri
         const uint64_t i = first + (uint64_t)(j * DEQUANT_THREADS);
         if (i < units) {
             if constexpr (BITS == 4) {
-                w[j][0] = __ldcs(q + i);
+                w[j][0] = ld_fresh<uint32_t, true>(q + i);
             } else {
-                const uint2 v = __ldcs(reinterpret_cast<const uint2*>(q) + i);
+                const uint2 v = ld_fresh<uint2, true>(reinterpret_cast<const uint2*>(q) + i);
                 w[j][0] = v.x, w[j][1] = v.y;
             }
-            sc[j] = __ldg(s + (i >> ushift));
-            bi[j] = __ldg(b + (i >> ushift));
+            sc[j] = ld_fresh(s + (i >> ushift));
+            bi[j] = ld_fresh(b + (i >> ushift));
         }
     }
 #pragma unroll
@@ -94,11 +94,11 @@ dequant_wide_kernel(const uint4* __restrict__ q, const uint16_t* __restrict__ s,
         if (i >= steps) return;
 #pragma unroll
         for (int k = 0; k < WORDS / 4; ++k) {
-            const uint4 v = __ldcs(q + i * (WORDS / 4) + k);
+            const uint4 v = ld_fresh<uint4, true>(q + i * (WORDS / 4) + k);
             l.w[4 * k] = v.x, l.w[4 * k + 1] = v.y, l.w[4 * k + 2] = v.z, l.w[4 * k + 3] = v.w;
         }
-        l.sc = __ldg(s + (i >> sshift));
-        l.bi = __ldg(b + (i >> sshift));
+        l.sc = ld_fresh(s + (i >> sshift));
+        l.bi = ld_fresh(b + (i >> sshift));
     };
     uint64_t i = (uint64_t)blockIdx.x * DEQUANT_THREADS + threadIdx.x;
     Step cur, next;

@@ -62,7 +62,7 @@ gemm_narrow_kernel(const uint16_t* __restrict__ A, const uint16_t* __restrict__ 
         for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int r = 0; r < 2 * MT; ++r)
-                a[u][r] = k_of(trip, u) < K ? __ldg(reinterpret_cast<const uint4*>(a_row[r] + k_of(trip, u))) : zero;
+                a[u][r] = k_of(trip, u) < K ? ld_fresh(reinterpret_cast<const uint4*>(a_row[r] + k_of(trip, u))) : zero;
         if (trip) load_b(trip);
 #pragma unroll
         for (int u = 0; u < U; ++u)

@@ -583,7 +583,7 @@ splitk_reduce_kernel(const float4* __restrict__ ws, void* __restrict__ Cout, siz
         float4 v[MAX_SPLITS];
 #pragma unroll
         for (uint32_t s = 0; s < (uint32_t)MAX_SPLITS; ++s)
-            if (s < splits) v[s] = __ldcg(ws + (size_t)s * quads + i);
+            if (s < splits) v[s] = ld_fresh(ws + (size_t)s * quads + i);
         float4 a = v[0];
 #pragma unroll
         for (uint32_t s = 1; s < (uint32_t)MAX_SPLITS; ++s)
@@ -829,8 +829,8 @@ gemm_bf16_simt_kernel(const uint16_t* __restrict__ A, const uint16_t* __restrict
         for (uint32_t r = 0; r < 4u; ++r) {
             const uint32_t row = ty + 8u * r, k = k0 + tx;
             const uint32_t m = m0 + row, n = n0 + row;
-            As[row][tx] = (m < M && k < K) ? bf16_bits_to_float(A[(size_t)m * lda + k]) : 0.0f;
-            Bs[row][tx] = (n < N && k < K) ? bf16_bits_to_float(B[(size_t)n * ldb + k]) : 0.0f;
+            As[row][tx] = (m < M && k < K) ? bf16_bits_to_float(ld_fresh(A + (size_t)m * lda + k)) : 0.0f;
+            Bs[row][tx] = (n < N && k < K) ? bf16_bits_to_float(ld_fresh(B + (size_t)n * ldb + k)) : 0.0f;
         }
         __syncthreads();
 #pragma unroll 8

@@ -139,7 +139,7 @@ gemv_cache_kernel(const __grid_constant__ CUtensorMap tmap_w, const uint16_t* __
             const uint32_t k = (uint32_t)s * KS + (kpart * NT + i) * 32u + t * 8u;
             xf[s % XF][i] = make_uint4(0u, 0u, 0u, 0u);
             if (warp < WARPS && m < M && k < K)  // K is a multiple of 8: whole pieces
-                xf[s % XF][i] = __ldg(reinterpret_cast<const uint4*>(x + (size_t)m * K + k));
+                xf[s % XF][i] = ld_fresh(reinterpret_cast<const uint4*>(x + (size_t)m * K + k));
         }
     };
 #pragma unroll

@@ -195,9 +195,9 @@ __device__ __noinline__ float plain_dot(const Args& A, uint32_t n, uint32_t m, f
             const uint32_t codes = q[g * (GROUP / 8u) + w];
             for (uint32_t i = 0; i < 8u; ++i) {
                 const size_t k = (size_t)g * GROUP + w * 8u + i, at = (size_t)m * A.K + k;
-                const float x = NORMED ? bf16_bits_to_float(float_to_bf16_bits(reinterpret_cast<const float*>(A.x)[at] * inv *
+                const float x = NORMED ? bf16_bits_to_float(float_to_bf16_bits(ld_fresh(reinterpret_cast<const float*>(A.x) + at) * inv *
                                                                                bf16_bits_to_float(A.pre.gamma[k])))
-                                       : bf16_bits_to_float(A.x[at]);
+                                       : bf16_bits_to_float(ld_fresh(A.x + at));
                 cx = __fmaf_rn((float)((codes >> (4u * i)) & 15u), x, cx);
                 sx += x;
             }
@@ -413,6 +413,8 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         if (pieces) take(test_stage(0u, 0u));
     };
 
+    uint4 gm = make_uint4(0u, 0u, 0u, 0u);  // RES: norm weights of this lane's activations
+    if (RES && normed && pieces && (pos * 32u + lane) * 8u < K) gm = __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + pos * 32u + lane);
     pdl_wait_prior();  // x (and y) belong to the predecessor until here
 
     // A CTA without rows keeps its place until the next launch has taken its own: at the head of a chain it would be gone
@@ -433,7 +435,6 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         // again (from L2)
         constexpr bool KEEP = RES;
         float4 xa4[ROWS], xc4[ROWS];
-        uint4 gm = make_uint4(0u, 0u, 0u, 0u);
         float inv[ROWS];
         if (normed) {
             const float4* x4 = reinterpret_cast<const float4*>(A.x);
@@ -452,9 +453,8 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 #pragma unroll
                 for (int m = 0; m < ROWS; ++m) {
                     xa4[m] = xc4[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (slabs && u < upr) xa4[m] = __ldg(x4 + (m * upr + u) * 2u), xc4[m] = __ldg(x4 + (m * upr + u) * 2u + 1u);
+                    if (slabs && u < upr) xa4[m] = ld_fresh(x4 + (m * upr + u) * 2u), xc4[m] = ld_fresh(x4 + (m * upr + u) * 2u + 1u);
                 }
-                if (slabs && u < upr) gm = __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + u);
                 first_piece();
 #pragma unroll
                 for (int m = 0; m < ROWS; ++m) add_up((uint32_t)m, squares(xa4[m], xc4[m], 0.0f));
@@ -463,7 +463,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     float ss = 0.0f;
                     for (uint32_t s = 0; s < slabs; ++s) {
                         const uint32_t u = (s * 8u + pos) * 32u + lane;
-                        if (u < upr) ss = squares(__ldg(x4 + ((size_t)m * upr + u) * 2u), __ldg(x4 + ((size_t)m * upr + u) * 2u + 1u), ss);
+                        if (u < upr) ss = squares(ld_fresh(x4 + ((size_t)m * upr + u) * 2u), ld_fresh(x4 + ((size_t)m * upr + u) * 2u + 1u), ss);
                     }
                     add_up(m, ss);
                 }
@@ -489,10 +489,10 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                     v = ROWS == 1 || m == 0u ? gemvtma::normed8(xa4[0], xc4[0], inv[0], gm) : gemvtma::normed8(xa4[ROWS - 1], xc4[ROWS - 1], inv[ROWS - 1], gm);
                 } else if (normed) {
                     const float4* x4 = reinterpret_cast<const float4*>(A.x) + 2u * i;
-                    v = gemvtma::normed8(__ldg(x4), __ldg(x4 + 1), ROWS == 1 || m == 0u ? inv[0] : inv[ROWS - 1],
+                    v = gemvtma::normed8(ld_fresh(x4), ld_fresh(x4 + 1), ROWS == 1 || m == 0u ? inv[0] : inv[ROWS - 1],
                                          __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + u));
                 } else {
-                    v = __ldg(reinterpret_cast<const uint4*>(A.x) + i);
+                    v = ld_fresh(reinterpret_cast<const uint4*>(A.x) + i);
                 }
             }
             return v;

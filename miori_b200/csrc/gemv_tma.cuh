@@ -291,7 +291,7 @@ __device__ __forceinline__ void stage_x(const XArea& xa, const uint16_t* __restr
             m[h] = S::ROWS == 1 ? 0u : __umulhi(i, inv_upr);
             u[h] = i - m[h] * upr;
             v[h] = make_uint4(0u, 0u, 0u, 0u);
-            if (i < total) v[h] = __ldg(reinterpret_cast<const uint4*>(x) + i);
+            if (i < total) v[h] = ld_fresh(reinterpret_cast<const uint4*>(x) + i);
         }
 #pragma unroll
         for (int h = 0; h < AHEAD; ++h) {
@@ -335,8 +335,8 @@ __device__ __forceinline__ void stage_x_normed(const XArea& xa, const float* __r
         for (uint32_t m = 0; m < R; ++m) {
             a[m] = c[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (mine && m < M) {
-                a[m] = __ldg(x4 + ((size_t)m * upr + tid) * 2u);
-                c[m] = __ldg(x4 + ((size_t)m * upr + tid) * 2u + 1u);
+                a[m] = ld_fresh(x4 + ((size_t)m * upr + tid) * 2u);
+                c[m] = ld_fresh(x4 + ((size_t)m * upr + tid) * 2u + 1u);
             }
         }
 #pragma unroll
@@ -370,7 +370,7 @@ __device__ __forceinline__ void stage_x_normed(const XArea& xa, const float* __r
 #pragma unroll
             for (uint32_t r = 0; r < 4u; ++r) {
                 if (m0 + r < M) {
-                    const float4 v = __ldg(x4 + (size_t)(m0 + r) * qpr + i);
+                    const float4 v = ld_fresh(x4 + (size_t)(m0 + r) * qpr + i);
                     ss[r] = __fmaf_rn(v.w, v.w, __fmaf_rn(v.z, v.z, __fmaf_rn(v.y, v.y, __fmaf_rn(v.x, v.x, ss[r]))));
                 }
             }
@@ -393,7 +393,7 @@ __device__ __forceinline__ void stage_x_normed(const XArea& xa, const float* __r
     for (uint32_t i0 = tid - lane; i0 < M * upr; i0 += COMPUTE) {  // whole warps
         const uint32_t i = i0 + lane, m = S::ROWS == 1 ? 0u : __umulhi(i, inv_upr), u = i - m * upr;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (i < M * upr) v = normed8(__ldg(x4 + 2 * (size_t)i), __ldg(x4 + 2 * (size_t)i + 1), inv_row[m], __ldg(g4 + u));
+        if (i < M * upr) v = normed8(ld_fresh(x4 + 2 * (size_t)i), ld_fresh(x4 + 2 * (size_t)i + 1), inv_row[m], __ldg(g4 + u));
         stage_unit_at<S>(xa, v, i < M * upr, m, u);
     }
 }

@@ -29,7 +29,7 @@ rmsnorm_kernel(const float* __restrict__ x, const uint16_t* __restrict__ w, uint
         pdl_wait_prior();
         const float inv = rsqrtf(row_sum_squares<0, false>(row, n, part) / (float)n + eps);
         for (uint32_t i = threadIdx.x; i < n; i += NORM_THREADS)
-            to[i] = (uint16_t)float_to_bf16_bits(row[i] * inv * bf16_bits_to_float(w[i]));
+            to[i] = (uint16_t)float_to_bf16_bits(ld_fresh(row + i) * inv * bf16_bits_to_float(w[i]));
     }
 }
 
@@ -59,12 +59,12 @@ silu_mul_kernel(const float* __restrict__ gate, const float* __restrict__ up, ui
     const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
     if constexpr (VEC) {
         for (size_t i = first; i < n / 4u; i += stride) {
-            const float4 g = reinterpret_cast<const float4*>(gate)[i], u = reinterpret_cast<const float4*>(up)[i];
+            const float4 g = ld_fresh(reinterpret_cast<const float4*>(gate) + i), u = ld_fresh(reinterpret_cast<const float4*>(up) + i);
             reinterpret_cast<uint2*>(out)[i] =
                 make_uint2(silu_mul_bits(g.x, u.x) | (silu_mul_bits(g.y, u.y) << 16), silu_mul_bits(g.z, u.z) | (silu_mul_bits(g.w, u.w) << 16));
         }
     } else {
-        for (size_t i = first; i < n; i += stride) out[i] = (uint16_t)silu_mul_bits(gate[i], up[i]);
+        for (size_t i = first; i < n; i += stride) out[i] = (uint16_t)silu_mul_bits(ld_fresh(gate + i), ld_fresh(up + i));
     }
 }
 
@@ -77,7 +77,7 @@ embed8_kernel(const uint4* __restrict__ q, const uint16_t* __restrict__ s, const
               uint32_t rows) {
     pdl_launch_dependents();
     pdl_wait_prior();
-    const uint32_t tok = tokens[blockIdx.x];
+    const uint32_t tok = ld_fresh(tokens + blockIdx.x);
     if (tok >= rows) return;  // an id outside the table leaves its output row untouched
     const uint32_t ng = K >> gshift;
     const uint4* qrow = q + (size_t)tok * (K / 16u);
@@ -144,6 +144,11 @@ __device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {  // of 
     asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
+template <bool BF16>
+__device__ __forceinline__ float fresh_value(const void* v, uint32_t i) {
+    if constexpr (BF16) return bf16_bits_to_float(ld_fresh(static_cast<const uint16_t*>(v) + i));
+    else return ld_fresh(static_cast<const float*>(v) + i);
+}
 // This CTA's best over its slice of v[0, n), in thread 0.  Ties go to the lower index.
 template <bool BF16>
 __device__ __forceinline__ unsigned long long block_argmax(const void* __restrict__ v, uint32_t n, uint32_t index0,
@@ -164,7 +169,7 @@ __device__ __forceinline__ unsigned long long block_argmax(const void* __restric
         const uint4* v4 = static_cast<const uint4*>(v);
 #pragma unroll 2
         for (uint32_t p = p0 + threadIdx.x; p < p1; p += ARGMAX_THREADS) {
-            const uint4 w = __ldg(v4 + p);
+            const uint4 w = ld_fresh(v4 + p);
             float m;  // NaN only if all of them are
             if constexpr (BF16) {
                 const uint32_t m2 = max_bf16x2(max_bf16x2(w.x, w.y), max_bf16x2(w.z, w.w));
@@ -192,7 +197,7 @@ __device__ __forceinline__ unsigned long long block_argmax(const void* __restric
     if (!vec_ok) s0 = cr * ARGMAX_THREADS + threadIdx.x, step = nct * ARGMAX_THREADS;
     else if (cr == nct - 1u) s0 = pieces * PER + threadIdx.x;
     for (uint32_t i = s0; i < n; i += step)
-        see(BF16 ? bf16_bits_to_float(static_cast<const uint16_t*>(v)[i]) : static_cast<const float*>(v)[i], index0 + i);
+        see(fresh_value<BF16>(v, i), index0 + i);
     const unsigned long long mine = warp_key_max(bi == 0xFFFFFFFFu ? 0ull : best_key(bv, bi));
     if ((threadIdx.x & 31u) == 0) warp_best[threadIdx.x >> 5] = mine;
     __syncthreads();
@@ -201,8 +206,7 @@ __device__ __forceinline__ unsigned long long block_argmax(const void* __restric
 // A candidate's value with the sign that its zero has in v (keys know one zero).
 template <bool BF16>
 __device__ __forceinline__ Best signed_zero(Best b, const void* __restrict__ v, uint32_t index0) {
-    if (b.v == 0.0f)
-        b.v = BF16 ? bf16_bits_to_float(static_cast<const uint16_t*>(v)[b.i - index0]) : static_cast<const float*>(v)[b.i - index0];
+    if (b.v == 0.0f) b.v = fresh_value<BF16>(v, b.i - index0);
     return b;
 }
 // Cluster-wide result, valid in thread 0 of CTA 0 of the cluster.  Every thread of every CTA of

@@ -21,7 +21,7 @@ __device__ __forceinline__ void norm_sync() {
 template <bool FRESH>
 __device__ __forceinline__ float norm_load(const float* row, uint32_t i) {
     if constexpr (FRESH) return __ldcg(row + i);
-    else return row[i];
+    else return ld_fresh(row + i);
 }
 
 // Sum of squares of a row, in a fixed order: every thread adds its strided elements, warps reduce
@@ -68,7 +68,7 @@ __device__ __forceinline__ void post_norm_add_row(const float* x, const float* s
                                                   uint32_t n, float eps, float* part) {
     const float inv = rsqrtf(row_sum_squares<BAR, FRESH>(src, n, part) / (float)n + eps);
     for (uint32_t i = threadIdx.x; i < n; i += NORM_THREADS)
-        out[i] = x[i] + norm_load<FRESH>(src, i) * inv * bf16_bits_to_float(w[i]);
+        out[i] = ld_fresh(x + i) + norm_load<FRESH>(src, i) * inv * bf16_bits_to_float(w[i]);
 }
 
 // The same for rows that divide into 16-byte pieces, at most PIECES of them per thread: every load of the
@@ -86,8 +86,8 @@ __device__ __forceinline__ void post_norm_add_row_vec(const float* x, const floa
         g[j] = make_uint2(0u, 0u);
         if (i < n / 4u) {
             if constexpr (FRESH) v[j] = __ldcg(reinterpret_cast<const float4*>(src) + i);
-            else v[j] = reinterpret_cast<const float4*>(src)[i];
-            r[j] = reinterpret_cast<const float4*>(x)[i];
+            else v[j] = ld_fresh(reinterpret_cast<const float4*>(src) + i);
+            r[j] = ld_fresh(reinterpret_cast<const float4*>(x) + i);
             g[j] = reinterpret_cast<const uint2*>(w)[i];
         }
     }
@@ -120,7 +120,7 @@ __device__ __forceinline__ void rmsnorm_row_vec(const float* x, const uint16_t* 
     for (int j = 0; j < PIECES; ++j) {
         const uint32_t i = threadIdx.x + (uint32_t)j * NORM_THREADS;
         v[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (i < n / 4u) v[j] = reinterpret_cast<const float4*>(x)[i];
+        if (i < n / 4u) v[j] = ld_fresh(reinterpret_cast<const float4*>(x) + i);
     }
     const float inv = rsqrtf(row_sum_of_pieces<0, PIECES>(v, part) / (float)n + eps);
 #pragma unroll

@@ -39,10 +39,10 @@ allgather_kernel(const PeerArgs pa, const uint8_t* __restrict__ src, uint32_t sr
         const size_t idx = m * n_total + row0 + c;
         uint32_t bits;
         if (BF16) {
-            bits = *reinterpret_cast<const uint16_t*>(src + m * src_pitch + c * 2u);
+            bits = ld_fresh(reinterpret_cast<const uint16_t*>(src + m * src_pitch + c * 2u));
             reinterpret_cast<uint16_t*>(y)[idx] = (uint16_t)bits;
         } else {
-            bits = *reinterpret_cast<const uint32_t*>(src + m * src_pitch + c * 4u);
+            bits = ld_fresh(reinterpret_cast<const uint32_t*>(src + m * src_pitch + c * 4u));
             reinterpret_cast<uint32_t*>(y)[idx] = bits;
         }
         for (uint32_t p = 0; p < pa.world; ++p)
