@@ -46,8 +46,7 @@ struct Batch {
         if constexpr (BITS == 4 && GROUP == 64) {
             // the class of one and two rows: exact integer sums (gemv_digits.cuh)
             if (M <= 2u && gemvdigits::takes(N, K))
-                return M == 1u ? gemvdigits::launch_rows<1>(q, s, b, x, y, N, K, flags, stream, sh)
-                               : gemvdigits::launch_rows<2>(q, s, b, x, y, N, K, flags, stream, sh);
+                return gemvdigits::launch_rows(q, s, b, x, y, N, K, M, flags, stream, sh);
         }
         uint32_t cls = class_of(M), kpar = 0;
         while (cls && (kpar = kpar_of(cls, N, K)) == 0u) cls >>= 1;

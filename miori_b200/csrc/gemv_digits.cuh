@@ -9,36 +9,44 @@
 //     are exact for everything of at least 2^-17 of the largest, the rest is rounded by less than 2^-25 of it
 //     -- times sixteen for the codes in low nibbles, cut into four digits of -128 .. 127, a column of the MMA
 //     each.  With one row the eight columns are the digits of two groups, with two rows those of one.
-// A row's sums are int32, then fp32 per group: its bits depend neither on the other row nor on N or the grid.
+// A row's sums are int32, then fp32 per group: its bits depend neither on the other row, nor on the launch, nor on the grid.
 // (The fp16 operands of gemv_tma.cuh take twice the MMAs and three times the ALU work for the unpacking, which
 // are worth it only where the columns are full of rows.)
 //
-// What bounds it: in a chain of dependent launches the steps that follow one another -- the hand-over from grid
-// to grid (0.7 us), the trip of x through L2 (0.35), its conversion (0.3; 0.25 a slab beyond), each piece of weights
-// (0.33) -- and
-// not HBM: with the weights in L2 the four projections of a layer took 13.4 instead of 13.8.  So nothing else is on that
-// path:
-//   * TWO CTAs of 256 threads fit an SM, one of this launch and one of the next, which fetches its weights
-//     while this one works.  Every launch is one CTA per SM, those without rows included: a launch of
-//     fewer would let the next one's double up, and every later launch would inherit the skew;
-//   * a 1-KiB slab of a row is cut into eight positions of 128 bytes, and warp w owns position w of every tile
-//     of the CTA: it fetches its own pieces (16 rows x 128 bytes by TMA, 128-byte swizzle, and their scales by
-//     cp.async) into its own ring, and converts the activations of its own position.  Warps meet once per
-//     batch of tiles, when the eight partial sums of an output are added in a fixed tree.  (With the
-//     activations staged by the whole CTA behind a barrier a layer took 4 % more.)
-//   * K <= 2048: the activations stay in registers from tile to tile;
-//   * the first piece is read while x is on its way.
-// After its first pieces a CTA holds the others back for 800 cycles: it starts when its predecessor fetches
-// x, whose loads would queue up behind them (four projections of a layer 15.2 us when all are fetched at once, 14.5 so).
+// What bounds it: the steps of a launch that follow one another -- the hand-over from grid to grid (0.7 us), the trip of x
+// through L2 (0.35), its conversion (0.3; 0.25 a slab beyond with eight warps), each piece of weights (0.33) -- and not HBM.
+//   * A 1-KiB slab of a row is cut into eight positions of 128 bytes, and a warp owns a position of the CTA's tiles: it
+//     fetches its own pieces (16 rows x 128 bytes by TMA, 128-byte swizzle, and their scales by cp.async) into its own
+//     ring, and converts the activations of its own position.  Warps meet once per batch of tiles, when the partial sums
+//     of an output are added in a fixed tree.  (With the activations staged by the whole CTA behind a barrier a layer
+//     took 4 % more.)
+//   * K <= 2048: the activations stay in registers from tile to tile.
+//   * The first piece is read while x is on its way.
+// Two frames, the same bits:
+//   * one row started early: EIGHT warps a CTA and two CTAs to an SM, one of this launch and one of the next, which
+//     fetches its weights while this one works.  Behind a norm that is fused into it a launch has one CTA fewer than there
+//     are SMs, else one per SM, those without rows included: a launch of fewer lets the next one's double up, and every
+//     later launch inherits the skew.  After its first pieces a CTA holds the others back for 800 cycles: it starts when
+//     its predecessor fetches x, whose loads would queue up behind them (four projections of a layer 15.2 us when all are
+//     fetched at once, 14.5 so);
+//   * two rows, launches that wait for the one before, launches over several GPUs: SIXTEEN warps and one CTA to an SM.  Two
+//     warps share a position: each converts one row of two, or half the slabs.  All pieces but the first are fetched behind
+//     x (16384 x 2048 at one row 7.0 us when all are fetched ahead, 6.3 with two first ones, 5.7 with one; none 5.9).  Beside
+//     launches that keep to neither rule -- norms, activations, other products -- it is the steadier one: with eight warps a
+//     layer's four projections that wait took 24.8 us, 17.1 so, and nine launches of a layer at two rows 28.8 and 24.3.
 //
-// Measured in chains over weights larger than L2, the kernel of gemv_tma.cuh and this one, us, one row: 2048 x 2048
-// 2.45 -> 2.16, 3072 x 2048 2.92 -> 2.43, 16384 x 2048 6.57 -> 4.86, 32768 x 512 6.55 -> 3.43, 2048 x 8192 4.63 -> 4.38, the four
-// projections of a layer 16.6 -> 13.4, with its norms and activation (six launches) 21.1 -> 17.8; launches that wait for the
-// one before, 2048 x 2048 2.86 -> 2.76, 16384 x 2048 7.69 -> 6.94.  Two rows 2.50 -> 2.44, 2.93 -> 2.85, 7.03 -> 5.88.
-// Behind, because converting a row takes 2.2 times the instructions of fp16's and is most of the time there: two rows
-// beyond one slab (2048 x 4096 3.46 -> 3.89, 2048 x 8192 4.89 -> 6.26), and launches that wait of such rows (one row 4.12 ->
-// 4.49 and 5.61 -> 6.93) or of two short ones (2048 x 2048 2.93 -> 3.19).  A row's bits must depend neither on the other row
-// nor on how it is launched, and a chain of dependent launches at one row is what this is for.
+// Measured in chains over weights larger than L2, the kernel of gemv_tma.cuh and this one, us:
+//                          one row early     one that waits    two rows early    two that wait
+//   2048 x 2048            2.50   2.09       2.93   2.48       2.51   2.76       2.94   2.77
+//   3072 x 2048            2.85   2.42       3.55   3.01       2.93   3.10       3.61   3.37
+//   16384 x 2048           6.63   4.88       7.62   5.70       7.05   5.95       7.81   6.42
+//   32768 x 512            6.60   3.44       7.19   4.28       6.83   4.36       7.46   4.72
+//   2048 x 4096            3.35   3.24       4.14   4.04       3.51   4.13       4.13   4.64
+//   2048 x 8192            4.63   4.55       5.64   5.49       4.87   5.92       5.65   6.69
+//   a layer's four        16.6   13.5       20.1   17.1       17.3   17.6       20.4   19.7
+//   with neighbours, six  21.2   18.4                         23.3   22.3
+// Two rows beyond one slab are behind: converting a row takes 2.2 times the instructions of fp16's and is most of the time
+// there.  They run here all the same: a row has the same bits alone and beside another, and one row gains.
 #pragma once
 #include "gemv_tma.cuh"
 
@@ -49,7 +57,6 @@ using gemvtma::Fuse;
 using gemvtma::lds128;
 using gemvtma::lds_words;
 
-constexpr int WARPS = 8, THREADS = 32 * WARPS;
 constexpr int MAX_STAGES = 8;
 constexpr uint32_t GROUP = 64;
 constexpr uint32_t SLAB = 1024, PIECE = 128, PIECE_BYTES = 16 * PIECE;  // bytes of a row; 16 rows
@@ -57,15 +64,17 @@ constexpr uint32_t PK = 2 * PIECE;          // codes of a row in a piece
 constexpr uint32_t NG = PK / GROUP;         // its scale groups
 constexpr uint32_t XPAD = 64;               // between digit planes: their 64-byte reads fall into different banks
 constexpr uint32_t MAX_K = 8192;
-constexpr int HEAD_PIECES = 2;              // fetched at once; the others after HOLD_CYCLES
+constexpr int HEAD_SHARING = 2, HEAD_ALONE = 1;  // pieces of a warp fetched at once; the others after HOLD_CYCLES, or behind x
 constexpr long long HOLD_CYCLES = 800, LINGER_CYCLES = 3500;
-// Two of these fit the 228 KB of an SM, three do not (and more than 77 KB keep other kernels' CTAs from taking
-// the successor's place).
-constexpr size_t SMEM_LIMIT = 112 * 1024, SMEM_FLOOR = 78 * 1024;
 
-template <int ROWS_>
+// W warps a CTA: eight, two CTAs to an SM, or sixteen, one CTA to an SM.
+template <int ROWS_, int W_>
 struct Shape {
-    static constexpr int ROWS = ROWS_;
+    static constexpr int ROWS = ROWS_, W = W_, THREADS = 32 * W;
+    static constexpr bool SHARING = W == 8;           // an SM with the launch before and after
+    // Two that share fit the 228 KB of an SM, three do not (and more than 77 KB keep other kernels' CTAs from taking the
+    // successor's place); the sixteen warps of the others take all registers.
+    static constexpr size_t SMEM_LIMIT = (SHARING ? 112 : 200) * 1024, SMEM_FLOOR = SHARING ? 78 * 1024 : 0;
     static constexpr int GS = 2 / ROWS;               // scale groups side by side in the eight columns
     static constexpr int NU = 2 * GS;                 // MMAs of a chain = units of eight activations per lane
     static constexpr int CH = (int)NG / GS;           // chains of a piece
@@ -74,38 +83,45 @@ struct Shape {
 };
 
 struct Args {
-    const uint16_t* x;      // activations, bf16 [M][K] (fp32 when normed)
+    const uint16_t* x;      // activations, bf16 [ROWS][K] (fp32 when normed)
     void* y;
     const uint16_t *s, *b;  // scales and biases, [N][K / 64]
     const uint8_t* q;
     gemvtma::PreNorm pre;
     gemvtma::PostNorm post;
-    uint32_t N, K, M, stages, out_bf16, gated, early;
+    uint32_t N, K, M, stages, out_bf16, gated, early;  // M is ROWS
     uint32_t n_total, row0;
     size_t y_off;
     unsigned long long* best;
     PeerArgs pa;
 };
 
+// How a row's slabs are dealt: beyond one slab, sixteen warps are two for each position, one for the slabs below HALF and one
+// for the others; eight warps sum the two parts apart, so that both kernels add in the same order.
+__host__ __device__ inline uint32_t slabs_of(uint32_t K) { return (K / 2u + SLAB - 1u) / SLAB; }
+__host__ __device__ inline uint32_t half_of(uint32_t nslab) { return (nslab + 1u) >> 1; }
+
 // Dynamic shared memory, from a 1024-byte aligned base.
 struct Layout {
-    uint32_t pitch, sc, x, ms, zeros, part, total;
+    uint32_t pitch, slabs, sc, x, ms, zeros, part, total;
 };
 constexpr uint32_t SC_ROW = 4u * NG, SC_BYTES = 16u * SC_ROW;  // scales and biases of a row of a piece, and of a piece
 template <class S>
-__host__ __device__ inline Layout layout(uint32_t K, uint32_t M, uint32_t stages, uint32_t parts) {
+__host__ __device__ inline Layout layout(uint32_t K, uint32_t stages, uint32_t parts) {
     Layout L;
-    const uint32_t nslab = (K / 2u + SLAB - 1u) / SLAB;
-    L.pitch = nslab * PK + XPAD;  // of a digit plane of one warp
-    uint32_t at = WARPS * stages * PIECE_BYTES;
+    const uint32_t nslab = slabs_of(K);
+    L.slabs = S::W == 16 ? half_of(nslab) : nslab;                           // of a warp
+    const uint32_t regions = S::W == 16 && nslab == 1u ? 8u : (uint32_t)S::W;  // of activations: one slab's are shared by two warps
+    L.pitch = L.slabs * PK + XPAD;  // of a digit plane
+    uint32_t at = S::W * stages * PIECE_BYTES;
     L.sc = at;
-    at += WARPS * stages * SC_BYTES;
+    at += S::W * stages * SC_BYTES;
     L.x = at;
-    at += WARPS * M * 4u * L.pitch;
+    at += regions * S::ROWS * 4u * L.pitch;
     L.ms = at;
-    at += WARPS * nslab * NG * S::ROWS * 16u;
+    at += regions * L.slabs * NG * S::ROWS * 16u;
     L.zeros = at;
-    at += WARPS * 16u;
+    at += S::W * 16u;
     L.part = at;
     at += parts * S::ROWS * 128u;  // partial sums of a tile's positions
     L.total = at + 1024u;
@@ -209,34 +225,42 @@ __device__ __noinline__ float plain_dot(const Args& A, uint32_t n, uint32_t m, f
 
 // RES: K <= 2048, one slab: the activations of a warp's position stay in registers.
 template <class S, Fuse F, bool RES>
-__global__ void __launch_bounds__(THREADS, 2)
+__global__ void __launch_bounds__(S::THREADS, S::SHARING ? 2 : 1)
 gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ Args A) {
     constexpr int ROWS = S::ROWS, CH = S::CH, NU = S::NU, GS = S::GS;
+    constexpr uint32_t WARPS = S::W;
+    constexpr bool PAIRED = RES && WARPS == 16u;    // two warps share a position's activations: each converts one row of two
+    constexpr bool HALVED = !RES && WARPS == 16u;   // two warps share a position's slabs
+    static_assert(!RES || PAIRED || ROWS == 1, "a warp converts one row of a slab, or all rows of several");
     constexpr bool SHARDED_ = F == gemvtma::SHARDED, ARGMAX_ = F == gemvtma::ARGMAX, POSTNORM_ = F == gemvtma::POSTNORM;
     const bool gated = F == gemvtma::FUSED && A.gated != 0u, normed = F == gemvtma::FUSED && A.pre.gamma != nullptr;
-    const uint32_t N = A.N, K = A.K, M = A.M, stages = A.stages;
+    const uint32_t N = A.N, K = A.K, stages = A.stages;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t tiles = (N + 15u) >> 4, row_bytes = K / 2u, ng = K / GROUP;
-    const uint32_t full_slabs = row_bytes / SLAB, rest = row_bytes % SLAB, nslab = (row_bytes + SLAB - 1u) / SLAB;
+    const uint32_t full_slabs = row_bytes / SLAB, rest = row_bytes % SLAB, half = half_of(slabs_of(K));
     // short rows have fewer positions, and the warps of a position share the tiles
     const uint32_t P = full_slabs ? 8u : (rest + PIECE - 1u) / PIECE;
-    const uint32_t pshift = P > 4u ? 3u : P > 2u ? 2u : P - 1u, TG = 8u >> pshift;
-    const uint32_t pos = warp & ((1u << pshift) - 1u), tg = warp >> pshift;
-    const uint32_t slabs = full_slabs + (pos * PIECE < rest ? 1u : 0u);
+    const uint32_t pshift = P > 4u ? 3u : P > 2u ? 2u : P - 1u, TG = HALVED ? 1u : WARPS >> pshift;
+    const uint32_t pos = warp & ((1u << pshift) - 1u), tg = HALVED ? 0u : warp >> pshift;
+    auto slabs_at = [&](uint32_t p) { return full_slabs + (p * PIECE < rest ? 1u : 0u); };
+    const uint32_t s0 = HALVED && warp >= 8u ? half : 0u;  // this warp's slabs of its position
+    const uint32_t slabs = HALVED ? (warp >= 8u ? max(slabs_at(pos), half) - half : min(slabs_at(pos), half)) : slabs_at(pos);
+    const uint32_t slots = pshift + (HALVED ? 1u : 0u);    // log2 of a tile's partial sums
 
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bars[WARPS * MAX_STAGES];
     __shared__ volatile uint32_t abort_flag;
     __shared__ uint32_t largest[WARPS][ROWS];  // magnitudes, in what each warp has seen of a row
 
+    const bool early = S::SHARING || A.early != 0u;
     const long long born = clock64();
-    if (A.early) pdl_launch_dependents();
+    if (early) pdl_launch_dependents();
 
     const uint32_t my_tiles = (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x;
     const uint32_t batch = TG * S::BATCH;
     const uint32_t wt = my_tiles > tg ? (my_tiles - tg + TG - 1u) / TG : 0u;  // tiles of this warp
     const uint32_t pieces = wt * slabs;
-    const Layout L = layout<S>(K, M, stages, (my_tiles > batch ? 2u * batch : my_tiles) << pshift);
+    const Layout L = layout<S>(K, stages, (my_tiles > batch ? 2u * batch : my_tiles) << slots);
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
     const uint32_t ring = base + warp * stages * PIECE_BYTES, bar0 = smem_addr(&bars[warp * MAX_STAGES]);
     const uint32_t sc_ring = base + L.sc + warp * stages * SC_BYTES;
@@ -246,9 +270,11 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     auto row_of = [&](uint32_t tile, uint32_t r) {
         return gated ? tile * 8u + (r & 7u) + (r >= 8u ? N >> 1 : 0u) : min(tile * 16u + r, N - 1u);
     };
-    uint32_t issued = 0, itile = tile_of(tg), ic0 = pos * (PIECE / 8u);
+    const uint32_t ic_first = pos * (PIECE / 8u) + s0 * (SLAB / 8u), ic_end = ic_first + slabs * (SLAB / 8u);
+    const uint32_t ie_first = pos * NG + s0 * (8u * NG);
+    uint32_t issued = 0, itile = tile_of(tg), ic0 = ic_first;
     const uint16_t* const sc_src = lane < 16u ? A.s : A.b;
-    size_t ie = (size_t)row_of(itile, lane & 15u) * ng + pos * NG;
+    size_t ie = (size_t)row_of(itile, lane & 15u) * ng + ie_first;
     const uint32_t sc_dst = sc_ring + (lane & 15u) * SC_ROW + (lane >> 4) * (SC_ROW / 2u);
     auto issue = [&](uint32_t st) {
         const uint32_t bar = bar0 + st * 8u;
@@ -267,10 +293,10 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
         ++issued;
         ic0 += SLAB / 8u, ie += 8u * NG;
-        if (RES || ic0 * 8u >= row_bytes) {
-            ic0 = pos * (PIECE / 8u);
+        if (RES || ic0 == ic_end) {
+            ic0 = ic_first;
             itile += TG * gridDim.x;
-            ie = (size_t)row_of(itile, lane & 15u) * ng + pos * NG;
+            ie = (size_t)row_of(itile, lane & 15u) * ng + ie_first;
         }
     };
     if (lane == 0) {
@@ -282,29 +308,31 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     __syncwarp();
     // A launch that may not start early waits here, and lets its dependents start only when its predecessor is
     // complete: they prefetch what that may have written.
-    if (A.early == 0u) {
+    if (!early) {
         pdl_wait_prior();
         pdl_launch_dependents();
     }
-    {
-        const uint32_t n = min(stages, pieces);
+    const uint32_t ahead = min(stages, pieces);
+    auto fill = [&](uint32_t n) {
 #pragma unroll 1  // one copy of the code: three copies of it cost a layer with its norms 0.5 to 1.6 us
-        for (uint32_t i = 0; i < n; ++i) {
-            if (i == (uint32_t)HEAD_PIECES && A.early) {
+        while (issued < n) {
+            if (S::SHARING && issued == (uint32_t)HEAD_SHARING) {
                 const long long t0 = clock64();
                 while (clock64() - t0 < HOLD_CYCLES) __nanosleep(40);
             }
-            issue(i);
+            issue(issued);
         }
-    }
+    };
+    fill(S::SHARING ? ahead : min(ahead, (uint32_t)HEAD_ALONE));
 
     // ---- this lane's place in the MMAs: tile rows prow and prow + 8 (in an order that spreads the swizzled rows which
     // a quarter- or half-warp reads over all banks); as a B operand column lane / 4 = (slot or row, digit)
     const uint32_t g = lane >> 2, t = lane & 3u;
     const uint32_t prow = ROWS == 1 ? ((g & 1u) << 2) | (g >> 1) : ((g & 3u) << 1) | (g >> 2);
-    const uint32_t xw = base + L.x + warp * M * 4u * L.pitch, msw = base + L.ms + warp * nslab * (NG * ROWS * 16u);
+    const uint32_t region = PAIRED ? ((tg >> 1) << pshift) + pos : warp;
+    const uint32_t xw = base + L.x + region * ROWS * 4u * L.pitch, msw = base + L.ms + region * L.slabs * (NG * ROWS * 16u);
     const bool mine = ROWS > 1 || (g >> 2) == (t >> 1);  // one row: the codes of this lane belong to its column's group
-    const uint32_t xb = mine ? xw + ((ROWS == 1 ? 0u : min(g >> 2, M - 1u)) * 4u + (g & 3u)) * L.pitch + t * (uint32_t)(NU * 8)
+    const uint32_t xb = mine ? xw + ((ROWS == 1 ? 0u : g >> 2) * 4u + (g & 3u)) * L.pitch + t * (uint32_t)(NU * 8)
                              : base + L.zeros + 16u * warp;
     const uint32_t xstep = mine ? 1u : 0u;
     const uint32_t ms0 = msw + (t >> 1) * 16u + (t & 1u) * 8u;  // one row: of group t / 2; two: of row t / 2
@@ -410,32 +438,41 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         if (issued != pieces) issue(st);
     };
     auto first_piece = [&] {  // once the loads of x are on their way
+        if (!S::SHARING) fill(ahead);
         if (pieces) take(test_stage(0u, 0u));
     };
 
+    // warps that share a position have pieces if the first of them has
+    const uint32_t work = !PAIRED ? pieces : my_tiles > (tg & ~1u) ? slabs : 0u;
     uint4 gm = make_uint4(0u, 0u, 0u, 0u);  // RES: norm weights of this lane's activations
-    if (RES && normed && pieces && (pos * 32u + lane) * 8u < K) gm = __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + pos * 32u + lane);
+    if (RES && normed && work && (pos * 32u + lane) * 8u < K) gm = __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + pos * 32u + lane);
     pdl_wait_prior();  // x (and y) belong to the predecessor until here
 
     // A CTA without rows keeps its place until the next launch has taken its own: at the head of a chain it would be gone
     // first, and leave its SM to two of the next launch's
-    if (my_tiles == 0u && A.early)
+    if (S::SHARING && my_tiles == 0u)
         while (clock64() - born < LINGER_CYCLES) __nanosleep(100);
 
     // ---- the activations of this warp's position: one unit of every row and slab a lane
-    __shared__ float nm_part[ROWS][WARPS], nm_inv[ROWS];
-    if (my_tiles && (pieces || normed)) {
-        const uint32_t upr = K >> 3, sets = M * slabs;
+    constexpr uint32_t NPART = RES ? WARPS : 16u;
+    __shared__ float nm_part[ROWS][NPART], nm_inv[ROWS];
+    constexpr uint32_t CR = PAIRED ? 1u : ROWS;                // rows that this warp converts, from row cr on
+    const uint32_t cr = PAIRED && ROWS > 1 ? tg & 1u : 0u;
+    const bool converts = !PAIRED || ROWS > 1 || (tg & 1u) == 0u;
+    uint32_t top[ROWS];
+#pragma unroll
+    for (int m = 0; m < ROWS; ++m) top[m] = 0u;
+    if (my_tiles && (work || normed)) {
+        const uint32_t upr = K >> 3, sets = converts ? CR * slabs : 0u;
         auto place = [&](uint32_t r, uint32_t& m, uint32_t& sl) {
-            m = ROWS > 1 && r >= slabs ? 1u : 0u;
-            sl = r - m * slabs;
-            return (sl * 8u + pos) * 32u + lane;
+            m = CR > 1u && r >= slabs ? 1u : cr;
+            sl = CR > 1u && r >= slabs ? r - slabs : r;
+            return ((s0 + sl) * 8u + pos) * 32u + lane;
         };
-        // normed: the squares first (of tg 0: every unit once), warps in order.  One slab's stay in registers, more are read
-        // again (from L2)
-        constexpr bool KEEP = RES;
-        float4 xa4[ROWS], xc4[ROWS];
-        float inv[ROWS];
+        // normed: the squares first (every unit once: of the first warps of a position), warps in order.  One slab's stay in
+        // registers, more are read again (from L2)
+        float4 xa4, xc4;
+        float inv[CR];
         if (normed) {
             const float4* x4 = reinterpret_cast<const float4*>(A.x);
             auto squares = [](const float4& a, const float4& c, float ss) {
@@ -443,40 +480,46 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 ss = __fmaf_rn(c.x, c.x, ss), ss = __fmaf_rn(c.y, c.y, ss), ss = __fmaf_rn(c.z, c.z, ss);
                 return __fmaf_rn(c.w, c.w, ss);
             };
-            auto add_up = [&](uint32_t m, float ss) {
+            auto warp_sum = [&](float ss) {
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-                if (lane == 0) nm_part[m][warp] = tg == 0u ? ss : 0.0f;
+                return ss;
             };
-            if constexpr (KEEP) {
+            if constexpr (RES) {
                 const uint32_t u = pos * 32u + lane;
-#pragma unroll
-                for (int m = 0; m < ROWS; ++m) {
-                    xa4[m] = xc4[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (slabs && u < upr) xa4[m] = ld_fresh(x4 + (m * upr + u) * 2u), xc4[m] = ld_fresh(x4 + (m * upr + u) * 2u + 1u);
-                }
+                xa4 = xc4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (sets && u < upr) xa4 = ld_fresh(x4 + (cr * upr + u) * 2u), xc4 = ld_fresh(x4 + (cr * upr + u) * 2u + 1u);
                 first_piece();
+                const float ss = warp_sum(squares(xa4, xc4, 0.0f));
+                if (lane == 0) {
 #pragma unroll
-                for (int m = 0; m < ROWS; ++m) add_up((uint32_t)m, squares(xa4[m], xc4[m], 0.0f));
+                    for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) nm_part[m][warp] = converts && m == cr && tg == cr ? ss : 0.0f;
+                }
             } else {
-                for (uint32_t m = 0; m < M; ++m) {
-                    float ss = 0.0f;
-                    for (uint32_t s = 0; s < slabs; ++s) {
-                        const uint32_t u = (s * 8u + pos) * 32u + lane;
-                        if (u < upr) ss = squares(ld_fresh(x4 + ((size_t)m * upr + u) * 2u), ld_fresh(x4 + ((size_t)m * upr + u) * 2u + 1u), ss);
+                for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) {
+#pragma unroll 1
+                    for (uint32_t h = 0; h < (HALVED ? 1u : 2u); ++h) {
+                        float ss = 0.0f;
+                        for (uint32_t s = h * half; s < (HALVED || h ? slabs : min(slabs, half)); ++s) {
+                            const uint32_t u = ((s0 + s) * 8u + pos) * 32u + lane;
+                            if (u < upr) ss = squares(ld_fresh(x4 + ((size_t)m * upr + u) * 2u), ld_fresh(x4 + ((size_t)m * upr + u) * 2u + 1u), ss);
+                        }
+                        ss = warp_sum(ss);
+                        if (lane == 0) nm_part[m][warp + 8u * h] = ss;
                     }
-                    add_up(m, ss);
                 }
                 first_piece();
             }
             __syncthreads();
 #pragma unroll
-            for (int m = 0; m < ROWS; ++m) {
+            for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) {
                 float tot = 0.0f;
 #pragma unroll
-                for (int w = 0; w < WARPS; ++w) tot += nm_part[m][w];
-                inv[m] = rsqrtf(tot / (float)K + A.pre.eps);
-                if (threadIdx.x == 0) nm_inv[m] = inv[m];
+                for (uint32_t w = 0; w < NPART; ++w) tot += nm_part[m][w];
+                const float in = rsqrtf(tot / (float)K + A.pre.eps);
+                if (CR > 1u) inv[m % CR] = in;
+                else if (m == cr) inv[0] = in;
+                if (threadIdx.x == 0) nm_inv[m] = in;
             }
         }
         auto load = [&](uint32_t r) {
@@ -485,11 +528,11 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
             if (r < sets && u < upr) {
                 const size_t i = (size_t)m * upr + u;
-                if (KEEP && normed) {
-                    v = ROWS == 1 || m == 0u ? gemvtma::normed8(xa4[0], xc4[0], inv[0], gm) : gemvtma::normed8(xa4[ROWS - 1], xc4[ROWS - 1], inv[ROWS - 1], gm);
+                if (RES && normed) {
+                    v = gemvtma::normed8(xa4, xc4, inv[0], gm);
                 } else if (normed) {
                     const float4* x4 = reinterpret_cast<const float4*>(A.x) + 2u * i;
-                    v = gemvtma::normed8(ld_fresh(x4), ld_fresh(x4 + 1), ROWS == 1 || m == 0u ? inv[0] : inv[ROWS - 1],
+                    v = gemvtma::normed8(ld_fresh(x4), ld_fresh(x4 + 1), CR == 1u || m == 0u ? inv[0] : inv[CR - 1u],
                                          __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + u));
                 } else {
                     v = ld_fresh(reinterpret_cast<const uint4*>(A.x) + i);
@@ -503,15 +546,16 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             return stage_unit(v, r < sets, xw + m * 4u * L.pitch + sl * PK + lane * 8u, L.pitch, (lane & 7u) == 0u,
                               msw + ((sl * NG + (lane >> 3)) * ROWS + m) * 16u);
         };
-        uint32_t top[ROWS];
-#pragma unroll
-        for (int m = 0; m < ROWS; ++m) top[m] = 0u;
-        if constexpr (RES && ROWS == 1) {
+        if constexpr (RES) {
             const uint4 v = load(0u);
             if (!normed) first_piece();
-            top[0] = stage(0u, v);
+            if (converts) {
+                const uint32_t t0 = stage(0u, v);
+#pragma unroll
+                for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) top[m] = m == cr ? t0 : 0u;
+            }
         } else {  // AHEAD loads in flight, PAIR units at a time (more would be straight code, which costs its fetches)
-            constexpr int AHEAD = RES ? 2 : 4, PAIR = 2;
+            constexpr int AHEAD = 4, PAIR = 2;
             uint4 v[AHEAD];
 #pragma unroll
             for (int h = 0; h < AHEAD; ++h) v[h] = load((uint32_t)h);
@@ -520,7 +564,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             for (uint32_t r = 0; r < sets; r += PAIR) {
                 uint4 w[PAIR];
 #pragma unroll
-                for (int h = 0; h < PAIR; ++h) w[h] = RES ? v[h] : load(r + (uint32_t)(AHEAD + h));
+                for (int h = 0; h < PAIR; ++h) w[h] = load(r + (uint32_t)(AHEAD + h));
                 const uint32_t t0 = stage(r, v[0]), t1 = stage(r + 1u, v[1]);
                 if (ROWS == 1 || r < slabs) top[0] = max(top[0], t0);
                 else top[ROWS - 1] = max(top[ROWS - 1], t0);
@@ -532,14 +576,14 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 for (int h = 0; h < PAIR; ++h) v[AHEAD - PAIR + h] = w[h];
             }
         }
+    }
 #pragma unroll
-        for (int m = 0; m < ROWS; ++m) {
-            const uint32_t all = __reduce_max_sync(0xFFFFFFFFu, top[m]);
-            if (lane == 0) largest[warp][m] = all;
-        }
-    } else if (lane == 0) {
-#pragma unroll
-        for (int m = 0; m < ROWS; ++m) largest[warp][m] = 0u;
+    for (int m = 0; m < ROWS; ++m) {
+        const uint32_t all = __reduce_max_sync(0xFFFFFFFFu, top[m]);
+        if (lane == 0) largest[warp][m] = all;
+    }
+    if constexpr (PAIRED) {
+        if (work) asm volatile("bar.sync %0, 64;" ::"r"(region + 1u) : "memory");
     }
     __syncwarp();
     Acts xa;
@@ -553,14 +597,21 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     uint32_t j = tg, left = pieces;
     for (uint32_t j0 = 0; j0 < my_tiles; j0 += batch) {
         const uint32_t jend = min(my_tiles, j0 + batch), buf = (j0 / batch) & 1u ? batch : 0u;  // two buffers: one meeting a batch
-        uint32_t at = base + L.part + (((buf + j - j0) << pshift) + pos) * (ROWS * 128u) + lane * (ROWS * 4u);
+        uint32_t at = base + L.part + (((buf + j - j0) << slots) + (HALVED ? warp : pos)) * (ROWS * 128u) + lane * (ROWS * 4u);
 #pragma unroll 1
-        for (; j < jend && slabs; j += TG, at += 8u * (ROWS * 128u)) {
+        for (; j < jend && slabs; j += TG, at += WARPS * (ROWS * 128u)) {
+            float below[PAR][2];  // eight warps: sums of the slabs below half
 #pragma unroll
             for (int p = 0; p < PAR; ++p) acc[p][0] = acc[p][1] = 0.0f;
 #pragma unroll 1
             for (uint32_t s = 0; s < (RES ? 1u : slabs); ++s) {
                 if constexpr (!RES) load_x(s, xa);
+                if constexpr (!RES && !HALVED) {
+                    if (s == half) {
+#pragma unroll
+                        for (int p = 0; p < PAR; ++p) below[p][0] = acc[p][0], below[p][1] = acc[p][1], acc[p][0] = acc[p][1] = 0.0f;
+                    }
+                }
                 Codes cur;
                 Sums sums;
                 if (++st == stages) st = 0u, par ^= 1u;
@@ -572,19 +623,22 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 apply(sums, now, xa);
             }
             // the digits' sums; lanes of even t go on with row prow, the others with row prow + 8
+            auto meet = [&](const float (&a)[2]) { return (t & 1u ? a[1] : a[0]) + __shfl_xor_sync(0xFFFFFFFFu, t & 1u ? a[0] : a[1], 1); };
 #pragma unroll
             for (int p = 0; p < PAR; ++p) {
-                const float send = t & 1u ? acc[p][0] : acc[p][1], keep = t & 1u ? acc[p][1] : acc[p][0];
-                const float v = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 1);
+                float v = meet(acc[p]);
+                if constexpr (!RES && !HALVED) {
+                    if (slabs > half) v += meet(below[p]);
+                }
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (uint32_t)p * 4u), "f"(v) : "memory");
             }
         }
         __syncthreads();
-        uint32_t top = 0u;  // of this lane's row
+        uint32_t tallest = 0u;  // of this lane's row
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) top = max(top, largest[w][ROWS == 1 ? 0u : t >> 1]);
+        for (uint32_t w = 0; w < WARPS; ++w) tallest = max(tallest, largest[w][ROWS == 1 ? 0u : t >> 1]);
         for (uint32_t jj = j0 + warp; jj < jend; jj += WARPS) {  // a tile a warp: positions in a fixed tree, even and odd groups last
-            const uint32_t from = base + L.part + ((buf + jj - j0) << pshift) * (ROWS * 128u) + lane * (ROWS * 4u);
+            const uint32_t from = base + L.part + ((buf + jj - j0) << slots) * (ROWS * 128u) + lane * (ROWS * 4u);
             float v[PAR];
 #pragma unroll
             for (int p = 0; p < PAR; ++p) {
@@ -593,13 +647,18 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 for (uint32_t i = 0; i < 8u; ++i) {
                     h[i] = 0.0f;
                     if (i < P) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(h[i]) : "r"(from + i * (ROWS * 128u) + (uint32_t)p * 4u));
+                    if (HALVED && slabs_at(i) > half) {
+                        float above;
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(above) : "r"(from + (8u + i) * (ROWS * 128u) + (uint32_t)p * 4u));
+                        h[i] = above + h[i];
+                    }
                 }
                 v[p] = ((h[0] + h[1]) + (h[2] + h[3])) + ((h[4] + h[5]) + (h[6] + h[7]));
             }
             float y = ROWS == 1 ? v[0] + __shfl_xor_sync(0xFFFFFFFFu, v[0], 2) : v[0] + v[PAR - 1];
             const uint32_t m = ROWS == 1 ? 0u : t >> 1, r = prow + 8u * (t & 1u), tile = tile_of(jj);
-            const bool live = m < M && (ROWS > 1 || t < 2u) && (gated || tile * 16u + r < N);
-            if (no_digits(top) && live) {
+            const bool live = (ROWS > 1 || t < 2u) && (gated || tile * 16u + r < N);
+            if (no_digits(tallest) && live) {
                 if (normed) y = plain_dot<true>(A, row_of(tile, r), m, nm_inv[m]);
                 else y = plain_dot<false>(A, row_of(tile, r), m, 0.0f);
             }
@@ -618,7 +677,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000LL) __nanosleep(1000);
     }
-    gemvtma::close_launch<F, WARPS, WARPS>(A, my_best);
+    gemvtma::close_launch<F, (int)WARPS, (int)WARPS>(A, my_best);
 }
 
 // Launch plan: stages of a warp's ring (0: does not fit) and shared memory.
@@ -627,33 +686,36 @@ struct Plan {
     size_t smem;
 };
 template <class S>
-Plan plan_launch(uint32_t N, uint32_t K, uint32_t M, bool normed) {
+Plan plan_launch(uint32_t N, uint32_t K, bool normed) {
     Plan p;
-    // One CTA per SM, but for the SM that the norm kernel before a normed projection is on: its CTAs take the room
-    // of one of ours there, and ours would join another SM's (a layer with its two norms at one row 21.7 us so, 18.3
-    // with one CTA fewer, at two rows 24.2, and 26.1 with two fewer; a chain of plain projections needs them all).
-    p.grid = std::max(1u, (uint32_t)sm_count() - (normed ? 1u : 0u));
-    const uint32_t tiles = (N + 15u) / 16u, tc = (tiles + p.grid - 1u) / p.grid, row_bytes = K / 2u;
-    const uint32_t P = row_bytes >= SLAB ? 8u : (row_bytes + PIECE - 1u) / PIECE, TG = P > 4u ? 1u : P > 2u ? 2u : P > 1u ? 4u : 8u;
-    const uint32_t slabs = (row_bytes + SLAB - 1u) / SLAB, batch = TG * S::BATCH, part = (tc > batch ? 2u * batch : tc) * (8u / TG);
-    for (p.stages = std::min<uint32_t>(MAX_STAGES, (tc + TG - 1u) / TG * slabs); p.stages > 0u; --p.stages) {
-        p.smem = layout<S>(K, M, p.stages, part).total;
-        if (p.smem <= SMEM_LIMIT) break;  // two rows of 8192 and several batches of tiles leave room for one
+    const uint32_t tiles = (N + 15u) / 16u;
+    // Sharing its SMs: one CTA per SM, but for the SM that the norm kernel before a normed projection is on: its CTAs take
+    // the room of one of ours there, and ours would join another SM's (a layer with its two norms at one row 21.7 us so, 18.3
+    // with one CTA fewer; a chain of plain projections needs them all).
+    p.grid = S::SHARING ? std::max(1u, (uint32_t)sm_count() - (normed ? 1u : 0u)) : std::min((uint32_t)sm_count(), tiles);
+    const uint32_t tc = (tiles + p.grid - 1u) / p.grid, row_bytes = K / 2u, nslab = slabs_of(K);
+    const uint32_t P = row_bytes >= SLAB ? 8u : (row_bytes + PIECE - 1u) / PIECE, pshift = P > 4u ? 3u : P > 2u ? 2u : P > 1u ? 1u : 0u;
+    const bool halved = S::W == 16 && nslab > 1u;
+    const uint32_t TG = halved ? 1u : (uint32_t)S::W >> pshift, batch = TG * S::BATCH;
+    const uint32_t part = (tc > batch ? 2u * batch : tc) << (pshift + (halved ? 1u : 0u));
+    for (p.stages = std::min<uint32_t>(MAX_STAGES, (tc + TG - 1u) / TG * (S::W == 16 ? half_of(nslab) : nslab)); p.stages > 0u; --p.stages) {
+        p.smem = layout<S>(K, p.stages, part).total;
+        if (p.smem <= S::SMEM_LIMIT) break;
     }
-    p.smem = std::max(p.smem, SMEM_FLOOR);
+    p.smem = std::max(p.smem, S::SMEM_FLOOR);
     return p;
 }
 
 template <class S, Fuse F, bool RES>
 int launch_one(const void* q, Args a, cudaStream_t stream) {
-    const Plan p = plan_launch<S>(a.N, a.K, a.M, a.pre.gamma != nullptr);
+    const Plan p = plan_launch<S>(a.N, a.K, a.pre.gamma != nullptr);
     if (!p.stages) return fail(MIORI_E_INVALID, "gemv: no plan for N=%u K=%u M=%u", a.N, a.K, a.M);
     a.stages = p.stages;
     CUtensorMap tq;
     const int rc = make_tmap_2d(&tq, q, CU_TENSOR_MAP_DATA_TYPE_UINT64, 8, (uint64_t)a.K / 16, a.N, PIECE / 8, a.gated ? 8 : 16,
                                 CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    const cudaError_t e = launch<Split::SHARED>(gemv_digits_kernel<S, F, RES>, dim3(p.grid), dim3(THREADS), p.smem, stream, true, tq, a);
+    const cudaError_t e = launch<Split::SHARED>(gemv_digits_kernel<S, F, RES>, dim3(p.grid), dim3(S::THREADS), p.smem, stream, true, tq, a);
     if (e != cudaSuccess) return cuda_fail(e, "gemv_digits launch");
     return MIORI_OK;
 }
@@ -665,35 +727,41 @@ int launch_k(const void* q, const Args& a, cudaStream_t stream) {
 
 // K that this kernel takes: whole pieces (a row of 6208 codes, with its last groups picked out one by one, took 11.3 us at
 // 5967 rows, 7.6 in gemv_tma.cuh), up to where its launches still pay.
-// Beyond one slab as long as there is one tile a CTA: what a layer's last projection is, which the
-// others of a chain start beside; with more, the conversion of x and the pieces take longer than there (8192 x 8192 at one
-// row 11.5 us, 10.1).
+// Beyond one slab as long as there is one tile a CTA: what a layer's last projection is, which the others of a chain of
+// early launches start beside (with this product in gemv_tma.cuh the four projections of a layer take 15.9 us at one row, 13.5
+// with it here); with more, the conversion of x and the pieces take longer than there (8192 x 8192 at one row 11.5 us,
+// 10.1).  So there the kernel, and with it a row's rounding, depends on N, as the order of its sums in gemv_tma.cuh does.
 inline bool takes(uint32_t N, uint32_t K) {
     return K % PK == 0u && (K <= 2u * SLAB || (K <= MAX_K && (N + 15u) / 16u <= (uint32_t)sm_count()));
 }
 
 // One or two rows, of a K that is taken.
-template <int ROWS>
-int launch_rows(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t flags,
-                cudaStream_t stream, const gemvtma::Shard& sh) {
-    using S = Shape<ROWS>;
+template <class S>
+int launch_form(const void* q, const Args& a, cudaStream_t stream) {
+    if (a.best) {
+        if constexpr (S::ROWS == 1) return launch_k<S, gemvtma::ARGMAX>(q, a, stream);
+    }
+    if (a.pa.world > 1) {
+        if constexpr (!S::SHARING) return launch_k<S, gemvtma::SHARDED>(q, a, stream);
+    }
+    if (a.post.residual) return launch_k<S, gemvtma::POSTNORM>(q, a, stream);
+    if (a.gated || a.pre.gamma) return launch_k<S, gemvtma::FUSED>(q, a, stream);
+    return launch_k<S, gemvtma::NONE>(q, a, stream);
+}
+inline int launch_rows(const void* q, const void* s, const void* b, const void* x, void* y, uint32_t N, uint32_t K, uint32_t M, uint32_t flags,
+                       cudaStream_t stream, const gemvtma::Shard& sh) {
     const bool placed = sh.pa.world > 1 || sh.best;  // y is a slice of an n_total-row output
     Args a;
     a.x = static_cast<const uint16_t*>(x), a.y = y;
     a.q = static_cast<const uint8_t*>(q), a.s = static_cast<const uint16_t*>(s), a.b = static_cast<const uint16_t*>(b);
     a.pre = sh.pre, a.post = sh.post;
-    a.N = N, a.K = K, a.M = ROWS, a.stages = 0u;
+    a.N = N, a.K = K, a.M = M, a.stages = 0u;
     a.out_bf16 = flags & MIORI_OUT_BF16 ? 1u : 0u, a.gated = sh.gated ? 1u : 0u, a.early = flags & MIORI_LAUNCH_PDL ? 1u : 0u;
     a.n_total = placed ? sh.n_total : N, a.row0 = placed ? sh.row0 : 0u, a.y_off = sh.y_off, a.best = sh.best, a.pa = sh.pa;
-    const int rc = gemvtma::check_fuse(sh, 4, N, ROWS, a.out_bf16 != 0u);
+    const int rc = gemvtma::check_fuse(sh, 4, N, M, a.out_bf16 != 0u);
     if (rc) return rc;
-    if (sh.best) {
-        if constexpr (ROWS == 1) return launch_k<S, gemvtma::ARGMAX>(q, a, stream);
-    }
-    if (sh.pa.world > 1) return launch_k<S, gemvtma::SHARDED>(q, a, stream);
-    if (sh.post.residual) return launch_k<S, gemvtma::POSTNORM>(q, a, stream);
-    if (sh.gated || sh.pre.gamma) return launch_k<S, gemvtma::FUSED>(q, a, stream);
-    return launch_k<S, gemvtma::NONE>(q, a, stream);
+    if (M == 2u) return launch_form<Shape<2, 16>>(q, a, stream);
+    return a.early && sh.pa.world <= 1 ? launch_form<Shape<1, 8>>(q, a, stream) : launch_form<Shape<1, 16>>(q, a, stream);
 }
 
 }  // namespace gemvdigits

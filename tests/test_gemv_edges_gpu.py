@@ -247,3 +247,27 @@ def test_fused_forms_of_activations_that_are_not_finite():
     z = miori_b200.gemv4_silu(q, s, b, x.to(torch.bfloat16), group=64)
     v = miori_b200.gemv4(q, s, b, x.to(torch.bfloat16), group=64)
     assert torch.equal(z[0], miori_b200.silu_mul(v[:, :N // 2].contiguous(), v[:, N // 2:].contiguous())[0])
+
+
+@pytest.mark.parametrize("K", [512, 1536, 2048, 2560, 4096, 6656, 8192])
+@pytest.mark.parametrize("N", [16, 2368, 5008])
+def test_launches_of_one_and_two_rows_agree(K, N):
+    """One row started early runs eight warps a CTA, one that waits and two rows run sixteen: the same bits in every form."""
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=N + K, device=DEV)
+    x, h, res = synth.make_activation(2, K, seed=K, device=DEV), torch.randn((2, K), device=DEV), torch.randn((2, N), device=DEV)
+    g, gn = (synth.make_activation(1, n, seed=n, device=DEV).reshape(-1) for n in (K, N))
+    counter = torch.zeros(1, dtype=torch.int32, device=DEV)
+    forms = [lambda r, f: miori_b200.gemv4(q, s, b, x[r], group=64, flags=f)]
+    if K % 512 == 0:  # what the fused entries take
+        forms += [lambda r, f: miori_b200.gemv4_rmsnorm(q, s, b, h[r], g, 1e-5, group=64, flags=f),
+                  lambda r, f: miori_b200.gemv4_silu(q, s, b, x[r], group=64, flags=f),
+                  lambda r, f: miori_b200.gemv4_rmsnorm_silu(q, s, b, h[r], g, 1e-5, group=64, flags=f),
+                  lambda r, f: miori_b200.gemv4_post_norm_add(q, s, b, x[r], res[r], gn, 1e-5, counter, group=64, flags=f)]
+    for i, form in enumerate(forms):
+        both = form(slice(0, 2), 0)
+        assert torch.isfinite(both.float()).all()
+        assert torch.equal(form(slice(0, 2), miori_b200.LAUNCH_PDL), both), i
+        for r in (0, 1):
+            for f in (0, miori_b200.LAUNCH_PDL):
+                assert torch.equal(form(slice(r, r + 1), f), both[r:r + 1]), (i, r, f)
+    assert miori_b200.lib.miori_device_error_poll() == 0
