@@ -173,7 +173,7 @@ __device__ __forceinline__ uint32_t stage_unit(const uint4& v, bool live, uint32
     uint32_t q[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)  // the bytes of (q + 0x80808080) are the digits + 128
-        q[i] = (uint32_t)(__float2int_rn(f[i] * (i & 1 ? up : up16)) + (int)0x80808080) ^ 0x80808080u;
+        q[i] = ((uint32_t)__float2int_rn(f[i] * (i & 1 ? up : up16)) + 0x80808080u) ^ 0x80808080u;
     uint32_t p[2][4];  // byte l of the even (odd) ones
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
