@@ -199,28 +199,81 @@ __device__ __noinline__ bool wait_on(uint32_t bar, uint32_t parity, volatile uin
     return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort, where));
 }
 
-// One output of a row of activations that are not all finite, or all next to nothing, in fp32: they have no digits.
+// Eight outputs of a row of activations that are not all finite, or all next to nothing, in fp32 by a whole warp: they have no
+// digits.  Tensor rows row0 .. row0 + 7, or, gated, row0 .. row0 + 3 and the up rows of the same outputs.  Lane i < 8 gets
+// the i-th.
 template <bool NORMED>
-__device__ __noinline__ float plain_dot(const Args& A, uint32_t n, uint32_t m, float inv) {
-    const uint32_t ng = A.K / GROUP;
-    const uint32_t* q = reinterpret_cast<const uint32_t*>(A.q) + (size_t)n * (A.K / 8u);
-    float y = 0.0f;
-    for (uint32_t g = 0; g < ng; ++g) {
-        float cx = 0.0f, sx = 0.0f;
-        for (uint32_t w = 0; w < GROUP / 8u; ++w) {
-            const uint32_t codes = q[g * (GROUP / 8u) + w];
-            for (uint32_t i = 0; i < 8u; ++i) {
-                const size_t k = (size_t)g * GROUP + w * 8u + i, at = (size_t)m * A.K + k;
-                const float x = NORMED ? bf16_bits_to_float(float_to_bf16_bits(ld_fresh(reinterpret_cast<const float*>(A.x) + at) * inv *
-                                                                               bf16_bits_to_float(A.pre.gamma[k])))
-                                       : bf16_bits_to_float(ld_fresh(A.x + at));
-                cx = __fmaf_rn((float)((codes >> (4u * i)) & 15u), x, cx);
-                sx += x;
-            }
+__device__ __forceinline__ float plain_dots(const Args& A, uint32_t row0, bool gated, uint32_t m, float inv) {
+    constexpr uint32_t DOTS = 8;
+    const uint32_t ng = A.K / GROUP, words = A.K / 8u, lane = threadIdx.x & 31u;
+    uint32_t row[DOTS];
+    float sum[DOTS];
+#pragma unroll
+    for (uint32_t d = 0; d < DOTS; ++d) {
+        row[d] = gated ? row0 + (d & 3u) + (d >= 4u ? A.N >> 1 : 0u) : min(row0 + d, A.N - 1u);
+        sum[d] = 0.0f;
+    }
+    for (uint32_t w = lane; w < words; w += 32u) {
+        const size_t at = (size_t)m * words + w;
+        uint4 v;
+        if constexpr (NORMED) {
+            const float4* x4 = reinterpret_cast<const float4*>(A.x) + 2u * at;
+            v = gemvtma::normed8(ld_fresh(x4), ld_fresh(x4 + 1), inv, __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + w));
+        } else {
+            v = ld_fresh(reinterpret_cast<const uint4*>(A.x) + at);
         }
-        y = __fmaf_rn(bf16_bits_to_float(A.s[(size_t)n * ng + g]), cx, __fmaf_rn(bf16_bits_to_float(A.b[(size_t)n * ng + g]), sx, y));
+        const float x[8] = {bf16lo(v.x), bf16hi(v.x), bf16lo(v.y), bf16hi(v.y), bf16lo(v.z), bf16hi(v.z), bf16lo(v.w), bf16hi(v.w)};
+        const float sx = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+        uint32_t codes[DOTS], s[DOTS], b[DOTS];
+#pragma unroll
+        for (uint32_t d = 0; d < DOTS; ++d) {
+            const size_t g = (size_t)row[d] * ng + w / (GROUP / 8u);
+            codes[d] = reinterpret_cast<const uint32_t*>(A.q)[(size_t)row[d] * words + w], s[d] = A.s[g], b[d] = A.b[g];
+        }
+#pragma unroll
+        for (uint32_t d = 0; d < DOTS; ++d) {
+            float cx = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) cx = __fmaf_rn((float)((codes[d] >> (4 * i)) & 15u), x[i], cx);
+            sum[d] = __fmaf_rn(bf16_bits_to_float(s[d]), cx, __fmaf_rn(bf16_bits_to_float(b[d]), sx, sum[d]));
+        }
+    }
+    float y = 0.0f;
+#pragma unroll
+    for (uint32_t d = 0; d < DOTS; ++d) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum[d] += __shfl_xor_sync(0xFFFFFFFFu, sum[d], o);
+        if (lane == d) y = sum[d];
     }
     return y;
+}
+
+// All outputs of the CTA's tiles in the rows of `wanting`, half a tile a warp.  Returns the arg-max form's best key.  (One
+// launch after the other with such a row, a thread an output and so, us: 2048 x 2048 35 -> 9, 16384 x 2048 47 -> 18, 2048 x
+// 8192 119 -> 28.)
+template <int ROWS, Fuse F>
+__device__ __noinline__ unsigned long long plain_rows(const Args& A, uint32_t wanting, uint32_t inv_at, unsigned long long my_best) {
+    const bool gated = F == gemvtma::FUSED && A.gated != 0u, normed = F == gemvtma::FUSED && A.pre.gamma != nullptr;
+    const uint32_t my_tiles = (((A.N + 15u) >> 4) - blockIdx.x + gridDim.x - 1u) / gridDim.x;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+#pragma unroll 1
+    for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) {
+        if (!(wanting >> m & 1u)) continue;
+        float inv = 0.0f;
+        if (normed) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(inv) : "r"(inv_at + 4u * m));
+#pragma unroll 1
+        for (uint32_t i = warp; i < 2u * my_tiles; i += warps) {
+            const uint32_t tile = blockIdx.x + (i >> 1) * gridDim.x, row0 = gated ? tile * 8u + (i & 1u) * 4u : tile * 16u + (i & 1u) * 8u;
+            const float y = normed ? plain_dots<true>(A, row0, gated, m, inv) : plain_dots<false>(A, row0, gated, m, 0.0f);
+            if (gated) {
+                const float up = __shfl_down_sync(0xFFFFFFFFu, y, 4);
+                if (lane < 4u) gemvtma::store_gated(A, m, row0 + lane, y, up);
+            } else if (lane < 8u && row0 + lane < A.N) {
+                gemvtma::store_out<F>(A, m, row0 + lane, y, my_best);
+            }
+        }
+    }
+    return my_best;
 }
 
 // RES: K <= 2048, one slab: the activations of a warp's position stay in registers.
@@ -594,7 +647,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     // y is one launch's output; ARGMAX: key of the best element this thread has stored
     unsigned long long my_best = 0ull;
     auto store_out = [&](uint32_t m, uint32_t row, float v) { gemvtma::store_out<F>(A, m, row, v, my_best); };
-    uint32_t j = tg, left = pieces;
+    uint32_t j = tg, left = pieces, wanting = 0u;  // wanting: rows without digits
     for (uint32_t j0 = 0; j0 < my_tiles; j0 += batch) {
         const uint32_t jend = min(my_tiles, j0 + batch), buf = (j0 / batch) & 1u ? batch : 0u;  // two buffers: one meeting a batch
         uint32_t at = base + L.part + (((buf + j - j0) << slots) + (HALVED ? warp : pos)) * (ROWS * 128u) + lane * (ROWS * 4u);
@@ -637,6 +690,8 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         uint32_t tallest = 0u;  // of this lane's row
 #pragma unroll
         for (uint32_t w = 0; w < WARPS; ++w) tallest = max(tallest, largest[w][ROWS == 1 ? 0u : t >> 1]);
+        const bool none = no_digits(tallest);
+        wanting = ROWS == 1 ? (none ? 1u : 0u) : (__any_sync(0xFFFFFFFFu, none && t < 2u) ? 1u : 0u) | (__any_sync(0xFFFFFFFFu, none && t >= 2u) ? 2u : 0u);
         for (uint32_t jj = j0 + warp; jj < jend; jj += WARPS) {  // a tile a warp: positions in a fixed tree, even and odd groups last
             const uint32_t from = base + L.part + ((buf + jj - j0) << slots) * (ROWS * 128u) + lane * (ROWS * 4u);
             float v[PAR];
@@ -657,11 +712,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
             float y = ROWS == 1 ? v[0] + __shfl_xor_sync(0xFFFFFFFFu, v[0], 2) : v[0] + v[PAR - 1];
             const uint32_t m = ROWS == 1 ? 0u : t >> 1, r = prow + 8u * (t & 1u), tile = tile_of(jj);
-            const bool live = (ROWS > 1 || t < 2u) && (gated || tile * 16u + r < N);
-            if (no_digits(tallest) && live) {
-                if (normed) y = plain_dot<true>(A, row_of(tile, r), m, nm_inv[m]);
-                else y = plain_dot<false>(A, row_of(tile, r), m, 0.0f);
-            }
+            const bool live = !none && (ROWS > 1 || t < 2u) && (gated || tile * 16u + r < N);
             if (gated) {  // even t: gate of output prow, odd t: its up
                 __syncwarp();
                 const float up = __shfl_xor_sync(0xFFFFFFFFu, y, 1);
@@ -671,6 +722,9 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
         }
     }
+
+    // rows without digits: here, where nothing of the above is wanted any more (among the stores it would be spilled)
+    if (__builtin_expect(wanting != 0u, 0)) my_best = plain_rows<ROWS, F>(A, wanting, smem_addr(nm_inv), my_best);
 
     if constexpr (POSTNORM_ || ARGMAX_ || SHARDED_) __syncthreads();
     if (abort_flag) {  // let copies still in flight land before the CTA's memory is released

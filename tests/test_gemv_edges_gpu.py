@@ -271,3 +271,74 @@ def test_launches_of_one_and_two_rows_agree(K, N):
             for f in (0, miori_b200.LAUNCH_PDL):
                 assert torch.equal(form(slice(r, r + 1), f), both[r:r + 1]), (i, r, f)
     assert miori_b200.lib.miori_device_error_poll() == 0
+
+
+@pytest.mark.parametrize("flags", [0, miori_b200.LAUNCH_PDL])
+@pytest.mark.parametrize("K", [512, 2048, 3072, 8192])
+def test_every_form_of_rows_next_to_nothing(K, flags):
+    """Rows of activations below 2^-98 through the forms that carry a neighbour: the sums of the plain product."""
+    N = 144
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=K, device=DEV)
+    s, b = s * 2.0 ** 100, b * 2.0 ** 100  # outputs of ordinary size
+    w = _weights64(q, s, b, 4, 64)
+    x = synth.make_activation(2, K, seed=1, device=DEV)
+    x[1] *= 2.0 ** -100
+    x[0] *= 2.0 ** -90
+    assert float(x[1].abs().max()) < 2.0 ** -97 and float(x[0].abs().max()) > 2.0 ** -98
+    v = miori_b200.gemv4(q, s, b, x, group=64, flags=flags)
+    want = x.double() @ w.T
+    for m in (0, 1):  # a row's terms in order at worst, growing as the root of their number
+        assert float((v[m].double() - want[m]).norm() / want[m].norm()) < 2.0 ** -24 * 4 * K ** 0.5
+    z = miori_b200.silu_mul(v[:, :N // 2].contiguous(), v[:, N // 2:].contiguous())
+    assert torch.equal(miori_b200.gemv4_silu(q, s, b, x, group=64, flags=flags), z) and (z[1] != 0).any()
+    res, gn = torch.randn((2, N), device=DEV), synth.make_activation(1, N, seed=1, device=DEV).reshape(-1)
+    counter = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got = miori_b200.gemv4_post_norm_add(q, s, b, x, res, gn, 1e-5, counter, group=64, flags=flags)
+    assert torch.equal(got, miori_b200.post_norm_add(res, v, gn, 1e-5)) and int(counter) == 0
+    for m in (0, 1):
+        one = slice(m, m + 1)
+        assert torch.equal(miori_b200.gemv4(q, s, b, x[one], group=64, flags=flags), v[one])
+        assert torch.equal(miori_b200.gemv4_silu(q, s, b, x[one], group=64, flags=flags), z[one])
+        assert torch.equal(miori_b200.gemv4_post_norm_add(q, s, b, x[one], res[one], gn, 1e-5, counter, group=64, flags=flags), got[one])
+    # the norm in front: normalised rows that small, and single roundings of them may tip over
+    h, g = torch.randn((2, K), device=DEV), (synth.make_activation(1, K, seed=2, device=DEV) * 2.0 ** -101).reshape(-1)
+    want = miori_b200.rmsnorm(h, g, 1e-5).double() @ w.T
+    y = miori_b200.gemv4_rmsnorm(q, s, b, h, g, 1e-5, group=64, flags=flags)
+    assert float((y.double() - want).norm() / want.norm()) < 1e-3
+    z = miori_b200.silu_mul(y[:, :N // 2].contiguous(), y[:, N // 2:].contiguous())
+    assert torch.equal(miori_b200.gemv4_rmsnorm_silu(q, s, b, h, g, 1e-5, group=64, flags=flags), z) and (z != 0).any()
+    assert torch.equal(miori_b200.gemv4_rmsnorm(q, s, b, h[1:], g, 1e-5, group=64, flags=flags), y[1:])
+    assert miori_b200.lib.miori_device_error_poll() == 0
+
+
+@pytest.mark.parametrize("K", [512, 2048, 8192])
+def test_gated_outputs_of_a_row_that_is_not_finite(K):
+    N = 144
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=3, device=DEV)
+    x = synth.make_activation(2, K, seed=4, device=DEV)
+    want = miori_b200.gemv4_silu(q, s, b, x, group=64)
+    x[1, 7] = float("inf")
+    z = miori_b200.gemv4_silu(q, s, b, x, group=64)
+    v = miori_b200.gemv4(q, s, b, x, group=64)
+    assert torch.equal(z[0], want[0]) and not torch.isfinite(v[1]).any()
+    pair = miori_b200.silu_mul(v[1:, :N // 2].contiguous(), v[1:, N // 2:].contiguous())
+    assert torch.equal(z[1:].view(torch.int16), pair.view(torch.int16))
+
+
+def test_greedy_pick_of_a_row_next_to_nothing():
+    from miori_b200.peers import PeerGroup
+    N, K = 1000, 2048
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=5, device=DEV)
+    s, b = s * 2.0 ** 100, b * 2.0 ** 100
+    x = (synth.make_activation(1, K, seed=1, device=DEV).float() * 2.0 ** -110).to(torch.bfloat16)
+    want = miori_b200.gemv4(q, s, b, x, group=64)[0]
+    grp = PeerGroup(0, 1, 1 << 16, torch.device("cuda", 0))
+    try:
+        off_y, off_b = grp.alloc(N * 4), grp.alloc(grp.gemv_argmax_bytes())
+        for flags in (0, miori_b200.LAUNCH_PDL):
+            grp.gemv_argmax(4, q, s, b, x, off_y, off_b, 0, N, group=64, flags=flags)
+            torch.cuda.synchronize()
+            assert torch.equal(grp.tensor(off_y, (1, N))[0], want)
+            assert grp.gemv_argmax_result(off_b) == (int(want.argmax()), float(want.max()))
+    finally:
+        grp.close()
