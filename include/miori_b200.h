@@ -96,9 +96,12 @@ int miori_stream_sync(void* stream);
  * (reference shaders/batch.metal:142-144) within a class of batch sizes, 1..2 and 3..8 rows (4-bit
  * weights in groups of 64) or 1..4 and 5..8 (others), 9..16, 17..32, nor on MIORI_LAUNCH_PDL.  Across
  * classes rows agree to fp32 rounding, not bit for bit, and so do a tensor's rows and the same rows of a
- * taller one (a shard and the whole): N, too, decides how a row is summed.  Requires K % group == 0,
- * group in {32,64}; q,s,b,x 16-byte aligned.  Only M rows of x are read and M rows of y written (the
- * reference's gemv4_b always touches four, shaders/batch.metal:178-179). */
+ * taller one (a shard and the whole): N, too, decides how a row is summed.  One and two rows of 4-bit
+ * weights in groups of 64, K a multiple of 256 up to 2048 (up to 8192 while N is at most 16 times the number
+ * of SMs), hold an activation to 2^-25 of the largest of its 64 and sum exactly what they hold; the others
+ * hold it exactly down to 2^-28 of it, and their sums cut it off.  Requires K % group == 0, group in
+ * {32,64}; q,s,b,x 16-byte aligned.  Only M rows of x are read and M rows of y written (the reference's
+ * gemv4_b always touches four, shaders/batch.metal:178-179). */
 int miori_gemv4(const void* q, const void* s, const void* b, const void* x, void* y,
                 uint32_t N, uint32_t K, uint32_t M, uint32_t group, uint32_t flags,
                 void* stream);

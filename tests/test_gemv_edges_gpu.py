@@ -342,3 +342,34 @@ def test_greedy_pick_of_a_row_next_to_nothing():
             assert grp.gemv_argmax_result(off_b) == (int(want.argmax()), float(want.max()))
     finally:
         grp.close()
+
+
+@pytest.mark.parametrize("exponent", [6, 12, 20])
+@pytest.mark.parametrize("code", [0, 1, 3, 8])
+@pytest.mark.parametrize("K", [2048, 4096])
+def test_outliers_whose_weights_are_zero(exponent, code, K):
+    """One activation of 2^exponent a group, the others normal, and its weight exactly zero: code * s + b = 0.  An activation
+    is held to 2^-25 of its group's largest, and that is all that is to be seen.  The rows of a batch of three, whose operands are
+    fp16, are exact there for code 0 alone, where nothing of the outlier meets a sum: for the others they are further off."""
+    N = 256
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(exponent)
+    at = torch.randint(0, 64, (K // 64,), generator=gen, device=DEV) + torch.arange(0, K, 64, device=DEV)
+    codes = torch.randint(0, 16, (N, K), generator=gen, device=DEV)
+    codes[:, at] = code
+    q = (codes.view(N, K // 8, 8) << (4 * torch.arange(8, device=DEV))).sum(-1)
+    q = torch.where(q >= 2 ** 31, q - 2 ** 32, q).to(torch.int32)
+    s = torch.randint(1, 16, (N, K // 64), generator=gen, device=DEV).to(torch.bfloat16) * 2.0 ** -10
+    b = -code * s  # exact: four bits times four
+    x = torch.randn((3, K), generator=gen, device=DEV).to(torch.bfloat16)
+    x[:, at] = 2.0 ** exponent
+    want = x.double() @ _weights64(q, s, b, 4, 64).T
+    reach = (codes.double() * s.double().repeat_interleave(64, 1)).sum(1) * 2.0 ** (exponent - 25)
+    # a group's sum of its codes and its bias term meet the outlier's code * s * 2^exponent each, and round it some three times
+    rounding = 6 * 2.0 ** -24 * ((code * s.double()).sum(1) * 2.0 ** exponent + 64 * s.double().sum(1))
+    for M in (1, 2):
+        got = miori_b200.gemv4(q, s, b, x[:M].contiguous(), group=64).double()
+        assert ((got - want[:M]).abs() <= reach + rounding).all()
+    if code:
+        wide = miori_b200.gemv4(q, s, b, x, group=64).double()
+        assert float((got - want[:2]).norm()) < float((wide[:2] - want[:2]).norm())
