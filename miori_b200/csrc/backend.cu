@@ -3,6 +3,8 @@
 // begin/submit); there is no pipeline cache because kernels are linked in.
 #include "common.cuh"
 
+#include <cuda.h>
+
 #include <mutex>
 #include <new>
 
@@ -29,6 +31,18 @@ int sm_count() {
         cached[dev] = n;
     }
     return cached[dev];
+}
+
+unsigned long long context_id() {
+    using Fn = CUresult (*)(CUcontext, unsigned long long*);
+    static const Fn get = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool ok = cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+        return ok ? reinterpret_cast<Fn>(p) : nullptr;
+    }();
+    unsigned long long id = 0;
+    return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0ull;
 }
 
 }  // namespace miori_b200

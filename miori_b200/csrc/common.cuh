@@ -32,29 +32,38 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // Number of SMs of the current device (cached per device ordinal).
 int sm_count();
 
-// What a kernel is set to before its first launch on a device: as much dynamic shared memory as there is beside its
-// static and, for the kernels of a decode step of few rows, the largest shared-memory share of an SM's memory.  They
-// all ask for the same share, because a change of it waits until the SM is empty, and none could start beside one
-// that wants another (four projections of a decode layer 24 us instead of 18).  The others leave it to the
-// driver: the largest share is the smallest L1 (a cache build of 8-bit weights 7.6 us, 11.3 with it).  The settings are
-// the same whoever makes them; what a thread has made it remembers (as launch attributes the share costs 1.4 us of host
-// time a launch, and each call here 0.1).
+// Number of the current context, which no other context of the process ever has (0: unknown).
+unsigned long long context_id();
+
+// What a kernel is set to before its first launch in a context: as much dynamic shared memory as there is beside its static
+// and, for the norms of a few rows and the GEMV of one and two 4-bit rows (gemv_digits.cuh), the largest shared-memory share
+// of an SM's memory: a change of it waits until the SM is empty, and none of them could start beside one that wants another
+// (four projections of a decode layer 24 us instead of 18).  The others leave it to the driver: the largest share is the
+// smallest L1 (a cache build of 8-bit weights 7.6 us, 11.3 with it; the activation between the projections of a layer at one
+// row: no difference).  The settings are the same whoever makes them; what a thread has made it remembers (as launch
+// attributes the share costs 1.4 us of host time a launch, and each call here 0.1).
 enum class Split { DRIVERS, SHARED };
 inline cudaError_t set_up_kernel(const void* kernel, Split split) {
-    constexpr uint32_t SLOTS = 128;
-    static thread_local struct { const void* kernel; int device; } made[SLOTS];
-    int device = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e != cudaSuccess) return e;
-    auto& m = made[(reinterpret_cast<uintptr_t>(kernel) >> 4) % SLOTS];
-    if (m.kernel == kernel && m.device == device) return cudaSuccess;
+    constexpr uint32_t SLOTS = 512;  // three times the kernels there are: probed, so that no two take turns in a slot
+    struct Made { const void* kernel; unsigned long long context; };
+    static thread_local Made made[SLOTS];
+    const unsigned long long context = context_id();
+    Made* free_slot = nullptr;
+    for (uint32_t i = 0, at = (uint32_t)(reinterpret_cast<uintptr_t>(kernel) >> 4); i < SLOTS && context; ++i, ++at) {
+        auto& m = made[at % SLOTS];
+        if (m.kernel == kernel && m.context == context) return cudaSuccess;
+        if (!m.kernel) {
+            free_slot = &m;
+            break;
+        }
+    }
     cudaFuncAttributes fa;
-    e = cudaFuncGetAttributes(&fa, kernel);
+    cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes);
     if (e == cudaSuccess && split == Split::SHARED)
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess) m = {kernel, device};
+    if (e == cudaSuccess && free_slot) *free_slot = {kernel, context};
     return e;
 }
 
