@@ -27,30 +27,35 @@
 //   * K <= 2048: the activations stay in registers from tile to tile.
 //   * The first piece is read while x is on its way.
 // Two frames, the same bits:
-//   * one row started early: EIGHT warps a CTA and two CTAs to an SM, one of this launch and one of the next, which
+//   * one row started early, up to 192 KiB of codes an SM: EIGHT warps a CTA and two CTAs to an SM, one of this launch and one of the next, which
 //     fetches its weights while this one works.  Behind a norm that is fused into it a launch has one CTA fewer than there
 //     are SMs, else one per SM, those without rows included: a launch of fewer lets the next one's double up, and every
 //     later launch inherits the skew.  After its first pieces a CTA holds the others back for 800 cycles: it starts when
-//     its predecessor fetches x, whose loads would queue up behind them (four projections of a layer 15.2 us when all are
-//     fetched at once, 14.5 so);
-//   * two rows, launches that wait for the one before, launches over several GPUs: SIXTEEN warps and one CTA to an SM.  Two
-//     warps share a position: each converts one row of two, or half the slabs.  All pieces but the first are fetched behind
-//     x (16384 x 2048 at one row 7.0 us when all are fetched ahead, 6.3 with two first ones, 5.7 with one; none 5.9).  Beside
-//     launches that keep to neither rule -- norms, activations, other products -- it is the steadier one: with eight warps a
-//     layer's four projections that wait took 24.8 us, 17.1 so, and nine launches of a layer at two rows 28.8 and 24.3.
+//     its predecessor fetches x, whose loads would queue up behind them (four projections of a layer 5 % slower when all are
+//     fetched at once);
+//   * two rows, longer launches, launches that wait for the one before or go over several GPUs: SIXTEEN warps and one CTA to
+//     an SM.  Two warps share a position: each converts one row of two, or half the slabs.  All pieces but the first are
+//     fetched behind x (16384 x 2048 at one row 7.0 us when all are fetched ahead, 6.3 with two first ones, 5.7 with one; none
+//     5.9).  Beside launches that keep to neither rule -- norms, activations, other products -- it is the steadier one: with
+//     eight warps a layer's four projections that wait took 24.8 us, 17.2 so, and nine launches of a layer at two rows 28.8
+//     and 24.1.
 //
-// Measured in chains over weights larger than L2, the kernel of gemv_tma.cuh and this one, us:
+// Measured in chains over weights larger than L2, the kernel of gemv_tma.cuh and this one in turns, us:
 //                          one row early     one that waits    two rows early    two that wait
-//   2048 x 2048            2.50   2.09       2.93   2.48       2.51   2.76       2.94   2.77
-//   3072 x 2048            2.85   2.42       3.55   3.01       2.93   3.10       3.61   3.37
-//   16384 x 2048           6.63   4.88       7.62   5.70       7.05   5.95       7.81   6.42
-//   32768 x 512            6.60   3.44       7.19   4.28       6.83   4.36       7.46   4.72
-//   2048 x 4096            3.35   3.24       4.14   4.04       3.51   4.13       4.13   4.64
-//   2048 x 8192            4.63   4.55       5.64   5.49       4.87   5.92       5.65   6.69
-//   a layer's four        16.6   13.5       20.1   17.1       17.3   17.6       20.4   19.7
-//   with neighbours, six  21.2   18.4                         23.3   22.3
-// Two rows beyond one slab are behind: converting a row takes 2.2 times the instructions of fp16's and is most of the time
-// there.  They run here all the same: a row has the same bits alone and beside another, and one row gains.
+//   2048 x 2048            2.70   2.05       3.41   2.89       2.71   2.83       3.43   3.08
+//   3072 x 2048            2.96   2.41       3.75   3.28       2.93   3.09       3.80   3.69
+//   16384 x 2048           6.67   5.04       7.70   5.71       7.05   5.66       7.83   6.30
+//   131072 x 2048         32.1   27.6       32.2   27.8       34.5   30.2       34.9   30.5
+//   32768 x 512            6.55   3.45       7.15   4.25       6.80   4.21       7.43   4.64
+//   2048 x 4096            3.29   3.18       4.10   3.96       3.41   4.29       4.10   4.84
+//   2048 x 8192            4.63   4.46       5.60   5.33       4.89   6.09       5.60   6.85
+//   a layer's four        16.8   13.6       20.4   17.2       17.4   17.6       20.6   19.8
+//   with neighbours, six  21.5   19.3       25.0   21.8       23.7   22.9       25.8   25.2
+//   nine launches         22.0   20.4       27.3   24.8       23.2   24.1       27.6   27.6
+// Two rows that start early are behind up to some 4000 outputs, and all beyond one slab: converting a row takes 2.2 times the
+// instructions of fp16's and is most of the time there.  They run here all the same: a row has the same bits alone and beside
+// another, and one row gains.  (Digits from two additions of a power of two, which leave out the conversion instructions, are
+// the same and 0.05 to 0.2 us slower: what counts is the number of instructions.)
 #pragma once
 #include "gemv_tma.cuh"
 
@@ -793,6 +798,16 @@ inline bool takes(uint32_t N, uint32_t K) {
     return K % PK == 0u && (K <= 2u * SLAB || (K <= MAX_K && (N + 15u) / 16u <= (uint32_t)sm_count()));
 }
 
+// Whether one row started early leaves half of its SMs to the next launch.  Beside a long stream that half is worth less than
+// eight more warps.  Early launches with eight and with sixteen warps, us, in chains of their own, and each with one of 2048 outputs
+// behind it, which has eight:
+//   24576 x 2048 (170 KiB of codes an SM) 7.5 and 7.2, 9.5 and 10.3    28672 x 2048 (194) 8.5 and 7.5, 10.4 and 10.5
+//   32768 x 2048 (226) 9.3 and 8.6, 11.2 and 10.9                      131072 x 2048 (908) 35.2 and 27.6, 36.8 and 29.7
+//   49152 x 1024 (170) 7.5 and 7.0, 9.2 and 9.4                        65536 x 1024 (226) 9.4 and 8.3, 11.0 and 10.5
+//   65536 x 512 (113) 5.3 and 5.4, 7.0 and 7.8                         131072 x 512 (226) 9.7 and 8.6, 11.4 and 10.7
+constexpr uint32_t SHARING_CODES = 192 * 1024;
+inline bool shares(uint32_t N, uint32_t K) { return (uint64_t)N * (K / 2u) <= (uint64_t)sm_count() * SHARING_CODES; }
+
 // One or two rows, of a K that is taken.
 template <class S>
 int launch_form(const void* q, const Args& a, cudaStream_t stream) {
@@ -819,7 +834,7 @@ inline int launch_rows(const void* q, const void* s, const void* b, const void* 
     const int rc = gemvtma::check_fuse(sh, 4, N, M, a.out_bf16 != 0u);
     if (rc) return rc;
     if (M == 2u) return launch_form<Shape<2, 16>>(q, a, stream);
-    return a.early && sh.pa.world <= 1 ? launch_form<Shape<1, 8>>(q, a, stream) : launch_form<Shape<1, 16>>(q, a, stream);
+    return a.early && sh.pa.world <= 1 && shares(N, K) ? launch_form<Shape<1, 8>>(q, a, stream) : launch_form<Shape<1, 16>>(q, a, stream);
 }
 
 }  // namespace gemvdigits

@@ -373,3 +373,19 @@ def test_outliers_whose_weights_are_zero(exponent, code, K):
     if code:
         wide = miori_b200.gemv4(q, s, b, x, group=64).double()
         assert float((got - want[:2]).norm()) < float((wide[:2] - want[:2]).norm())
+
+
+@pytest.mark.parametrize("K", [256, 1536, 2048])
+@pytest.mark.parametrize("more", [0, 1])
+def test_early_rows_about_the_length_at_which_they_stop_sharing_an_sm(K, more):
+    """192 KiB of codes an SM and one row of the tensor more: eight warps a CTA, sixteen beyond, the same bits."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    N = sms * 192 * 1024 // (K // 2) + more
+    q, s, b = synth.make_weight(N, K, 4, 64, seed=K, device=DEV)
+    x = synth.make_activation(2, K, seed=K, device=DEV)
+    both = miori_b200.gemv4(q, s, b, x, group=64)
+    want = x.double() @ _weights64(q, s, b, 4, 64).T
+    assert float((both - want).norm() / want.norm()) < 2.0 ** -24 * 4 * K ** 0.5  # a row's terms in order at worst, at random
+    for r in (0, 1):
+        assert torch.equal(miori_b200.gemv4(q, s, b, x[r:r + 1], group=64, flags=miori_b200.LAUNCH_PDL), both[r:r + 1])
+    assert miori_b200.lib.miori_device_error_poll() == 0
