@@ -97,10 +97,11 @@ int miori_stream_sync(void* stream);
  * weights in groups of 64) or 1..4 and 5..8 (others), 9..16, 17..32, nor on MIORI_LAUNCH_PDL.  Across
  * classes rows agree to fp32 rounding, not bit for bit, and so do a tensor's rows and the same rows of a
  * taller one (a shard and the whole): N, too, decides how a row is summed.  One and two rows of 4-bit
- * weights in groups of 64, K a multiple of 256 up to 2048 (up to 8192 while N is at most 16 times the number
- * of SMs), hold an activation to 2^-25 of the largest of its 64 and sum exactly what they hold; the others
- * hold it exactly down to 2^-28 of it, and their sums cut it off.  Requires K % group == 0, group in
- * {32,64}; q,s,b,x 16-byte aligned.  Only M rows of x are read and M rows of y written (the reference's
+ * weights in groups of 64, K a multiple of 256 up to 2048 (without a norm in front up to 8192 while N is
+ * at most 16 times the number of SMs), hold an activation to 2^-25 of the largest of its 64 and sum
+ * exactly what they hold; the others hold it exactly down to 2^-28 of it, and their sums cut it off.
+ * Requires K % group == 0, group in {32,64}; q,s,b,x 16-byte aligned.  Only M rows of x are read and M
+ * rows of y written (the reference's
  * gemv4_b always touches four, shaders/batch.metal:178-179). */
 int miori_gemv4(const void* q, const void* s, const void* b, const void* x, void* y,
                 uint32_t N, uint32_t K, uint32_t M, uint32_t group, uint32_t flags,
@@ -357,7 +358,7 @@ int miori_gemv4_post_norm_add(const void* q, const void* s, const void* b, const
  * round trip of its output (the fusion the reference planned, docs/MILESTONES.md:87): every CTA sums
  * the rows' squares for itself, then normalises while it stages.  Requires (K / group) % 8 == 0; other
  * shapes get MIORI_E_INVALID.  The result is the unfused pair's up to the fp32 order of the sum
- * of squares. */
+ * of squares and, beyond K = 2048, that of the products. */
 int miori_gemv4_rmsnorm(const void* q, const void* s, const void* b, const void* x, const void* gamma,
                         float eps, void* y, uint32_t N, uint32_t K, uint32_t M, uint32_t group,
                         uint32_t flags, void* stream);

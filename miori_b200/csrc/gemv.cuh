@@ -45,7 +45,7 @@ struct Batch {
                    uint32_t flags, cudaStream_t stream, Shard sh) {
         if constexpr (BITS == 4 && GROUP == 64) {
             // the class of one and two rows: exact integer sums (gemv_digits.cuh)
-            if (M <= 2u && gemvdigits::takes(N, K))
+            if (M <= 2u && gemvdigits::takes(N, K, sh.pre.gamma != nullptr))
                 return gemvdigits::launch_rows(q, s, b, x, y, N, K, M, flags, stream, sh);
         }
         uint32_t cls = class_of(M), kpar = 0;

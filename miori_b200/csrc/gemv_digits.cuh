@@ -49,6 +49,7 @@
 //   32768 x 512            6.55   3.45       7.15   4.25       6.80   4.21       7.43   4.64
 //   2048 x 4096            3.29   3.18       4.10   3.96       3.41   4.29       4.10   4.84
 //   2048 x 8192            4.63   4.46       5.60   5.33       4.89   6.09       5.60   6.85
+//   norm and 3072 x 2048   3.21   3.43       3.95   3.92       3.82   4.08       4.11   4.61
 //   a layer's four        16.8   13.6       20.4   17.2       17.4   17.6       20.6   19.8
 //   with neighbours, six  21.5   19.3       25.0   21.8       23.7   22.9       25.8   25.2
 //   nine launches         22.0   20.4       27.3   24.8       23.2   24.1       27.6   27.6
@@ -295,7 +296,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     constexpr bool HALVED = !RES && WARPS == 16u;   // two warps share a position's slabs
     static_assert(!RES || PAIRED || ROWS == 1, "a warp converts one row of a slab, or all rows of several");
     constexpr bool SHARDED_ = F == gemvtma::SHARDED, ARGMAX_ = F == gemvtma::ARGMAX, POSTNORM_ = F == gemvtma::POSTNORM;
-    const bool gated = F == gemvtma::FUSED && A.gated != 0u, normed = F == gemvtma::FUSED && A.pre.gamma != nullptr;
+    const bool gated = F == gemvtma::FUSED && A.gated != 0u, normed = F == gemvtma::FUSED && RES && A.pre.gamma != nullptr;
     const uint32_t N = A.N, K = A.K, stages = A.stages;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t tiles = (N + 15u) >> 4, row_bytes = K / 2u, ng = K / GROUP;
@@ -506,8 +507,8 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 
     // warps that share a position have pieces if the first of them has
     const uint32_t work = !PAIRED ? pieces : my_tiles > (tg & ~1u) ? slabs : 0u;
-    uint4 gm = make_uint4(0u, 0u, 0u, 0u);  // RES: norm weights of this lane's activations
-    if (RES && normed && work && (pos * 32u + lane) * 8u < K) gm = __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + pos * 32u + lane);
+    uint4 gm = make_uint4(0u, 0u, 0u, 0u);  // norm weights of this lane's activations
+    if (normed && work && (pos * 32u + lane) * 8u < K) gm = __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + pos * 32u + lane);
     pdl_wait_prior();  // x (and y) belong to the predecessor until here
 
     // A CTA without rows keeps its place until the next launch has taken its own: at the head of a chain it would be gone
@@ -516,8 +517,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         while (clock64() - born < LINGER_CYCLES) __nanosleep(100);
 
     // ---- the activations of this warp's position: one unit of every row and slab a lane
-    constexpr uint32_t NPART = RES ? WARPS : 16u;
-    __shared__ float nm_part[ROWS][NPART], nm_inv[ROWS];
+    __shared__ float nm_part[ROWS][WARPS], nm_inv[ROWS];
     constexpr uint32_t CR = PAIRED ? 1u : ROWS;                // rows that this warp converts, from row cr on
     const uint32_t cr = PAIRED && ROWS > 1 ? tg & 1u : 0u;
     const bool converts = !PAIRED || ROWS > 1 || (tg & 1u) == 0u;
@@ -531,56 +531,32 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             sl = CR > 1u && r >= slabs ? r - slabs : r;
             return ((s0 + sl) * 8u + pos) * 32u + lane;
         };
-        // normed: the squares first (every unit once: of the first warps of a position), warps in order.  One slab's stay in
-        // registers, more are read again (from L2)
+        // normed (one slab): the squares first (every unit once: of the first warps of a position), warps in order
         float4 xa4, xc4;
-        float inv[CR];
+        float inv = 0.0f;
         if (normed) {
             const float4* x4 = reinterpret_cast<const float4*>(A.x);
-            auto squares = [](const float4& a, const float4& c, float ss) {
-                ss = __fmaf_rn(a.x, a.x, ss), ss = __fmaf_rn(a.y, a.y, ss), ss = __fmaf_rn(a.z, a.z, ss), ss = __fmaf_rn(a.w, a.w, ss);
-                ss = __fmaf_rn(c.x, c.x, ss), ss = __fmaf_rn(c.y, c.y, ss), ss = __fmaf_rn(c.z, c.z, ss);
-                return __fmaf_rn(c.w, c.w, ss);
-            };
-            auto warp_sum = [&](float ss) {
+            const uint32_t u = pos * 32u + lane;
+            xa4 = xc4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (sets && u < upr) xa4 = ld_fresh(x4 + (cr * upr + u) * 2u), xc4 = ld_fresh(x4 + (cr * upr + u) * 2u + 1u);
+            first_piece();
+            float ss = 0.0f;
+            ss = __fmaf_rn(xa4.x, xa4.x, ss), ss = __fmaf_rn(xa4.y, xa4.y, ss), ss = __fmaf_rn(xa4.z, xa4.z, ss), ss = __fmaf_rn(xa4.w, xa4.w, ss);
+            ss = __fmaf_rn(xc4.x, xc4.x, ss), ss = __fmaf_rn(xc4.y, xc4.y, ss), ss = __fmaf_rn(xc4.z, xc4.z, ss), ss = __fmaf_rn(xc4.w, xc4.w, ss);
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-                return ss;
-            };
-            if constexpr (RES) {
-                const uint32_t u = pos * 32u + lane;
-                xa4 = xc4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (sets && u < upr) xa4 = ld_fresh(x4 + (cr * upr + u) * 2u), xc4 = ld_fresh(x4 + (cr * upr + u) * 2u + 1u);
-                first_piece();
-                const float ss = warp_sum(squares(xa4, xc4, 0.0f));
-                if (lane == 0) {
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+            if (lane == 0) {
 #pragma unroll
-                    for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) nm_part[m][warp] = converts && m == cr && tg == cr ? ss : 0.0f;
-                }
-            } else {
-                for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) {
-#pragma unroll 1
-                    for (uint32_t h = 0; h < (HALVED ? 1u : 2u); ++h) {
-                        float ss = 0.0f;
-                        for (uint32_t s = h * half; s < (HALVED || h ? slabs : min(slabs, half)); ++s) {
-                            const uint32_t u = ((s0 + s) * 8u + pos) * 32u + lane;
-                            if (u < upr) ss = squares(ld_fresh(x4 + ((size_t)m * upr + u) * 2u), ld_fresh(x4 + ((size_t)m * upr + u) * 2u + 1u), ss);
-                        }
-                        ss = warp_sum(ss);
-                        if (lane == 0) nm_part[m][warp + 8u * h] = ss;
-                    }
-                }
-                first_piece();
+                for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) nm_part[m][warp] = converts && m == cr && tg == cr ? ss : 0.0f;
             }
             __syncthreads();
 #pragma unroll
             for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) {
                 float tot = 0.0f;
 #pragma unroll
-                for (uint32_t w = 0; w < NPART; ++w) tot += nm_part[m][w];
+                for (uint32_t w = 0; w < WARPS; ++w) tot += nm_part[m][w];
                 const float in = rsqrtf(tot / (float)K + A.pre.eps);
-                if (CR > 1u) inv[m % CR] = in;
-                else if (m == cr) inv[0] = in;
+                if (m == cr) inv = in;
                 if (threadIdx.x == 0) nm_inv[m] = in;
             }
         }
@@ -590,15 +566,8 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
             if (r < sets && u < upr) {
                 const size_t i = (size_t)m * upr + u;
-                if (RES && normed) {
-                    v = gemvtma::normed8(xa4, xc4, inv[0], gm);
-                } else if (normed) {
-                    const float4* x4 = reinterpret_cast<const float4*>(A.x) + 2u * i;
-                    v = gemvtma::normed8(ld_fresh(x4), ld_fresh(x4 + 1), CR == 1u || m == 0u ? inv[0] : inv[CR - 1u],
-                                         __ldg(reinterpret_cast<const uint4*>(A.pre.gamma) + u));
-                } else {
-                    v = ld_fresh(reinterpret_cast<const uint4*>(A.x) + i);
-                }
+                if (normed) v = gemvtma::normed8(xa4, xc4, inv, gm);
+                else v = ld_fresh(reinterpret_cast<const uint4*>(A.x) + i);
             }
             return v;
         };
@@ -794,8 +763,10 @@ int launch_k(const void* q, const Args& a, cudaStream_t stream) {
 // early launches start beside (with this product in gemv_tma.cuh the four projections of a layer take 15.9 us at one row, 13.5
 // with it here); with more, the conversion of x and the pieces take longer than there (8192 x 8192 at one row 11.5 us,
 // 10.1).  So there the kernel, and with it a row's rounding, depends on N, as the order of its sums in gemv_tma.cuh does.
-inline bool takes(uint32_t N, uint32_t K) {
-    return K % PK == 0u && (K <= 2u * SLAB || (K <= MAX_K && (N + 15u) / 16u <= (uint32_t)sm_count()));
+// Never with the norm in front: the squares are a trip to L2 of their own there (norm and 2048 x 4096 at one row and at two
+// 5.2 and 6.1 us, 3.7 and 4.5 there; 2048 x 8192 8.0 and 9.2, 6.5 and 7.8).
+inline bool takes(uint32_t N, uint32_t K, bool normed) {
+    return K % PK == 0u && (K <= 2u * SLAB || (!normed && K <= MAX_K && (N + 15u) / 16u <= (uint32_t)sm_count()));
 }
 
 // Whether one row started early leaves half of its SMs to the next launch.  Beside a long stream that half is worth less than
