@@ -683,18 +683,18 @@ def main():
 
     peaks, peak_kind = measured_peaks()
     m1 = per_m["1"]
-    # DRAM bytes (read + write) per algorithmic byte of gemv_tma_kernel, from an ncu capture of
-    # the N=8192, K=2048, M=1 launch over a pool larger than L2 (9.486 MB read, nothing written --
-    # the 32 KB of y stay in L2 -- for 9.437 MB of weights); traffic grows in proportion to the
-    # weights a launch streams
+    # DRAM bytes (read + write) per algorithmic byte of gemv_digits_kernel, from ncu captures of early
+    # one-row launches over pools larger than L2 (N=8192, K=2048 9.476 MB and N=2048, K=8192 9.495 MB
+    # read, nothing written -- y stays in L2 -- for 9.437 MB of weights); traffic grows in proportion
+    # to the weights a launch streams (another kernel runs groups of 32: not captured)
     DRAM_PER_ALGO_BYTE = 1.005
     roofline = {
-        "kernel": "gemv_tma_kernel, one row of 4-bit weights (M=1 pass of the stack, 96 launches per pass)",
+        "kernel": ("gemv_digits_kernel" if G == 64 else "gemv_tma_kernel") + ", one row of 4-bit weights (M=1 pass of the stack, 96 launches per pass)",
         "bound": "hbm", "achieved": m1["gbs"] / world, "peak": peaks["hbm_gbs"], "unit": "GB/s",
         "frac": m1["gbs"] / world / peaks["hbm_gbs"], "peak_kind": peak_kind,
         "bytes_per_launch": bytes_pass / launches_pass / world,
         "us_per_launch": m1["us_per_launch"],
-        "traffic": DRAM_PER_ALGO_BYTE * bytes_pass / launches_pass / world,
+        "traffic": DRAM_PER_ALGO_BYTE * bytes_pass / launches_pass / world if G == 64 else None,
     }
     out = {
         "metric": METRIC, "value": value, "unit": "GB/s",
@@ -933,7 +933,7 @@ def extras(torch, miori_b200, synth, dev, G, peaks, timed):
     by = packed_bytes(N, K, 4, G)
     ex["stream_gemv4_m1_n131072_k2048"] = {"us": 1e3 * ms, "gbs": by / (ms * 1e-3) / 1e9,
                                            "frac_of_hbm_peak": by / (ms * 1e-3) / 1e9 / peaks["hbm_gbs"],
-                                           "kernel": "gemv_tma_kernel, one activation row"}
+                                           "kernel": ("gemv_digits_kernel" if G == 64 else "gemv_tma_kernel") + ", one activation row"}
     del big
     # RMSNorm in front of a projection: norm kernel + GEMV against the GEMV with the norm fused into
     # its activation staging, M=1, one layer's four shapes over pools of distinct weights (> L2)

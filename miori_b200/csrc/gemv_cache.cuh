@@ -6,7 +6,7 @@
 // projection of 2048 outputs, splits K over a cluster to fill the SMs, and pays TMEM allocation, a
 // pipeline fill and the exchange: 5.3 us where the cache streams in 1.3.  Here the cache is
 // streamed once in 16-row tiles, exactly like the packed weights of the decode GEMV -- 128 of
-// them, 3.1-4.2 us -- with no unpack at all: 16 bytes of a cache row ARE an A
+// them, 3.1-5.0 us -- with no unpack at all: 16 bytes of a cache row ARE an A
 // fragment of mma.sync.m16n8k16 (under the fixed k permutation "slot 2t, 2t+1, 2t+8, 2t+9 of lane
 // t = elements 8t .. 8t+3"), and the same 16 bytes of an activation row are the matching B
 // fragment, so x needs no permutation either.
@@ -21,7 +21,8 @@
 //     fragments are therefore the same for all tiles and live in REGISTERS: after the wait every
 //     lane loads its 16 bytes of x per (k-slab, 32-k step) straight from global memory, once -- at
 //     most 16 of them, 64 registers -- and x never touches shared memory, which is left to the
-//     ring (eight stages, 139 KB in flight per SM);
+//     ring (eight stages, 139 KB in flight per SM).  That is up to 128 KB an SM, some 1 us (8192 -> 2048 at 8 rows 8.5 us),
+//     and cannot start before the wait: the launch before writes x;
 //   * per stage and 32-k step a warp issues two 16-byte loads (the tile's rows g and g + 8) and two
 //     MMAs; after the last slab of a tile the 16 / NT warps that share a set add their 16 x 8
 //     partial sums through shared memory in a fixed order, so a row's value depends neither on M

@@ -26,8 +26,8 @@
 // ones.  Measured in chains of dependent launches over weights larger than L2, with codes as bf16 128 + code
 // and one producer, and now, us: 8-bit head 131072 x 2048 at 1, 4, 16 rows 53.1, 60.3, 93 -> 42.7
 // (6.7 TB/s, what a plain copy does), 44.2, 72.5; 4-bit 16384 x 2048 at 1, 4, 8 rows 7.44, 8.80, 10.2 ->
-// 6.56, 7.19, 7.72; 2048 x 8192 at 1, 4 rows 6.58, 9.56 -> 4.63, 6.27.  2048 x 2048 at 1 row is no faster: 2.68
-// and 2.76 (2.71 with less exact sums, see above).
+// 6.67, 7.28, 7.94; 2048 x 8192 at 1, 4 rows 6.58, 9.56 -> 4.63, 6.31.  2048 x 2048 at 1 row is no faster: 2.68
+// and 2.70.
 //
 // One CTA per SM owns every gridDim-th 16-row tile.  A slab -- 16 rows x up to 1 KiB of codes -- is one
 // 2-D TMA copy into a shared-memory ring; a tile's scales and biases (contiguous in memory) are two

@@ -163,20 +163,21 @@ MIORI_API int miori_gemv_bf16_cache(const void* x, const void* cache, void* y, u
 // Where miori_linear4 sends a projection: 0 = packed-weight GEMV, 1 = narrow-batch kernel on the
 // bf16 cache, 2 = tcgen05 GEMM on the bf16 cache.  Measured on B200 in chains of dependent
 // launches (group 64; us per launch, 2048 -> 3072 / 2048 -> 2048 / 8192 -> 2048 / 2048 -> 16384):
-//   M = 5:  packed 3.4 / 3.0 / 6.9 / 7.4,    narrow 3.8 / 3.0 / 7.2 / 11.2,  GEMM 5.8 / 5.3 / 9.6 / 12.9
-//   M = 8:  packed 3.7 / 3.2 / 8.3 / 7.8,    narrow 4.1 / 3.1 / 7.2 / 11.4,  GEMM 5.8 / 5.4 / 9.6 / 12.9
-//   M = 9:  packed 4.8 / 4.2 / 12.7 / 10.2,  narrow 4.2 / 3.2 / 8.3 / 11.5,  GEMM 5.9 / 5.3 / 9.6 / 13.0
-//   M = 16: packed 5.6 / 5.0 / 16.2 / 10.7,  narrow 4.4 / 3.3 / 9.1 / 11.7,  GEMM 5.9 / 5.3 / 9.6 / 13.1
-//   M = 17: packed 7.3 / 6.5 / 20.9 / 15.2,  narrow 5.2 / 3.9 / 13.1 / 16.4, GEMM 6.3 / 5.4 / 9.7 / 13.6
-//   M = 32: packed 9.4 / 8.4 / 32.3 / 21.2,  narrow 5.7 / 4.2 / 14.6 / 16.8, GEMM 6.5 / 5.3 / 9.7 / 14.0
-// (the packed GEMV at group 32: 0.2-0.4 more at K = 2048, up to 4 more at 8192.)
+//   M = 5:  packed 3.3 / 3.0 / 6.9 / 7.4,    narrow 4.0 / 3.1 / 8.0 / 12.1,  GEMM 5.9 / 5.3 / 10.0 / 13.7
+//   M = 8:  packed 3.7 / 3.2 / 8.3 / 8.0,    narrow 4.1 / 3.1 / 8.5 / 12.1,  GEMM 5.9 / 5.4 / 10.0 / 13.8
+//   M = 9:  packed 4.8 / 4.2 / 12.9 / 10.2,  narrow 4.4 / 3.3 / 8.5 / 12.5,  GEMM 5.9 / 5.3 / 10.0 / 13.7
+//   M = 16: packed 5.5 / 5.0 / 16.3 / 10.7,  narrow 4.7 / 3.6 / 9.0 / 12.9,  GEMM 6.0 / 5.3 / 10.0 / 14.1
+//   M = 17: packed 7.3 / 6.5 / 20.9 / 15.2,  narrow 5.7 / 4.3 / 12.9 / 17.7, GEMM 6.4 / 5.3 / 10.0 / 14.4
+//   M = 32: packed 9.4 / 8.4 / 32.3 / 21.3,  narrow 6.4 / 5.0 / 14.7 / 18.6, GEMM 6.6 / 5.3 / 10.2 / 14.6
+// (the packed GEMV at group 32: 0.1-0.5 more at K = 2048 and 3072 outputs, 1.3-2.9 at 16384, up to 4 at 8192.)
 // Up to four rows stay on the packed weights with fp32 dequantization, as in the reference
 // (src/batch.cpp:223-230 cuts over to the cache above four rows).  Above that the cache is used
 // when given: by the narrow-batch kernel while the projection is short (at most two 16-row tiles
 // per SM: its launch is cheap, but it streams four times the bytes and its mma.sync rate caps it
 // on long streams) and for 9..16 rows of any width, else by the packed GEMV up to 8 rows, else by
-// the tensor-core GEMM.  By time alone the packed GEMV would also take 2048 -> 3072 up to 8 rows (0.4 us) and
-// 2048 -> 16384 up to 16 (1.0-1.3 us); a caller who gives a cache gets its rounding of the weights there.
+// the tensor-core GEMM.  By time alone the packed GEMV would also take 2048 -> 3072 (0.4-0.7 us) and
+// 8192 -> 2048 (0.2-1.1) up to 8 rows and 2048 -> 16384 up to 16 (2.2); a caller who gives a cache gets its rounding of the
+// weights there.
 static int linear4_route(uint32_t M, uint32_t N, uint32_t K, bool has_cache) {
     if (M <= 4 || !has_cache) return 0;
     const uint32_t tiles = (N + 15u) / 16u, slabs = (K + 511u) / 512u;
@@ -187,7 +188,7 @@ static int linear4_route(uint32_t M, uint32_t N, uint32_t K, bool has_cache) {
         // activations resident in registers: short projections, and 9..16 rows of any width
         if (frags <= (uint32_t)gemvcache::MAX_FRAGS && (short_proj || nt == 2u)) return 1;
         // activations streamed per tile (long rows): pays up to 16 rows on short projections
-        // (8192 -> 2048 at 16 rows: 9.1 us against 9.6 us for the GEMM; at 17 rows 13.1 against 9.7)
+        // (8192 -> 2048 at 16 rows: 9.0 us against 10.0 us for the GEMM; at 17 rows 12.9 against 10.0)
         if (frags > (uint32_t)gemvcache::MAX_FRAGS && short_proj && nt == 2u) return 1;
     }
     if (M <= 8) return 0;
