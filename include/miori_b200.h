@@ -40,9 +40,10 @@ extern "C" {
 #define MIORI_OUT_F32 0u       /* y / C written as fp32 (what the reference's kernels write) */
 #define MIORI_OUT_BF16 1u      /* y / C rounded to bf16 (RNE) in the epilogue */
 #define MIORI_LAUNCH_PDL 2u    /* programmatic dependent launch: the kernel may start while its
-                                  predecessor on the stream drains; it prefetches weights (which
-                                  must be immutable while in flight) and waits for the
-                                  predecessor before touching x / A or writing y / C */
+                                  predecessor on the stream drains; it prefetches weights (a
+                                  norm's among them), which must be immutable while in flight,
+                                  and waits for the predecessor before touching x / A or
+                                  writing y / C */
 #define MIORI_GEMV_EXACT 4u    /* fp32 dequantization for every M (what every launch does) */
 const char* miori_last_error(void);
 /* Library version string, e.g. "miori_b200 0.1 sm_100a". */
