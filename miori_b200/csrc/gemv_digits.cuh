@@ -34,25 +34,26 @@
 //     its predecessor fetches x, whose loads would queue up behind them (four projections of a layer 5 % slower when all are
 //     fetched at once);
 //   * two rows, longer launches, launches that wait for the one before or go over several GPUs: SIXTEEN warps and one CTA to
-//     an SM.  Two warps share a position: each converts one row of two, or half the slabs.  All pieces but the first are
-//     fetched behind x (16384 x 2048 at one row 7.0 us when all are fetched ahead, 6.3 with two first ones, 5.7 with one; none
-//     5.9).  Beside launches that keep to neither rule -- norms, activations, other products -- it is the steadier one: with
-//     eight warps a layer's four projections that wait took 24.8 us, 17.2 so, and nine launches of a layer at two rows 28.8
-//     and 24.1.
+//     an SM.  Two warps share a position: each converts one row of two, or half the slabs, and beyond one slab only the first
+//     multiplies, slabs in order, as with eight warps (with half of them for each warp 2048 x 8192 that waits took 5.3 and
+//     6.9 us at one and at two rows, 5.1 and 6.3 so).  All pieces but the first are fetched behind x (16384 x 2048 at one row
+//     7.0 us when all are fetched ahead, 6.3 with two first ones, 5.7 with one; none 5.9).  Beside launches that keep to
+//     neither rule -- norms, activations, other products -- it is the steadier one: with eight warps a layer's four projections
+//     that wait took 24.8 us, 16.9 so, and nine launches of a layer at two rows 28.8 and 22.8.
 //
 // Measured in chains over weights larger than L2, the kernel of gemv_tma.cuh and this one in turns, us:
 //                          one row early     one that waits    two rows early    two that wait
-//   2048 x 2048            2.70   2.05       3.41   2.89       2.71   2.83       3.43   3.08
-//   3072 x 2048            2.96   2.41       3.75   3.28       2.93   3.09       3.80   3.69
-//   16384 x 2048           6.67   5.04       7.70   5.71       7.05   5.66       7.83   6.30
+//   2048 x 2048            2.70   2.04       3.41   2.89       2.71   2.79       3.43   3.06
+//   3072 x 2048            2.96   2.38       3.75   3.30       2.93   3.07       3.80   3.64
+//   16384 x 2048           6.67   5.05       7.70   5.77       7.05   5.75       7.83   6.27
 //   131072 x 2048         32.1   27.6       32.2   27.8       34.5   30.2       34.9   30.5
-//   32768 x 512            6.55   3.45       7.15   4.25       6.80   4.21       7.43   4.64
-//   2048 x 4096            3.29   3.18       4.10   3.96       3.41   4.29       4.10   4.84
-//   2048 x 8192            4.63   4.46       5.60   5.33       4.89   6.09       5.60   6.85
+//   32768 x 512            6.55   3.42       7.15   4.26       6.80   4.26       7.43   4.65
+//   2048 x 4096            3.29   3.07       4.10   3.72       3.41   3.91       4.10   4.22
+//   2048 x 8192            4.63   4.30       5.60   5.07       4.89   5.75       5.60   6.28
 //   norm and 3072 x 2048   3.21   3.43       3.95   3.92       3.82   4.08       4.11   4.61
-//   a layer's four        16.8   13.6       20.4   17.2       17.4   17.6       20.6   19.8
-//   with neighbours, six  21.5   19.3       25.0   21.8       23.7   22.9       25.8   25.2
-//   nine launches         22.0   20.4       27.3   24.8       23.2   24.1       27.6   27.6
+//   a layer's four        16.8   13.4       20.4   16.9       17.4   17.3       20.6   19.1
+//   with neighbours, six  21.5   19.0       25.0   21.4       23.7   22.3       25.8   24.4
+//   nine launches         22.0   19.5       27.3   24.4       23.2   22.8       27.6   26.8
 // Two rows that start early are behind up to some 4000 outputs, and all beyond one slab: converting a row takes 2.2 times the
 // instructions of fp16's and is most of the time there.  They run here all the same: a row has the same bits alone and beside
 // another, and one row gains.  (Digits from two additions of a power of two, which leave out the conversion instructions, are
@@ -106,30 +107,29 @@ struct Args {
     PeerArgs pa;
 };
 
-// How a row's slabs are dealt: beyond one slab, sixteen warps are two for each position, one for the slabs below HALF and one
-// for the others; eight warps sum the two parts apart, so that both kernels add in the same order.
 __host__ __device__ inline uint32_t slabs_of(uint32_t K) { return (K / 2u + SLAB - 1u) / SLAB; }
-__host__ __device__ inline uint32_t half_of(uint32_t nslab) { return (nslab + 1u) >> 1; }
+// Warps with a ring: beyond one slab a CTA has one tile, and the second warps of the positions only convert.
+template <class S>
+__host__ __device__ inline uint32_t rings_of(uint32_t nslab) { return nslab > 1u ? 8u : (uint32_t)S::W; }
 
 // Dynamic shared memory, from a 1024-byte aligned base.
 struct Layout {
-    uint32_t pitch, slabs, sc, x, ms, zeros, part, total;
+    uint32_t pitch, sc, x, ms, zeros, part, total;
 };
 constexpr uint32_t SC_ROW = 4u * NG, SC_BYTES = 16u * SC_ROW;  // scales and biases of a row of a piece, and of a piece
 template <class S>
 __host__ __device__ inline Layout layout(uint32_t K, uint32_t stages, uint32_t parts) {
     Layout L;
     const uint32_t nslab = slabs_of(K);
-    L.slabs = S::W == 16 ? half_of(nslab) : nslab;                           // of a warp
-    const uint32_t regions = S::W == 16 && nslab == 1u ? 8u : (uint32_t)S::W;  // of activations: one slab's are shared by two warps
-    L.pitch = L.slabs * PK + XPAD;  // of a digit plane
-    uint32_t at = S::W * stages * PIECE_BYTES;
+    const uint32_t rings = rings_of<S>(nslab);
+    L.pitch = nslab * PK + XPAD;  // of a digit plane
+    uint32_t at = rings * stages * PIECE_BYTES;
     L.sc = at;
-    at += S::W * stages * SC_BYTES;
+    at += rings * stages * SC_BYTES;
     L.x = at;
-    at += regions * S::ROWS * 4u * L.pitch;
+    at += 8u * S::ROWS * 4u * L.pitch;  // of eight warps, or of eight pairs of them
     L.ms = at;
-    at += regions * L.slabs * NG * S::ROWS * 16u;
+    at += 8u * nslab * NG * S::ROWS * 16u;
     L.zeros = at;
     at += S::W * 16u;
     L.part = at;
@@ -292,23 +292,19 @@ __global__ void __launch_bounds__(S::THREADS, S::SHARING ? 2 : 1)
 gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ Args A) {
     constexpr int ROWS = S::ROWS, CH = S::CH, NU = S::NU, GS = S::GS;
     constexpr uint32_t WARPS = S::W;
-    constexpr bool PAIRED = RES && WARPS == 16u;    // two warps share a position's activations: each converts one row of two
-    constexpr bool HALVED = !RES && WARPS == 16u;   // two warps share a position's slabs
-    static_assert(!RES || PAIRED || ROWS == 1, "a warp converts one row of a slab, or all rows of several");
+    constexpr bool PAIRED = WARPS == 16u;  // two warps share a position's activations: each converts one row of two, or half the slabs
+    static_assert(PAIRED || ROWS == 1, "a warp converts one row");
     constexpr bool SHARDED_ = F == gemvtma::SHARDED, ARGMAX_ = F == gemvtma::ARGMAX, POSTNORM_ = F == gemvtma::POSTNORM;
     const bool gated = F == gemvtma::FUSED && A.gated != 0u, normed = F == gemvtma::FUSED && RES && A.pre.gamma != nullptr;
     const uint32_t N = A.N, K = A.K, stages = A.stages;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t tiles = (N + 15u) >> 4, row_bytes = K / 2u, ng = K / GROUP;
-    const uint32_t full_slabs = row_bytes / SLAB, rest = row_bytes % SLAB, half = half_of(slabs_of(K));
+    const uint32_t full_slabs = row_bytes / SLAB, rest = row_bytes % SLAB, nslab = slabs_of(K);
     // short rows have fewer positions, and the warps of a position share the tiles
     const uint32_t P = full_slabs ? 8u : (rest + PIECE - 1u) / PIECE;
-    const uint32_t pshift = P > 4u ? 3u : P > 2u ? 2u : P - 1u, TG = HALVED ? 1u : WARPS >> pshift;
-    const uint32_t pos = warp & ((1u << pshift) - 1u), tg = HALVED ? 0u : warp >> pshift;
-    auto slabs_at = [&](uint32_t p) { return full_slabs + (p * PIECE < rest ? 1u : 0u); };
-    const uint32_t s0 = HALVED && warp >= 8u ? half : 0u;  // this warp's slabs of its position
-    const uint32_t slabs = HALVED ? (warp >= 8u ? max(slabs_at(pos), half) - half : min(slabs_at(pos), half)) : slabs_at(pos);
-    const uint32_t slots = pshift + (HALVED ? 1u : 0u);    // log2 of a tile's partial sums
+    const uint32_t pshift = P > 4u ? 3u : P > 2u ? 2u : P - 1u, TG = WARPS >> pshift;
+    const uint32_t pos = warp & ((1u << pshift) - 1u), tg = warp >> pshift;
+    const uint32_t slabs = full_slabs + (pos * PIECE < rest ? 1u : 0u);
 
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bars[WARPS * MAX_STAGES];
@@ -323,7 +319,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     const uint32_t batch = TG * S::BATCH;
     const uint32_t wt = my_tiles > tg ? (my_tiles - tg + TG - 1u) / TG : 0u;  // tiles of this warp
     const uint32_t pieces = wt * slabs;
-    const Layout L = layout<S>(K, stages, (my_tiles > batch ? 2u * batch : my_tiles) << slots);
+    const Layout L = layout<S>(K, stages, (my_tiles > batch ? 2u * batch : my_tiles) << pshift);
     const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
     const uint32_t ring = base + warp * stages * PIECE_BYTES, bar0 = smem_addr(&bars[warp * MAX_STAGES]);
     const uint32_t sc_ring = base + L.sc + warp * stages * SC_BYTES;
@@ -333,8 +329,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     auto row_of = [&](uint32_t tile, uint32_t r) {
         return gated ? tile * 8u + (r & 7u) + (r >= 8u ? N >> 1 : 0u) : min(tile * 16u + r, N - 1u);
     };
-    const uint32_t ic_first = pos * (PIECE / 8u) + s0 * (SLAB / 8u), ic_end = ic_first + slabs * (SLAB / 8u);
-    const uint32_t ie_first = pos * NG + s0 * (8u * NG);
+    const uint32_t ic_first = pos * (PIECE / 8u), ic_end = ic_first + slabs * (SLAB / 8u), ie_first = pos * NG;
     uint32_t issued = 0, itile = tile_of(tg), ic0 = ic_first;
     const uint16_t* const sc_src = lane < 16u ? A.s : A.b;
     size_t ie = (size_t)row_of(itile, lane & 15u) * ng + ie_first;
@@ -393,7 +388,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     const uint32_t g = lane >> 2, t = lane & 3u;
     const uint32_t prow = ROWS == 1 ? ((g & 1u) << 2) | (g >> 1) : ((g & 3u) << 1) | (g >> 2);
     const uint32_t region = PAIRED ? ((tg >> 1) << pshift) + pos : warp;
-    const uint32_t xw = base + L.x + region * ROWS * 4u * L.pitch, msw = base + L.ms + region * L.slabs * (NG * ROWS * 16u);
+    const uint32_t xw = base + L.x + region * ROWS * 4u * L.pitch, msw = base + L.ms + region * nslab * (NG * ROWS * 16u);
     const bool mine = ROWS > 1 || (g >> 2) == (t >> 1);  // one row: the codes of this lane belong to its column's group
     const uint32_t xb = mine ? xw + ((ROWS == 1 ? 0u : g >> 2) * 4u + (g & 3u)) * L.pitch + t * (uint32_t)(NU * 8)
                              : base + L.zeros + 16u * warp;
@@ -518,19 +513,12 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 
     // ---- the activations of this warp's position: one unit of every row and slab a lane
     __shared__ float nm_part[ROWS][WARPS], nm_inv[ROWS];
-    constexpr uint32_t CR = PAIRED ? 1u : ROWS;                // rows that this warp converts, from row cr on
-    const uint32_t cr = PAIRED && ROWS > 1 ? tg & 1u : 0u;
-    const bool converts = !PAIRED || ROWS > 1 || (tg & 1u) == 0u;
-    uint32_t top[ROWS];
-#pragma unroll
-    for (int m = 0; m < ROWS; ++m) top[m] = 0u;
+    const uint32_t cr = ROWS > 1 ? tg & 1u : 0u;             // the row that this warp converts, and its slabs c0 .. c0 + sets - 1
+    const uint32_t below = PAIRED && ROWS == 1 ? (slabs + 1u) >> 1 : slabs;
+    const uint32_t c0 = PAIRED && ROWS == 1 && (tg & 1u) ? below : 0u, sets = c0 ? slabs - below : below;
+    uint32_t top = 0u;
     if (my_tiles && (work || normed)) {
-        const uint32_t upr = K >> 3, sets = converts ? CR * slabs : 0u;
-        auto place = [&](uint32_t r, uint32_t& m, uint32_t& sl) {
-            m = CR > 1u && r >= slabs ? 1u : cr;
-            sl = CR > 1u && r >= slabs ? r - slabs : r;
-            return ((s0 + sl) * 8u + pos) * 32u + lane;
-        };
+        const uint32_t upr = K >> 3;
         // normed (one slab): the squares first (every unit once: of the first warps of a position), warps in order
         float4 xa4, xc4;
         float inv = 0.0f;
@@ -547,7 +535,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
             if (lane == 0) {
 #pragma unroll
-                for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) nm_part[m][warp] = converts && m == cr && tg == cr ? ss : 0.0f;
+                for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) nm_part[m][warp] = m == cr && tg == cr ? ss : 0.0f;
             }
             __syncthreads();
 #pragma unroll
@@ -561,57 +549,41 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
         }
         auto load = [&](uint32_t r) {
-            uint32_t m, sl;
-            const uint32_t u = place(r, m, sl);
+            const uint32_t u = ((c0 + r) * 8u + pos) * 32u + lane;
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
             if (r < sets && u < upr) {
-                const size_t i = (size_t)m * upr + u;
                 if (normed) v = gemvtma::normed8(xa4, xc4, inv, gm);
-                else v = ld_fresh(reinterpret_cast<const uint4*>(A.x) + i);
+                else v = ld_fresh(reinterpret_cast<const uint4*>(A.x) + (size_t)cr * upr + u);
             }
             return v;
         };
         auto stage = [&](uint32_t r, const uint4& v) {
-            uint32_t m, sl;
-            place(r, m, sl);
-            return stage_unit(v, r < sets, xw + m * 4u * L.pitch + sl * PK + lane * 8u, L.pitch, (lane & 7u) == 0u,
-                              msw + ((sl * NG + (lane >> 3)) * ROWS + m) * 16u);
+            return stage_unit(v, r < sets, xw + cr * 4u * L.pitch + (c0 + r) * PK + lane * 8u, L.pitch, (lane & 7u) == 0u,
+                              msw + (((c0 + r) * NG + (lane >> 3)) * ROWS + cr) * 16u);
         };
         if constexpr (RES) {
             const uint4 v = load(0u);
             if (!normed) first_piece();
-            if (converts) {
-                const uint32_t t0 = stage(0u, v);
-#pragma unroll
-                for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) top[m] = m == cr ? t0 : 0u;
-            }
-        } else {  // AHEAD loads in flight, PAIR units at a time (more would be straight code, which costs its fetches)
+            if (sets) top = stage(0u, v);
+        } else {  // AHEAD loads in flight (all of them), PAIR units at a time (more would be straight code, which costs its fetches)
             constexpr int AHEAD = 4, PAIR = 2;
+            static_assert(MAX_K <= AHEAD * 2u * SLAB, "a slab of the row for each");
             uint4 v[AHEAD];
 #pragma unroll
             for (int h = 0; h < AHEAD; ++h) v[h] = load((uint32_t)h);
-            if (!normed) first_piece();
+            first_piece();
 #pragma unroll 1
             for (uint32_t r = 0; r < sets; r += PAIR) {
-                uint4 w[PAIR];
-#pragma unroll
-                for (int h = 0; h < PAIR; ++h) w[h] = load(r + (uint32_t)(AHEAD + h));
-                const uint32_t t0 = stage(r, v[0]), t1 = stage(r + 1u, v[1]);
-                if (ROWS == 1 || r < slabs) top[0] = max(top[0], t0);
-                else top[ROWS - 1] = max(top[ROWS - 1], t0);
-                if (ROWS == 1 || r + 1u < slabs) top[0] = max(top[0], t1);
-                else top[ROWS - 1] = max(top[ROWS - 1], t1);
+                top = max(top, max(stage(r, v[0]), stage(r + 1u, v[1])));
 #pragma unroll
                 for (int h = 0; h + PAIR < AHEAD; ++h) v[h] = v[h + PAIR];
-#pragma unroll
-                for (int h = 0; h < PAIR; ++h) v[AHEAD - PAIR + h] = w[h];
             }
         }
     }
+    top = __reduce_max_sync(0xFFFFFFFFu, top);
+    if (lane == 0) {
 #pragma unroll
-    for (int m = 0; m < ROWS; ++m) {
-        const uint32_t all = __reduce_max_sync(0xFFFFFFFFu, top[m]);
-        if (lane == 0) largest[warp][m] = all;
+        for (uint32_t m = 0; m < (uint32_t)ROWS; ++m) largest[warp][m] = m == cr ? top : 0u;
     }
     if constexpr (PAIRED) {
         if (work) asm volatile("bar.sync %0, 64;" ::"r"(region + 1u) : "memory");
@@ -628,21 +600,14 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     uint32_t j = tg, left = pieces, wanting = 0u;  // wanting: rows without digits
     for (uint32_t j0 = 0; j0 < my_tiles; j0 += batch) {
         const uint32_t jend = min(my_tiles, j0 + batch), buf = (j0 / batch) & 1u ? batch : 0u;  // two buffers: one meeting a batch
-        uint32_t at = base + L.part + (((buf + j - j0) << slots) + (HALVED ? warp : pos)) * (ROWS * 128u) + lane * (ROWS * 4u);
+        uint32_t at = base + L.part + (((buf + j - j0) << pshift) + pos) * (ROWS * 128u) + lane * (ROWS * 4u);
 #pragma unroll 1
         for (; j < jend && slabs; j += TG, at += WARPS * (ROWS * 128u)) {
-            float below[PAR][2];  // eight warps: sums of the slabs below half
 #pragma unroll
             for (int p = 0; p < PAR; ++p) acc[p][0] = acc[p][1] = 0.0f;
 #pragma unroll 1
             for (uint32_t s = 0; s < (RES ? 1u : slabs); ++s) {
                 if constexpr (!RES) load_x(s, xa);
-                if constexpr (!RES && !HALVED) {
-                    if (s == half) {
-#pragma unroll
-                        for (int p = 0; p < PAR; ++p) below[p][0] = acc[p][0], below[p][1] = acc[p][1], acc[p][0] = acc[p][1] = 0.0f;
-                    }
-                }
                 Codes cur;
                 Sums sums;
                 if (++st == stages) st = 0u, par ^= 1u;
@@ -657,10 +622,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             auto meet = [&](const float (&a)[2]) { return (t & 1u ? a[1] : a[0]) + __shfl_xor_sync(0xFFFFFFFFu, t & 1u ? a[0] : a[1], 1); };
 #pragma unroll
             for (int p = 0; p < PAR; ++p) {
-                float v = meet(acc[p]);
-                if constexpr (!RES && !HALVED) {
-                    if (slabs > half) v += meet(below[p]);
-                }
+                const float v = meet(acc[p]);
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + (uint32_t)p * 4u), "f"(v) : "memory");
             }
         }
@@ -671,7 +633,7 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const bool none = no_digits(tallest);
         wanting = ROWS == 1 ? (none ? 1u : 0u) : (__any_sync(0xFFFFFFFFu, none && t < 2u) ? 1u : 0u) | (__any_sync(0xFFFFFFFFu, none && t >= 2u) ? 2u : 0u);
         for (uint32_t jj = j0 + warp; jj < jend; jj += WARPS) {  // a tile a warp: positions in a fixed tree, even and odd groups last
-            const uint32_t from = base + L.part + ((buf + jj - j0) << slots) * (ROWS * 128u) + lane * (ROWS * 4u);
+            const uint32_t from = base + L.part + ((buf + jj - j0) << pshift) * (ROWS * 128u) + lane * (ROWS * 4u);
             float v[PAR];
 #pragma unroll
             for (int p = 0; p < PAR; ++p) {
@@ -680,11 +642,6 @@ gemv_digits_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 for (uint32_t i = 0; i < 8u; ++i) {
                     h[i] = 0.0f;
                     if (i < P) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(h[i]) : "r"(from + i * (ROWS * 128u) + (uint32_t)p * 4u));
-                    if (HALVED && slabs_at(i) > half) {
-                        float above;
-                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(above) : "r"(from + (8u + i) * (ROWS * 128u) + (uint32_t)p * 4u));
-                        h[i] = above + h[i];
-                    }
                 }
                 v[p] = ((h[0] + h[1]) + (h[2] + h[3])) + ((h[4] + h[5]) + (h[6] + h[7]));
             }
@@ -727,10 +684,12 @@ Plan plan_launch(uint32_t N, uint32_t K, bool normed) {
     p.grid = S::SHARING ? std::max(1u, (uint32_t)sm_count() - (normed ? 1u : 0u)) : std::min((uint32_t)sm_count(), tiles);
     const uint32_t tc = (tiles + p.grid - 1u) / p.grid, row_bytes = K / 2u, nslab = slabs_of(K);
     const uint32_t P = row_bytes >= SLAB ? 8u : (row_bytes + PIECE - 1u) / PIECE, pshift = P > 4u ? 3u : P > 2u ? 2u : P > 1u ? 1u : 0u;
-    const bool halved = S::W == 16 && nslab > 1u;
-    const uint32_t TG = halved ? 1u : (uint32_t)S::W >> pshift, batch = TG * S::BATCH;
-    const uint32_t part = (tc > batch ? 2u * batch : tc) << (pshift + (halved ? 1u : 0u));
-    for (p.stages = std::min<uint32_t>(MAX_STAGES, (tc + TG - 1u) / TG * (S::W == 16 ? half_of(nslab) : nslab)); p.stages > 0u; --p.stages) {
+    const uint32_t TG = (uint32_t)S::W >> pshift, batch = TG * S::BATCH, part = (tc > batch ? 2u * batch : tc) << pshift;
+    if (nslab > 1u && tc > 1u) {  // takes() has none (see rings_of)
+        p.stages = 0u;
+        return p;
+    }
+    for (p.stages = std::min<uint32_t>(MAX_STAGES, (tc + TG - 1u) / TG * nslab); p.stages > 0u; --p.stages) {
         p.smem = layout<S>(K, p.stages, part).total;
         if (p.smem <= S::SMEM_LIMIT) break;
     }

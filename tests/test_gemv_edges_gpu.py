@@ -389,3 +389,20 @@ def test_early_rows_about_the_length_at_which_they_stop_sharing_an_sm(K, more):
     for r in (0, 1):
         assert torch.equal(miori_b200.gemv4(q, s, b, x[r:r + 1], group=64, flags=miori_b200.LAUNCH_PDL), both[r:r + 1])
     assert miori_b200.lib.miori_device_error_poll() == 0
+
+
+@pytest.mark.parametrize("K,values", [(8192, (2.0 ** 24, 1.0, 1.0, -2.0 ** 24)), (6144, (2.0 ** 24, 1.0, -2.0 ** 24)), (6144, (1.0, 2.0 ** 24, -2.0 ** 24))])
+@pytest.mark.parametrize("flags", [0, miori_b200.LAUNCH_PDL])
+def test_slabs_of_a_row_are_added_in_order(K, values, flags):
+    """2048 activations at a time, from the first on: 2^24 + 1 is 2^24 in fp32, with the ones by themselves the sums were others."""
+    N = 48
+    x = torch.zeros((2, K), dtype=torch.bfloat16, device=DEV)
+    x[:, ::2048] = torch.tensor(values, device=DEV).to(torch.bfloat16)
+    q = torch.full((N, K // 8), 0x11111111, dtype=torch.int32, device=DEV)
+    s = torch.ones((N, K // 64), dtype=torch.bfloat16, device=DEV)
+    b = torch.zeros_like(s)
+    want = torch.zeros((), device=DEV)
+    for v in values:
+        want = want + v
+    for M in (1, 2):
+        assert (miori_b200.gemv4(q, s, b, x[:M].contiguous(), group=64, flags=flags) == want).all()
