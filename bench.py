@@ -684,7 +684,7 @@ def main():
     peaks, peak_kind = measured_peaks()
     m1 = per_m["1"]
     # DRAM bytes (read + write) per algorithmic byte of gemv_digits_kernel, from ncu captures of early
-    # one-row launches over pools larger than L2 (N=8192, K=2048 9.476 MB and N=2048, K=8192 9.495 MB
+    # one-row launches over pools larger than L2 (N=8192, K=2048 9.476 MB and N=2048, K=8192 9.494 MB
     # read, nothing written -- y stays in L2 -- for 9.437 MB of weights); traffic grows in proportion
     # to the weights a launch streams (another kernel runs groups of 32: not captured)
     DRAM_PER_ALGO_BYTE = 1.005
